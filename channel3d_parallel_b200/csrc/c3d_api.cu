@@ -262,7 +262,7 @@ static void free_handle(Handle* h) {
   ib_free(h);
   mlp_free(h);
   mixed_free(h);
-  if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
+  drop_step_graphs(h);
   for (void* p : h->allocations) cudaFree(p);
   if (h->h2d) cudaStreamSynchronize(h->h2d);
   if (h->d2h) cudaStreamSynchronize(h->d2h);
@@ -477,42 +477,112 @@ static int sync_scalars_from_device(Handle* h) {
   return 0;
 }
 
+void drop_step_graphs(Handle* h) {
+  for (Handle::StepGraph& g : h->graphs) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g = Handle::StepGraph{};
+  }
+}
+
 // ---------------------------------------------------------------------------
 // one RK3 step, src/time_integration.f90:86-213
 // ---------------------------------------------------------------------------
-static int enqueue_step(Handle* h, double dt, double to) {
+// The constant x mass flow (:187-193) inside the last stage: over the
+// periodic, uniformly spaced x grid the bulk flux of d(phi)/dx telescopes to
+// zero, so the flux of the projected u is that of U* (up to rounding); the
+// stage-3 divergence kernel reduces it and the projection adds the shift.
+static bool flux_in_step(const Handle* h) { return h->p.x_mass_cte == 1 && h->ib == nullptr && h->x_uniform; }
+
+// the constant-flux corrections that follow the step (:187-211)
+static bool corrections_after(const Handle* h) {
+  return (h->p.x_mass_cte == 1 && !flux_in_step(h)) || h->p.y_mass_cte == 1 || h->p.z_mass_cte == 1;
+}
+
+// without immersed body: stages whose projection is formed inside the next
+// stage's update (launch_rhs_stage_projected).  The stage fields alternate
+// between U*, V*, W* and the arrays of U, V, W, which hold no velocity until
+// the last projection writes them.
+//   open:  start from U, V, W (else from U* of the step before, in `a`)
+//   close: end with the projection into U, V, W
+// Leaves the last stage's field in b and its potential in rhs_p.
+static int enqueue_stages(Handle* h, double dt, bool open, bool close, double* const a[3], double* const b[3]) {
+  const bool flux = flux_in_step(h);
+  const double* shift = flux ? &h->sc->shift : nullptr;
+  double* const* in = a;       // stage field of the step before (not open)
+  double* const* out = b;
+  double* phi = h->rhs_p;
+  int rc;
+  for (int s = 1; s <= 3; ++s) {
+    if (s == 1 && open) rc = launch_rhs_stage(h, 1, dt);    // U -> Us
+    else rc = launch_rhs_stage_projected(h, s, dt, in, phi, s == 1 ? shift : nullptr, out);
+    if (rc) return rc;
+    if ((rc = launch_stage_solve(h, out, s, dt, flux && s == 3, &phi))) return rc;
+    std::swap(in, out);
+  }
+  if (!close) return 0;
+  if ((rc = launch_gradient_subtract(h, in[0], in[1], in[2], phi, dt, h->U, h->V, h->W, false, true, shift)))
+    return rc;
+  return corrections_after(h) ? launch_massflow_correction(h, dt, false, flux) : 0;
+}
+
+// with an immersed body
+static int enqueue_ib_step(Handle* h, double dt, double to) {
   static const double rk_t[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
   int rc, warn = 0;
-  // The constant x mass flow (:187-193) inside the last stage: over the
-  // periodic, uniformly spaced x grid the bulk flux of d(phi)/dx telescopes
-  // to zero, so the flux of the projected u is that of U* (up to rounding);
-  // the stage-3 divergence kernel reduces it and the projection adds the shift.
-  const bool xflux = h->p.x_mass_cte == 1 && h->ib == nullptr && h->x_uniform && !h->write_pinterim;
   for (int s = 1; s <= 3; ++s) {
-    const bool fx = xflux && s == 3;
     if ((rc = launch_rhs_stage(h, s, dt))) return rc;
-    // the projection reads the ghosts of U*, V*, W* as the boundary
-    // conditions define them; the immersed-boundary operators need them set
-    if (h->ib && (rc = launch_fill_ghosts3(h, h->Us, h->Vs, h->Ws))) return rc;
+    // the immersed-boundary operators need the ghosts of U*, V*, W*
+    if ((rc = launch_fill_ghosts3(h, h->Us, h->Vs, h->Ws))) return rc;
     const double ts = to + rk_t[s - 1] * dt;
-    if (h->ib && ib_moving(h)) {                         // :111-115
+    if (ib_moving(h)) {                                  // :111-115
       if ((rc = ib_setup_geometry(h, ts))) return rc;
       if ((rc = ib_setup_operators(h))) return rc;
       if ((rc = ib_heaviside(h))) return rc;
     }
-    if ((rc = launch_projection_step(h, s, dt, fx ? &h->sc->shift : nullptr))) return rc;   // :117-118, :123
-    if (h->ib) {
-      // a Schur solve that reached cg_max_iter is a warning: the reference
-      // stops iterating and completes the step (src/projection.f90:60)
-      rc = ib_projection(h, dt, s);                           // :119-122
-      if (rc < 0) return rc;
-      if (rc > 0) warn = rc;
-    }
+    if ((rc = launch_projection_step(h, s, dt))) return rc;   // :117-118, :123
+    // a Schur solve that reached cg_max_iter is a warning: the reference
+    // stops iterating and completes the step (src/projection.f90:60)
+    rc = ib_projection(h, dt, s);                             // :119-122
+    if (rc < 0) return rc;
+    if (rc > 0) warn = rc;
   }
-  if ((h->p.x_mass_cte == 1 && !xflux) || h->p.y_mass_cte == 1 || h->p.z_mass_cte == 1) {   // :187-211
-    if ((rc = launch_massflow_correction(h, dt, false, xflux))) return rc;
-  }
+  if (corrections_after(h) && (rc = launch_massflow_correction(h, dt))) return rc;
   return warn;
+}
+
+// launch one of the step's graphs, captured on first use
+static int launch_step_graph(Handle* h, int which, double dt) {
+  double* const star[3] = {h->Us, h->Vs, h->Ws};
+  double* const vel[3] = {h->U, h->V, h->W};
+  Handle::StepGraph& g = h->graphs[which];
+  int rc;
+  if (g.exec == nullptr) {
+    cudaGraph_t gr = nullptr;
+    const int64_t l0 = h->launches, p0 = h->stats.poisson_solves;
+    C3D_CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    if (which == Handle::G_PAIR) {
+      rc = enqueue_stages(h, dt, false, false, star, vel);          // star -> vel -> star -> vel
+      if (!rc) rc = enqueue_stages(h, dt, false, false, vel, star);
+    } else {
+      rc = enqueue_stages(h, dt, true, which == Handle::G_STEP, vel, star);   // vel -> star -> vel -> star
+    }
+    cudaError_t e = cudaStreamEndCapture(h->stream, &gr);
+    if (rc) { if (gr) cudaGraphDestroy(gr); return rc; }
+    if (e != cudaSuccess) { h->last_error = std::string("graph capture: ") + cudaGetErrorString(e); return C3D_ERR_CUDA; }
+    e = cudaGraphInstantiate(&g.exec, gr, 0);
+    cudaGraphDestroy(gr);
+    if (e != cudaSuccess) { h->last_error = std::string("graph instantiate: ") + cudaGetErrorString(e); return C3D_ERR_CUDA; }
+    g.launches = h->launches - l0;
+    g.solves = h->stats.poisson_solves - p0;
+    h->launches = l0;
+    h->stats.poisson_solves = p0;
+  }
+  C3D_CUDA_TRY(h, cudaGraphLaunch(g.exec, h->stream));
+  h->launches += g.launches;
+  h->stats.poisson_solves += g.solves;
+  h->P_pending = true;
+  h->P_pending_dt = dt;
+  return 0;
 }
 
 // one explicit Euler step, src/time_integration.f90:25-81: rk_step = 3 (no
@@ -543,38 +613,33 @@ static int run_steps(Handle* h, int nsteps, bool euler = false) {
       h->stats.steps++;
       continue;
     }
-    const bool graphable = h->use_graph && h->ib == nullptr;
-    if (graphable) {
-      if (h->step_exec == nullptr || h->graph_dt != dt) {
-        if (h->step_exec) { cudaGraphExecDestroy(h->step_exec); h->step_exec = nullptr; }
-        cudaGraph_t g = nullptr;
-        const int64_t l0 = h->launches, p0 = h->stats.poisson_solves;
-        C3D_CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        rc = enqueue_step(h, dt, to);
-        cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-        if (rc) { if (g) cudaGraphDestroy(g); return rc; }
-        if (e != cudaSuccess) { h->last_error = std::string("graph capture: ") + cudaGetErrorString(e); return C3D_ERR_CUDA; }
-        e = cudaGraphInstantiate(&h->step_exec, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) { h->last_error = std::string("graph instantiate: ") + cudaGetErrorString(e); return C3D_ERR_CUDA; }
-        h->graph_dt = dt;
-        h->graph_launches = h->launches - l0;
-        h->graph_solves = h->stats.poisson_solves - p0;
-        h->launches = l0;
-        h->stats.poisson_solves = p0;
+    int taken = 1;
+    if (h->ib == nullptr) {
+      if (h->graph_dt != dt) drop_step_graphs(h);
+      h->graph_dt = dt;
+      // With a fixed dt and no correction after the step, an odd number of
+      // steps runs through with one projection at the very end: the stage
+      // fields swap arrays with every step, and U* has to end in its own.
+      const int left = nsteps - n;
+      if (h->p.CFL < 0 && !corrections_after(h) && left >= 3 && left % 2 == 1) {
+        if ((rc = launch_step_graph(h, Handle::G_OPEN, dt))) return rc;
+        for (int q = 0; q < left / 2; ++q)
+          if ((rc = launch_step_graph(h, Handle::G_PAIR, dt))) return rc;
+        rc = launch_gradient_subtract(h, h->Us, h->Vs, h->Ws, h->rhs_p, dt, h->U, h->V, h->W, false, true,
+                                      flux_in_step(h) ? &h->sc->shift : nullptr);
+        if (rc) return rc;
+        taken = left;
+      } else if ((rc = launch_step_graph(h, Handle::G_STEP, dt))) {
+        return rc;
       }
-      C3D_CUDA_TRY(h, cudaGraphLaunch(h->step_exec, h->stream));
-      h->launches += h->graph_launches;
-      h->stats.poisson_solves += h->graph_solves;
-      h->P_pending = true;
-      h->P_pending_dt = dt;
     } else {
-      rc = enqueue_step(h, dt, to);
+      rc = enqueue_ib_step(h, dt, to);
       if (rc < 0) return rc;
       if (rc > 0) warn = rc;
     }
-    h->t = to + 1.0 * dt;
-    h->stats.steps++;
+    for (int q = 0; q < taken; ++q) h->t += dt;
+    h->stats.steps += taken;
+    n += taken - 1;
   }
   C3D_CUDA_TRY(h, cudaEventRecord(h->ev1, h->stream));
   C3D_CUDA_TRY(h, cudaEventSynchronize(h->ev1));
@@ -745,7 +810,7 @@ int c3d_set_grid(int id, const double* x, const double* y, const double* z) {
   // rebuild the spectral tables for the new spacings
   rc = poisson_setup(h);
   if (rc) RET(h, rc);
-  if (h->step_exec) { cudaGraphExecDestroy(h->step_exec); h->step_exec = nullptr; }
+  drop_step_graphs(h);
   if (h->ib) {
     ib_grids_changed(h);
     rc = ib_setup_geometry(h, h->t);
@@ -785,7 +850,7 @@ int c3d_download(int id, int field, double* host, const int64_t lb[3], const int
 int c3d_set_scalars(int id, double dPdx, double dPdy, double dPdz, double t, double q0) {
   GET_HANDLE(id);
   h->dPdx = dPdx; h->dPdy = dPdy; h->dPdz = dPdz; h->t = t; h->Qflow_x_0 = q0;
-  if (h->step_exec) { cudaGraphExecDestroy(h->step_exec); h->step_exec = nullptr; }
+  drop_step_graphs(h);
   RET(h, sync_scalars_to_device(h));
 }
 
@@ -843,7 +908,7 @@ int c3d_compute_mean_mass_flow_w(int id, double* q) {
 int c3d_set_flow_targets(int id, double qx, double qy, double qz) {
   GET_HANDLE(id);
   h->Qflow_x_0 = qx; h->Qflow_y_0 = qy; h->Qflow_z_0 = qz;
-  if (h->step_exec) { cudaGraphExecDestroy(h->step_exec); h->step_exec = nullptr; }
+  drop_step_graphs(h);
   RET(h, 0);
 }
 
@@ -1009,7 +1074,7 @@ int c3d_set_mode(int id, int poisson_mode, int precond_mode) {
   if (poisson_mode == C3D_POISSON_MIXED_UNREFINED) poisson_mode = C3D_POISSON_MIXED;
   h->poisson_mode = poisson_mode;
   h->precond_mode = precond_mode;
-  if (h->step_exec) { cudaGraphExecDestroy(h->step_exec); h->step_exec = nullptr; }
+  drop_step_graphs(h);
   RET(h, 0);
 }
 
@@ -1060,17 +1125,19 @@ int c3d_kernel_launches(int id, int64_t* count) {
 int c3d_profile_kernels(int id, int nrep, double* ms, int nmax) {
   GET_HANDLE(id);
   if (!ms || nrep <= 0) return C3D_ERR_PARAM;
-  if (h->step_exec) { cudaGraphExecDestroy(h->step_exec); h->step_exec = nullptr; }
+  drop_step_graphs(h);
   const double dt = h->dt > 0 ? h->dt : 1e-3;
   const int ncls = 7;
   double out[ncls] = {0};
+  double* const star[3] = {h->Us, h->Vs, h->Ws};
+  double* const vel[3] = {h->U, h->V, h->W};
   for (int c = 0; c < ncls; ++c) {
     int rc = 0;
     // one untimed launch, then nrep timed ones
     for (int r = 0; r <= nrep; ++r) {
       if (r == 1) C3D_CUDA_TRY(h, cudaEventRecord(h->ev0, h->stream));
       switch (c) {
-        case 0: rc = launch_rhs_stage(h, 2, dt); break;
+        case 0: rc = launch_rhs_stage_projected(h, 2, dt, star, h->rhs_p, nullptr, vel); break;
         case 1: rc = launch_fill_ghosts3(h, h->Us, h->Vs, h->Ws); break;
         case 2: case 3: case 4: rc = profile_spectral(h, c - 2); break;
         case 5: rc = launch_gradient_subtract(h, h->Us, h->Vs, h->Ws, h->rhs_p, dt, h->U, h->V, h->W, false, true); break;

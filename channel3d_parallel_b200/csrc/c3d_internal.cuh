@@ -201,20 +201,24 @@ struct Handle {
   IbState* ib = nullptr;
   MixedState* mixed = nullptr;
   MlpState* mlp = nullptr;
-  // one RK3 step captured as a CUDA graph (valid for graph_dt)
-  cudaGraphExec_t step_exec = nullptr;
+  // the time step's captured CUDA graphs (valid for graph_dt): a whole step,
+  // a step that leaves its last projection to the next one, and two steps
+  // that continue from such a step and leave theirs
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    int64_t launches = 0, solves = 0;   // kernels and Poisson solves inside
+  };
+  enum { G_STEP = 0, G_OPEN = 1, G_PAIR = 2, G_COUNT = 3 };
+  StepGraph graphs[G_COUNT];
   double graph_dt = 0;
-  int64_t graph_launches = 0;     // kernels per captured step
-  int64_t graph_solves = 0;       // Poisson solves per captured step
-  bool use_graph = true;
   bool write_pinterim = false;   // projection also stores P_interim = phi/dt
-  int rhs_kernel = 0;             // 0: shared-memory tiled stage kernel, 1: per-point kernel
   // programmatic dependent launch of the time step's kernels: off, the
   // captured step graph ran slower with it (1118 against 1124 steps/s at
   // 192x129x192) although each kernel alone starts 2-3 us earlier
   bool use_pdl = false;
 };
 
+void drop_step_graphs(Handle* h);   // after any change of what they bake in
 const double* ib_hu(Handle* h);
 const double* ib_hv(Handle* h);
 const double* ib_hw(Handle* h);
@@ -279,6 +283,8 @@ int launch_fill_ghosts3(Handle* h, double* U, double* V, double* W);
 // rhs (k_rhs.cu)
 int rhs_setup(Handle* h);
 int launch_rhs_stage(Handle* h, int stage, double dt);
+int launch_rhs_stage_projected(Handle* h, int stage, double dt, double* const in[3], const double* phi,
+                               const double* ushift, double* const out[3]);
 int launch_rhs_euler(Handle* h, double dt);
 int launch_rhs_only(Handle* h, int component);
 // poisson + projection (k_poisson.cu)
@@ -289,6 +295,7 @@ int launch_poisson_of_div(Handle* h, const double* U, const double* V, const dou
                           int rk_step, double dt);
 int launch_poisson_of_div_band(Handle* h, const double* U, const double* V, const double* W, double* out,
                                int jlo, int jhi);
+int launch_stage_solve(Handle* h, double* const star[3], int rk_step, double dt, bool flux, double** phi);
 int launch_projection_step(Handle* h, int rk_step, double dt, const double* ushift = nullptr);
 int launch_gradient_subtract(Handle* h, const double* Ui, const double* Vi, const double* Wi,
                              const double* phi, double dt, double* Uo, double* Vo, double* Wo,

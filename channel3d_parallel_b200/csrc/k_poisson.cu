@@ -155,7 +155,8 @@ struct XfwdArgs {
   const double* __restrict__ U;
   const double* __restrict__ V;
   const double* __restrict__ W;
-  const double* __restrict__ rhs;             // right-hand side when not fused with div
+  const double* __restrict__ rhs;             // right-hand side when not fused with div,
+                                              // or the potential phi of the residual div(U - grad phi)
   typename cplx<T>::t* __restrict__ spec;
   const typename cplx<T>::t* __restrict__ tw;
   double* __restrict__ linesum;               // FP64 line sums (mixed path) or null
@@ -204,7 +205,12 @@ __device__ __forceinline__ XfftSmem<T> xfft_carve(unsigned char* base, int N, in
 // from the u values this kernel reads (compute_time_step_RK3's correction,
 // src/time_integration.f90:187-193, then needs no pass of its own): weights
 // wq(j) + wq(j+1) per row and plane 2 twice (plane nzg-1 is its copy).
-template <bool FROM_DIV, typename T, bool FLUX = false>
+//
+// RESID (refinement of the FP32 solve): the divergence of U - grad(phi), the
+// projection of (U, V, W) with the potential in rhs, formed as the projection
+// update forms it, so that field is neither written nor read back (32 bytes a
+// cell read in place of 56 for the update and 24 for its divergence).
+template <bool FROM_DIV, typename T, bool FLUX = false, bool RESID = false>
 __global__ void __launch_bounds__(kMaxNx) k_xfft_fwd(XfwdArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char xf_smem[];
@@ -216,6 +222,10 @@ __global__ void __launch_bounds__(kMaxNx) k_xfft_fwd(XfwdArgs<T> a) {
   __shared__ int64_t s_bu[2 * kLinesX], s_bv[2 * kLinesX], s_bvm[2 * kLinesX];
   __shared__ int64_t s_bw[2 * kLinesX], s_bwm[2 * kLinesX];
   __shared__ double s_ry[2 * kLinesX], s_rz[2 * kLinesX];
+  // RESID: phi of the line, of its y and z neighbours, and the gradient's 1/dyg, 1/dzg
+  constexpr int kRes = RESID ? 2 * kLinesX : 1;
+  __shared__ int64_t s_p[kRes], s_pym[kRes], s_pzm[kRes];
+  __shared__ double s_gy[kRes], s_gym[kRes], s_gz[kRes], s_gzm[kRes];
   const Dims& d = a.d;
   const int N = d.Nx, RS = a.rs;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -247,6 +257,16 @@ __global__ void __launch_bounds__(kMaxNx) k_xfft_fwd(XfwdArgs<T> a) {
         ry = a.m.rdy[j];
         rz = a.m.rdz[k];
         if (FLUX) s_cq[tid] = a.m.cqu[j] * (k == 2 ? 2.0 : 1.0);
+        if (RESID) {
+          const int km = k == 2 ? d.Nz + 1 : k - 1;
+          s_p[tid] = idxR(d, 2, j, k);
+          s_pym[tid] = j == 2 ? s_p[tid] : idxR(d, 2, j - 1, k);
+          s_pzm[tid] = idxR(d, 2, j, km);
+          s_gy[tid] = j == d.ny ? 0.0 : a.m.rdyg[j];
+          s_gym[tid] = j == 2 ? 0.0 : a.m.rdyg[j - 1];
+          s_gz[tid] = a.m.rdzg[k];
+          s_gzm[tid] = a.m.rdzg[km];
+        }
       } else {
         bu = idxR(d, 2, j, k);
       }
@@ -267,6 +287,7 @@ __global__ void __launch_bounds__(kMaxNx) k_xfft_fwd(XfwdArgs<T> a) {
   const int ii = tid % N, rls = nt / N;
   const int xo = ii == 0 ? N - 1 : ii - 1;
   const double rdx_i = FROM_DIV ? a.m.rdx[2 + ii] : 0.0;
+  const double gx = RESID ? a.m.rdxg[2 + ii] : 0.0, gxm = RESID ? a.m.rdxg[2 + xo] : 0.0;
   constexpr int kBatch = 4;
   for (int rb = tid / N; rb < 2 * kLinesX; rb += kBatch * rls) {
     double x0[kBatch], x1[kBatch], y0[kBatch], y1[kBatch], z0[kBatch], z1[kBatch];
@@ -282,6 +303,18 @@ __global__ void __launch_bounds__(kMaxNx) k_xfft_fwd(XfwdArgs<T> a) {
           if (bv >= 0) y1[q] = a.V[bv + ii];
           if (bvm >= 0) y0[q] = a.V[bvm + ii];
           z1[q] = a.W[s_bw[rl] + ii]; z0[q] = a.W[s_bwm[rl] + ii];
+          if (RESID) {
+            const double* ph = a.rhs + s_p[rl];
+            const int ny1 = s_gy[rl] == 0.0 ? 0 : N + 1;     // rows of phi are Nx+1 long
+            const double* pm = a.rhs + s_pzm[rl];
+            const double p0 = ph[ii];
+            x1[q] -= (ph[ii + 1] - p0) * gx;
+            x0[q] -= (ph[xo + 1] - ph[xo]) * gxm;
+            y1[q] -= (ph[ny1 + ii] - p0) * s_gy[rl];
+            y0[q] -= (p0 - a.rhs[s_pym[rl] + ii]) * s_gym[rl];
+            z1[q] -= (ph[(int64_t)(N + 1) * d.Ny + ii] - p0) * s_gz[rl];
+            z0[q] -= (pm[(int64_t)(N + 1) * d.Ny + ii] - pm[ii]) * s_gzm[rl];
+          }
         } else {
           x1[q] = a.rhs[bu + ii];
         }
@@ -1168,6 +1201,7 @@ static int set_limits(Handle* h, int smem_yz, int cs) {
   C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<true, T>>(smx)));
   C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<false, T>>(smx)));
   C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<true, T, true>>(smx)));
+  if (sizeof(T) == 4) C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<true, float, false, true>>(smx)));
   C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_inv<T>>(smx)));
   C3D_CUDA_TRY(h, (raise_smem_limit<k_spectral_yz<T, true>>(smem_yz)));
   C3D_CUDA_TRY(h, (raise_smem_limit<k_spectral_yz<T, false>>(smem_yz)));
@@ -1224,6 +1258,9 @@ static int run_spectral_t(Handle* h, bool from_div, const double* U, const doubl
       a.flux_part = h->flux_part; a.scw = h->sc;
       a.q0 = h->Qflow_x_0; a.norm = h->norm_u; a.dt = flux_dt;
       C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_fwd<true, T, true>, nbx, ntx, smx, s, a));
+    } else if (from_div && rhs_in) {
+      if constexpr (sizeof(T) == 4)
+        C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_fwd<true, T, false, true>, nbx, ntx, smx, s, a));
     } else if (from_div) {
       C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_fwd<true, T>, nbx, ntx, smx, s, a));
     } else {
@@ -1483,43 +1520,40 @@ int launch_gradient_subtract(Handle* h, const double* Ui, const double* Vi, cons
   return with_ghosts ? launch_fill_ghosts3(h, Uo, Vo, Wo) : 0;
 }
 
-// compute_non_IB_projection with U* in (Us,Vs,Ws) and the result in (U,V,W),
-// ghosts filled.  FP64: one solve.  Mixed: an FP32 solve, then refinement
-// sweeps that solve again for the FP64 residual div(U) and re-project U* with
-// the accumulated potential.
-int launch_projection_step(Handle* h, int rk_step, double dt, const double* ushift) {
-  const bool stage1 = (rk_step == 1 && h->ib == nullptr);
+// The potential of div(star) for one stage (rk_step 1..3), star an interior
+// field whose ghosts are taken as the boundary conditions define them; *phi is
+// where it lies.  The stage-1 potential, kept for the pressure
+// (src/poisson.f90:91-99), goes into its own array.  Mixed: an FP32 solve, then
+// refinement sweeps that solve for the FP64 residual div(star - grad phi) and
+// add to phi.  flux: the first forward x FFT also yields the constant-x-mass-
+// flow shift (the bulk flux of d(phi)/dx over the periodic uniform x grid is
+// zero, so the flux of the projected u is that of star).
+int launch_stage_solve(Handle* h, double* const star[3], int rk_step, double dt, bool flux, double** phi) {
+  const bool stage1 = rk_step == 1 && h->ib == nullptr;
+  double* p = stage1 ? h->phi1 : h->rhs_p;
   int rc;
-  double* phi = h->rhs_p;
   if (h->poisson_mode == C3D_POISSON_MIXED) {
-    // with ushift the first forward transform (of U*) also yields the x
-    // mass-flow correction: the flux of the refined projection is still U*'s
-    const int sweeps = h->refine_sweeps;
-    rc = run_spectral_t<float>(h, true, h->Us, h->Vs, h->Ws, nullptr, h->rhs_p,
-                               (stage1 && sweeps == 0) ? h->phi1 : nullptr, 0, 7, 0, -1, ushift ? dt : 0.0);
-    if (rc) return rc;
-    for (int sw = 1; sw <= sweeps; ++sw) {
-      rc = launch_gradient_subtract(h, h->Us, h->Vs, h->Ws, h->rhs_p, dt, h->U, h->V, h->W, false, true);
-      if (rc) return rc;
-      rc = run_spectral_t<float>(h, true, h->U, h->V, h->W, nullptr, h->rhs_p,
-                                 (stage1 && sw == sweeps) ? h->phi1 : nullptr, 1, 7);
-      if (rc) return rc;
-    }
-    h->stats.refinement_sweeps = sweeps;
+    rc = run_spectral_t<float>(h, true, star[0], star[1], star[2], nullptr, p, nullptr, 0, 7, 0, -1, flux ? dt : 0.0);
+    for (int sw = 1; sw <= h->refine_sweeps && !rc; ++sw)
+      rc = run_spectral_t<float>(h, true, star[0], star[1], star[2], p, p, nullptr, 1, 7);
+    h->stats.refinement_sweeps = h->refine_sweeps;
   } else {
-    // with ushift, the forward x FFT also yields the x mass-flow correction
-    // (the bulk flux of d(phi)/dx over the periodic uniform x grid is zero,
-    // so the flux of the projected u is that of U*).  The stage-1 potential,
-    // kept for the pressure (src/poisson.f90:91-99), is solved straight into
-    // its own array, which the update then reads: no second copy.
-    phi = stage1 ? h->phi1 : h->rhs_p;
-    rc = run_spectral_t<double>(h, true, h->Us, h->Vs, h->Ws, nullptr, phi, nullptr, 0, 7, 0, -1,
-                                ushift ? dt : 0.0);
-    if (rc) return rc;
+    rc = run_spectral_t<double>(h, true, star[0], star[1], star[2], nullptr, p, nullptr, 0, 7, 0, -1, flux ? dt : 0.0);
   }
+  if (rc) return rc;
   if (stage1) { h->P_pending = true; h->P_pending_dt = dt; }
-  // the projected fields with all their ghost entries (and the x mass-flow
-  // correction when ushift is given)
+  *phi = p;
+  return 0;
+}
+
+// compute_non_IB_projection with U* in (Us,Vs,Ws) and the result in (U,V,W),
+// all ghost entries included (and the x mass-flow correction when ushift is
+// given)
+int launch_projection_step(Handle* h, int rk_step, double dt, const double* ushift) {
+  double* const star[3] = {h->Us, h->Vs, h->Ws};
+  double* phi = nullptr;
+  const int rc = launch_stage_solve(h, star, rk_step, dt, ushift != nullptr, &phi);
+  if (rc) return rc;
   return launch_gradient_subtract(h, h->Us, h->Vs, h->Ws, phi, dt, h->U, h->V, h->W, false, true, ushift);
 }
 

@@ -38,11 +38,13 @@ struct RhsArgs {
   double cs;   // coefficient of F for U*
   double cg;   // coefficient of F for G (stage 1)
   int comp_mask;  // rhs-only mode: which components to write (bit0 u, bit1 v, bit2 w)
+  const double* __restrict__ phi;   // potential of the projection formed on the way in
+  const double* ushift;             // constant-mass-flow shift of u, or null
+  int kc;                           // z planes per CTA
 };
 
-// MODE 0: write F into rhs_u/v/w arrays (fine entries), incl. the duplicated
-// periodic planes the reference also computes.  MODE 1: stage 1.  MODE 2: stage 2/3.
-template <int MODE>
+// F into the rhs_u/v/w arrays (fine entries), incl. the duplicated periodic
+// planes the reference also computes
 __global__ void __launch_bounds__(256) k_rhs(RhsArgs a) {
   const Dims& d = a.d;
   const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -122,258 +124,346 @@ __global__ void __launch_bounds__(256) k_rhs(RhsArgs a) {
 #undef LV
 #undef LW
 
-  if (MODE == 0) {
-    // rhs_u(2:nx-1, 2:nyg-1, 2:nzg-1): x 2..Nx+1, z 2..Nz+2 (plane Nz+2 duplicates 2)
-    const int nu1 = d.nx - 2, nu2 = d.nyg - 2;
-    if (a.comp_mask & 1) {
-      double* R = a.Us;
-      R[(i - 2) + (int64_t)nu1 * ((j - 2) + (int64_t)nu2 * (k - 2))] = Fu;
-      if (k == 2) R[(i - 2) + (int64_t)nu1 * ((j - 2) + (int64_t)nu2 * (d.Nz))] = Fu;
-    }
-    // rhs_v(2:nxg-1, 2:ny-1, 2:nzg-1): x 2..Nx+2
-    if ((a.comp_mask & 2) && hasv) {
-      double* R = a.Vs;
-      const int n1 = d.nxg - 2, n2 = d.ny - 2;
-      const int64_t o = (int64_t)n1 * n2;
-      R[(i - 2) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fv;
-      if (i == 2) R[(d.Nx) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fv;
-      if (k == 2) {
-        R[(i - 2) + (int64_t)n1 * (j - 2) + o * d.Nz] = Fv;
-        if (i == 2) R[(d.Nx) + (int64_t)n1 * (j - 2) + o * d.Nz] = Fv;
-      }
-    }
-    // rhs_w(2:nxg-1, 2:nyg-1, 2:nz-1): x 2..Nx+2
-    if (a.comp_mask & 4) {
-      double* R = a.Ws;
-      const int n1 = d.nxg - 2, n2 = d.nyg - 2;
-      const int64_t o = (int64_t)n1 * n2;
-      R[(i - 2) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fw;
-      if (i == 2) R[(d.Nx) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fw;
-    }
-    return;
+  // rhs_u(2:nx-1, 2:nyg-1, 2:nzg-1): x 2..Nx+1, z 2..Nz+2 (plane Nz+2 duplicates 2)
+  const int nu1 = d.nx - 2, nu2 = d.nyg - 2;
+  if (a.comp_mask & 1) {
+    double* R = a.Us;
+    R[(i - 2) + (int64_t)nu1 * ((j - 2) + (int64_t)nu2 * (k - 2))] = Fu;
+    if (k == 2) R[(i - 2) + (int64_t)nu1 * ((j - 2) + (int64_t)nu2 * (d.Nz))] = Fu;
   }
-
-  const int64_t iu = idxU(d, i, j, k), iw = idxW(d, i, j, k);
-  if (MODE == 1) {
-    a.Us[iu] = u0 + a.cs * Fu;
-    a.Gu_out[iu] = u0 + a.cg * Fu;
-    a.Ws[iw] = w0 + a.cs * Fw;
-    a.Gw_out[iw] = w0 + a.cg * Fw;
-    if (hasv) {
-      const int64_t iv = idxV(d, i, j, k);
-      a.Vs[iv] = v0 + a.cs * Fv;
-      a.Gv_out[iv] = v0 + a.cg * Fv;
+  // rhs_v(2:nxg-1, 2:ny-1, 2:nzg-1): x 2..Nx+2
+  if ((a.comp_mask & 2) && hasv) {
+    double* R = a.Vs;
+    const int n1 = d.nxg - 2, n2 = d.ny - 2;
+    const int64_t o = (int64_t)n1 * n2;
+    R[(i - 2) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fv;
+    if (i == 2) R[(d.Nx) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fv;
+    if (k == 2) {
+      R[(i - 2) + (int64_t)n1 * (j - 2) + o * d.Nz] = Fv;
+      if (i == 2) R[(d.Nx) + (int64_t)n1 * (j - 2) + o * d.Nz] = Fv;
     }
-  } else {
-    a.Us[iu] = __ldg(a.Gu + iu) + a.cs * Fu;
-    a.Ws[iw] = __ldg(a.Gw + iw) + a.cs * Fw;
-    if (hasv) {
-      const int64_t iv = idxV(d, i, j, k);
-      a.Vs[iv] = __ldg(a.Gv + iv) + a.cs * Fv;
-    }
+  }
+  // rhs_w(2:nxg-1, 2:nyg-1, 2:nz-1): x 2..Nx+2
+  if (a.comp_mask & 4) {
+    double* R = a.Ws;
+    const int n1 = d.nxg - 2, n2 = d.nyg - 2;
+    const int64_t o = (int64_t)n1 * n2;
+    R[(i - 2) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fw;
+    if (i == 2) R[(d.Nx) + (int64_t)n1 * (j - 2) + o * (k - 2)] = Fw;
   }
 }
 
 // ---------------------------------------------------------------------------
-// Tiled stage kernel: a CTA owns a TX x TY tile of (i, j) columns and marches
-// over a run of KC z planes, keeping planes k-1, k, k+1 of U, V and W (tile
-// plus a one-cell halo in x and y) in a rolling shared-memory window.  Every
-// field value is read from HBM once per CTA (halo overhead (TX+2)(TY+2)/(TX*TY));
-// the arithmetic is that of k_rhs.
+// Stage kernel of the time step.  A CTA owns a TX x TY tile of (i, j) columns
+// and marches over a chunk of z planes, one cell per thread and plane.
+//
+// PROJ: the input is the previous stage's U*, V*, W* with its potential phi,
+// and the velocities are formed on the way in, u = u* - d(phi)/dx (+ the
+// mass-flow shift) with the boundary conditions as index folds and signs
+// (projection, src/projection.f90:40-44; boundary_conditions.f90:20-252), so
+// between two stages the projected fields are neither written nor read:
+// 80 bytes a cell (u*, phi, G in; u* out) in place of the 56 of a separate
+// projection plus 72.  Without PROJ the input is U, V, W with their ghosts.
+//
+// The planes (tile plus halo) come by cp.async into a ring of NSLOT slots,
+// three planes ahead of the one whose velocities are formed, which in turn is
+// two ahead of the one that is computed, so one barrier a plane orders
+// everything; each thread forms the velocities of its own cell and some
+// threads those of one halo cell, in place.  Loads one plane ahead into
+// registers took 166-197 us a stage at 192 x 128 x 192 (two to three
+// microseconds a plane: the memory's latency under load).
+//
+// Measured (B200, us a stage): 192 x 128 x 192 97 in stage 1 and 105 in 2 and
+// 3, where the separate projection took 53 and the update 92; 384 x 256 x 384
+// 785 (369 and 692); 32 x 64 x 32 8 (6 and 31: that update marched 64 planes
+// whatever the grid).  Bound by instruction issue (0.55 a cycle at 16 warps,
+// 400 a cell) and by the shared-memory pipe (0.7 busy: an 8-byte access of a
+// warp is two wavefronts); memory runs at 3.5 TB/s.
+//
+// The momentum fluxes live on cell edges and centres,
+//   Exy = (u + u(j+1)) (v + v(i+1)),  Exz = (u + u(k+1)) (w + w(i+1)),
+//   Eyz = (v + v(k+1)) (w + w(j+1)),  and the squares of the face sums,
+// each shared by two components; those on a z face, and the viscous z
+// differences, are carried in registers from one plane to the next, so plane
+// k-1 is not read again.
 // ---------------------------------------------------------------------------
-constexpr int TX = 32, TY = 8, KC = 64;
+constexpr int TX = 32, TY = 8;
 constexpr int PX = TX + 2, PY = TY + 2, PN = PX * PY;
-constexpr int NSLOT = 8;   // planes k-1, k, k+1 in use, k+2..k+4 in flight
-constexpr int AHEAD = 3;   // planes issued beyond k+1
+constexpr int FX = PX + 1, FY = PY + 1, FN = FX * FY;     // phi: one more column and row
+constexpr int RHS_THREADS = TX * TY;
+constexpr int NHALO = PN - TX * TY;       // halo cells of a tile, at most one a thread
+constexpr int RHS_CTAS = 2;               // resident CTAs per SM
+constexpr int NSLOT = 7;                  // planes k .. k+6
+static_assert(NHALO <= RHS_THREADS && FN - TX * TY <= RHS_THREADS, "one halo cell per thread");
 
-__device__ __forceinline__ void cp_async8(double* sdst, const double* gsrc, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-  const int n = valid ? 8 : 0;   // src-size 0 zero-fills the destination
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gsrc), "r"(n));
+__device__ __forceinline__ void cp_async8(unsigned sdst, const double* gsrc) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sdst), "l"(gsrc));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-template <int MODE>
-__global__ void __launch_bounds__(TX * TY, 2) k_rhs_tiled(RhsArgs a) {
-  extern __shared__ double rhs_smem[];
-  double (*sU)[PN] = reinterpret_cast<double (*)[PN]>(rhs_smem);
-  double (*sV)[PN] = reinterpret_cast<double (*)[PN]>(rhs_smem + NSLOT * PN);
-  double (*sW)[PN] = reinterpret_cast<double (*)[PN]>(rhs_smem + 2 * NSLOT * PN);
-  double* sZ = rhs_smem + 3 * NSLOT * PN;     // z factors of planes k0..k1: [6][KC]
+// Products and sums rounded as written here, so that both forms of the kernel
+// (and the separate projection followed by the plain one) give the same bits.
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double sqdiff(double a, double b) { return __fma_rn(a, a, -__dmul_rn(b, b)); }
+__device__ __forceinline__ double wdiff(double p, double a, double q, double b) {
+  return __fma_rn(p, a, -__dmul_rn(q, b));
+}
+
+// shared memory: NSLOT planes of U, V, W (PN each) and phi (FN, PROJ), the z
+// factors of planes k0..k1: (rdz/4, rdzg/4), (czpC, czmC), (czpF, czmF), and
+// 1/dzg of k0-1..k1+1
+template <bool PROJ>
+struct RhsSmem {
+  static constexpr int SLOT = 3 * PN + (PROJ ? FN : 0);
+  static constexpr int Z0 = NSLOT * SLOT + ((NSLOT * SLOT) & 1);
+  static size_t bytes(int kc) { return sizeof(double) * (size_t)(Z0 + 6 * kc + kc + 2); }
+};
+
+template <int MODE, bool PROJ>
+__global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) {
+  using L = RhsSmem<PROJ>;
+  extern __shared__ __align__(16) double rhs_smem[];
+  // 1/dxg per tile column, 1/dyg per tile row (gradient of phi); y factors per
+  // row: (rdy/4, rdyg/4), (cypC, cymC), (cypF, cymF)
+  __shared__ double sGx[PX], sGy[PY];
+  __shared__ double2 sY[3][TY];
+  double2* sZ = reinterpret_cast<double2*>(rhs_smem + L::Z0);
+  double* sGz = rhs_smem + L::Z0 + 6 * a.kc;
   const Dims& d = a.d;
   const Metric& m = a.m;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int tid = ty * TX + tx;
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
   const int i0 = 2 + blockIdx.x * TX, j0 = 2 + blockIdx.y * TY;
-  const int k0 = 2 + blockIdx.z * KC;
-  const int k1 = min(k0 + KC - 1, d.Nz + 1);
+  const int k0 = 2 + blockIdx.z * a.kc, k1 = min(k0 + a.kc - 1, d.Nz + 1);
   const int i = i0 + tx, j = j0 + ty;
-  const bool active = (i <= d.Nx + 1) && (j <= d.Ny + 1);
-  const bool hasv = active && (j <= d.Ny);
+  const int plU = d.nx * d.nyg, plV = d.nxg * d.ny, plW = d.nxg * d.nyg, plR = (d.nxg - 2) * (d.nyg - 2);
+  auto at = [](int z, int pl) { return (int64_t)z * pl; };     // 32 x 32 -> 64 bits
+  auto xfold = [&](int gi) { return gi == 1 ? d.Nx + 1 : (gi >= d.Nx + 2 ? gi - d.Nx : gi); };
+  auto zfold = [&](int k) { return PROJ ? (k == 1 ? d.Nz + 1 : (k >= d.Nz + 2 ? k - d.Nz : k)) : k; };
 
-  // halo-tile positions of this thread (at most two: PN <= 2 * TX * TY): the
-  // offset of plane 1 and the x/y validity are fixed, plane k adds k-1 planes
-  constexpr int kPos = (PN + TX * TY - 1) / (TX * TY);
-  int64_t offU[kPos], offV[kPos], offW[kPos];
-  bool okU[kPos], okV[kPos], okW[kPos];
-#pragma unroll
-  for (int q = 0; q < kPos; ++q) {
-    const int t = tid + q * TX * TY;
-    const int li = t % PX, lj = t / PX;
-    const int gi = i0 - 1 + li, gj = j0 - 1 + lj;
-    const bool in = t < PN;
-    okU[q] = in && gi <= d.nx && gj <= d.nyg;
-    okV[q] = in && gi <= d.nxg && gj <= d.ny;
-    okW[q] = in && gi <= d.nxg && gj <= d.nyg;
-    offU[q] = okU[q] ? idxU(d, gi, gj, 1) : 0;
-    offV[q] = okV[q] ? idxV(d, gi, gj, 1) : 0;
-    offW[q] = okW[q] ? idxW(d, gi, gj, 1) : 0;
-  }
-  const int64_t plU = (int64_t)d.nx * d.nyg, plV = (int64_t)d.nxg * d.ny, plW = (int64_t)d.nxg * d.nyg;
-  for (int t = tid; t < 6 * KC; t += TX * TY) {
-    const int q = t / KC, kk = k0 + (t - q * KC);
-    const double* f = q == 0 ? m.rdz : q == 1 ? m.rdzg : q == 2 ? m.czpC : q == 3 ? m.czmC : q == 4 ? m.czpF : m.czmF;
-    sZ[t] = kk <= k1 ? f[kk] : 0.0;
-  }
-  pdl_wait();
-  pdl_trigger();
-  // asynchronous copy of plane k (tile + halo) of U, V, W into a slot
-  auto issue_plane = [&](int k) {
-    const int slot = k & (NSLOT - 1);
-    const int64_t kk = k - 1;
-#pragma unroll
-    for (int q = 0; q < kPos; ++q) {
-      const int t = tid + q * TX * TY;
-      if (t < PN) {
-        const bool vu = okU[q] && k <= d.nzg, vv = okV[q] && k <= d.nzg, vw = okW[q] && k <= d.nz;
-        cp_async8(&sU[slot][t], vu ? a.U + offU[q] + kk * plU : a.U, vu);
-        cp_async8(&sV[slot][t], vv ? a.V + offV[q] + kk * plV : a.V, vv);
-        cp_async8(&sW[slot][t], vw ? a.W + offW[q] + kk * plW : a.W, vw);
-      }
-    }
-    cp_async_commit();
+  // places in the fields, inside a plane (always legal; what is read at a
+  // position that is not needed is not used)
+  struct Pos {
+    int u, v, w;
+    bool neg, wall;          // u, w: wall reflection; v: zero
   };
+  auto place = [&](int x, int y) {
+    Pos p;
+    int gi = min(i0 - 1 + x, d.Nx + 2), gj = min(j0 - 1 + y, d.Ny + 2), gv = min(gj, d.Ny + 1);
+    p.neg = p.wall = false;
+    if (PROJ) {
+      p.neg = gj == 1 || gj == d.Ny + 2;
+      p.wall = gj < 2 || gj > d.Ny;
+      gi = xfold(gi);
+      gj = gj == 1 ? 2 : (gj == d.Ny + 2 ? d.Ny + 1 : gj);
+      gv = min(gj, d.Ny);
+    }
+    p.u = (int)idxU(d, gi, gj, 1);
+    p.v = (int)idxV(d, gi, gv, 1);
+    p.w = (int)idxW(d, gi, gj, 1);
+    return p;
+  };
+  auto phi_place = [&](int x, int y) {      // rows 1 and ny+1: the gradient there is not used as it stands
+    const int gi = xfold(min(i0 - 1 + x, d.Nx + 3)), gj = min(max(j0 - 1 + y, 2), d.Ny + 1);
+    return (int)idxR(d, gi, gj, 2);
+  };
+  // second position of this thread: rows 0 and PY-1 of the tile, then the side
+  // columns; of phi: row 0, the last two rows, the side columns
+  int hx = 1, hy = 1, fx = 1, fy = 1;
+  const bool halo = tid < NHALO, fhalo = PROJ && tid < FN - TX * TY;
+  if (tid < 2 * PX) { hy = tid < PX ? 0 : PY - 1; hx = tid < PX ? tid : tid - PX; }
+  else if (halo) { const int t = tid - 2 * PX; hx = t < TY ? 0 : PX - 1; hy = 1 + (t < TY ? t : t - TY); }
+  if (tid < 3 * FX) { const int r = tid / FX; fy = r == 0 ? 0 : PY - 2 + r; fx = tid - r * FX; }
+  else if (fhalo) { const int t = tid - 3 * FX, q = t / TY; fx = q == 0 ? 0 : PX - 2 + q; fy = 1 + (t - q * TY); }
+  const int c = (ty + 1) * PX + (tx + 1), ch = hy * PX + hx;
+  const int cf = (ty + 1) * FX + (tx + 1), chf = hy * FX + hx;      // the same places in phi's tile
+  const Pos P0 = place(tx + 1, ty + 1), P1 = place(hx, hy);
+  const int f0 = PROJ ? phi_place(tx + 1, ty + 1) : 0, f1 = PROJ ? phi_place(fx, fy) : 0;
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(rhs_smem);
+
+  // plane k of the inputs into ring slot `slot`
+  auto issue = [&](int k, int slot) {
+    const int z = zfold(k) - 1;
+    const unsigned s = sbase + 8u * (unsigned)(slot * L::SLOT);
+    const double *Uz = a.U + at(z, plU), *Vz = a.V + at(z, plV), *Wz = a.W + at(z, plW);
+    cp_async8(s + 8 * c, Uz + P0.u);
+    cp_async8(s + 8 * (PN + c), Vz + P0.v);
+    cp_async8(s + 8 * (2 * PN + c), Wz + P0.w);
+    if (halo) {
+      cp_async8(s + 8 * ch, Uz + P1.u);
+      cp_async8(s + 8 * (PN + ch), Vz + P1.v);
+      cp_async8(s + 8 * (2 * PN + ch), Wz + P1.w);
+    }
+    if (PROJ) {
+      const double* Fz = a.phi + at(z - 1, plR);
+      cp_async8(s + 8 * (3 * PN + cf), Fz + f0);
+      if (fhalo) cp_async8(s + 8 * (3 * PN + fy * FX + fx), Fz + f1);
+    }
+  };
+  // the last plane whose velocities are needed is k1+1; its w needs phi of k1+2
+  const int kend = PROJ ? k1 + 2 : k1 + 1;
+  for (int q = 0; q < 7; ++q) {
+    if (k0 - 1 + q <= kend) issue(k0 - 1 + q, q);
+    cp_async_commit();
+  }
+
+  // tables
+  if (tid < PX) sGx[tid] = i0 - 1 + tid <= d.Nx + 2 ? m.rdxg[xfold(i0 - 1 + tid)] : 0.0;
+  if (tid < PY) sGy[tid] = j0 - 1 + tid >= 2 && j0 - 1 + tid <= d.Ny ? m.rdyg[j0 - 1 + tid] : 0.0;
+  if (tid < TY) {
+    const int gj = j0 + tid <= d.Ny + 1 ? j0 + tid : 2;
+    sY[0][tid] = make_double2(0.25 * m.rdy[gj], 0.25 * m.rdyg[gj]);
+    sY[1][tid] = make_double2(m.cypC[gj], m.cymC[gj]);
+    sY[2][tid] = make_double2(m.cypF[gj], m.cymF[gj]);
+  }
+  for (int t = tid; t < a.kc; t += RHS_THREADS) {
+    const int kk = min(k0 + t, k1);
+    sZ[t] = make_double2(0.25 * m.rdz[kk], 0.25 * m.rdzg[kk]);
+    sZ[a.kc + t] = make_double2(m.czpC[kk], m.czmC[kk]);
+    sZ[2 * a.kc + t] = make_double2(m.czpF[kk], m.czmF[kk]);
+  }
+  if (PROJ)
+    for (int t = tid; t < a.kc + 2; t += RHS_THREADS) sGz[t] = m.rdzg[zfold(min(k0 - 1 + t, k1 + 1))];
+  const bool edge = j0 + TY > d.Ny + 1;     // the tile holds wall rows of v or rows past them
+  const int ic = min(i, d.Nx + 1);
+  const double2 x0 = make_double2(0.25 * m.rdxg[ic], 0.25 * m.rdx[ic]);
+  const double2 x1 = make_double2(m.cxpF[ic], m.cxmF[ic]), x2 = make_double2(m.cxpC[ic], m.cxmC[ic]);
+  const double shift = MODE == 1 && PROJ && a.ushift ? *a.ushift : 0.0;
   const double dPdx = a.sc->dPdx, dPdy = a.sc->dPdy, dPdz = a.sc->dPdz;
-  issue_plane(k0 - 1);
-  issue_plane(k0);
-  for (int q = 1; q <= AHEAD; ++q) {
-    if (k0 + q <= k1 + 1) issue_plane(k0 + q);
-    else cp_async_commit();
+
+  // velocities of plane k0-1+kz in place: slot s, phi of the next plane in slot
+  // sn; p0, ph: phi of the own and the halo cell (carried from plane to plane);
+  // the own cell's velocities to u, v, w
+  double p0 = 0.0, ph = 0.0;
+  auto form = [&](const Pos& p, double* S, const double* Sn, int at, int atf, double gx, double gy, double gz, bool bc,
+                  double& pc, double& u, double& v, double& w) {
+    const double pz = Sn[3 * PN + atf];
+    u = __fma_rn(pc - S[3 * PN + atf + 1], gx, S[at]);
+    v = __fma_rn(pc - S[3 * PN + atf + FX], gy, S[PN + at]);
+    w = __fma_rn(pc - pz, gz, S[2 * PN + at]);
+    pc = pz;
+    if (MODE == 1) u += shift;
+    if (bc) {
+      if (p.neg) { u = -u; w = -w; }
+      if (p.wall) v = 0.0;
+    }
+    S[at] = u;
+    S[PN + at] = v;
+    S[2 * PN + at] = w;
+  };
+  auto form_plane = [&](int kz, int s, int sn, double& u, double& v, double& w) {
+    double* S = rhs_smem + s * L::SLOT;
+    if (!PROJ) {
+      u = S[c];
+      v = S[PN + c];
+      w = S[2 * PN + c];
+      return;
+    }
+    const double* Sn = rhs_smem + sn * L::SLOT;
+    const double gz = sGz[kz];
+    form(P0, S, Sn, c, cf, sGx[tx + 1], sGy[ty + 1], gz, edge, p0, u, v, w);
+    double hu, hv, hw;
+    if (halo) form(P1, S, Sn, ch, chf, sGx[hx], sGy[hy], gz, true, ph, hu, hv, hw);
+  };
+
+  // planes k0-1, k0, k0+1 formed (k0+2 has landed), slots 0, 1, 2
+  cp_async_wait<3>();
+  __syncthreads();
+  if (PROJ) {
+    p0 = rhs_smem[3 * PN + cf];
+    ph = rhs_smem[3 * PN + chf];
   }
-  const int c = (ty + 1) * PX + (tx + 1);     // own cell in the padded tile
-  // x- and y-indexed metric factors of this column, constant over the march
-  const int ic = active ? i : 2, jc = active ? j : 2;
-  const double rdxg_i = m.rdxg[ic], rdx_i = m.rdx[ic];
-  const double cxpF_i = m.cxpF[ic], cxmF_i = m.cxmF[ic], cxpC_i = m.cxpC[ic], cxmC_i = m.cxmC[ic];
-  const double rdy_j = m.rdy[jc], rdyg_j = m.rdyg[jc];
-  const double cypC_j = m.cypC[jc], cymC_j = m.cymC[jc], cypF_j = m.cypF[jc], cymF_j = m.cymF[jc];
-  const int64_t iu0 = idxU(d, ic, jc, 1), iv0 = idxV(d, ic, jc, 1), iw0 = idxW(d, ic, jc, 1);
-  // accumulators, loaded one plane ahead of their use
-  double gu = 0.0, gv = 0.0, gw = 0.0;
-  if (MODE == 2 && active) {
-    const int64_t kk = k0 - 1;
-    gu = __ldg(a.Gu + iu0 + kk * plU);
-    gw = __ldg(a.Gw + iw0 + kk * plW);
-    if (hasv) gv = __ldg(a.Gv + iv0 + kk * plV);
-  }
+  double ua, va, wa, u0, v0, w0, u1, v1, w1;
+  form_plane(0, 0, 1, ua, va, wa);
+  form_plane(1, 1, 2, u0, v0, w0);
+  form_plane(2, 2, 3, u1, v1, w1);
+  __syncthreads();
+  // fluxes and differences on the cell's lower z face
+  double Exz = mul(ua + u0, wa + rhs_smem[2 * PN + c + 1]);
+  double Eyz = mul(va + v0, wa + rhs_smem[2 * PN + c + PX]);
+  double Cz = mul(wa + w0, wa + w0);
+  double du = u0 - ua, dv = v0 - va, dw = w0 - wa;
+  double gu = 0.0, gv = 0.0, gw = 0.0;        // accumulators, one plane ahead
+  auto load_G = [&](int k) {                  // legal at every position
+    const int z = k - 1;
+    gu = __ldg(a.Gu + at(z, plU) + P0.u);
+    gv = __ldg(a.Gv + at(z, plV) + P0.v);
+    gw = __ldg(a.Gw + at(z, plW) + P0.w);
+  };
+  if (MODE == 2) load_G(k0);
+  const bool active = i <= d.Nx + 1 && j <= d.Ny + 1, hasv = active && j <= d.Ny;
+  auto next = [](int s) { return s == NSLOT - 1 ? 0 : s + 1; };
+  int s0 = 1;                // slot of plane k
   for (int k = k0; k <= k1; ++k) {
-    if (k + 1 + AHEAD <= k1 + 1) issue_plane(k + 1 + AHEAD);
-    else cp_async_commit();                   // keep the group count uniform
-    cp_async_wait<AHEAD>();                   // planes up to k+1 have landed
+    const int t = k - k0;
+    const int s1 = next(s0), s2 = next(s1), s3 = next(s2);
+    // planes up to k+3 have landed and those up to k+1 are formed; every
+    // thread is done with plane k-1, whose slot takes plane k+6
+    cp_async_wait<2>();
     __syncthreads();
-    const int sm = (k - 1) & (NSLOT - 1), s0 = k & (NSLOT - 1), sp = (k + 1) & (NSLOT - 1);
-    const int kz = k - k0;
-    const double rdz_k = sZ[kz], rdzg_k = sZ[KC + kz];
-    const double czpC_k = sZ[2 * KC + kz], czmC_k = sZ[3 * KC + kz];
-    const double czpF_k = sZ[4 * KC + kz], czmF_k = sZ[5 * KC + kz];
+    if (k + 6 <= kend) issue(k + 6, s0 == 0 ? NSLOT - 1 : s0 - 1);
+    cp_async_commit();
+    double u2 = 0.0, v2 = 0.0, w2 = 0.0;
+    if (k < k1) form_plane(t + 3, s2, s3, u2, v2, w2);
+    const double *U0 = rhs_smem + s0 * L::SLOT + c, *V0 = U0 + PN, *W0 = U0 + 2 * PN;
+    const double *U1 = rhs_smem + s1 * L::SLOT + c, *V1 = U1 + PN;
+    const double2 z0 = sZ[t], z1 = sZ[a.kc + t];
+    const double2 y0 = sY[0][ty], y1 = sY[1][ty];
+    const double uxm = U0[-1], uxp = U0[1], uym = U0[-PX], uyp = U0[PX];
+    const double vxm = V0[-1], vxp = V0[1], vym = V0[-PX], vyp = V0[PX];
+    const double wxp = W0[1], wym = W0[-PX], wyp = W0[PX];
+    const double exy = mul(u0 + uyp, v0 + vxp), exz = mul(u0 + u1, w0 + wxp), eyz = mul(v0 + v1, w0 + wyp);
+    const double eu = u1 - u0, ev = v1 - v0, ew = w1 - w0;
+    const int64_t zu = at(k - 1, plU), zv = at(k - 1, plV), zw = at(k - 1, plW);
+    auto store = [&](double* S, const double* Hm, double dP, double* Go, double conv, double visc, double f, double g,
+                     int64_t z, int o) {
+      const double F = Hm ? __fma_rn(dP, __ldg(Hm + z + o), conv + visc) : (conv + visc) + dP;
+      if (MODE == 1) {
+        (S + z)[o] = __fma_rn(a.cs, F, f);
+        (Go + z)[o] = __fma_rn(a.cg, F, f);
+      } else {
+        (S + z)[o] = __fma_rn(a.cs, F, g);
+      }
+    };
     if (active) {
-      const int64_t kk = k - 1;
-      const int64_t iu = iu0 + kk * plU, iw = iw0 + kk * plW;
-      const int64_t iv = iv0 + kk * plV;
-      double gu_n = 0.0, gv_n = 0.0, gw_n = 0.0;
-      if (MODE == 2 && k < k1) {              // the next plane's accumulators
-        gu_n = __ldg(a.Gu + iu + plU);
-        gw_n = __ldg(a.Gw + iw + plW);
-        if (hasv) gv_n = __ldg(a.Gv + iv + plV);
-      }
-#define AU(s, di, dj) sU[s][c + (di) + (dj) * PX]
-#define AV(s, di, dj) sV[s][c + (di) + (dj) * PX]
-#define AW(s, di, dj) sW[s][c + (di) + (dj) * PX]
-      const double u0 = AU(s0, 0, 0), uxm = AU(s0, -1, 0), uxp = AU(s0, 1, 0);
-      const double uym = AU(s0, 0, -1), uyp = AU(s0, 0, 1);
-      const double uzm = AU(sm, 0, 0), uzp = AU(sp, 0, 0);
-      const double v0 = AV(s0, 0, 0), vxp = AV(s0, 1, 0), vym = AV(s0, 0, -1);
-      const double w0 = AW(s0, 0, 0), wxp = AW(s0, 1, 0), wzm = AW(sm, 0, 0);
-      double Fu, Fv = 0.0, Fw;
       {
-        const double v1m = AV(s0, 1, -1);
-        const double w1m = AW(sm, 1, 0);
-        // independent partial sums (short dependency chains)
-        const double ap = u0 + uxp, am = uxm + u0;
-        const double cx = (am * am - ap * ap) * (0.25 * rdxg_i);
-        const double cy = ((uym + u0) * (vym + v1m) - (u0 + uyp) * (v0 + vxp)) * (0.25 * rdy_j);
-        const double cz = ((uzm + u0) * (wzm + w1m) - (u0 + uzp) * (w0 + wxp)) * (0.25 * rdz_k);
-        const double vx = cxpF_i * (uxp - u0) - cxmF_i * (u0 - uxm);
-        const double vy = cypC_j * (uyp - u0) - cymC_j * (u0 - uym);
-        const double vz = czpC_k * (uzp - u0) - czmC_k * (u0 - uzm);
-        const double f = a.Hu ? dPdx * __ldg(a.Hu + iu) : dPdx;
-        Fu = ((cx + cy) + (cz + f)) + ((vx + vy) + vz);
+        const double exym = mul(uym + u0, vym + V0[1 - PX]);
+        const double conv = __fma_rn(sqdiff(uxm + u0, u0 + uxp), x0.x,
+                                     __fma_rn(exym - exy, y0.x, mul(Exz - exz, z0.x)));
+        const double visc = (wdiff(x1.x, uxp - u0, x1.y, u0 - uxm) + wdiff(y1.x, uyp - u0, y1.y, u0 - uym)) +
+                            wdiff(z1.x, eu, z1.y, du);
+        store(a.Us, a.Hu, dPdx, a.Gu_out, conv, visc, u0, gu, zu, P0.u);
       }
       {
-        const double wxm = AW(s0, -1, 0), wym = AW(s0, 0, -1), wyp = AW(s0, 0, 1);
-        const double wzp = AW(sp, 0, 0);
-        const double umzp = AU(sp, -1, 0);
-        const double vzp = AV(sp, 0, 0), vymzp = AV(sp, 0, -1);
-        const double am = wzm + w0, ap = w0 + wzp;
-        const double cz = (am * am - ap * ap) * (0.25 * rdzg_k);
-        const double cx = ((uxm + umzp) * (wxm + w0) - (u0 + uzp) * (w0 + wxp)) * (0.25 * rdx_i);
-        const double cy = ((vym + vymzp) * (wym + w0) - (v0 + vzp) * (w0 + wyp)) * (0.25 * rdy_j);
-        const double vx = cxpC_i * (wxp - w0) - cxmC_i * (w0 - wxm);
-        const double vy = cypC_j * (wyp - w0) - cymC_j * (w0 - wym);
-        const double vz = czpF_k * (wzp - w0) - czmF_k * (w0 - wzm);
-        const double f = a.Hw ? dPdz * __ldg(a.Hw + iw) : dPdz;
-        Fw = ((cz + cx) + (cy + f)) + ((vx + vy) + vz);
+        const double2 z2 = sZ[2 * a.kc + t];
+        const double wxm = W0[-1];
+        const double exzm = mul(uxm + U1[-1], wxm + w0), eyzm = mul(vym + V1[-PX], wym + w0);
+        const double cz = mul(w0 + w1, w0 + w1);
+        const double conv = __fma_rn(Cz - cz, z0.y, __fma_rn(exzm - exz, x0.y, mul(eyzm - eyz, y0.x)));
+        const double visc = (wdiff(x2.x, wxp - w0, x2.y, w0 - wxm) + wdiff(y1.x, wyp - w0, y1.y, w0 - wym)) +
+                            wdiff(z2.x, ew, z2.y, dw);
+        store(a.Ws, a.Hw, dPdz, a.Gw_out, conv, visc, w0, gw, zw, P0.w);
+        Cz = cz;
       }
       if (hasv) {
-        const double vxm = AV(s0, -1, 0), vyp = AV(s0, 0, 1);
-        const double vzm = AV(sm, 0, 0), vzp = AV(sp, 0, 0);
-        const double um1 = AU(s0, -1, 1);
-        const double wyp = AW(s0, 0, 1), wypzm = AW(sm, 0, 1);
-        const double am = vym + v0, ap = v0 + vyp;
-        const double cy = (am * am - ap * ap) * (0.25 * rdyg_j);
-        const double cx = ((uxm + um1) * (vxm + v0) - (u0 + uyp) * (v0 + vxp)) * (0.25 * rdx_i);
-        const double cz = ((vzm + v0) * (wzm + wypzm) - (v0 + vzp) * (w0 + wyp)) * (0.25 * rdz_k);
-        const double vx = cxpC_i * (vxp - v0) - cxmC_i * (v0 - vxm);
-        const double vy = cypF_j * (vyp - v0) - cymF_j * (v0 - vym);
-        const double vz = czpC_k * (vzp - v0) - czmC_k * (v0 - vzm);
-        const double f = a.Hv ? dPdy * __ldg(a.Hv + iv) : dPdy;
-        Fv = ((cy + cx) + (cz + f)) + ((vx + vy) + vz);
-      }
-#undef AU
-#undef AV
-#undef AW
-      if (MODE == 1) {
-        a.Us[iu] = u0 + a.cs * Fu;
-        a.Gu_out[iu] = u0 + a.cg * Fu;
-        a.Ws[iw] = w0 + a.cs * Fw;
-        a.Gw_out[iw] = w0 + a.cg * Fw;
-        if (hasv) {
-          a.Vs[iv] = v0 + a.cs * Fv;
-          a.Gv_out[iv] = v0 + a.cg * Fv;
-        }
-      } else {
-        a.Us[iu] = gu + a.cs * Fu;
-        a.Ws[iw] = gw + a.cs * Fw;
-        if (hasv) a.Vs[iv] = gv + a.cs * Fv;
-        gu = gu_n; gv = gv_n; gw = gw_n;
+        const double2 y2 = sY[2][ty];
+        const double exym = mul(uxm + U0[PX - 1], vxm + v0);
+        const double conv = __fma_rn(sqdiff(vym + v0, v0 + vyp), y0.y,
+                                     __fma_rn(exym - exy, x0.y, mul(Eyz - eyz, z0.x)));
+        const double visc = (wdiff(x2.x, vxp - v0, x2.y, v0 - vxm) + wdiff(y2.x, vyp - v0, y2.y, v0 - vym)) +
+                            wdiff(z1.x, ev, z1.y, dv);
+        store(a.Vs, a.Hv, dPdy, a.Gv_out, conv, visc, v0, gv, zv, P0.v);
       }
     }
-    // No barrier here: the slot the next iteration refills, (k+5) mod 8, held
-    // plane k-3, last read in iteration k-2; every thread finished that
-    // iteration before it reached this iteration's barrier.
+    if (MODE == 2 && k < k1) load_G(k + 1);
+    Exz = exz; Eyz = eyz;
+    du = eu; dv = ev; dw = ew;
+    u0 = u1; v0 = v1; w0 = w1;
+    u1 = u2; v1 = v2; w1 = w2;
+    s0 = s1;
   }
+  cp_async_wait<0>();
 }
 
 static RhsArgs base_args(Handle* h) {
@@ -394,11 +484,44 @@ static dim3 rhs_grid(const Dims& d) {
   return dim3((d.Nx + b.x - 1) / b.x, (d.Ny + b.y - 1) / b.y, (d.Nz + b.z - 1) / b.z);
 }
 
-static const int kRhsSmem = (3 * NSLOT * PN + 6 * KC) * (int)sizeof(double);
+constexpr int kMaxChunk = 128;   // the chunk's z factors stay in shared memory
+
+// z planes per CTA: the chunk count whose waves of resident CTAs march the
+// fewest planes; a chunk also forms the planes on its two sides and fills its
+// pipeline, worth about four planes
+static int rhs_chunk(const Dims& d, int tiles) {
+  const int slots = RHS_CTAS * 148;
+  int best = 1, cost = 1 << 30;
+  for (int n = 1; n <= d.Nz; ++n) {
+    const int kc = (d.Nz + n - 1) / n;
+    if (kc > kMaxChunk) continue;
+    const int ctas = tiles * ((d.Nz + kc - 1) / kc);
+    const int t = ((ctas + slots - 1) / slots) * (kc + 4);
+    if (t < cost) { cost = t; best = kc; }
+  }
+  return best;
+}
+
+template <int MODE, bool PROJ>
+static int launch_march(Handle* h, RhsArgs& a) {
+  const Dims& d = h->d;
+  const int gx = (d.Nx + TX - 1) / TX, gy = (d.Ny + TY - 1) / TY;
+  a.kc = rhs_chunk(d, gx * gy);
+  const dim3 grid(gx, gy, (d.Nz + a.kc - 1) / a.kc);
+  const size_t smem = RhsSmem<PROJ>::bytes(a.kc);
+  k_rhs_march<MODE, PROJ><<<grid, dim3(TX, TY), smem, h->stream>>>(a);
+  C3D_LAUNCH_CHECK(h);
+  return 0;
+}
 
 int rhs_setup(Handle* h) {
-  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_rhs_tiled<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRhsSmem));
-  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_rhs_tiled<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRhsSmem));
+  auto limit = [&](auto* k, size_t b) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+  };
+  C3D_CUDA_TRY(h, limit(k_rhs_march<1, false>, RhsSmem<false>::bytes(kMaxChunk)));
+  C3D_CUDA_TRY(h, limit(k_rhs_march<2, false>, RhsSmem<false>::bytes(kMaxChunk)));
+  C3D_CUDA_TRY(h, limit(k_rhs_march<1, true>, RhsSmem<true>::bytes(kMaxChunk)));
+  C3D_CUDA_TRY(h, limit(k_rhs_march<2, true>, RhsSmem<true>::bytes(kMaxChunk)));
   return 0;
 }
 
@@ -406,23 +529,36 @@ int rhs_setup(Handle* h) {
 int launch_rhs_stage(Handle* h, int stage, double dt) {
   RhsArgs a = base_args(h);
   a.Us = h->Us; a.Vs = h->Vs; a.Ws = h->Ws;
-  const Dims& d = h->d;
-  const dim3 tb(TX, TY, 1);
-  const dim3 tg((d.Nx + TX - 1) / TX, (d.Ny + TY - 1) / TY, (d.Nz + KC - 1) / KC);
   if (stage == 1) {
     a.Gu_out = h->Gu; a.Gv_out = h->Gv; a.Gw_out = h->Gw;
     a.cs = dt * (8.0 / 15.0);
     a.cg = dt * (1.0 / 4.0);
-    if (h->rhs_kernel == 0) C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_rhs_tiled<1>, tg, tb, kRhsSmem, h->stream, a));
-    else k_rhs<1><<<rhs_grid(d), rhs_block(), 0, h->stream>>>(a);
-  } else {
-    a.Gu = h->Gu; a.Gv = h->Gv; a.Gw = h->Gw;
-    a.cs = (stage == 2) ? dt * (5.0 / 12.0) : dt * (3.0 / 4.0);
-    if (h->rhs_kernel == 0) C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_rhs_tiled<2>, tg, tb, kRhsSmem, h->stream, a));
-    else k_rhs<2><<<rhs_grid(d), rhs_block(), 0, h->stream>>>(a);
+    return launch_march<1, false>(h, a);
   }
-  C3D_LAUNCH_CHECK(h);
-  return 0;
+  a.Gu = h->Gu; a.Gv = h->Gv; a.Gw = h->Gw;
+  a.cs = (stage == 2) ? dt * (5.0 / 12.0) : dt * (3.0 / 4.0);
+  return launch_march<2, false>(h, a);
+}
+
+// the same from the previous stage's U* (in, interior only) and potential:
+// the velocities are the projected ones, plus *ushift for u when given, with
+// the boundary conditions applied; out must not be in
+int launch_rhs_stage_projected(Handle* h, int stage, double dt, double* const in[3], const double* phi,
+                               const double* ushift, double* const out[3]) {
+  RhsArgs a = base_args(h);
+  a.U = in[0]; a.V = in[1]; a.W = in[2];
+  a.phi = phi;
+  a.ushift = ushift;
+  a.Us = out[0]; a.Vs = out[1]; a.Ws = out[2];
+  if (stage == 1) {
+    a.Gu_out = h->Gu; a.Gv_out = h->Gv; a.Gw_out = h->Gw;
+    a.cs = dt * (8.0 / 15.0);
+    a.cg = dt * (1.0 / 4.0);
+    return launch_march<1, true>(h, a);
+  }
+  a.Gu = h->Gu; a.Gv = h->Gv; a.Gw = h->Gw;
+  a.cs = (stage == 2) ? dt * (5.0 / 12.0) : dt * (3.0 / 4.0);
+  return launch_march<2, true>(h, a);
 }
 
 // compute_time_step_Euler (src/time_integration.f90:34-52): U* = U + dt*F
@@ -434,13 +570,7 @@ int launch_rhs_euler(Handle* h, double dt) {
   a.Gu_out = h->Gu; a.Gv_out = h->Gv; a.Gw_out = h->Gw;
   a.cs = dt;
   a.cg = dt;
-  const Dims& d = h->d;
-  const dim3 tb(TX, TY, 1);
-  const dim3 tg((d.Nx + TX - 1) / TX, (d.Ny + TY - 1) / TY, (d.Nz + KC - 1) / KC);
-  if (h->rhs_kernel == 0) k_rhs_tiled<1><<<tg, tb, kRhsSmem, h->stream>>>(a);
-  else k_rhs<1><<<rhs_grid(d), rhs_block(), 0, h->stream>>>(a);
-  C3D_LAUNCH_CHECK(h);
-  return 0;
+  return launch_march<1, false>(h, a);
 }
 
 // fine entries: component 1/2/3 -> rhsU/rhsV/rhsW
@@ -448,7 +578,7 @@ int launch_rhs_only(Handle* h, int component) {
   RhsArgs a = base_args(h);
   a.Us = h->rhsU; a.Vs = h->rhsV; a.Ws = h->rhsW;
   a.comp_mask = 1 << (component - 1);
-  k_rhs<0><<<rhs_grid(h->d), rhs_block(), 0, h->stream>>>(a);
+  k_rhs<<<rhs_grid(h->d), rhs_block(), 0, h->stream>>>(a);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
