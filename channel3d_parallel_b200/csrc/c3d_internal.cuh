@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <map>
 #include <string>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -88,11 +89,19 @@ struct DevScalars {
   unsigned int pad;
 };
 
+// cluster of CTAs that holds a kx slab: cs CTAs of jc rows of j, shared memory
+// row stride rs complex values, nt threads, smem bytes; narrow CTAs or not
+struct SlabCluster {
+  int cs = 1, jc = 1, rs = 0, nt = 256, smem = 0, narrow = 0;
+};
+
 // Spectral Poisson state: twiddles, Thomas factor tables and spectra for the
 // FP64 path and the FP32 (mixed-precision) path.
 struct SpectralState {
   double2 *twx = nullptr, *twz = nullptr;    // exp(-2 pi i m / n) (device)
   float2 *twx32 = nullptr, *twz32 = nullptr;
+  double2* tw1x = nullptr;                   // first-stage twiddles of the x transform, [r][q]
+  float2* tw1x32 = nullptr;
   int* posx = nullptr;                       // digit-reversed position of x coefficient m
   // Thomas factors of every (kx, kz') mode, layout [(m*Ny + j)*nkzs + kz']:
   // multipliers DL(j)/D'(j) and reciprocal pivots 1/D'(j)
@@ -111,10 +120,7 @@ struct SpectralState {
   // FP64 kx = kz = 0 mode of the FP32 path
   double* linesum = nullptr;                 // per (j, k) line sum of the right-hand side
   double* phi00 = nullptr;                   // mean solution / (Nx*Nz) per j
-  // cluster decomposition of a kx slab: cs CTAs of jc rows of j, shared
-  // memory row stride rs complex values, nt threads, smem bytes
-  int cs64 = 1, jc64 = 1, rs64 = 0, nt64 = 256, smem64 = 0, nw64 = 0;   // nw: narrow slab CTAs
-  int cs32 = 1, jc32 = 1, rs32 = 0, nt32 = 256, smem32 = 0, nw32 = 0;
+  SlabCluster cluster, cluster32;
 };
 
 struct Params {
@@ -306,6 +312,20 @@ int compute_pressure(Handle* h);
 int profile_spectral(Handle* h, int part);   // 0 div_xfft, 1 spectral_yz, 2 xfft inv
 int mixed_setup(Handle* h);
 void mixed_free(Handle* h);
+// x transforms (k_xfft.cu)
+int64_t xfft_blocks(const Dims& d);
+template <typename T>
+int xfft_setup(Handle* h);
+template <typename T>
+int launch_xfft_fwd(Handle* h, bool from_div, const double* U, const double* V, const double* W, const double* rhs,
+                    double* linesum, int blo, int bhi, double flux_dt);
+template <typename T>
+int launch_xfft_inv(Handle* h, double* out, double* phi1, const double* phi00, int accumulate, int blo, int bhi);
+// z transforms and y solves (k_slab_cluster.cu)
+template <typename T>
+int cluster_setup(Handle* h);
+template <typename T>
+int launch_cluster(Handle* h, std::conditional_t<sizeof(T) == 8, double2, float2>* spec, int zero00, int rlo, int rhi);
 // mass flow and reductions (k_massflow.cu)
 int launch_massflow_correction(Handle* h, double dt, bool euler = false, bool skip_x = false);
 int massflow(Handle* h, int comp, bool u_view, double* q_out);

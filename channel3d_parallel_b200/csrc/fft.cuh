@@ -16,7 +16,16 @@ struct FftPasses {
   int n;
   int npass;
   int radix[8];
+  // per stage: span L of its blocks, butterfly stride M = L/R, N/L, and
+  // ceil(2^32 / M) (0: M = 1)
+  int span[8], stride[8], tws[8];
+  unsigned rec[8];
 };
+
+// x / M for x * M < 2^32, rec = ceil(2^32 / M)
+__host__ __device__ inline int div_by(int x, unsigned rec) {
+  return rec == 0u ? x : (int)(((unsigned long long)(unsigned)x * rec) >> 32);
+}
 
 template <typename T> struct cplx;
 template <> struct cplx<double> { using t = double2; };
@@ -173,15 +182,27 @@ template <typename T, bool INV> struct Dft<T, INV, 16> : DftSplit<T, INV, 4, 4> 
 // an odd row stride (in complex values) eight threads of a quarter warp touch
 // eight different 16-byte bank groups, and the twiddle reads of a warp are
 // broadcasts.
-template <typename T, bool INV, int R>
+// NR: the row count where it is known when compiling (0: nrows).
+template <typename T, bool INV, int R, int NR = 0>
 __device__ __forceinline__ void ct_stage(typename cplx<T>::t* data, int nrows, int rs,
-                                         const typename cplx<T>::t* tw, int N, int L) {
+                                         const typename cplx<T>::t* tw, const FftPasses& P, int st) {
   using C = typename cplx<T>::t;
-  const int M = L / R, nb = N / R, tws = N / L;
-  const int total = nrows * nb;
+  const int L = P.span[st], M = P.stride[st], nb = P.n / R, tws = P.tws[st];
+  const unsigned rec = P.rec[st];
+  const int total = (NR ? NR : nrows) * nb;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
-    const int bb = t / nrows, l = t - bb * nrows;
-    const int blk = bb / M, q = bb - blk * M;
+    const int bb = t / (NR ? NR : nrows), l = t - bb * (NR ? NR : nrows);
+    if (rec == 0u) {              // M = 1: neighbouring elements, no twiddles
+      C* p = data + l * rs + bb * R;
+      C v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = p[r];
+      Dft<T, INV, R>::run(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) p[r] = v[r];
+      continue;
+    }
+    const int blk = div_by(bb, rec), q = bb - blk * M;
     C* p = data + l * rs + blk * L + q;
     C v[R];
 #pragma unroll
@@ -205,45 +226,100 @@ __device__ __forceinline__ void ct_stage(typename cplx<T>::t* data, int nrows, i
   __syncthreads();
 }
 
+// The stage of the whole span (L = N: the first of the forward transform, the
+// last of the inverse) with its ends wherever the caller keeps the data: ld(l,
+// e) gives and st(l, e, v) takes element e of row l.  Consecutive threads take
+// consecutive q, so global rows are read and written in runs of M elements and
+// shared-memory rows without bank conflicts; tw1[r*M + q] = w_N^(q*r).  A row
+// then goes from memory to its first stage, and from its last stage to
+// memory, through registers alone.  No barrier: the caller's ends decide.
+template <typename T, bool INV, int R, typename Ld, typename St>
+__device__ __forceinline__ void ct_edge(int nrows, int N, const typename cplx<T>::t* tw1, unsigned rec, Ld ld, St st) {
+  using C = typename cplx<T>::t;
+  const int M = N / R;
+  for (int t = threadIdx.x; t < nrows * M; t += blockDim.x) {
+    const int l = div_by(t, rec), q = t - l * M;
+    C v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = ld(l, q + r * M);
+    if (INV) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        C w = tw1[r * M + q];
+        w.y = -w.y;
+        v[r] = cmul(v[r], w);
+      }
+    }
+    Dft<T, INV, R>::run(v);
+    if (!INV) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw1[r * M + q]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) st(l, q + r * M, v[r]);
+  }
+}
+
+// radices of plans with maxr = 8
+template <typename T, bool INV, typename Ld, typename St>
+__device__ __forceinline__ void ct_edge_any(int nrows, const typename cplx<T>::t* tw1, const FftPasses& P, Ld ld,
+                                            St st) {
+  switch (P.radix[0]) {
+    case 8: ct_edge<T, INV, 8>(nrows, P.n, tw1, P.rec[0], ld, st); break;
+    case 6: ct_edge<T, INV, 6>(nrows, P.n, tw1, P.rec[0], ld, st); break;
+    case 4: ct_edge<T, INV, 4>(nrows, P.n, tw1, P.rec[0], ld, st); break;
+    case 3: ct_edge<T, INV, 3>(nrows, P.n, tw1, P.rec[0], ld, st); break;
+    default: ct_edge<T, INV, 2>(nrows, P.n, tw1, P.rec[0], ld, st); break;
+  }
+}
+
 // radices above MAXR are not compiled in (a kernel's register budget)
-template <typename T, bool INV, int MAXR>
+template <typename T, bool INV, int MAXR, int NR>
 __device__ __forceinline__ void ct_stage_any(typename cplx<T>::t* data, int nrows, int rs,
-                                             const typename cplx<T>::t* tw, int N, int L, int R) {
-  if (MAXR >= 16 && R == 16) ct_stage<T, INV, (MAXR >= 16 ? 16 : 2)>(data, nrows, rs, tw, N, L);
-  else if (MAXR >= 12 && R == 12) ct_stage<T, INV, (MAXR >= 12 ? 12 : 2)>(data, nrows, rs, tw, N, L);
-  else if (MAXR >= 8 && R == 8) ct_stage<T, INV, (MAXR >= 8 ? 8 : 2)>(data, nrows, rs, tw, N, L);
-  else if (MAXR >= 6 && R == 6) ct_stage<T, INV, (MAXR >= 6 ? 6 : 2)>(data, nrows, rs, tw, N, L);
-  else if (R == 4) ct_stage<T, INV, 4>(data, nrows, rs, tw, N, L);
-  else if (R == 3) ct_stage<T, INV, 3>(data, nrows, rs, tw, N, L);
-  else ct_stage<T, INV, 2>(data, nrows, rs, tw, N, L);
+                                             const typename cplx<T>::t* tw, const FftPasses& P, int st) {
+  const int R = P.radix[st];
+  if (MAXR >= 16 && R == 16) ct_stage<T, INV, (MAXR >= 16 ? 16 : 2), NR>(data, nrows, rs, tw, P, st);
+  else if (MAXR >= 12 && R == 12) ct_stage<T, INV, (MAXR >= 12 ? 12 : 2), NR>(data, nrows, rs, tw, P, st);
+  else if (MAXR >= 8 && R == 8) ct_stage<T, INV, (MAXR >= 8 ? 8 : 2), NR>(data, nrows, rs, tw, P, st);
+  else if (MAXR >= 6 && R == 6) ct_stage<T, INV, (MAXR >= 6 ? 6 : 2), NR>(data, nrows, rs, tw, P, st);
+  else if (R == 4) ct_stage<T, INV, 4, NR>(data, nrows, rs, tw, P, st);
+  else if (R == 3) ct_stage<T, INV, 3, NR>(data, nrows, rs, tw, P, st);
+  else ct_stage<T, INV, 2, NR>(data, nrows, rs, tw, P, st);
 }
 
 // forward transform of nrows rows; output in digit-reversed order.  The plan
-// P must come from make_fft_passes with the same MAXR.
-template <typename T, int MAXR>
+// P must come from make_fft_passes with the same MAXR.  from / to: only the
+// stages from..to-1
+template <typename T, int MAXR, int NR = 0>
 __device__ void fft_rows_dif(typename cplx<T>::t* data, int nrows, int rs,
-                             const typename cplx<T>::t* tw, const FftPasses& P) {
-  int L = P.n;
-  for (int p = 0; p < P.npass; ++p) {
-    ct_stage_any<T, false, MAXR>(data, nrows, rs, tw, P.n, L, P.radix[p]);
-    L /= P.radix[p];
-  }
+                             const typename cplx<T>::t* tw, const FftPasses& P, int from = 0, int to = 8) {
+  for (int p = from; p < P.npass && p < to; ++p) ct_stage_any<T, false, MAXR, NR>(data, nrows, rs, tw, P, p);
 }
 
-// inverse transform of nrows digit-reversed rows; output in natural order
-template <typename T, int MAXR>
+// inverse transform of nrows digit-reversed rows; output in natural order.
+// from / to: only the stages to-1 down to from
+template <typename T, int MAXR, int NR = 0>
 __device__ void fft_rows_dit_inv(typename cplx<T>::t* data, int nrows, int rs,
-                                 const typename cplx<T>::t* tw, const FftPasses& P) {
-  int L = 1;
-  for (int p = P.npass - 1; p >= 0; --p) {
-    L *= P.radix[p];
-    ct_stage_any<T, true, MAXR>(data, nrows, rs, tw, P.n, L, P.radix[p]);
-  }
+                                 const typename cplx<T>::t* tw, const FftPasses& P, int from = 0, int to = 8) {
+  for (int p = (P.npass < to ? P.npass : to) - 1; p >= from; --p)
+    ct_stage_any<T, true, MAXR, NR>(data, nrows, rs, tw, P, p);
 }
 
 // Stage plan of an N-point transform: the largest radix of 16, 12, 8, 6, 4,
 // 3, 2 (not above maxr) that divides what is left, first.  False when N is
 // not 2^a 3^b.
+__host__ inline void set_strides(FftPasses& P) {
+  int L = P.n;
+  for (int p = 0; p < P.npass; ++p) {
+    const int M = L / P.radix[p];
+    P.span[p] = L;
+    P.stride[p] = M;
+    P.tws[p] = P.n / L;
+    P.rec[p] = M > 1 ? (unsigned)(((1ull << 32) + M - 1) / M) : 0u;
+    L = M;
+  }
+}
+
 __host__ inline bool make_fft_passes(int n, FftPasses& P, int maxr) {
   static const int kRadices[] = {16, 12, 8, 6, 4, 3, 2};
   P.n = n;
@@ -257,6 +333,7 @@ __host__ inline bool make_fft_passes(int n, FftPasses& P, int maxr) {
     P.radix[P.npass++] = r;
     m /= r;
   }
+  set_strides(P);
   return m == 1 && n >= 2;
 }
 

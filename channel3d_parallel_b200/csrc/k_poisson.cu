@@ -1,25 +1,21 @@
 // Pseudo-pressure Poisson solve and projection.
 //
 // solve_poisson_equation (src/poisson.f90:33-101) restated for one GPU:
-//   per y-plane 2-D DFT over (x, z)   -> k_xfft_fwd: x real-to-complex FFT of
-//                                        each (j, k) line (two real lines per
-//                                        complex FFT), divergence fused in;
-//   per (kx, kz) tridiagonal in y     -> k_spectral_yz: one thread-block
-//   (Zgtsv, :50-75)                      cluster per kx slab; each CTA brings
-//                                        its rows of the slab into shared
-//                                        memory with bulk copies, does the z
-//                                        FFT in place, the Thomas elimination
-//                                        in j (carried across the cluster's
-//                                        CTAs through distributed shared
-//                                        memory), the inverse z FFT, and
-//                                        copies the rows back;
-//   inverse DFT / (nxp*nzp), real     -> k_xfft_inv: complex-to-real x FFT of
-//   part, periodic copies (:78-88)       the Hermitian half spectrum.
+//   per y-plane 2-D DFT over (x, z)   -> k_xfft_fwd (k_xfft.cu): x
+//                                        real-to-complex FFT of each (j, k)
+//                                        line, divergence fused in;
+//   per (kx, kz) tridiagonal in y     -> k_spectral_yz (k_slab_cluster.cu): one
+//   (Zgtsv, :50-75)                      thread-block cluster per kx slab, z
+//                                        FFT, partitioned elimination over the
+//                                        cluster's CTAs, inverse z FFT;
+//   inverse DFT / (nxp*nzp), real     -> k_xfft_inv (k_xfft.cu):
+//   part, periodic copies (:78-88)       complex-to-real x FFT of the Hermitian
+//                                        half spectrum.
 // gradient (src/differential_operators.f90:16-52) and the projection update
 // (src/projection.f90:22-46) are k_grad_sub; in the time step k_grad_sub2,
 // which also writes every ghost entry of u, v, w (the boundary conditions)
 // and, in the last stage, adds the constant-x-mass-flow shift whose bulk
-// flux the forward x FFT reduced (k_xfft_fwd<.., FLUX>).
+// flux the forward x FFT reduced (k_xfft_fwd<FROM_DIV_FLUX>).
 //
 // Two precisions share the kernels (template T): FP64, and FP32 for the
 // mixed-precision solve, where the kx = kz = 0 wall-normal mode is computed
@@ -29,32 +25,24 @@
 //
 // Spectrum layout in HBM: spec[(m*Ny + (j-2))*pz + (k-2)], m = 0..Nx/2: a kx
 // slab is Ny contiguous rows of pz >= Nz complex values.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
-#include "bulk.cuh"
 #include "c3d_internal.cuh"
 #include "fft.cuh"
 #include "ghost_images.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace c3d {
 
 // ---------------------------------------------------------------------------
 // host set-up
 // ---------------------------------------------------------------------------
-// largest FFT radix compiled into the x-FFT kernels and the two slab shapes
-// (register budgets: 64-96 registers for the x kernels and the narrow slab
-// CTAs, 128 for the wide ones)
-constexpr int kXMaxR = 8;
-constexpr int kYzMaxRWide = 16;
-constexpr int kYzMaxRNarrow = 8;
+constexpr int kBandMaxR = 16;       // largest FFT radix of the band solve (128 registers)
 
 static bool make_passes(int n, FftPasses& P) { return make_fft_passes(n, P, 8); }
+
+constexpr int kMaxNx = 512;         // longest x row
 
 static FftPasses get_passes(int n, int maxr) {
   FftPasses P{};
@@ -139,585 +127,6 @@ static int build_tri_table(Handle* h) {
 }
 
 // ---------------------------------------------------------------------------
-// kernel 1: (divergence |) x real-to-complex FFT of (j, k) lines
-// ---------------------------------------------------------------------------
-// Two real x-lines form one complex line; a block transforms kLinesX complex
-// lines in place (rows of stride rs in shared memory) with a thread count
-// that is a multiple of Nx, so every FFT stage keeps one butterfly position
-// per thread.
-constexpr int kLinesX = 8;      // complex x-lines per block
-constexpr int kMaxNx = 512;
-
-template <typename T>
-struct XfwdArgs {
-  Dims d;
-  Metric m;
-  const double* __restrict__ U;
-  const double* __restrict__ V;
-  const double* __restrict__ W;
-  const double* __restrict__ rhs;             // right-hand side when not fused with div,
-                                              // or the potential phi of the residual div(U - grad phi)
-  typename cplx<T>::t* __restrict__ spec;
-  const typename cplx<T>::t* __restrict__ tw;
-  double* __restrict__ linesum;               // FP64 line sums (mixed path) or null
-  const int* __restrict__ pos;                // digit-reversed position of coefficient m
-  FftPasses P;
-  int pz;                                     // spectrum row pitch
-  int rs;                                     // shared-memory row stride
-  int64_t rbase, nlines;                      // lines rbase .. rbase+nlines-1 (a band of j rows)
-  // x bulk flux of u (FLUX kernels): per-block partials, the last block
-  // writes the constant-mass-flow correction to scw
-  double* flux_part;
-  DevScalars* scw;
-  double q0, norm, dt;
-};
-
-// real x-line r = (k-2) + Nz*(j-2); its spectrum goes to slab offset
-// (j-2)*pz + (k-2)
-__device__ __forceinline__ void line_info(const Dims& d, int pz, int64_t r, int* j, int* k, int* off) {
-  const int jj = (int)(r / d.Nz), kk = (int)(r - (int64_t)jj * d.Nz);
-  *j = 2 + jj;
-  *k = 2 + kk;
-  *off = jj * pz + kk;
-}
-
-// shared-memory carve-up of the x-FFT kernels
-template <typename T>
-struct XfftSmem {
-  typename cplx<T>::t* tw;     // [N]
-  typename cplx<T>::t* buf;    // [kLinesX][rs]
-  int* pos;                    // [N] digit-reversed position of coefficient m
-  double* sval;                // [2*kLinesX][N] FP64 values for line sums (FP32 path)
-};
-
-template <typename T>
-__device__ __forceinline__ XfftSmem<T> xfft_carve(unsigned char* base, int N, int rs) {
-  using C = typename cplx<T>::t;
-  XfftSmem<T> s;
-  s.tw = reinterpret_cast<C*>(base);
-  s.buf = s.tw + N;
-  s.pos = reinterpret_cast<int*>(s.buf + (size_t)kLinesX * rs);
-  s.sval = reinterpret_cast<double*>(s.pos + N + (N & 1));   // FP32 path only
-  return s;
-}
-
-// FLUX: the bulk flux of u (src/mass_flow.f90:24-53, 144-175) is reduced
-// from the u values this kernel reads (compute_time_step_RK3's correction,
-// src/time_integration.f90:187-193, then needs no pass of its own): weights
-// wq(j) + wq(j+1) per row and plane 2 twice (plane nzg-1 is its copy).
-//
-// RESID (refinement of the FP32 solve): the divergence of U - grad(phi), the
-// projection of (U, V, W) with the potential in rhs, formed as the projection
-// update forms it, so that field is neither written nor read back (32 bytes a
-// cell read in place of 56 for the update and 24 for its divergence).
-template <bool FROM_DIV, typename T, bool FLUX = false, bool RESID = false>
-__global__ void __launch_bounds__(kMaxNx) k_xfft_fwd(XfwdArgs<T> a) {
-  using C = typename cplx<T>::t;
-  extern __shared__ __align__(16) unsigned char xf_smem[];
-  __shared__ int s_j[2 * kLinesX], s_off[2 * kLinesX];
-  __shared__ double s_cq[FLUX ? 2 * kLinesX : 1];
-  // per real line: offsets of the x = 2 cell of u(j,k), v(j,k), v(j-1,k),
-  // w(j,k), w(j,k-1) (FROM_DIV) or of the right-hand side; -1: a zero wall
-  // value of v (j-1 = 1 or j = ny), or no line
-  __shared__ int64_t s_bu[2 * kLinesX], s_bv[2 * kLinesX], s_bvm[2 * kLinesX];
-  __shared__ int64_t s_bw[2 * kLinesX], s_bwm[2 * kLinesX];
-  __shared__ double s_ry[2 * kLinesX], s_rz[2 * kLinesX];
-  // RESID: phi of the line, of its y and z neighbours, and the gradient's 1/dyg, 1/dzg
-  constexpr int kRes = RESID ? 2 * kLinesX : 1;
-  __shared__ int64_t s_p[kRes], s_pym[kRes], s_pzm[kRes];
-  __shared__ double s_gy[kRes], s_gym[kRes], s_gz[kRes], s_gzm[kRes];
-  const Dims& d = a.d;
-  const int N = d.Nx, RS = a.rs;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  XfftSmem<T> sm = xfft_carve<T>(xf_smem, N, RS);
-  for (int t = tid; t < N; t += nt) {
-    sm.tw[t] = a.tw[t];
-    sm.pos[t] = a.pos[t];
-  }
-  const int64_t nreal = a.rbase + a.nlines;
-  const int64_t r0 = a.rbase + (int64_t)blockIdx.x * kLinesX * 2;
-  if (tid < 2 * kLinesX) {
-    const int64_t r = r0 + tid;
-    int j = -1, k = -1, off = 0;
-    int64_t bu = -1, bv = -1, bvm = -1, bw = 0, bwm = 0;
-    double ry = 0.0, rz = 0.0;
-    if (r < nreal) {
-      line_info(d, a.pz, r, &j, &k, &off);
-      if (FROM_DIV) {
-        // the ghost values are read as the boundary conditions define them
-        // (periodic images in x and z, zero V walls), so the fields need no
-        // ghost fill after the stage update
-        const int64_t plw = (int64_t)d.nxg * d.nyg;
-        const int64_t iv = idxV(d, 2, j, k), iw = idxW(d, 2, j, k);
-        bu = idxU(d, 2, j, k);
-        bv = j == d.ny ? -1 : iv;
-        bvm = j == 2 ? -1 : iv - d.nxg;
-        bw = iw;
-        bwm = k == 2 ? iw + (int64_t)(d.Nz - 1) * plw : iw - plw;
-        ry = a.m.rdy[j];
-        rz = a.m.rdz[k];
-        if (FLUX) s_cq[tid] = a.m.cqu[j] * (k == 2 ? 2.0 : 1.0);
-        if (RESID) {
-          const int km = k == 2 ? d.Nz + 1 : k - 1;
-          s_p[tid] = idxR(d, 2, j, k);
-          s_pym[tid] = j == 2 ? s_p[tid] : idxR(d, 2, j - 1, k);
-          s_pzm[tid] = idxR(d, 2, j, km);
-          s_gy[tid] = j == d.ny ? 0.0 : a.m.rdyg[j];
-          s_gym[tid] = j == 2 ? 0.0 : a.m.rdyg[j - 1];
-          s_gz[tid] = a.m.rdzg[k];
-          s_gzm[tid] = a.m.rdzg[km];
-        }
-      } else {
-        bu = idxR(d, 2, j, k);
-      }
-    }
-    s_j[tid] = j;
-    s_off[tid] = off;
-    s_bu[tid] = bu; s_bv[tid] = bv; s_bvm[tid] = bvm; s_bw[tid] = bw; s_bwm[tid] = bwm;
-    s_ry[tid] = ry; s_rz[tid] = rz;
-    if (FLUX && r >= nreal) s_cq[tid] = 0.0;
-  }
-  pdl_wait();
-  pdl_trigger();
-  __syncthreads();
-  double facc = 0.0;
-  // nt is a multiple of N: thread -> x index ii, real lines rl0, rl0 + nt/N, ...
-  // taken four at a time: all loads of a batch are issued before any use.
-  // u(i-1) of i = 2 is the periodic image i = N+1.
-  const int ii = tid % N, rls = nt / N;
-  const int xo = ii == 0 ? N - 1 : ii - 1;
-  const double rdx_i = FROM_DIV ? a.m.rdx[2 + ii] : 0.0;
-  const double gx = RESID ? a.m.rdxg[2 + ii] : 0.0, gxm = RESID ? a.m.rdxg[2 + xo] : 0.0;
-  constexpr int kBatch = 4;
-  for (int rb = tid / N; rb < 2 * kLinesX; rb += kBatch * rls) {
-    double x0[kBatch], x1[kBatch], y0[kBatch], y1[kBatch], z0[kBatch], z1[kBatch];
-#pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
-      const int rl = rb + q * rls;
-      const int64_t bu = rl < 2 * kLinesX ? s_bu[rl] : -1;
-      x0[q] = x1[q] = y0[q] = y1[q] = z0[q] = z1[q] = 0.0;
-      if (bu >= 0) {
-        if (FROM_DIV) {
-          const int64_t bv = s_bv[rl], bvm = s_bvm[rl];
-          x1[q] = a.U[bu + ii]; x0[q] = a.U[bu + xo];
-          if (bv >= 0) y1[q] = a.V[bv + ii];
-          if (bvm >= 0) y0[q] = a.V[bvm + ii];
-          z1[q] = a.W[s_bw[rl] + ii]; z0[q] = a.W[s_bwm[rl] + ii];
-          if (RESID) {
-            const double* ph = a.rhs + s_p[rl];
-            const int ny1 = s_gy[rl] == 0.0 ? 0 : N + 1;     // rows of phi are Nx+1 long
-            const double* pm = a.rhs + s_pzm[rl];
-            const double p0 = ph[ii];
-            x1[q] -= (ph[ii + 1] - p0) * gx;
-            x0[q] -= (ph[xo + 1] - ph[xo]) * gxm;
-            y1[q] -= (ph[ny1 + ii] - p0) * s_gy[rl];
-            y0[q] -= (p0 - a.rhs[s_pym[rl] + ii]) * s_gym[rl];
-            z1[q] -= (ph[(int64_t)(N + 1) * d.Ny + ii] - p0) * s_gz[rl];
-            z0[q] -= (pm[(int64_t)(N + 1) * d.Ny + ii] - pm[ii]) * s_gzm[rl];
-          }
-        } else {
-          x1[q] = a.rhs[bu + ii];
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
-      const int rl = rb + q * rls;
-      if (rl >= 2 * kLinesX) continue;
-      const double val = FROM_DIV ? (x1[q] - x0[q]) * rdx_i + (y1[q] - y0[q]) * s_ry[rl] + (z1[q] - z0[q]) * s_rz[rl]
-                                  : x1[q];
-      if (FLUX) facc += s_cq[rl] * x1[q];
-      C& zz = sm.buf[(rl >> 1) * RS + ii];
-      if (rl & 1) zz.y = (T)val; else zz.x = (T)val;
-      if (a.linesum) sm.sval[rl * N + ii] = val;
-    }
-  }
-  __syncthreads();
-  if (a.linesum) {   // FP64 line sums: one full warp per line, a fixed shuffle tree
-    const int warp = tid >> 5, lane = tid & 31;
-    for (int rl = warp; rl < 2 * kLinesX && (warp + 1) * 32 <= nt; rl += nt >> 5) {
-      double sum = 0.0;
-      for (int q = lane; q < N; q += 32) sum += sm.sval[rl * N + q];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane == 0 && r0 + rl < nreal) a.linesum[r0 + rl] = sum;
-    }
-  }
-  fft_rows_dif<T, kXMaxR>(sm.buf, kLinesX, RS, sm.tw, a.P);
-  // split Z = A + iB of the two real lines: A = (Z_m + conj Z_{N-m})/2,
-  // B = (Z_m - conj Z_{N-m})/(2i), m = 0..N/2
-  const int nk = d.nkx;
-  for (int t = tid; t < kLinesX * nk; t += nt) {
-    const int pl = t % kLinesX;
-    const int mm = t / kLinesX;
-    const int64_t ra = r0 + 2 * pl;
-    if (ra >= nreal) continue;
-    const C Z = sm.buf[pl * RS + sm.pos[mm]];
-    const C Zr = sm.buf[pl * RS + sm.pos[mm == 0 ? 0 : N - mm]];
-    C A, B;
-    A.x = (T)0.5 * (Z.x + Zr.x);
-    A.y = (T)0.5 * (Z.y - Zr.y);
-    B.x = (T)0.5 * (Z.y + Zr.y);
-    B.y = (T)-0.5 * (Z.x - Zr.x);
-    C* out = a.spec + (int64_t)mm * d.Ny * a.pz;
-    out[s_off[2 * pl]] = A;
-    if (ra + 1 < nreal) out[s_off[2 * pl + 1]] = B;
-  }
-  if (FLUX) {
-    // block partial by a fixed tree (any thread count up to kMaxNx); the last
-    // block adds the partials the same way, then shift = Qflow_x_0 -
-    // flux/norm and dPdx = (dPdx + shift/dt)/2
-    __shared__ double red[kMaxNx];
-    __shared__ bool last;
-    auto tree = [&](double v) {
-      red[tid] = v;
-      __syncthreads();
-      for (int st = kMaxNx / 2; st > 0; st >>= 1) {
-        if (tid < st && tid + st < nt) red[tid] += red[tid + st];
-        __syncthreads();
-      }
-      const double r = red[0];
-      __syncthreads();
-      return r;
-    };
-    const double bsum = tree(facc);
-    if (tid == 0) {
-      a.flux_part[blockIdx.x] = bsum;
-      __threadfence();
-      last = atomicAdd(&a.scw->ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last) {
-      __threadfence();
-      double t = 0.0;
-      for (unsigned b = tid; b < gridDim.x; b += nt) t += __ldcg(a.flux_part + b);
-      const double q = tree(t) / a.norm;
-      if (tid == 0) {
-        const double shift = a.q0 - q;
-        DevScalars* sc = a.scw;
-        sc->qflow = q;
-        sc->shift = shift;
-        sc->dpdx_prev = sc->dPdx;
-        sc->dPdx = 0.5 * (sc->dPdx + shift / a.dt);
-        sc->ticket = 0u;
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// kernel 2: z FFT, Thomas in y, inverse z FFT of one kx slab per cluster
-// ---------------------------------------------------------------------------
-// Two launch shapes: wide CTAs (at most 256 threads, two per SM) and narrow
-// CTAs (at most 192 threads, three per SM, half the rows).  The whole FP64
-// spectrum does not fit the aggregate shared memory at once, so the grid runs
-// in two waves either way; narrow CTAs keep more warps per SM in flight and
-// shorten each CTA's sequential sweeps.  yz_jmax: rows of j per CTA (the
-// pivots of one column are held in registers).
-template <typename T, bool NARROW>
-__host__ __device__ constexpr int yz_jmax() { return (sizeof(T) == 8 ? 32 : 64) / (NARROW ? 2 : 1); }
-template <bool NARROW>
-__host__ __device__ constexpr int yz_threads() { return NARROW ? 192 : 256; }
-template <bool NARROW>
-__host__ __device__ constexpr int yz_min_blocks() { return NARROW ? 3 : 2; }
-
-template <typename T>
-struct YzArgs {
-  Dims d;
-  typename cplx<T>::t* __restrict__ spec;
-  const typename cplx<T>::t* __restrict__ tw;
-  const T* __restrict__ rdp;     // 1/D'(j) per (m, j, kz')
-  const T* __restrict__ dl;      // Dyy(j+1, j)
-  const T* __restrict__ du;      // Dyy(j, j+1)
-  unsigned long long* err;       // sticky error bits
-  FftPasses P;
-  int cs;        // CTAs per cluster
-  int jc;        // j rows per CTA
-  int rs;        // shared-memory row stride (complex values)
-  int pz;        // HBM row pitch (complex values)
-  int zero00;    // 1: leave the kx = kz = 0 column to the FP64 mean-mode solve
-  int rlo, rhi;  // rows (j-2) with a nonzero right-hand side and rows of the
-                 // solution needed: the band [rlo, rhi]; other rows start at
-                 // zero and are not transformed back or stored
-};
-
-// CTA c of the cluster owns rows j0 = c*jc .. j0+jn-1 of the slab.  Shared
-// memory: rows [jc][rs] (the z FFT runs along a row), twiddles, DL and DU.
-// The Thomas sweeps walk a column (one kz per thread) down the rows, CTA by
-// CTA: forward elimination from CTA 0 to cs-1, back substitution from cs-1 to
-// 0, each CTA starting from the neighbour row read through distributed
-// shared memory.  After the forward transform column `col` holds wavenumber
-// kz = dif_position_to_k(col); the inverse transform takes that order back.
-template <typename T, bool NARROW>
-__global__ void __launch_bounds__(yz_threads<NARROW>(), yz_min_blocks<NARROW>()) k_spectral_yz(YzArgs<T> a) {
-  using C = typename cplx<T>::t;
-  constexpr int JM = yz_jmax<T, NARROW>();
-  extern __shared__ __align__(128) unsigned char yz_smem[];
-  __shared__ __align__(8) uint64_t bar;
-  cg::cluster_group cl = cg::this_cluster();
-  const Dims& d = a.d;
-  const int cs = a.cs;
-  const int crank = (int)cl.block_rank();
-  const int m = blockIdx.x / cs;
-  const int Ny = d.Ny, Nz = d.Nz, nkzs = d.nkzs;
-  const int RS = a.rs, Jc = a.jc;
-  const int j0 = crank * Jc;
-  const int jn = min(Jc, Ny - j0);             // rows owned by this CTA (>= 1)
-  C* data = reinterpret_cast<C*>(yz_smem);
-  C* tw = data + (size_t)Jc * RS;
-  C* ylast = tw + Nz;                          // local forward value of the last row
-  C* xfirst = ylast + Nz;                      // local back-substituted first row
-  C* yin = xfirst + Nz;                        // carry Y_in of this CTA
-  T* sdl = reinterpret_cast<T*>(yin + Nz);
-  T* sdu = sdl + Ny;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  C* g = a.spec + ((int64_t)m * Ny + j0) * a.pz;
-  const unsigned rowbytes = (unsigned)(a.pz * sizeof(C));
-
-  if (tid == 0) {
-    mbar_init(&bar, 1);
-    fence_mbar_init();
-  }
-  pdl_wait();
-  pdl_trigger();
-  __syncthreads();
-  // this CTA's rows of the band: [blo, bhi)
-  const int blo = min(max(a.rlo - j0, 0), jn), bhi = max(min(a.rhi + 1 - j0, jn), blo);
-  if (tid < 32) {
-    if (tid == 0) mbar_arrive_expect_tx(&bar, rowbytes * (unsigned)(bhi - blo));
-    __syncwarp();
-    for (int r = blo + tid; r < bhi; r += 32)
-      bulk_load(data + (size_t)r * RS, g + (int64_t)r * a.pz, rowbytes, &bar);
-  }
-  for (int t = tid; t < (jn - (bhi - blo)) * Nz; t += nt) {   // rows outside the band start at zero
-    const int rr = t / Nz, col = t - rr * Nz;
-    const int r = rr < blo ? rr : rr + (bhi - blo);
-    data[(size_t)r * RS + col] = C{(T)0, (T)0};
-  }
-  for (int t = tid; t < Nz; t += nt) tw[t] = a.tw[t];
-  for (int t = tid; t < Ny; t += nt) { sdl[t] = a.dl[t]; sdu[t] = a.du[t]; }
-
-  const bool loaded = mbar_wait(&bar, 0, kWaitCycles);
-  if (!loaded) atomicOr(a.err, 1ull);
-  __syncthreads();
-
-  fft_rows_dif<T, (NARROW ? kYzMaxRNarrow : kYzMaxRWide)>(data + (size_t)blo * RS, bhi - blo, RS, tw, a.P);
-
-  // pivots of this thread's column for rows j0-1 .. j0+jn-1 (one column per
-  // thread when Nz <= blockDim; otherwise reloaded per column below)
-  const T* rdp_m = a.rdp + (int64_t)m * Ny * nkzs;
-  const bool one_col = Nz <= nt;
-  T rdv[JM];
-  T rdm1 = (T)0;                               // pivot of row j0-1 (previous CTA)
-  auto load_pivots = [&](int col) {
-    const int kz = dif_position_to_k(col, a.P);
-    const int kzs = kz <= Nz - kz ? kz : Nz - kz;
-#pragma unroll
-    for (int jl = 0; jl < JM; ++jl)
-      rdv[jl] = jl < jn ? __ldg(rdp_m + (int64_t)(j0 + jl) * nkzs + kzs) : (T)0;
-    rdm1 = j0 > 0 ? __ldg(rdp_m + (int64_t)(j0 - 1) * nkzs + kzs) : (T)0;
-  };
-  if (one_col && tid < Nz) load_pivots(tid);
-
-  // Partitioned elimination: every CTA sweeps its own rows at once, then
-  // corrects them with carries from its neighbours (no tables):
-  //   forward: y(j) = yl(j) + h(j) Y_in,  h(j0-1) = 1, h(j) = -MULT(j-1) h(j-1),
-  //            Y_in(c+1) = yl_c(j1) + h_c(j1) Y_in(c);
-  //   backward (on the corrected y): x(j) = xl(j) + g(j) X_in,  g(j1+1) = 1,
-  //            g(j) = -DU(j)/D'(j) g(j+1),  X_in(c-1) = xl_c(j0) + g_c(j0) X_in(c).
-  // The sweeps take rows in chunks of kCh: loads of a chunk are issued
-  // together, the recurrence runs in registers, then the chunk is stored.
-  constexpr int kCh = 4;
-  // ylast / xfirst: published end values; hg[col] = (h(j1), g(j0))
-  C* hg = yin;
-  for (int col = tid; col < Nz; col += nt) {
-    if (!one_col) load_pivots(col);
-    // local forward elimination B(j) -= DL(j-1)/D'(j-1) * B(j-1) from y(j0-1) = 0
-    C prev = C{(T)0, (T)0};
-    T hcur = (T)1;
-#pragma unroll
-    for (int c0 = 0; c0 < JM; c0 += kCh) {
-      if (c0 < jn) {
-        C bv[kCh];
-        T dlv[kCh];
-#pragma unroll
-        for (int u = 0; u < kCh; ++u) {
-          const int jl = c0 + u;
-          bv[u] = C{(T)0, (T)0};
-          dlv[u] = (T)0;
-          if (jl < jn) {
-            bv[u] = data[jl * RS + col];
-            if (j0 + jl > 0) dlv[u] = sdl[j0 + jl - 1];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kCh; ++u) {
-          const int jl = c0 + u;
-          if (jl < jn) {
-            const T mu = dlv[u] * (jl == 0 ? rdm1 : rdv[jl > 0 ? jl - 1 : 0]);
-            if (jl > 0) {
-              bv[u].x = bv[u].x - mu * prev.x;
-              bv[u].y = bv[u].y - mu * prev.y;
-            }
-            hcur = -mu * hcur;
-            prev = bv[u];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kCh; ++u)
-          if (c0 + u < jn) data[(c0 + u) * RS + col] = bv[u];
-      }
-    }
-    ylast[col] = prev;
-    hg[col].x = hcur;
-  }
-  cl.sync();
-  for (int col = tid; col < Nz; col += nt) {
-    if (!one_col) load_pivots(col);
-    // Y_in = y(j0-1) from the predecessors' end values
-    C Y = C{(T)0, (T)0};
-    for (int c = 0; c < crank; ++c) {
-      const C yl = cl.map_shared_rank(ylast, c)[col];
-      const T he = cl.map_shared_rank(hg, c)[col].x;
-      const T yx = yl.x + he * Y.x, yy = yl.y + he * Y.y;
-      Y.x = yx;
-      Y.y = yy;
-    }
-    // forward correction y += h Y_in (h recomputed), then the local back
-    // substitution x(j) = (y(j) - DU(j) x(j+1)) / D'(j) from x(j1+1) = 0
-    T hcur = (T)1;
-#pragma unroll
-    for (int c0 = 0; c0 < JM; c0 += kCh) {
-      if (c0 < jn && crank > 0) {
-        C bv[kCh];
-        T dlv[kCh];
-#pragma unroll
-        for (int u = 0; u < kCh; ++u) {
-          const int jl = c0 + u;
-          bv[u] = C{(T)0, (T)0};
-          dlv[u] = (T)0;
-          if (jl < jn) {
-            bv[u] = data[jl * RS + col];
-            dlv[u] = sdl[j0 + jl - 1];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kCh; ++u) {
-          const int jl = c0 + u;
-          if (jl < jn) {
-            const T mu = dlv[u] * (jl == 0 ? rdm1 : rdv[jl > 0 ? jl - 1 : 0]);
-            hcur = -mu * hcur;
-            bv[u].x += hcur * Y.x;
-            bv[u].y += hcur * Y.y;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kCh; ++u)
-          if (c0 + u < jn) data[(c0 + u) * RS + col] = bv[u];
-      }
-    }
-    C xn = C{(T)0, (T)0};
-    T gcur = (T)1;
-#pragma unroll
-    for (int c0 = JM - kCh; c0 >= 0; c0 -= kCh) {
-      if (c0 < jn) {
-        C bv[kCh];
-        T duv[kCh];
-#pragma unroll
-        for (int u = 0; u < kCh; ++u) {
-          const int jl = c0 + u;
-          bv[u] = C{(T)0, (T)0};
-          duv[u] = (T)0;
-          if (jl < jn) {
-            bv[u] = data[jl * RS + col];
-            duv[u] = sdu[j0 + jl];
-          }
-        }
-#pragma unroll
-        for (int u = kCh - 1; u >= 0; --u) {
-          const int jl = c0 + u;
-          if (jl < jn) {
-            bv[u].x = (bv[u].x - duv[u] * xn.x) * rdv[jl];
-            bv[u].y = (bv[u].y - duv[u] * xn.y) * rdv[jl];
-            gcur = -duv[u] * rdv[jl] * gcur;
-            xn = bv[u];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kCh; ++u)
-          if (c0 + u < jn) data[(c0 + u) * RS + col] = bv[u];
-      }
-    }
-    xfirst[col] = xn;
-    hg[col].y = gcur;
-  }
-  cl.sync();
-  for (int col = tid; col < Nz; col += nt) {
-    if (!one_col) load_pivots(col);
-    // X_in = x(j1+1) from the successors' first values
-    C X = C{(T)0, (T)0};
-    for (int c = cs - 1; c > crank; --c) {
-      const C xf = cl.map_shared_rank(xfirst, c)[col];
-      const T ge = cl.map_shared_rank(hg, c)[col].y;
-      const T xx = xf.x + ge * X.x, xy = xf.y + ge * X.y;
-      X.x = xx;
-      X.y = xy;
-    }
-    // backward correction x += g X_in (g recomputed from the last row up)
-    T gcur = (T)1;
-#pragma unroll
-    for (int c0 = JM - kCh; c0 >= 0; c0 -= kCh) {
-      if (c0 < jn && crank < cs - 1) {
-        C bv[kCh];
-        T duv[kCh];
-#pragma unroll
-        for (int u = 0; u < kCh; ++u) {
-          const int jl = c0 + u;
-          bv[u] = C{(T)0, (T)0};
-          duv[u] = (T)0;
-          if (jl < jn) {
-            bv[u] = data[jl * RS + col];
-            duv[u] = sdu[j0 + jl];
-          }
-        }
-#pragma unroll
-        for (int u = kCh - 1; u >= 0; --u) {
-          const int jl = c0 + u;
-          if (jl < jn) {
-            gcur = -duv[u] * rdv[jl] * gcur;
-            bv[u].x += gcur * X.x;
-            bv[u].y += gcur * X.y;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kCh; ++u)
-          if (c0 + u < jn) data[(c0 + u) * RS + col] = bv[u];
-      }
-    }
-    if (a.zero00 && m == 0 && col == 0)
-      for (int jl = 0; jl < jn; ++jl) data[jl * RS] = C{(T)0, (T)0};
-  }
-  __syncthreads();
-
-  fft_rows_dit_inv<T, (NARROW ? kYzMaxRNarrow : kYzMaxRWide)>(data + (size_t)blo * RS, bhi - blo, RS, tw, a.P);
-  // no CTA leaves while another may still read its ylast / xfirst
-  cl.sync();
-
-  fence_async_shared();
-  __syncthreads();
-  if (tid < 32) {
-    if (loaded) {
-      for (int r = blo + tid; r < bhi; r += 32) bulk_store(g + (int64_t)r * a.pz, data + (size_t)r * RS, rowbytes);
-      bulk_commit();
-      bulk_wait_read_all();
-    } else {
-      // the rows never arrived: let the copies in flight finish before exit
-      mbar_wait(&bar, 0, kWaitCycles);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Band-restricted z transform and y solve (FP64), for the Poisson solve of
 // the Schur complement: the right-hand side is zero outside the rows
 // [rlo, rhi] and only those rows of the solution are read.  Thomas on the
@@ -725,7 +134,7 @@ __global__ void __launch_bounds__(yz_threads<NARROW>(), yz_min_blocks<NARROW>())
 // substitution starts from x(rhi+1) = S(rhi+1) y(rhi+1), y(rhi+1) =
 // -MULT(rhi) y(rhi), where S(j) = x(j)/y(j) of the homogeneous tail is
 // tabulated once (build_tail_table).  One CTA per kx slab, the band rows in
-// shared memory; the same z transform as k_spectral_yz.
+// shared memory; the band's own z transform, there and back.
 // ---------------------------------------------------------------------------
 struct BandYzArgs {
   Dims d;
@@ -767,7 +176,7 @@ __global__ void __launch_bounds__(256) k_spectral_band(BandYzArgs a) {
     }
   }
   __syncthreads();
-  fft_rows_dif<double, kYzMaxRWide>(data, nr, RS, tw, a.P);
+  fft_rows_dif<double, kBandMaxR>(data, nr, RS, tw, a.P);
   const double* rdp_m = a.rdp + (int64_t)m * Ny * nkzs;
   const double* tail_m = a.tail + (int64_t)m * Ny * nkzs;
   for (int col = tid; col < Nz; col += nt) {
@@ -807,7 +216,7 @@ __global__ void __launch_bounds__(256) k_spectral_band(BandYzArgs a) {
     }
   }
   __syncthreads();
-  fft_rows_dit_inv<double, kYzMaxRWide>(data, nr, RS, tw, a.P);
+  fft_rows_dit_inv<double, kBandMaxR>(data, nr, RS, tw, a.P);
   for (int t = tid; t < nr * Nz; t += nt) {
     const int r = t / Nz, c = t - r * Nz;
     g[(int64_t)r * a.pz + c] = data[r * RS + c];
@@ -857,7 +266,9 @@ static int launch_band_yz(Handle* h, int blo, int bhi, bool* done) {
   SpectralState& S = h->sp;
   *done = false;
   const int nr = bhi - blo + 1;
-  const size_t smem = band_yz_smem(d, S.rs64, nr);
+  int rs = d.Nz;
+  while (rs % 8 != 1) ++rs;
+  const size_t smem = band_yz_smem(d, rs, nr);
   if (nr <= 0 || smem > kBandYzSmemMax) return 0;
   int rc;
   if (!S.tail) {   // first use (outside any graph capture: the table build synchronises)
@@ -867,7 +278,7 @@ static int launch_band_yz(Handle* h, int blo, int bhi, bool* done) {
   }
   BandYzArgs a{};
   a.d = d; a.spec = S.spec; a.tw = S.twz; a.rdp = S.rdp; a.tail = S.tail; a.dl = S.dl; a.du = S.du;
-  a.P = get_passes(d.Nz, kYzMaxRWide); a.rs = S.rs64; a.pz = S.pz64; a.rlo = blo; a.rhi = bhi;
+  a.P = get_passes(d.Nz, kBandMaxR); a.rs = rs; a.pz = S.pz64; a.rlo = blo; a.rhi = bhi;
   C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_spectral_band, dim3((unsigned)d.nkx), dim3(256), smem, h->stream, a));
   C3D_LAUNCH_CHECK(h);
   *done = true;
@@ -917,381 +328,44 @@ __global__ void __launch_bounds__(1024) k_mode00(Dims d, const double* __restric
 }
 
 // ---------------------------------------------------------------------------
-// kernel 3: x complex-to-real inverse FFT, write phi into rhs_p layout
-// ---------------------------------------------------------------------------
-template <typename T>
-struct XinvArgs {
-  Dims d;
-  const typename cplx<T>::t* __restrict__ spec;
-  const typename cplx<T>::t* __restrict__ tw;
-  double* __restrict__ rhs;      // output phi (rhs_p layout)
-  double* __restrict__ phi1;     // optional second copy (P side effect)
-  const double* __restrict__ phi00;   // FP64 mean mode added to the output (mixed path)
-  int accumulate;                // 1: rhs += result (refinement)
-  const int* __restrict__ pos;   // digit-reversed position of coefficient m
-  FftPasses P;
-  int pz;                        // spectrum row pitch
-  int rs;                        // shared-memory row stride
-  int64_t rbase, nlines;         // lines rbase .. rbase+nlines-1 (a band of j rows)
-  double inv_scale;              // 1/(nxp*nzp)
-};
-
-template <typename T>
-__global__ void __launch_bounds__(kMaxNx) k_xfft_inv(XinvArgs<T> a) {
-  using C = typename cplx<T>::t;
-  extern __shared__ __align__(16) unsigned char xi_smem[];
-  __shared__ int s_j[2 * kLinesX], s_off[2 * kLinesX];
-  // per real line: offset of the x = 2 value of phi(j,k), and of phi(j,nzp+2)
-  // for the plane k = 2 that the reference duplicates (else -1)
-  __shared__ int64_t s_bo[2 * kLinesX], s_bo2[2 * kLinesX];
-  __shared__ double s_p00[2 * kLinesX];   // FP64 mean mode of each line's row (mixed path)
-  const Dims& d = a.d;
-  const int N = d.Nx, nk = d.nkx, RS = a.rs;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  XfftSmem<T> sm = xfft_carve<T>(xi_smem, N, RS);
-  for (int t = tid; t < N; t += nt) {
-    sm.tw[t] = a.tw[t];
-    sm.pos[t] = a.pos[t];
-  }
-  const int64_t nreal = a.rbase + a.nlines;
-  const int64_t r0 = a.rbase + (int64_t)blockIdx.x * kLinesX * 2;
-  if (tid < 2 * kLinesX) {
-    const int64_t r = r0 + tid;
-    int j = -1, k = -1, off = 0;
-    int64_t bo = -1, bo2 = -1;
-    if (r < nreal) {
-      line_info(d, a.pz, r, &j, &k, &off);
-      bo = idxR(d, 2, j, k);
-      if (k == 2) bo2 = idxR(d, 2, j, d.Nz + 2);
-    }
-    s_j[tid] = j;
-    s_off[tid] = off;
-    s_bo[tid] = bo;
-    s_bo2[tid] = bo2;
-  }
-  pdl_wait();
-  pdl_trigger();
-  if (a.phi00 && tid < 2 * kLinesX) s_p00[tid] = s_j[tid] >= 2 ? a.phi00[s_j[tid] - 2] : 0.0;
-  __syncthreads();
-  // Z = A + iB on the full circle from the two half spectra, placed at the
-  // digit-reversed positions the inverse transform expects
-  // the spectrum values of kU items are loaded before any of them is placed
-  constexpr int kU = 4;
-  for (int t0 = tid; t0 < kLinesX * nk; t0 += kU * nt) {
-    C Ab[kU], Bb[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int t = t0 + u * nt;
-      Ab[u] = Bb[u] = C{(T)0, (T)0};
-      if (t < kLinesX * nk) {
-        const int pl = t % kLinesX, mm = t / kLinesX;
-        const int64_t ra = r0 + 2 * pl;
-        const C* in = a.spec + (int64_t)mm * d.Ny * a.pz;
-        if (ra < nreal) Ab[u] = in[s_off[2 * pl]];
-        if (ra + 1 < nreal) Bb[u] = in[s_off[2 * pl + 1]];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int t = t0 + u * nt;
-      if (t >= kLinesX * nk) break;
-      const int pl = t % kLinesX, mm = t / kLinesX;
-      C A = Ab[u], B = Bb[u];
-      if (mm == 0 || 2 * mm == N) { A.y = (T)0; B.y = (T)0; }   // Hermitian projection
-      C Z;
-      Z.x = A.x - B.y;
-      Z.y = A.y + B.x;
-      sm.buf[pl * RS + sm.pos[mm]] = Z;
-      if (mm > 0 && 2 * mm < N) {
-        C Zc;
-        Zc.x = A.x + B.y;
-        Zc.y = -A.y + B.x;
-        sm.buf[pl * RS + sm.pos[N - mm]] = Zc;
-      }
-    }
-  }
-  __syncthreads();
-  fft_rows_dit_inv<T, kXMaxR>(sm.buf, kLinesX, RS, sm.tw, a.P);
-  const double rsd = a.inv_scale;
-  const int ii = tid % N, rls = nt / N;
-  // apply_periodic_xz_centers (src/poisson.f90:106-125): x plane nxg-1 and
-  // z plane nzp+2 duplicate plane 2
-#pragma unroll 4
-  for (int rl = tid / N; rl < 2 * kLinesX; rl += rls) {
-    const int64_t bo = s_bo[rl], bo2 = s_bo2[rl];
-    if (bo < 0) continue;
-    const C z = sm.buf[(rl >> 1) * RS + ii];
-    double v = (double)((rl & 1) ? z.y : z.x) * rsd;
-    if (a.phi00) v += s_p00[rl];
-    const int64_t o = bo + ii;
-    if (a.accumulate) v += a.rhs[o];
-    a.rhs[o] = v;
-    if (ii == 0) a.rhs[bo + N] = v;
-    if (bo2 >= 0) {
-      a.rhs[bo2 + ii] = v;
-      if (ii == 0) a.rhs[bo2 + N] = v;
-    }
-    if (a.phi1) {
-      a.phi1[o] = v;
-      if (ii == 0) a.phi1[bo + N] = v;
-      if (bo2 >= 0) {
-        a.phi1[bo2 + ii] = v;
-        if (ii == 0) a.phi1[bo2 + N] = v;
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // host drivers
 // ---------------------------------------------------------------------------
-// x-FFT launch shape: threads a multiple of Nx (at least 128), shared-memory
-// rows padded (FP64: rs = 1 mod 8, FP32: rs odd) so that the line-parallel
-// accesses are conflict-free
-static int xfft_threads(const Dims& d) {
-  int nt = d.Nx;
-  while (nt < 128) nt += d.Nx;
-  return nt;
-}
-
-template <typename T>
-static int xfft_rs(const Dims& d) {
-  int rs = d.Nx;
-  if (sizeof(T) == 8) { while (rs % 8 != 1) ++rs; }
-  else { while (rs % 2 != 1) ++rs; }
-  return rs;
-}
-
-template <typename T>
-static int xfft_smem(const Dims& d) {
-  return (int)(sizeof(typename cplx<T>::t) * ((size_t)d.Nx + (size_t)kLinesX * xfft_rs<T>(d)) +
-               sizeof(int) * (d.Nx + (d.Nx & 1)) +
-               (sizeof(T) == 4 ? sizeof(double) * 2 * kLinesX * d.Nx : 0));
-}
-
-// cluster decomposition of a kx slab: the narrow shape when it fits (Nz <=
-// 192, a CTA within 72 KB so three share an SM), else the wide shape (two
-// CTAs per SM within 112 KB; 16-CTA clusters may use up to one SM each); in
-// each the smallest power-of-two cluster whose CTAs own at most yz_jmax rows.
-// Row stride: FP64 rows of 16-byte values padded to rs = 1 (mod 8) make
-// row-to-row steps conflict-free; FP32 rows stay 16-byte aligned for the
-// bulk copies (rs even) with rs = 2 (mod 4).
-template <typename T, bool NARROW>
-static bool choose_shape(const Dims& d, int rs, int& cs, int& jc, int& nt, int& smem) {
-  const size_t esz = sizeof(typename cplx<T>::t);
-  const int ntmax = yz_threads<NARROW>();
-  // a multiple of Nz (one column per thread, fixed FFT butterflies) when
-  // Nz <= ntmax
-  nt = ntmax;
-  if (d.Nz <= ntmax) {
-    nt = d.Nz * (ntmax / d.Nz);
-    if (nt > 128 && d.Nz >= 128) nt = d.Nz;
-  } else if (NARROW) {
-    return false;
-  }
-  const size_t limit = NARROW ? 72 * 1024 : 112 * 1024;
-  for (cs = 1; cs <= 16; cs *= 2) {
-    jc = (d.Ny + cs - 1) / cs;
-    if ((cs - 1) * jc >= d.Ny) continue;      // every CTA must own a row
-    if (jc > yz_jmax<T, NARROW>()) continue;
-    const size_t bytes = esz * ((size_t)jc * rs + 4 * (size_t)d.Nz) + 2 * sizeof(T) * d.Ny;
-    if (bytes <= limit || (!NARROW && cs == 16 && bytes <= 224 * 1024)) {
-      smem = (int)bytes;
-      return true;
-    }
-  }
-  return false;
-}
-
-// Function attributes are process-wide and handles of different sizes share
-// them, so a kernel's dynamic shared-memory limit only ever grows (per
-// device; handles are created from one host thread at a time).
-template <auto KERN>
-static cudaError_t raise_smem_limit(int bytes) {
-  static int cur[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  if (bytes <= cur[dev]) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) cur[dev] = bytes;
-  return e;
-}
-
-template <typename T, bool NARROW>
-static int active_clusters(int cs, int nt, int smem) {
-  if (raise_smem_limit<k_spectral_yz<T, NARROW>>(smem) != cudaSuccess) return 0;
-  if (cs > 8 &&
-      cudaFuncSetAttribute(k_spectral_yz<T, NARROW>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-    return 0;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)cs, 1, 1);
-  cfg.blockDim = dim3((unsigned)nt, 1, 1);
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_spectral_yz<T, NARROW>, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n;
-}
-
-// Picks the shape whose kx slabs (one cluster each) run in fewer waves of
-// co-resident clusters, as the device reports them; the narrow shape on a tie.
-template <typename T>
-static bool choose_cluster(const Dims& d, int pz, int& cs, int& jc, int& rs, int& nt, int& smem, int& narrow) {
-  rs = pz;
-  if (sizeof(T) == 8) { while (rs % 8 != 1) ++rs; }
-  else { while (rs % 4 != 2) ++rs; }
-  int ncs, njc, nnt, nsm, wcs, wjc, wnt, wsm;
-  const bool okn = choose_shape<T, true>(d, rs, ncs, njc, nnt, nsm);
-  const bool okw = choose_shape<T, false>(d, rs, wcs, wjc, wnt, wsm);
-  auto waves = [&](int active) { return active > 0 ? (d.nkx + active - 1) / active : 1 << 30; };
-  const int wn = okn ? waves(active_clusters<T, true>(ncs, nnt, nsm)) : 1 << 30;
-  const int ww = okw ? waves(active_clusters<T, false>(wcs, wnt, wsm)) : 1 << 30;
-  if (okn && (!okw || wn <= ww)) {
-    narrow = 1; cs = ncs; jc = njc; nt = nnt; smem = nsm;
-    return true;
-  }
-  if (!okw) return false;
-  narrow = 0; cs = wcs; jc = wjc; nt = wnt; smem = wsm;
-  return true;
-}
-
-template <typename T>
-static int launch_yz(Handle* h, typename cplx<T>::t* spec, const typename cplx<T>::t* tw, const T* rdp,
-                     const T* dl, const T* du, int cs, int jc, int rs, int pz, int nt, int smem, int narrow,
-                     int zero00, int rlo, int rhi) {
-  const Dims& d = h->d;
-  YzArgs<T> a{};
-  a.d = d; a.spec = spec; a.tw = tw; a.rdp = rdp; a.dl = dl; a.du = du;
-  a.err = &h->sc->err;
-  a.P = get_passes(d.Nz, narrow ? kYzMaxRNarrow : kYzMaxRWide); a.cs = cs; a.jc = jc; a.rs = rs; a.pz = pz; a.zero00 = zero00;
-  a.rlo = rlo; a.rhi = rhi;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(cs * d.nkx), 1, 1);
-  cfg.blockDim = dim3((unsigned)nt, 1, 1);
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cfg.stream = h->stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = h->use_pdl ? 2 : 1;
-  if (narrow) C3D_CUDA_TRY(h, cudaLaunchKernelEx(&cfg, k_spectral_yz<T, true>, a));
-  else C3D_CUDA_TRY(h, cudaLaunchKernelEx(&cfg, k_spectral_yz<T, false>, a));
-  C3D_LAUNCH_CHECK(h);
-  return 0;
-}
-
-template <typename T>
-static int set_limits(Handle* h, int smem_yz, int cs) {
-  const Dims& d = h->d;
-  const int smx = xfft_smem<T>(d);
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<true, T>>(smx)));
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<false, T>>(smx)));
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<true, T, true>>(smx)));
-  if (sizeof(T) == 4) C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_fwd<true, float, false, true>>(smx)));
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_xfft_inv<T>>(smx)));
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_spectral_yz<T, true>>(smem_yz)));
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_spectral_yz<T, false>>(smem_yz)));
-  if (cs > 8) {
-    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_spectral_yz<T, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_spectral_yz<T, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  }
-  return 0;
-}
-
-// parts: bit0 x FFT, bit1 yz, bit2 inverse x FFT
+// parts: bit0 x FFT, bit1 y-z solve, bit2 inverse x FFT.  rhs_in: the
+// right-hand side, or with from_div the potential whose residual
+// div((U, V, W) - grad rhs_in) is solved for (FP32).
 template <typename T>
 static int run_spectral_t(Handle* h, bool from_div, const double* U, const double* V, const double* W,
                           const double* rhs_in, double* out, double* phi1, int accumulate, int parts,
                           int blo = 0, int bhi = -1, double flux_dt = 0.0) {
   const Dims& d = h->d;
   SpectralState& S = h->sp;
-  cudaStream_t s = h->stream;
-  const bool f32 = sizeof(T) == 4;
-  using C = typename cplx<T>::t;
-  C* spec;
-  const C *twx, *twz;
-  const T *rdp, *dl, *du;
-  int cs, jc, rs, pz, nt, smem, narrow;
-  if (f32) {
-    spec = (C*)S.spec32; twx = (const C*)S.twx32; twz = (const C*)S.twz32;
-    rdp = (const T*)S.rdp32; dl = (const T*)S.dl32; du = (const T*)S.du32;
-    cs = S.cs32; jc = S.jc32; rs = S.rs32; pz = S.pz32; nt = S.nt32; smem = S.smem32; narrow = S.nw32;
-  } else {
-    spec = (C*)S.spec; twx = (const C*)S.twx; twz = (const C*)S.twz;
-    rdp = (const T*)S.rdp; dl = (const T*)S.dl; du = (const T*)S.du;
-    cs = S.cs64; jc = S.jc64; rs = S.rs64; pz = S.pz64; nt = S.nt64; smem = S.smem64; narrow = S.nw64;
-  }
-  const FftPasses Px = get_passes(d.Nx, kXMaxR);
+  constexpr bool f32 = sizeof(T) == 4;
+  int rc;
   if (bhi < 0) bhi = d.Ny - 1;                 // band of j rows (0-based j-2); full by default
-  const int64_t rbase = (int64_t)blo * d.Nz, nlines = (int64_t)(bhi - blo + 1) * d.Nz;
-  const int64_t npairs = (nlines + 1) / 2;
-  const unsigned nbx = (unsigned)((npairs + kLinesX - 1) / kLinesX);
-  const int smx = xfft_smem<T>(d);
-  const int ntx = xfft_threads(d);
-  const int rsx = xfft_rs<T>(d);
   if (parts & 1) {
-    XfwdArgs<T> a{};
-    a.d = d; a.m = h->m; a.U = U; a.V = V; a.W = W; a.rhs = rhs_in;
-    a.spec = spec; a.tw = twx; a.P = Px; a.pz = pz; a.rs = rsx; a.rbase = rbase; a.nlines = nlines;
-    a.linesum = f32 ? S.linesum : nullptr;
-    a.pos = S.posx;
-    if (flux_dt > 0.0 && from_div && nlines == (int64_t)d.Ny * d.Nz) {
-      // the x bulk flux of U reduced on the way (constant x mass flow)
-      if (h->flux_part_len < (int64_t)nbx) {
-        h->last_error = "x bulk-flux partials not allocated";
-        return C3D_ERR_CUDA;
-      }
-      a.flux_part = h->flux_part; a.scw = h->sc;
-      a.q0 = h->Qflow_x_0; a.norm = h->norm_u; a.dt = flux_dt;
-      C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_fwd<true, T, true>, nbx, ntx, smx, s, a));
-    } else if (from_div && rhs_in) {
-      if constexpr (sizeof(T) == 4)
-        C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_fwd<true, T, false, true>, nbx, ntx, smx, s, a));
-    } else if (from_div) {
-      C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_fwd<true, T>, nbx, ntx, smx, s, a));
-    } else {
-      C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_fwd<false, T>, nbx, ntx, smx, s, a));
-    }
-    C3D_LAUNCH_CHECK(h);
+    const bool whole = blo == 0 && bhi == d.Ny - 1;
+    if ((rc = launch_xfft_fwd<T>(h, from_div, U, V, W, rhs_in, f32 ? S.linesum : nullptr, blo, bhi,
+                                 from_div && whole ? flux_dt : 0.0)))
+      return rc;
     if (f32) {
-      k_mode00<<<1, 1024, 4 * sizeof(double) * d.Ny, s>>>(d, S.linesum, S.mult, S.rdp, S.du, S.phi00);
+      k_mode00<<<1, 1024, 4 * sizeof(double) * d.Ny, h->stream>>>(d, S.linesum, S.mult, S.rdp, S.du, S.phi00);
       C3D_LAUNCH_CHECK(h);
     }
   }
   if (parts & 2) {
     bool band_done = false;
     if (!f32 && (blo > 0 || bhi < d.Ny - 1)) {   // a band of rows: the band-restricted solve
-      int rc = launch_band_yz(h, blo, bhi, &band_done);
-      if (rc) return rc;
+      if ((rc = launch_band_yz(h, blo, bhi, &band_done))) return rc;
     }
     if (!band_done) {
-      int rc = launch_yz<T>(h, spec, twz, rdp, dl, du, cs, jc, rs, pz, nt, smem, narrow, f32 ? 1 : 0, blo, bhi);
+      std::conditional_t<f32, float2, double2>* spec;
+      if constexpr (f32) spec = S.spec32; else spec = S.spec;
+      rc = launch_cluster<T>(h, spec, f32 ? 1 : 0, blo, bhi);
       if (rc) return rc;
     }
   }
   if (parts & 4) {
-    XinvArgs<T> a{};
-    a.d = d; a.spec = spec; a.tw = twx; a.rhs = out; a.phi1 = phi1;
-    a.phi00 = f32 ? S.phi00 : nullptr; a.accumulate = accumulate;
-    a.pos = S.posx;
-    a.P = Px; a.pz = pz; a.rs = rsx; a.rbase = rbase; a.nlines = nlines;
-    a.inv_scale = 1.0 / ((double)d.Nx * (double)d.Nz);
-    C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_xfft_inv<T>, nbx, ntx, smx, s, a));
-    C3D_LAUNCH_CHECK(h);
+    if ((rc = launch_xfft_inv<T>(h, out, phi1, f32 ? S.phi00 : nullptr, accumulate, blo, bhi))) return rc;
   }
   if (parts == 7) h->stats.poisson_solves++;
   return 0;
@@ -1604,23 +678,13 @@ int poisson_setup(Handle* h) {
   int rc;
   if (S.spec == nullptr) {
     S.pz64 = d.Nz;
-    if (!choose_cluster<double>(d, S.pz64, S.cs64, S.jc64, S.rs64, S.nt64, S.smem64, S.nw64)) {
-      h->last_error = "ny_global too large for one 16-CTA cluster per kx slab";
-      return C3D_ERR_UNSUPPORTED;
-    }
+    if ((rc = cluster_setup<double>(h))) return rc;
     if ((rc = make_twiddles(h, d.Nx, &S.twx))) return rc;
     if ((rc = make_twiddles(h, d.Nz, &S.twz))) return rc;
-    {
-      const FftPasses Px = get_passes(d.Nx, kXMaxR);
-      std::vector<int> pos(d.Nx);
-      for (int m = 0; m < d.Nx; ++m) pos[m] = dif_k_to_position(m, Px);
-      if ((rc = dev_alloc(h, &S.posx, d.Nx))) return rc;
-      C3D_CUDA_TRY(h, cudaMemcpy(S.posx, pos.data(), sizeof(int) * d.Nx, cudaMemcpyHostToDevice));
-    }
+    if ((rc = xfft_setup<double>(h))) return rc;
     const int64_t ns = (int64_t)d.Ny * S.pz64 * d.nkx;
     if ((rc = dev_alloc(h, &S.spec, ns))) return rc;
-    if ((rc = set_limits<double>(h, S.smem64, S.cs64))) return rc;
-    const int64_t nbx = (((int64_t)d.Ny * d.Nz + 1) / 2 + kLinesX - 1) / kLinesX;
+    const int64_t nbx = xfft_blocks(d);
     if ((rc = dev_alloc(h, &h->flux_part, nbx))) return rc;
     h->flux_part_len = nbx;
   }
@@ -1632,18 +696,15 @@ int mixed_setup(Handle* h) {
   SpectralState& S = h->sp;
   if (S.spec32 != nullptr) return 0;
   S.pz32 = d.Nz + (d.Nz & 1);
-  if (!choose_cluster<float>(d, S.pz32, S.cs32, S.jc32, S.rs32, S.nt32, S.smem32, S.nw32)) {
-    h->last_error = "ny_global too large for the FP32 cluster decomposition";
-    return C3D_ERR_UNSUPPORTED;
-  }
   int rc;
+  if ((rc = cluster_setup<float>(h))) return rc;
   if ((rc = make_twiddles(h, d.Nx, &S.twx32))) return rc;
   if ((rc = make_twiddles(h, d.Nz, &S.twz32))) return rc;
   const int64_t ns = (int64_t)d.Ny * S.pz32 * d.nkx;
   if ((rc = dev_alloc(h, &S.spec32, ns))) return rc;
   if ((rc = dev_alloc(h, &S.linesum, (int64_t)d.Ny * d.Nz))) return rc;
   if ((rc = dev_alloc(h, &S.phi00, d.Ny))) return rc;
-  if ((rc = set_limits<float>(h, S.smem32, S.cs32))) return rc;
+  if ((rc = xfft_setup<float>(h))) return rc;
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return 0;
 }
