@@ -89,6 +89,18 @@ struct DevScalars {
   unsigned int pad;
 };
 
+// tables and workspaces of the slab kernels (k_slab.cu), per precision
+template <typename T>
+struct SlabTables {
+  using C = std::conditional_t<sizeof(T) == 8, double2, float2>;
+  C* tw1 = nullptr;             // first-stage twiddles of the z transform
+  int* kzs = nullptr;           // kz' of each transformed position
+  T* link = nullptr;            // factors across a block of rows
+  C* ends = nullptr;            // end values of the blocks
+  unsigned* ticket = nullptr;   // per slab, zero between solves
+  int jr = 0, nblk = 0;         // rows per block, blocks of a slab
+};
+
 // cluster of CTAs that holds a kx slab: cs CTAs of jc rows of j, shared memory
 // row stride rs complex values, nt threads, smem bytes; narrow CTAs or not
 struct SlabCluster {
@@ -102,6 +114,8 @@ struct SpectralState {
   float2 *twx32 = nullptr, *twz32 = nullptr;
   double2* tw1x = nullptr;                   // first-stage twiddles of the x transform, [r][q]
   float2* tw1x32 = nullptr;
+  SlabTables<double> slab;
+  SlabTables<float> slab32;
   int* posx = nullptr;                       // digit-reversed position of x coefficient m
   // Thomas factors of every (kx, kz') mode, layout [(m*Ny + j)*nkzs + kz']:
   // multipliers DL(j)/D'(j) and reciprocal pivots 1/D'(j)
@@ -321,11 +335,15 @@ int launch_xfft_fwd(Handle* h, bool from_div, const double* U, const double* V, 
                     double* linesum, int blo, int bhi, double flux_dt);
 template <typename T>
 int launch_xfft_inv(Handle* h, double* out, double* phi1, const double* phi00, int accumulate, int blo, int bhi);
-// z transforms and y solves (k_slab_cluster.cu)
+// z transforms and y solves (k_slab.cu)
+int slab_setup(Handle* h, bool f32);
+template <typename T>
+int launch_slab(Handle* h, typename SlabTables<T>::C* spec, int zero00, int rlo, int rhi);
+// the same in one kernel (k_slab_cluster.cu)
 template <typename T>
 int cluster_setup(Handle* h);
 template <typename T>
-int launch_cluster(Handle* h, std::conditional_t<sizeof(T) == 8, double2, float2>* spec, int zero00, int rlo, int rhi);
+int launch_cluster(Handle* h, typename SlabTables<T>::C* spec, int zero00, int rlo, int rhi);
 // mass flow and reductions (k_massflow.cu)
 int launch_massflow_correction(Handle* h, double dt, bool euler = false, bool skip_x = false);
 int massflow(Handle* h, int comp, bool u_view, double* q_out);

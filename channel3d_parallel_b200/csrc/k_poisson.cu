@@ -4,10 +4,9 @@
 //   per y-plane 2-D DFT over (x, z)   -> k_xfft_fwd (k_xfft.cu): x
 //                                        real-to-complex FFT of each (j, k)
 //                                        line, divergence fused in;
-//   per (kx, kz) tridiagonal in y     -> k_spectral_yz (k_slab_cluster.cu): one
-//   (Zgtsv, :50-75)                      thread-block cluster per kx slab, z
-//                                        FFT, partitioned elimination over the
-//                                        cluster's CTAs, inverse z FFT;
+//   per (kx, kz) tridiagonal in y     -> k_slab_fwd, k_slab_inv (k_slab.cu):
+//   (Zgtsv, :50-75)                      z FFT, partitioned elimination over
+//                                        blocks of rows, inverse z FFT;
 //   inverse DFT / (nxp*nzp), real     -> k_xfft_inv (k_xfft.cu):
 //   part, periodic copies (:78-88)       complex-to-real x FFT of the Hermitian
 //                                        half spectrum.
@@ -330,6 +329,15 @@ __global__ void __launch_bounds__(1024) k_mode00(Dims d, const double* __restric
 // ---------------------------------------------------------------------------
 // host drivers
 // ---------------------------------------------------------------------------
+// Which form of the z transforms and y solves: the cluster that keeps a slab on
+// chip moves the spectrum once in place of twice, but needs 16 CTAs of an SM
+// each for the large slabs, and past 256 columns a thread has several.
+// Measured, cluster against blocks (us, B200): 192x128x192 49 / 67,
+// 256x128x256 97 / 114, 64x256x64 19 / 33; 16 CTAs: 192x256x192 156 / 134,
+// 256x192x256 276 / 165, 384x256x384 1237 / 533; 8 CTAs with Nz = 384:
+// 128x64x384 89 / 65, 384x64x384 222 / 145.
+static bool slab_by_blocks(const Dims& d, const SlabCluster& c) { return c.cs > 8 || d.Nz > 256; }
+
 // parts: bit0 x FFT, bit1 y-z solve, bit2 inverse x FFT.  rhs_in: the
 // right-hand side, or with from_div the potential whose residual
 // div((U, V, W) - grad rhs_in) is solved for (FP32).
@@ -358,9 +366,11 @@ static int run_spectral_t(Handle* h, bool from_div, const double* U, const doubl
       if ((rc = launch_band_yz(h, blo, bhi, &band_done))) return rc;
     }
     if (!band_done) {
-      std::conditional_t<f32, float2, double2>* spec;
+      typename SlabTables<T>::C* spec;
       if constexpr (f32) spec = S.spec32; else spec = S.spec;
-      rc = launch_cluster<T>(h, spec, f32 ? 1 : 0, blo, bhi);
+      const SlabCluster& c = f32 ? S.cluster32 : S.cluster;
+      rc = slab_by_blocks(d, c) ? launch_slab<T>(h, spec, f32 ? 1 : 0, blo, bhi)
+                                : launch_cluster<T>(h, spec, f32 ? 1 : 0, blo, bhi);
       if (rc) return rc;
     }
   }
@@ -688,7 +698,9 @@ int poisson_setup(Handle* h) {
     if ((rc = dev_alloc(h, &h->flux_part, nbx))) return rc;
     h->flux_part_len = nbx;
   }
-  return build_tri_table(h);
+  if ((rc = build_tri_table(h))) return rc;
+  if (S.spec32 && (rc = slab_setup(h, true))) return rc;
+  return slab_setup(h, false);
 }
 
 int mixed_setup(Handle* h) {
@@ -705,6 +717,7 @@ int mixed_setup(Handle* h) {
   if ((rc = dev_alloc(h, &S.linesum, (int64_t)d.Ny * d.Nz))) return rc;
   if ((rc = dev_alloc(h, &S.phi00, d.Ny))) return rc;
   if ((rc = xfft_setup<float>(h))) return rc;
+  if ((rc = slab_setup(h, true))) return rc;
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return 0;
 }

@@ -1,6 +1,7 @@
 // The z transforms and wall-normal solves of the Poisson equation
 // (src/poisson.f90:45-80), one thread-block cluster per kx slab: the slab stays
-// in the cluster's shared memory from its first read to its last write.
+// in the cluster's shared memory from its first read to its last write (the
+// two-kernel form in k_slab.cu is for slabs that this holds badly).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -423,7 +424,7 @@ static bool choose_cluster(const Dims& d, int pz, int& cs, int& jc, int& rs, int
 
 // z transforms and y solves of the whole spectrum in place, one launch
 template <typename T>
-int launch_cluster(Handle* h, std::conditional_t<sizeof(T) == 8, double2, float2>* spec, int zero00, int rlo, int rhi) {
+int launch_cluster(Handle* h, typename SlabTables<T>::C* spec, int zero00, int rlo, int rhi) {
   const Dims& d = h->d;
   SpectralState& S = h->sp;
   constexpr bool f32 = sizeof(T) == 4;
