@@ -237,7 +237,12 @@ static int setup_metric(Handle* h, const double* xf, const double* yf, const dou
     czpF[k] = nu / ((z[k + 1] - z[k]) * (zg[k + 1] - zg[k]));
     czmF[k] = nu / ((z[k] - z[k - 1]) * (zg[k + 1] - zg[k]));
   }
+  std::vector<double> dxg(LX, 0), dyg(LY, 0), dzg(LZ, 0);
+  for (int i = 1; i <= nxg - 1; ++i) dxg[i] = xg[i + 1] - xg[i];
+  for (int j = 1; j <= nyg - 1; ++j) dyg[j] = yg[j + 1] - yg[j];
+  for (int k = 1; k <= nzg - 1; ++k) dzg[k] = zg[k + 1] - zg[k];
   Metric& m = h->m;
+  add(dxg, &m.dxg); add(dyg, &m.dyg); add(dzg, &m.dzg);
   add(rdx, &m.rdx); add(rdxg, &m.rdxg); add(cxpF, &m.cxpF); add(cxmF, &m.cxmF);
   add(cxpC, &m.cxpC); add(cxmC, &m.cxmC);
   add(rdy, &m.rdy); add(rdyg, &m.rdyg); add(cypC, &m.cypC); add(cymC, &m.cymC);
@@ -1096,7 +1101,7 @@ int c3d_get_stats(int id, c3d_stats* out) {
 int c3d_check_divergence(int id, double* mx) {
   GET_HANDLE(id);
   if (!mx) return C3D_ERR_PARAM;
-  RET(h, max_abs_divergence(h, h->U, h->V, h->W, mx));
+  RET(h, max_abs_divergence(h, mx));
 }
 
 int c3d_check_finite(int id) {

@@ -72,6 +72,8 @@ struct Metric {
   const double *czpF, *czmF;   // viscous z for z-face fields (W)
   // mass-flow weights 0.5*(yg(j)-yg(j-1)) (U, W) and 0.5*(y(j)-y(j-1)) (V)
   const double *wq, *wqv;
+  // centre spacings xg(i+1) - xg(i) and so on (compute_dt)
+  const double *dxg, *dyg, *dzg;
   // weight of u(j) in the x bulk flux, wq(j) + wq(j+1) (zero outside the pairs)
   const double *cqu;
 };
@@ -188,6 +190,7 @@ struct Handle {
   double* pbc = nullptr;          // compute_pressure wall conditions bc_1, bc_2 (2 x nxg x nzg)
   double* stat_buf = nullptr;     // compute_statistics partials and profiles
   int64_t stat_cap = 0;
+  double* mon_buf = nullptr;      // output_monitor partials
   double *Gu = nullptr, *Gv = nullptr, *Gw = nullptr;       // RK accumulators
   double *rhs_p = nullptr;                                  // rhs_p / phi
   double *P_interim = nullptr;
@@ -347,11 +350,13 @@ int launch_cluster(Handle* h, typename SlabTables<T>::C* spec, int zero00, int r
 // mass flow and reductions (k_massflow.cu)
 int launch_massflow_correction(Handle* h, double dt, bool euler = false, bool skip_x = false);
 int massflow(Handle* h, int comp, bool u_view, double* q_out);
-int massflow_w_as_v(Handle* h, double* q_out);
+int launch_statistics_flows(Handle* h, double* q_dev);
+int launch_maxdiv(Handle* h, double* part);
+int launch_finite(Handle* h, int* flag);
 // diagnostics (k_stats.cu)
 int compute_statistics(Handle* h, double* profiles, double* scalars);
 int monitor_values(Handle* h, double* out);
-int max_abs_divergence(Handle* h, const double* U, const double* V, const double* W, double* out);
+int max_abs_divergence(Handle* h, double* out);
 int check_finite(Handle* h, bool* ok);
 int compute_dt_cfl(Handle* h, double* dt);
 // immersed boundary (k_ib.cu)

@@ -12,6 +12,9 @@
 // The z range includes plane nzg-1, the periodic duplicate of plane 2, exactly
 // as the reference's last rank does.  Reductions are deterministic: a fixed
 // grid writes per-block partials that one block sums in a fixed order.
+#include <algorithm>
+#include <cmath>
+
 #include "c3d_internal.cuh"
 
 namespace c3d {
@@ -97,7 +100,8 @@ static FluxView flux_view(Handle* h, int comp, const double* F, const double* H,
 //           (RK3, src/time_integration.f90:187-211);
 //   mode 2: the same with dPd{x,y} = shift/dt (Euler, :65-78).
 __global__ void __launch_bounds__(kRedThreads) k_flux(FluxView v, double2* __restrict__ part, DevScalars* sc,
-                                                     double q0, double dt, int mode, int comp) {
+                                                     double q0, double dt, int mode, int comp,
+                                                     double* __restrict__ q_out) {
   const int nrows = v.nj * v.nk;
   const int lane = threadIdx.x & 31;
   const int wpb = kRedThreads / 32;
@@ -141,6 +145,7 @@ __global__ void __launch_bounds__(kRedThreads) k_flux(FluxView v, double2* __res
   if (threadIdx.x == 0) {
     const double q = t.x / t.y;
     sc->qflow = q;
+    if (q_out) *q_out = q;
     if (mode >= 1) {
       const double shift = q0 - t.x / t.y;
       double* dp = comp == 0 ? &sc->dPdx : (comp == 1 ? &sc->dPdy : &sc->dPdz);
@@ -197,7 +202,8 @@ int launch_massflow_correction(Handle* h, double dt, bool euler, bool skip_x) {
     if (on[c] != 1) continue;
     // with an immersed body the flux is H-weighted (src/mass_flow.f90:160-163)
     const FluxView v = flux_view(h, c, F[c], flux_weight(h, c), true);
-    k_flux<<<kRedBlocks, kRedThreads, 0, h->stream>>>(v, (double2*)h->red, h->sc, q0[c], dt, euler ? 2 : 1, c);
+    k_flux<<<kRedBlocks, kRedThreads, 0, h->stream>>>(v, (double2*)h->red, h->sc, q0[c], dt, euler ? 2 : 1, c,
+                                                      nullptr);
     C3D_LAUNCH_CHECK(h);
     k_shift_field<<<148 * 8, 256, 0, h->stream>>>(F[c], n1[c], n2[c], n3[c], c == 1 ? 1 : 0, sh[c]);
     C3D_LAUNCH_CHECK(h);
@@ -205,13 +211,20 @@ int launch_massflow_correction(Handle* h, double dt, bool euler, bool skip_x) {
   return 0;
 }
 
-// bulk flux of component comp (flux/norm) of the handle's field; u_view: the
-// mis-shaped view of the z correction (comp 2 only)
-int massflow(Handle* h, int comp, bool u_view, double* q_out) {
+// bulk flux of component comp (flux/norm) of the handle's field into *q_dev
+// (device); u_view: the mis-shaped view of the z correction (comp 2 only)
+static int launch_flux(Handle* h, int comp, bool u_view, double* q_dev) {
   const double* F = comp == 0 ? h->U : (comp == 1 ? h->V : h->W);
   const FluxView v = flux_view(h, comp, F, flux_weight(h, comp), u_view);
-  k_flux<<<kRedBlocks, kRedThreads, 0, h->stream>>>(v, (double2*)h->red, h->sc, 0.0, 1.0, 0, comp);
+  k_flux<<<kRedBlocks, kRedThreads, 0, h->stream>>>(v, (double2*)h->red, h->sc, 0.0, 1.0, 0, comp, q_dev);
   C3D_LAUNCH_CHECK(h);
+  return 0;
+}
+
+// the same to the host
+int massflow(Handle* h, int comp, bool u_view, double* q_out) {
+  const int rc = launch_flux(h, comp, u_view, nullptr);
+  if (rc) return rc;
   double q = 0;
   C3D_CUDA_TRY(h, cudaMemcpyAsync(&q, &h->sc->qflow, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -219,15 +232,17 @@ int massflow(Handle* h, int comp, bool u_view, double* q_out) {
   return 0;
 }
 
-// compute_mean_mass_flow_V applied to W, as compute_statistics calls it
-// (src/statistics.f90:133): W read through V's declared extents (nxg, ny,
-// nzg) with V's loops and weights (every offset reached lies inside W)
-int massflow_w_as_v(Handle* h, double* q_out) {
-  FluxView v = flux_view(h, 1, h->W, flux_weight(h, 1), false);
-  k_flux<<<kRedBlocks, kRedThreads, 0, h->stream>>>(v, (double2*)h->red, h->sc, 0.0, 1.0, 0, 1);
+// The bulk flows of compute_statistics (src/statistics.f90:130-133) into
+// q_dev[3]; the z flow is compute_mean_mass_flow_V applied to W, as the
+// reference calls it: W read through V's declared extents (nxg, ny, nzg) with
+// V's loops and weights (every offset reached lies inside W)
+int launch_statistics_flows(Handle* h, double* q_dev) {
+  int rc;
+  if ((rc = launch_flux(h, 0, false, q_dev))) return rc;
+  if ((rc = launch_flux(h, 1, false, q_dev + 1))) return rc;
+  const FluxView v = flux_view(h, 1, h->W, flux_weight(h, 1), false);
+  k_flux<<<kRedBlocks, kRedThreads, 0, h->stream>>>(v, (double2*)h->red, h->sc, 0.0, 1.0, 0, 1, q_dev + 2);
   C3D_LAUNCH_CHECK(h);
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(q_out, &h->sc->qflow, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return 0;
 }
 
@@ -236,18 +251,22 @@ __global__ void __launch_bounds__(kRedThreads) k_maxdiv(Dims d, Metric m, const 
                                                        const double* __restrict__ V,
                                                        const double* __restrict__ W,
                                                        double* __restrict__ part) {
-  const int ni = d.nxg - 2, nj = d.nyg - 2, nk = d.nzg - 2;
-  const int64_t tot = (int64_t)ni * nj * nk;
+  // one warp per x row, so that a row's index arithmetic is done once
+  const int nrows = (d.nyg - 2) * (d.nzg - 2), lane = threadIdx.x & 31;
   double mx = 0.0;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = 2 + (int)(t % ni);
-    const int j = 2 + (int)((t / ni) % nj);
-    const int k = 2 + (int)(t / ((int64_t)ni * nj));
-    const double v = (U[idxU(d, i, j, k)] - U[idxU(d, i - 1, j, k)]) * m.rdx[i]
-                   + (V[idxV(d, i, j, k)] - V[idxV(d, i, j - 1, k)]) * m.rdy[j]
-                   + (W[idxW(d, i, j, k)] - W[idxW(d, i, j, k - 1)]) * m.rdz[k];
-    mx = fmax(mx, fabs(v));
+  for (int row = blockIdx.x * (kRedThreads / 32) + (threadIdx.x >> 5); row < nrows;
+       row += gridDim.x * (kRedThreads / 32)) {
+    const int kk = row / (d.nyg - 2), k = 2 + kk, j = 2 + row - kk * (d.nyg - 2);
+    const double ry = m.rdy[j], rz = m.rdz[k];
+    const double* u = U + idxU(d, 2, j, k);
+    const double* v = V + idxV(d, 2, j, k);
+    const double* w = W + idxW(d, 2, j, k);
+    const double* wm = W + idxW(d, 2, j, k - 1);
+#pragma unroll 2
+    for (int i = lane; i < d.nxg - 2; i += 32) {
+      const double x = (u[i] - u[i - 1]) * m.rdx[2 + i] + (v[i] - v[i - d.nxg]) * ry + (w[i] - wm[i]) * rz;
+      mx = fmax(mx, fabs(x));
+    }
   }
   __shared__ double sm[kRedThreads];
   sm[threadIdx.x] = mx;
@@ -259,9 +278,16 @@ __global__ void __launch_bounds__(kRedThreads) k_maxdiv(Dims d, Metric m, const 
   if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
 }
 
-int max_abs_divergence(Handle* h, const double* U, const double* V, const double* W, double* out) {
-  k_maxdiv<<<kRedBlocks, kRedThreads, 0, h->stream>>>(h->d, h->m, U, V, W, h->red);
+// kRedBlocks partial maxima into part (device)
+int launch_maxdiv(Handle* h, double* part) {
+  k_maxdiv<<<kRedBlocks, kRedThreads, 0, h->stream>>>(h->d, h->m, h->U, h->V, h->W, part);
   C3D_LAUNCH_CHECK(h);
+  return 0;
+}
+
+int max_abs_divergence(Handle* h, double* out) {
+  const int rc = launch_maxdiv(h, h->red);
+  if (rc) return rc;
   std::vector<double> part(kRedBlocks);
   C3D_CUDA_TRY(h, cudaMemcpyAsync(part.data(), h->red, sizeof(double) * kRedBlocks,
                                   cudaMemcpyDeviceToHost, h->stream));
@@ -273,22 +299,29 @@ int max_abs_divergence(Handle* h, const double* U, const double* V, const double
 }
 
 // ---- finiteness scan of U, V, W ----
-__global__ void k_finite(const double* __restrict__ a, int64_t n, int* flag) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    if (!isfinite(a[t])) { *flag = 1; return; }
-  }
+__global__ void k_finite(const double* __restrict__ a, int64_t na, const double* __restrict__ b, int64_t nb,
+                         const double* __restrict__ c, int64_t nc, int* flag) {
+  const double* f = blockIdx.y == 0 ? a : (blockIdx.y == 1 ? b : c);
+  const int64_t n = blockIdx.y == 0 ? na : (blockIdx.y == 1 ? nb : nc);
+  bool bad = false;
+#pragma unroll 4
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
+    bad = bad || !isfinite(f[t]);
+  if (bad) *flag = 1;
+}
+
+// *flag (device) = 1 if U, V or W holds a NaN or infinity, else 0
+int launch_finite(Handle* h, int* flag) {
+  C3D_CUDA_TRY(h, cudaMemsetAsync(flag, 0, sizeof(int), h->stream));
+  k_finite<<<dim3(148 * 4, 3), 256, 0, h->stream>>>(h->U, sizeU(h->d), h->V, sizeV(h->d), h->W, sizeW(h->d), flag);
+  C3D_LAUNCH_CHECK(h);
+  return 0;
 }
 
 int check_finite(Handle* h, bool* ok) {
   int* flag = (int*)(h->red + 2 * kRedBlocks + 8);
-  C3D_CUDA_TRY(h, cudaMemsetAsync(flag, 0, sizeof(int), h->stream));
-  k_finite<<<148 * 4, 256, 0, h->stream>>>(h->U, sizeU(h->d), flag);
-  C3D_LAUNCH_CHECK(h);
-  k_finite<<<148 * 4, 256, 0, h->stream>>>(h->V, sizeV(h->d), flag);
-  C3D_LAUNCH_CHECK(h);
-  k_finite<<<148 * 4, 256, 0, h->stream>>>(h->W, sizeW(h->d), flag);
-  C3D_LAUNCH_CHECK(h);
+  const int rc = launch_finite(h, flag);
+  if (rc) return rc;
   int f = 0;
   C3D_CUDA_TRY(h, cudaMemcpyAsync(&f, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -297,62 +330,59 @@ int check_finite(Handle* h, bool* ok) {
 }
 
 // ---- compute_dt with CFL > 0 (src/time_integration.f90:227-262) ----
-__global__ void __launch_bounds__(kRedThreads) k_cfl(Dims d, const double* __restrict__ xg,
-                                                    const double* __restrict__ yg,
-                                                    const double* __restrict__ zg,
-                                                    const double* __restrict__ U,
-                                                    const double* __restrict__ V,
-                                                    const double* __restrict__ W,
-                                                    double* __restrict__ part) {
-  const int ni = d.nxg - 2, nj = d.nyg - 2, nk = d.nzg - 2;
-  const int64_t tot = (int64_t)ni * nj * nk;
-  double mu = 0.0, mv = 0.0, mw = 0.0;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = 2 + (int)(t % ni);
-    const int j = 2 + (int)((t / ni) % nj);
-    const int k = 2 + (int)(t / ((int64_t)ni * nj));
-    mu = fmax(mu, (xg[i + 1] - xg[i]) / fabs(U[idxU(d, i, j, k)]));
-    mv = fmax(mv, (yg[j + 1] - yg[j]) / fabs(V[idxV(d, i, j, k)]));
-    mw = fmax(mw, (zg[k + 1] - zg[k]) / fabs(W[idxW(d, i, j, k)]));
+// max over the interior of spacing/|velocity|, per component.  The spacing
+// belongs to one index (i for U, j for V, k for W), so a thread keeps the
+// smallest |velocity| over a run of points with the same spacing and divides
+// once: the quotient of the smallest is the largest quotient, rounding
+// included, and NaNs drop out either way.
+// U, V: thread (i, j), a run of z planes; W: thread (i, k), a run of rows.
+constexpr int kCflRun = 24;
+__global__ void __launch_bounds__(256) k_cfl(Dims d, Metric m, const double* __restrict__ U,
+                                             const double* __restrict__ V, const double* __restrict__ W,
+                                             unsigned long long* __restrict__ out) {
+  const int comp = blockIdx.z % 3, chunk = blockIdx.z / 3;
+  const int i = 2 + blockIdx.x * 32 + threadIdx.x;
+  const int r = 2 + blockIdx.y * 8 + threadIdx.y;              // j (U, V) or k (W)
+  const int rend = comp == 2 ? d.nzg - 1 : d.nyg - 1, cend = comp == 2 ? d.nyg - 1 : d.nzg - 1;
+  const int c0 = 2 + chunk * kCflRun, c1 = min(c0 + kCflRun - 1, cend);
+  double q = 0.0;
+  if (i <= d.nxg - 1 && r <= rend && c0 <= c1) {
+    const double* f;
+    int64_t step;
+    double h;
+    if (comp == 0) { f = U + idxU(d, i, r, c0); step = (int64_t)d.nx * d.nyg; h = m.dxg[i]; }
+    else if (comp == 1) { f = V + idxV(d, i, r, c0); step = (int64_t)d.nxg * d.ny; h = m.dyg[r]; }
+    else { f = W + idxW(d, i, c0, r); step = d.nxg; h = m.dzg[r]; }
+    double least = INFINITY;
+#pragma unroll 8
+    for (int c = 0; c <= c1 - c0; ++c) least = fmin(least, fabs(f[c * step]));
+    q = fmax(q, h / least);
   }
-  __shared__ double s[3][kRedThreads];
-  s[0][threadIdx.x] = mu; s[1][threadIdx.x] = mv; s[2][threadIdx.x] = mw;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) q = fmax(q, __shfl_xor_sync(0xffffffffu, q, o));
+  __shared__ double s[8];
+  if (threadIdx.x == 0) s[threadIdx.y] = q;
   __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
-      for (int c = 0; c < 3; ++c) s[c][threadIdx.x] = fmax(s[c][threadIdx.x], s[c][threadIdx.x + st]);
-    __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    for (int w = 1; w < 8; ++w) q = fmax(q, s[w]);
+    // nonnegative doubles order as their bits
+    atomicMax(out + comp, (unsigned long long)__double_as_longlong(q));
   }
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; ++c) part[3 * blockIdx.x + c] = s[c][0];
 }
 
 int compute_dt_cfl(Handle* h, double* dt) {
   const Params& p = h->p;
   if (p.CFL < 0) { *dt = -p.CFL; return 0; }
-  double* xg = nullptr;
-  // grids on device: reuse the tail of the reduction buffer for xg, yg, zg
   const Dims& d = h->d;
-  double* g = h->red + 4 * kRedBlocks;
-  xg = g;
-  double* yg = xg + d.nxg + 2;
-  double* zg = yg + d.nyg + 2;
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(xg, h->xg.data(), sizeof(double) * (d.nxg + 1), cudaMemcpyHostToDevice, h->stream));
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(yg, h->yg.data(), sizeof(double) * (d.nyg + 1), cudaMemcpyHostToDevice, h->stream));
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(zg, h->zg.data(), sizeof(double) * (d.nzg + 1), cudaMemcpyHostToDevice, h->stream));
-  k_cfl<<<kRedBlocks, kRedThreads, 0, h->stream>>>(d, xg, yg, zg, h->U, h->V, h->W, h->red);
+  C3D_CUDA_TRY(h, cudaMemsetAsync(h->red, 0, 3 * sizeof(double), h->stream));
+  const int rows = std::max(d.nyg, d.nzg) - 2, runs = (rows + kCflRun - 1) / kCflRun;
+  k_cfl<<<dim3((d.nxg - 2 + 31) / 32, (rows + 7) / 8, 3 * runs), dim3(32, 8), 0, h->stream>>>(
+      d, h->m, h->U, h->V, h->W, (unsigned long long*)h->red);
   C3D_LAUNCH_CHECK(h);
-  std::vector<double> part(3 * kRedBlocks);
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(part.data(), h->red, sizeof(double) * 3 * kRedBlocks,
-                                  cudaMemcpyDeviceToHost, h->stream));
+  double part[3];
+  C3D_CUDA_TRY(h, cudaMemcpyAsync(part, h->red, sizeof(part), cudaMemcpyDeviceToHost, h->stream));
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  double lu = 0, lv = 0, lw = 0;
-  for (int b = 0; b < kRedBlocks; ++b) {
-    lu = part[3 * b] > lu ? part[3 * b] : lu;
-    lv = part[3 * b + 1] > lv ? part[3 * b + 1] : lv;
-    lw = part[3 * b + 2] > lw ? part[3 * b + 2] : lw;
-  }
+  const double lu = part[0], lv = part[1], lw = part[2];
   double dtc = p.CFL * lu;
   dtc = p.CFL * lv < dtc ? p.CFL * lv : dtc;
   dtc = p.CFL * lw < dtc ? p.CFL * lw : dtc;

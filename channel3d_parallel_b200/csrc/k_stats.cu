@@ -8,7 +8,9 @@
 // term_1*term_2, divided by (nxg-3)(nzg-3) (W: (nxg-3)(nz-2)); the wall
 // derivatives of the mean profiles give utau, wtau and Retau.  Row sums are
 // per (row, z chunk) block partials added in chunk order (deterministic).
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "c3d_internal.cuh"
@@ -31,17 +33,21 @@ __global__ void __launch_bounds__(kStatThreads) k_stat_rows(Dims d, const double
   const int ni = d.nxg - 3, nk = d.nzg - 3;
   const int k0 = 2 + (int)((int64_t)c * nk / gridDim.y), k1 = 2 + (int)((int64_t)(c + 1) * nk / gridDim.y);
   double s[kStatQ] = {0, 0, 0, 0, 0, 0, 0};
-  for (int t = threadIdx.x; t < ni * (k1 - k0); t += blockDim.x) {
-    const int i = 2 + t % ni, k = k0 + t / ni;
-    const double t1 = 0.5 * (U[idxU(d, i - 1, j, k)] + U[idxU(d, i, j, k)]);
-    double t2;
-    if (j == 1) t2 = -(0.5 * (V[idxV(d, i, 1, k)] + V[idxV(d, i, 2, k)]));
-    else if (j == d.nyg) t2 = -(0.5 * (V[idxV(d, i, d.nyg - 2, k)] + V[idxV(d, i, d.nyg - 1, k)]));
-    else t2 = 0.5 * (V[idxV(d, i, j - 1, k)] + V[idxV(d, i, j, k)]);
-    const double w = W[idxW(d, i, j, k)];
-    s[0] += t1; s[1] += t2; s[2] += w;
-    s[3] += t1 * t1; s[4] += t2 * t2; s[5] += w * w;
-    s[6] += t1 * t2;
+  // one warp per x row of the chunk; rows of V either side of the row (the
+  // walls' own for the ghost rows, with the opposite sign)
+  const int ja = j == 1 ? 1 : (j == d.nyg ? d.nyg - 2 : j - 1);
+  const double sg = j == 1 || j == d.nyg ? -0.5 : 0.5;
+  for (int k = k0 + (int)(threadIdx.x >> 5); k < k1; k += kStatThreads / 32) {
+    const double* u = U + idxU(d, 2, j, k);
+    const double* va = V + idxV(d, 2, ja, k);
+    const double* wr = W + idxW(d, 2, j, k);
+#pragma unroll 2
+    for (int i = threadIdx.x & 31; i < ni; i += 32) {
+      const double t1 = 0.5 * (u[i - 1] + u[i]), t2 = sg * (va[i] + va[i + d.nxg]), w = wr[i];
+      s[0] += t1; s[1] += t2; s[2] += w;
+      s[3] += t1 * t1; s[4] += t2 * t2; s[5] += w * w;
+      s[6] += t1 * t2;
+    }
   }
   __shared__ double red[kStatQ][kStatThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -70,35 +76,41 @@ __global__ void k_stat_final(int nyg, int nch, double cnt_uv, double cnt_w, cons
   out[t] = v / ((q == 2 || q == 5) ? cnt_w : cnt_uv);
 }
 
-// (sum, max) of F(i,j,k) over the box, F of extents (n1, n2, .)
-__global__ void __launch_bounds__(256) k_box_sum_max(const double* __restrict__ F, int n1, int n2, int i0, int ni,
-                                                    int j0, int nj, int k0, int nk, double2* __restrict__ part) {
-  const int64_t tot = (int64_t)ni * nj * nk;
+// Sums and maxima of U, V, W over the interior boxes of output_monitor
+// (blockIdx.y: component), one warp per x row; per block (sum, max)
+__global__ void __launch_bounds__(256) k_box_sum_max(Dims d, const double* __restrict__ U,
+                                                    const double* __restrict__ V, const double* __restrict__ W,
+                                                    double2* __restrict__ part) {
+  const int c = blockIdx.y, lane = threadIdx.x & 31;
+  const double* F = c == 0 ? U : (c == 1 ? V : W);
+  const int n1 = c == 0 ? d.nx : d.nxg, n2 = c == 1 ? d.ny : d.nyg, n3 = c == 2 ? d.nz : d.nzg;
+  const int nrows = (n2 - 2) * (n3 - 2);
   double s = 0.0, mx = -INFINITY;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = i0 + (int)(t % ni);
-    const int j = j0 + (int)((t / ni) % nj);
-    const int k = k0 + (int)(t / ((int64_t)ni * nj));
-    const double v = F[(int64_t)(i - 1) + (int64_t)n1 * ((j - 1) + (int64_t)n2 * (k - 1))];
-    s += v;
-    mx = fmax(mx, v);
+  for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < nrows; row += gridDim.x * 8) {
+    const int k = row / (n2 - 2), j = row - k * (n2 - 2);
+    const double* f = F + 1 + (int64_t)n1 * (j + 1 + (int64_t)n2 * (k + 1));
+#pragma unroll 4
+    for (int i = lane; i < n1 - 2; i += 32) {
+      const double v = f[i];
+      s += v;
+      mx = fmax(mx, v);
+    }
   }
   __shared__ double ss[8], sm[8];
   for (int o = 16; o > 0; o >>= 1) {
     s += __shfl_down_sync(0xffffffffu, s, o);
     mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int wid = threadIdx.x >> 5;
   if (lane == 0) { ss[wid] = s; sm[wid] = mx; }
   __syncthreads();
   if (threadIdx.x == 0) {
     double a = 0.0, b = -INFINITY;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { a += ss[w]; b = fmax(b, sm[w]); }
-    part[blockIdx.x] = make_double2(a, b);
+    part[blockIdx.y * gridDim.x + blockIdx.x] = make_double2(a, b);
   }
 }
 
-int massflow_w_as_v(Handle* h, double* q_out);
 
 // compute_statistics: profiles[7*nyg] (Umean, Vmean, Wmean, U2mean, V2mean,
 // W2mean, UVmean at yg(1:nyg)); scalars[8] = utau, wtau, Retau_u, Retau_w,
@@ -107,23 +119,29 @@ int massflow_w_as_v(Handle* h, double* q_out);
 int compute_statistics(Handle* h, double* profiles, double* scalars) {
   const Dims& d = h->d;
   const int nyg = d.nyg;
-  double* part = nullptr;
+  // device results: the profiles, then the three flows and the finiteness
+  // flag; one copy and one synchronisation bring them all
   int rc;
-  const int64_t need = (int64_t)nyg * kStatChunks * kStatQ + (int64_t)nyg * kStatQ;
+  const int64_t nout = (int64_t)nyg * kStatQ + 4;
+  const int64_t need = (int64_t)nyg * kStatChunks * kStatQ + nout;
   if (h->stat_cap < need) {
     if ((rc = dev_alloc(h, &h->stat_buf, need))) return rc;
     h->stat_cap = need;
   }
-  part = h->stat_buf;
+  double* part = h->stat_buf;
   double* out = h->stat_buf + (int64_t)nyg * kStatChunks * kStatQ;
   k_stat_rows<<<dim3((unsigned)nyg, kStatChunks), kStatThreads, 0, h->stream>>>(d, h->U, h->V, h->W, part);
   C3D_LAUNCH_CHECK(h);
   const double cnt = (double)(d.nxg - 3) * (double)(d.nzg - 3), cntw = (double)(d.nxg - 3) * (double)(d.nz - 2);
   k_stat_final<<<(nyg * kStatQ + 127) / 128, 128, 0, h->stream>>>(nyg, kStatChunks, cnt, cntw, part, out);
   C3D_LAUNCH_CHECK(h);
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(profiles, out, sizeof(double) * nyg * kStatQ, cudaMemcpyDeviceToHost,
-                                  h->stream));
+  double* flows = out + (int64_t)nyg * kStatQ;
+  if ((rc = launch_statistics_flows(h, flows))) return rc;
+  if ((rc = launch_finite(h, (int*)(flows + 3)))) return rc;
+  std::vector<double> res(nout);
+  C3D_CUDA_TRY(h, cudaMemcpyAsync(res.data(), out, sizeof(double) * nout, cudaMemcpyDeviceToHost, h->stream));
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  std::memcpy(profiles, res.data(), sizeof(double) * nyg * kStatQ);
   const double* Um = profiles;
   const double* Wm = profiles + 2 * nyg;
   const std::vector<double>& yg = h->yg;
@@ -140,30 +158,10 @@ int compute_statistics(Handle* h, double* profiles, double* scalars) {
   scalars[1] = wtau;
   scalars[2] = utau * (y[d.ny] - y[1]) / 2.0 / nu;
   scalars[3] = wtau * (y[d.ny] - y[1]) / 2.0 / nu;
-  // src/statistics.f90:130-133; the z flow is compute_mean_mass_flow_V
-  // applied to W, as the reference calls it
-  if ((rc = massflow(h, 0, false, &scalars[4]))) return rc;
-  if ((rc = massflow(h, 1, false, &scalars[5]))) return rc;
-  if ((rc = massflow_w_as_v(h, &scalars[6]))) return rc;
-  bool ok = true;
-  if ((rc = check_finite(h, &ok))) return rc;
-  scalars[7] = ok ? 0.0 : 1.0;
-  return 0;
-}
-
-static int box_sum_max(Handle* h, const double* F, int n1, int n2, int i0, int i1, int j0, int j1, int k0, int k1,
-                       double* sum, double* mx) {
-  double2* part = (double2*)h->red;
-  k_box_sum_max<<<kBoxBlocks, 256, 0, h->stream>>>(F, n1, n2, i0, i1 - i0 + 1, j0, j1 - j0 + 1, k0, k1 - k0 + 1,
-                                                  part);
-  C3D_LAUNCH_CHECK(h);
-  std::vector<double2> p(kBoxBlocks);
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(p.data(), part, sizeof(double2) * kBoxBlocks, cudaMemcpyDeviceToHost, h->stream));
-  C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  double s = 0.0, m = -INFINITY;
-  for (const double2& v : p) { s += v.x; m = v.y > m ? v.y : m; }
-  *sum = s;
-  *mx = m;
+  int bad = 0;
+  std::memcpy(&bad, &res[(size_t)nyg * kStatQ + 3], sizeof(bad));
+  for (int c = 0; c < 3; ++c) scalars[4 + c] = res[(size_t)nyg * kStatQ + c];
+  scalars[7] = bad ? 1.0 : 0.0;
   return 0;
 }
 
@@ -174,14 +172,28 @@ int monitor_values(Handle* h, double* out) {
   const Dims& d = h->d;
   int rc;
   const double vol = (double)(d.nx - 1) * (double)(d.ny - 1) * (double)(d.nz - 1);
-  double s, m;
-  if ((rc = box_sum_max(h, h->U, d.nx, d.nyg, 2, d.nx - 1, 2, d.nyg - 1, 2, d.nzg - 1, &s, &m))) return rc;
-  out[0] = s / vol; out[3] = m;
-  if ((rc = box_sum_max(h, h->V, d.nxg, d.ny, 2, d.nxg - 1, 2, d.ny - 1, 2, d.nzg - 1, &s, &m))) return rc;
-  out[1] = s / vol; out[4] = m;
-  if ((rc = box_sum_max(h, h->W, d.nxg, d.nyg, 2, d.nxg - 1, 2, d.nyg - 1, 2, d.nz - 1, &s, &m))) return rc;
-  out[2] = s / vol; out[5] = m;
-  return max_abs_divergence(h, h->U, h->V, h->W, &out[6]);
+  // partials of the three components, then those of the divergence, in one copy
+  constexpr int64_t nbox = 3 * 2 * (int64_t)kBoxBlocks, nres = nbox + kBoxBlocks;
+  if (h->mon_buf == nullptr && (rc = dev_alloc(h, &h->mon_buf, nres))) return rc;
+  k_box_sum_max<<<dim3(kBoxBlocks, 3), 256, 0, h->stream>>>(d, h->U, h->V, h->W, (double2*)h->mon_buf);
+  C3D_LAUNCH_CHECK(h);
+  if ((rc = launch_maxdiv(h, h->mon_buf + nbox))) return rc;
+  std::vector<double> p(nres);
+  C3D_CUDA_TRY(h, cudaMemcpyAsync(p.data(), h->mon_buf, sizeof(double) * nres, cudaMemcpyDeviceToHost, h->stream));
+  C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  for (int c = 0; c < 3; ++c) {
+    double s = 0.0, m = -INFINITY;
+    for (int b = 0; b < kBoxBlocks; ++b) {
+      s += p[2 * ((size_t)c * kBoxBlocks + b)];
+      m = std::max(m, p[2 * ((size_t)c * kBoxBlocks + b) + 1]);
+    }
+    out[c] = s / vol;
+    out[3 + c] = m;
+  }
+  double mx = 0.0;
+  for (int b = 0; b < kBoxBlocks; ++b) mx = p[nbox + b] > mx ? p[nbox + b] : mx;
+  out[6] = mx;
+  return 0;
 }
 
 }  // namespace c3d
