@@ -120,9 +120,11 @@ struct SpectralState {
   SlabTables<float> slab32;
   int* posx = nullptr;                       // digit-reversed position of x coefficient m
   // Thomas factors of every (kx, kz') mode, layout [(m*Ny + j)*nkzs + kz']:
-  // multipliers DL(j)/D'(j) and reciprocal pivots 1/D'(j)
-  double *mult = nullptr, *rdp = nullptr;
-  float *mult32 = nullptr, *rdp32 = nullptr;
+  // reciprocal pivots 1/D'(j)
+  double* rdp = nullptr;
+  float* rdp32 = nullptr;
+  double* mult00 = nullptr;                  // multipliers DL(j)/D'(j) of mode (0, 0)
+  double* tri = nullptr;                     // diagonal, kxx and kzz behind the tables
   double *dl = nullptr, *du = nullptr;       // Dyy(j+1, j) and Dyy(j, j+1), j = 0..Ny-1 (0 past the end)
   // x(j)/y(j) of the homogeneous tail (right-hand side zero from row j on),
   // same layout as rdp; built on first use by the band-restricted solve

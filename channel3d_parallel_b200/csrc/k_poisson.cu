@@ -67,16 +67,52 @@ static int make_twiddles(Handle* h, int n, C** out) {
 }
 
 // Thomas factorisation of every mode, the no-pivot path of the reference's
-// LAPACK zgtsv call (src/poisson.f90:72): MULT = DL(k)/D(k), D(k+1) -= MULT*DU(k).
-// Stored: mult_j and 1/d'_j, layout [(m*Ny + j)*nkzs + kz'].
+// LAPACK zgtsv call (src/poisson.f90:72): MULT = DL(k)/D(k), D(k+1) -= MULT*DU(k),
+// one thread per mode.  Stored: 1/d'_j, layout [(m*Ny + j)*nkzs + kz'], FP64
+// and (if given) FP32, and the multipliers of mode (0, 0).  Rounded operation
+// by operation as written.
+__global__ void k_tri_table(Dims d, const double* __restrict__ dd, const double* __restrict__ dl,
+                            const double* __restrict__ du, const double* __restrict__ kxx,
+                            const double* __restrict__ kzz, double* __restrict__ rdp, float* __restrict__ rdp32,
+                            double* __restrict__ mult00) {
+  const int kz = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
+  if (kz >= d.nkzs) return;
+  const double kx2 = kxx[m], kz2 = kzz[kz];
+  double up = 0.0;                          // MULT(j-1)*DU(j-1)
+  for (int j = 0; j < d.Ny; ++j) {
+    double D = (dd[j] + kx2) + kz2;
+    if (m == 0 && kz == 0 && j == 0) D = 3.0 / 2.0 * D;       // src/poisson.f90:69
+    if (j > 0) D = __dsub_rn(D, up);
+    const int64_t o = ((int64_t)m * d.Ny + j) * d.nkzs + kz;
+    const double r = __ddiv_rn(1.0, D);
+    rdp[o] = r;
+    if (rdp32) rdp32[o] = (float)r;
+    if (j + 1 < d.Ny) {
+      const double mu = __ddiv_rn(dl[j], D);
+      up = __dmul_rn(mu, du[j]);
+      if (m == 0 && kz == 0) mult00[j] = mu;
+    }
+  }
+}
+
+// the tables of the current grid (FP32 copies once the mixed path is set up)
 static int build_tri_table(Handle* h) {
   const Dims& d = h->d;
   SpectralState& S = h->sp;
   const int Ny = d.Ny, nkx = d.nkx, nkzs = d.nkzs;
   const int64_t nt = (int64_t)Ny * nkzs * nkx;
-  std::vector<double> rdp(nt), mult(nt);
-  std::vector<float> rdp32(nt), mult32(nt);
-  std::vector<double> D(Ny), dl(Ny, 0.0), du(Ny, 0.0);
+  int rc;
+  if (S.rdp == nullptr) {
+    if ((rc = dev_alloc(h, &S.rdp, nt))) return rc;
+    if ((rc = dev_alloc(h, &S.mult00, Ny))) return rc;
+    if ((rc = dev_alloc(h, &S.dl, Ny))) return rc;
+    if ((rc = dev_alloc(h, &S.du, Ny))) return rc;
+    if ((rc = dev_alloc(h, &S.dl32, Ny))) return rc;
+    if ((rc = dev_alloc(h, &S.du32, Ny))) return rc;
+    if ((rc = dev_alloc(h, &S.tri, Ny + nkx + nkzs))) return rc;
+  }
+  if (S.spec32 != nullptr && S.rdp32 == nullptr && (rc = dev_alloc(h, &S.rdp32, nt))) return rc;
+  std::vector<double> dl(Ny, 0.0), du(Ny, 0.0), tri(Ny + nkx + nkzs);
   std::vector<float> dl32(Ny, 0.0f), du32(Ny, 0.0f);
   for (int jj = 0; jj + 1 < Ny; ++jj) {
     dl[jj] = h->Dl[jj + 3];   // Dyy(j+1, j), j = jj+2
@@ -84,45 +120,20 @@ static int build_tri_table(Handle* h) {
     dl32[jj] = (float)dl[jj];
     du32[jj] = (float)du[jj];
   }
-  for (int m = 0; m < nkx; ++m) {
-    for (int kzs = 0; kzs < nkzs; ++kzs) {
-      for (int jj = 0; jj < Ny; ++jj) D[jj] = (h->Dd[jj + 2] + h->kxx[m]) + h->kzz[kzs];
-      if (m == 0 && kzs == 0) D[0] = 3.0 / 2.0 * D[0];       // src/poisson.f90:69
-      for (int jj = 0; jj < Ny; ++jj) {
-        const int64_t o = ((int64_t)m * Ny + jj) * nkzs + kzs;
-        double mu = 0.0;
-        if (jj + 1 < Ny) {
-          mu = dl[jj] / D[jj];
-          D[jj + 1] = D[jj + 1] - mu * du[jj];
-        }
-        rdp[o] = 1.0 / D[jj];
-        mult[o] = mu;
-        rdp32[o] = (float)rdp[o];
-        mult32[o] = (float)mu;
-      }
-    }
-  }
-  int rc;
-  if (S.rdp == nullptr) {
-    if ((rc = dev_alloc(h, &S.rdp, nt))) return rc;
-    if ((rc = dev_alloc(h, &S.mult, nt))) return rc;
-    if ((rc = dev_alloc(h, &S.rdp32, nt))) return rc;
-    if ((rc = dev_alloc(h, &S.mult32, nt))) return rc;
-    if ((rc = dev_alloc(h, &S.dl, Ny))) return rc;
-    if ((rc = dev_alloc(h, &S.du, Ny))) return rc;
-    if ((rc = dev_alloc(h, &S.dl32, Ny))) return rc;
-    if ((rc = dev_alloc(h, &S.du32, Ny))) return rc;
-  }
+  for (int jj = 0; jj < Ny; ++jj) tri[jj] = h->Dd[jj + 2];
+  for (int m = 0; m < nkx; ++m) tri[Ny + m] = h->kxx[m];
+  for (int k = 0; k < nkzs; ++k) tri[Ny + nkx + k] = h->kzz[k];
   cudaStream_t s = h->stream;
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(S.rdp, rdp.data(), nt * 8, cudaMemcpyHostToDevice, s));
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(S.mult, mult.data(), nt * 8, cudaMemcpyHostToDevice, s));
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(S.rdp32, rdp32.data(), nt * 4, cudaMemcpyHostToDevice, s));
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(S.mult32, mult32.data(), nt * 4, cudaMemcpyHostToDevice, s));
   C3D_CUDA_TRY(h, cudaMemcpyAsync(S.dl, dl.data(), Ny * 8, cudaMemcpyHostToDevice, s));
   C3D_CUDA_TRY(h, cudaMemcpyAsync(S.du, du.data(), Ny * 8, cudaMemcpyHostToDevice, s));
   C3D_CUDA_TRY(h, cudaMemcpyAsync(S.dl32, dl32.data(), Ny * 4, cudaMemcpyHostToDevice, s));
   C3D_CUDA_TRY(h, cudaMemcpyAsync(S.du32, du32.data(), Ny * 4, cudaMemcpyHostToDevice, s));
-  return cudaStreamSynchronize(s) == cudaSuccess ? 0 : C3D_ERR_CUDA;
+  C3D_CUDA_TRY(h, cudaMemcpyAsync(S.tri, tri.data(), tri.size() * 8, cudaMemcpyHostToDevice, s));
+  k_tri_table<<<dim3((nkzs + 63) / 64, nkx), 64, 0, s>>>(d, S.tri, S.dl, S.du, S.tri + Ny, S.tri + Ny + nkx, S.rdp,
+                                                         S.rdp32, S.mult00);
+  C3D_LAUNCH_CHECK(h);
+  C3D_CUDA_TRY(h, cudaStreamSynchronize(s));   // the host copies end here
+  return 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -288,7 +299,7 @@ static int launch_band_yz(Handle* h, int blo, int bhi, bool* done) {
 // FP64 kx = kz = 0 mode of the mixed path: plane sums and the pinned solve
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_mode00(Dims d, const double* __restrict__ linesum,
-                                                 const double* __restrict__ mult, const double* __restrict__ rdp,
+                                                 const double* __restrict__ mult00, const double* __restrict__ rdp,
                                                  const double* __restrict__ du, double* __restrict__ phi00) {
   extern __shared__ double m00[];
   const int Ny = d.Ny, Nz = d.Nz, nkzs = d.nkzs;
@@ -306,7 +317,7 @@ __global__ void __launch_bounds__(1024) k_mode00(Dims d, const double* __restric
     if (lane == 0) b00[j] = s;
   }
   for (int j = threadIdx.x; j < Ny; j += blockDim.x) {
-    sm_[j] = j > 0 ? mult[(int64_t)(j - 1) * nkzs] : 0.0;
+    sm_[j] = j > 0 ? mult00[j - 1] : 0.0;
     sr[j] = rdp[(int64_t)j * nkzs];
     su[j] = du[j];
   }
@@ -332,9 +343,9 @@ __global__ void __launch_bounds__(1024) k_mode00(Dims d, const double* __restric
 // Which form of the z transforms and y solves: the cluster that keeps a slab on
 // chip moves the spectrum once in place of twice, but needs 16 CTAs of an SM
 // each for the large slabs, and past 256 columns a thread has several.
-// Measured, cluster against blocks (us, B200): 192x128x192 49 / 67,
-// 256x128x256 97 / 114, 64x256x64 19 / 33; 16 CTAs: 192x256x192 156 / 134,
-// 256x192x256 276 / 165, 384x256x384 1237 / 533; 8 CTAs with Nz = 384:
+// Measured, cluster against blocks (us, B200): 192x128x192 45 / 67,
+// 256x128x256 93 / 114, 64x256x64 19 / 33; 16 CTAs: 192x256x192 156 / 134,
+// 256x192x256 276 / 165, 384x256x384 1237 / 467; 8 CTAs with Nz = 384:
 // 128x64x384 89 / 65, 384x64x384 222 / 145.
 static bool slab_by_blocks(const Dims& d, const SlabCluster& c) { return c.cs > 8 || d.Nz > 256; }
 
@@ -356,7 +367,7 @@ static int run_spectral_t(Handle* h, bool from_div, const double* U, const doubl
                                  from_div && whole ? flux_dt : 0.0)))
       return rc;
     if (f32) {
-      k_mode00<<<1, 1024, 4 * sizeof(double) * d.Ny, h->stream>>>(d, S.linesum, S.mult, S.rdp, S.du, S.phi00);
+      k_mode00<<<1, 1024, 4 * sizeof(double) * d.Ny, h->stream>>>(d, S.linesum, S.mult00, S.rdp, S.du, S.phi00);
       C3D_LAUNCH_CHECK(h);
     }
   }
@@ -717,6 +728,7 @@ int mixed_setup(Handle* h) {
   if ((rc = dev_alloc(h, &S.linesum, (int64_t)d.Ny * d.Nz))) return rc;
   if ((rc = dev_alloc(h, &S.phi00, d.Ny))) return rc;
   if ((rc = xfft_setup<float>(h))) return rc;
+  if ((rc = build_tri_table(h))) return rc;       // with the FP32 pivots
   if ((rc = slab_setup(h, true))) return rc;
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return 0;
