@@ -686,6 +686,15 @@ __global__ void k_lb_scatter(LbArgs a, const float* __restrict__ out, const doub
   }
 }
 
+// n groups of four FP32 values rounded to BF16 (nearest even, as on the host)
+__global__ void k_to_bf16(int64_t n, const float4* __restrict__ x, uint2* __restrict__ y) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    const float4 v = x[t];
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    y[t] = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+  }
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -1062,16 +1071,22 @@ extern "C" int c3d_precond_eval(int id, const float* feats, const float* mom, in
   if ((rc = mlp_ensure(h))) return rc;
   if ((rc = ensure_rows(h, m))) return rc;
   MlpState* S = h->mlp;
-  std::vector<__nv_bfloat16> fb((size_t)m * kF);
-  for (size_t i = 0; i < fb.size(); ++i) fb[i] = __float2bfloat16_rn(feats[i]);
+  const int64_t nf = (int64_t)m * kF;
   if (S->eval_cap < m) {
-    if ((rc = dev_alloc(h, &S->eval_f, (int64_t)m * kF))) return rc;
+    if ((rc = dev_alloc(h, &S->eval_f, nf))) return rc;
     if ((rc = dev_alloc(h, &S->eval_m, (int64_t)m * kMom))) return rc;
     S->eval_cap = m;
   }
   for (int i = 0; i < 4; ++i) { S->sig_r[i] = sig[i]; S->sig_e[i] = sig[4 + i]; }
   if ((rc = upload_sig(h))) return rc;
-  C3D_CUDA_TRY(h, cudaMemcpyAsync(S->eval_f, fb.data(), 2 * fb.size(), cudaMemcpyHostToDevice, h->stream));
+  // the features as given pass through H1 (256 bytes a row), which the forward
+  // pass writes next
+  float* const fx = reinterpret_cast<float*>(S->H1);
+  static_assert(kH * sizeof(__nv_bfloat16) >= kF * sizeof(float), "a row of features fits a row of H1");
+  C3D_CUDA_TRY(h, cudaMemcpyAsync(fx, feats, 4 * nf, cudaMemcpyHostToDevice, h->stream));
+  k_to_bf16<<<(unsigned)std::min<int64_t>((nf / 4 + 255) / 256, 148 * 8), 256, 0, h->stream>>>(
+      nf / 4, (const float4*)fx, (uint2*)S->eval_f);
+  C3D_LAUNCH_CHECK(h);
   C3D_CUDA_TRY(h, cudaMemcpyAsync(S->eval_m, mom, 4 * (size_t)m * kMom, cudaMemcpyHostToDevice, h->stream));
   double l = 0, nrm = 0;
   if ((rc = mlp_train_pass(h, S->eval_f, S->eval_m, m, S->sig_d, &l, &nrm))) return rc;
