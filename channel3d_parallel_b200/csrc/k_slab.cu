@@ -24,6 +24,10 @@
 // slab of 128 x 192 values takes 2 SMs' shared memory and one of 256 x 384
 // takes 7, so a cluster that holds it runs 8 to 12 warps per SM, in whole
 // waves of clusters, with the sweeps of 16 to 32 rows one after another.
+// 384 x 256 x 384: 1237 us in clusters, 467 here (1.5 GB moved: 230 us at the
+// copy rate); what is left is latency at 24 warps per SM and about 130
+// instructions a value.  Four rounds of 64 registers or 16 rows a block were
+// slower there (553 and 603 us with 256 threads, against 539).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -38,7 +42,9 @@ namespace {
 
 constexpr int kRows = 8;            // rows of j per block, held in registers per column
 constexpr int kMaxR = 8;            // largest FFT radix
-constexpr int kSlabThreads = 256;
+// one column per thread up to 384: the row's columns in two rounds of 192
+// threads took 539 us at 384 x 256 x 384 against 467
+constexpr int kSlabThreads = 384;
 
 template <typename T>
 struct SlabArgs {
@@ -240,7 +246,7 @@ __device__ __forceinline__ void slab_correct(const SlabArgs<T>& a, const SlabSme
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kSlabThreads, 3) k_slab_fwd(SlabArgs<T> a) {
+__global__ void __launch_bounds__(kSlabThreads, 2) k_slab_fwd(SlabArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char slab_smem_raw[];
   __shared__ bool s_last;
@@ -279,7 +285,7 @@ __global__ void __launch_bounds__(kSlabThreads, 3) k_slab_fwd(SlabArgs<T> a) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kSlabThreads, 3) k_slab_inv(SlabArgs<T> a) {
+__global__ void __launch_bounds__(kSlabThreads, 2) k_slab_inv(SlabArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char slab_smem_raw[];
   const int m = blockIdx.y, b = a.b0 + blockIdx.x;
