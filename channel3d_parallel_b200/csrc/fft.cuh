@@ -10,6 +10,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <initializer_list>
+
 namespace c3d {
 
 struct FftPasses {
@@ -303,6 +305,63 @@ __device__ void fft_rows_dit_inv(typename cplx<T>::t* data, int nrows, int rs,
                                  const typename cplx<T>::t* tw, const FftPasses& P, int from = 0, int to = 8) {
   for (int p = (P.npass < to ? P.npass : to) - 1; p >= from; --p)
     ct_stage_any<T, true, MAXR, NR>(data, nrows, rs, tw, P, p);
+}
+
+// The same transforms with the length N compiled in (radices, strides and
+// twiddle steps become constants, and only this length's stages are code): the
+// plan of make_fft_passes(N, P, MAXR).  nrec: ceil(2^32 / nrows).
+__host__ __device__ constexpr int plan_radix(int m, int maxr) {
+  for (int c : {16, 12, 8, 6, 4, 3, 2})
+    if (c <= maxr && m % c == 0) return c;
+  return m;
+}
+template <typename T, bool INV, int N, int R, int L>
+__device__ __forceinline__ void ct_stage_fixed(typename cplx<T>::t* data, int nrows, unsigned nrec, int rs,
+                                               const typename cplx<T>::t* tw) {
+  using C = typename cplx<T>::t;
+  constexpr int M = L / R, nb = N / R, tws = N / L;
+  for (int t = threadIdx.x; t < nrows * nb; t += blockDim.x) {
+    const int bb = div_by(t, nrec), l = t - bb * nrows;
+    const int blk = bb / M, q = bb - blk * M;
+    C* p = data + l * rs + blk * L + q;
+    C v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = p[r * M];
+    if (INV && M > 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        C w = tw[q * r * tws];
+        w.y = -w.y;
+        v[r] = cmul(v[r], w);
+      }
+    }
+    Dft<T, INV, R>::run(v);
+    if (!INV && M > 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw[q * r * tws]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) p[r * M] = v[r];
+  }
+  __syncthreads();
+}
+template <typename T, int N, int MAXR, int L = N>
+__device__ __forceinline__ void fft_fixed_dif(typename cplx<T>::t* data, int nrows, unsigned nrec, int rs,
+                                              const typename cplx<T>::t* tw) {
+  if constexpr (L > 1) {
+    constexpr int R = plan_radix(L, MAXR);
+    ct_stage_fixed<T, false, N, R, L>(data, nrows, nrec, rs, tw);
+    fft_fixed_dif<T, N, MAXR, L / R>(data, nrows, nrec, rs, tw);
+  }
+}
+template <typename T, int N, int MAXR, int L = N>
+__device__ __forceinline__ void fft_fixed_dit_inv(typename cplx<T>::t* data, int nrows, unsigned nrec, int rs,
+                                                  const typename cplx<T>::t* tw) {
+  if constexpr (L > 1) {
+    constexpr int R = plan_radix(L, MAXR);
+    fft_fixed_dit_inv<T, N, MAXR, L / R>(data, nrows, nrec, rs, tw);
+    ct_stage_fixed<T, true, N, R, L>(data, nrows, nrec, rs, tw);
+  }
 }
 
 // Stage plan of an N-point transform: the largest radix of 16, 12, 8, 6, 4,

@@ -14,6 +14,10 @@ namespace cg = cooperative_groups;
 
 namespace c3d {
 
+__host__ __device__ inline unsigned reciprocal(int n) {
+  return n > 1 ? (unsigned)(((1ull << 32) + n - 1) / n) : 0u;
+}
+
 constexpr int kYzMaxRWide = 16;     // largest FFT radix (register budget)
 constexpr int kYzMaxRNarrow = 8;
 
@@ -43,6 +47,7 @@ struct YzArgs {
   const T* __restrict__ du;      // Dyy(j, j+1)
   unsigned long long* err;       // sticky error bits
   FftPasses P;
+  unsigned rec_jc;   // ceil(2^32 / jc)
   int cs;        // CTAs per cluster
   int jc;        // j rows per CTA
   int rs;        // shared-memory row stride (complex values)
@@ -60,7 +65,7 @@ struct YzArgs {
 // 0, each CTA starting from the neighbour row read through distributed
 // shared memory.  After the forward transform column `col` holds wavenumber
 // kz = dif_position_to_k(col); the inverse transform takes that order back.
-template <typename T, bool NARROW>
+template <typename T, bool NARROW, int NZ = 0>
 __global__ void __launch_bounds__(yz_threads<NARROW>(), yz_min_blocks<NARROW>()) k_spectral_yz(YzArgs<T> a) {
   using C = typename cplx<T>::t;
   constexpr int JM = yz_jmax<T, NARROW>();
@@ -71,7 +76,7 @@ __global__ void __launch_bounds__(yz_threads<NARROW>(), yz_min_blocks<NARROW>())
   const int cs = a.cs;
   const int crank = (int)cl.block_rank();
   const int m = blockIdx.x / cs;
-  const int Ny = d.Ny, Nz = d.Nz, nkzs = d.nkzs;
+  const int Ny = d.Ny, Nz = NZ ? NZ : d.Nz, nkzs = d.nkzs;
   const int RS = a.rs, Jc = a.jc;
   const int j0 = crank * Jc;
   const int jn = min(Jc, Ny - j0);             // rows owned by this CTA (>= 1)
@@ -111,7 +116,10 @@ __global__ void __launch_bounds__(yz_threads<NARROW>(), yz_min_blocks<NARROW>())
   if (!loaded) atomicOr(a.err, 1ull);
   __syncthreads();
 
-  fft_rows_dif<T, (NARROW ? kYzMaxRNarrow : kYzMaxRWide)>(data + (size_t)blo * RS, bhi - blo, RS, tw, a.P);
+  constexpr int MAXR = NARROW ? kYzMaxRNarrow : kYzMaxRWide;
+  const unsigned nrec = bhi - blo == Jc ? a.rec_jc : reciprocal(bhi - blo);
+  if constexpr (NZ > 0) fft_fixed_dif<T, NZ, MAXR>(data + (size_t)blo * RS, bhi - blo, nrec, RS, tw);
+  else fft_rows_dif<T, MAXR>(data + (size_t)blo * RS, bhi - blo, RS, tw, a.P);
 
   // pivots of this thread's column for rows j0-1 .. j0+jn-1 (one column per
   // thread when Nz <= blockDim; otherwise reloaded per column below)
@@ -309,7 +317,8 @@ __global__ void __launch_bounds__(yz_threads<NARROW>(), yz_min_blocks<NARROW>())
   }
   __syncthreads();
 
-  fft_rows_dit_inv<T, (NARROW ? kYzMaxRNarrow : kYzMaxRWide)>(data + (size_t)blo * RS, bhi - blo, RS, tw, a.P);
+  if constexpr (NZ > 0) fft_fixed_dit_inv<T, NZ, MAXR>(data + (size_t)blo * RS, bhi - blo, nrec, RS, tw);
+  else fft_rows_dit_inv<T, MAXR>(data + (size_t)blo * RS, bhi - blo, RS, tw, a.P);
   // no CTA leaves while another may still read its ylast / xfirst
   cl.sync();
 
@@ -422,6 +431,28 @@ static bool choose_cluster(const Dims& d, int pz, int& cs, int& jc, int& rs, int
   return true;
 }
 
+// The kernel for rows of Nz columns.  FP64 rows of 64 to 256 columns have the
+// length compiled in: the kernel passes through its code about once, so its
+// size costs instruction fetches (49 -> 45 us at 192 x 128 x 192 on its own, 710
+// -> 673 us a time step, where other kernels run in between).  Shorter rows and
+// FP32 take the form with run-time stages.
+template <typename T>
+using YzKernel = void (*)(YzArgs<T>);
+template <typename T, bool NARROW, int... NZ>
+static YzKernel<T> yz_pick(int Nz) {
+  YzKernel<T> k = k_spectral_yz<T, NARROW>;
+  ((Nz == NZ ? (void)(k = k_spectral_yz<T, NARROW, NZ>) : (void)0), ...);
+  return k;
+}
+template <typename T>
+static YzKernel<T> yz_kernel(int Nz, int narrow) {
+  if constexpr (sizeof(T) == 8) {
+    return narrow ? yz_pick<T, true, 64, 72, 96, 108, 128, 144, 162, 192>(Nz)
+                  : yz_pick<T, false, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256>(Nz);
+  }
+  return narrow ? yz_pick<T, true>(Nz) : yz_pick<T, false>(Nz);
+}
+
 // z transforms and y solves of the whole spectrum in place, one launch
 template <typename T>
 int launch_cluster(Handle* h, typename SlabTables<T>::C* spec, int zero00, int rlo, int rhi) {
@@ -453,8 +484,8 @@ int launch_cluster(Handle* h, typename SlabTables<T>::C* spec, int zero00, int r
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (c.narrow) C3D_CUDA_TRY(h, cudaLaunchKernelEx(&cfg, k_spectral_yz<T, true>, a));
-  else C3D_CUDA_TRY(h, cudaLaunchKernelEx(&cfg, k_spectral_yz<T, false>, a));
+  a.rec_jc = reciprocal(c.jc);
+  C3D_CUDA_TRY(h, cudaLaunchKernelEx(&cfg, yz_kernel<T>(d.Nz, c.narrow), a));
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
@@ -473,12 +504,10 @@ int cluster_setup(Handle* h) {
                         : "ny_global too large for one 16-CTA cluster per kx slab";
     return C3D_ERR_UNSUPPORTED;
   }
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_spectral_yz<T, true>>(c.smem)));
-  C3D_CUDA_TRY(h, (raise_smem_limit<k_spectral_yz<T, false>>(c.smem)));
-  if (c.cs > 8) {
-    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_spectral_yz<T, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_spectral_yz<T, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  }
+  // process-wide, and handles of one Nz may differ in Ny: the most any needs
+  const YzKernel<T> k = yz_kernel<T>(d.Nz, c.narrow);
+  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+  if (c.cs > 8) C3D_CUDA_TRY(h, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return 0;
 }
 template int cluster_setup<double>(Handle*);
