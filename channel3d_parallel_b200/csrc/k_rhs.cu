@@ -193,7 +193,7 @@ constexpr int FX = PX + 1, FY = PY + 1, FN = FX * FY;     // phi: one more colum
 constexpr int RHS_THREADS = TX * TY;
 constexpr int NHALO = PN - TX * TY;       // halo cells of a tile, at most one a thread
 constexpr int RHS_CTAS = 2;               // resident CTAs per SM
-constexpr int NSLOT = 7;                  // planes k .. k+6
+constexpr int NSLOT = 6;                  // planes k .. k+6
 static_assert(NHALO <= RHS_THREADS && FN - TX * TY <= RHS_THREADS, "one halo cell per thread");
 
 __device__ __forceinline__ void cp_async8(unsigned sdst, const double* gsrc) {
@@ -212,13 +212,13 @@ __device__ __forceinline__ double wdiff(double p, double a, double q, double b) 
 }
 
 // shared memory: NSLOT planes of U, V, W (PN each) and phi (FN, PROJ), the z
-// factors of planes k0..k1: (rdz/4, rdzg/4), (czpC, czmC), (czpF, czmF), and
-// 1/dzg of k0-1..k1+1
+// factors (rdz/4, rdzg/4) of planes k0-1..k1+1 and (czpC, czmC), (czpF, czmF)
+// of planes k0..k1
 template <bool PROJ>
 struct RhsSmem {
   static constexpr int SLOT = 3 * PN + (PROJ ? FN : 0);
   static constexpr int Z0 = NSLOT * SLOT + ((NSLOT * SLOT) & 1);
-  static size_t bytes(int kc) { return sizeof(double) * (size_t)(Z0 + 6 * kc + kc + 2); }
+  static size_t bytes(int kc) { return sizeof(double) * (size_t)(Z0 + 2 * (kc + 2) + 4 * kc); }
 };
 
 template <int MODE, bool PROJ>
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
   __shared__ double sGx[PX], sGy[PY];
   __shared__ double2 sY[3][TY];
   double2* sZ = reinterpret_cast<double2*>(rhs_smem + L::Z0);
-  double* sGz = rhs_smem + L::Z0 + 6 * a.kc;
+  double2* sZ1 = sZ + a.kc + 2;
   const Dims& d = a.d;
   const Metric& m = a.m;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
@@ -239,18 +239,21 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
   const int i = i0 + tx, j = j0 + ty;
   const int plU = d.nx * d.nyg, plV = d.nxg * d.ny, plW = d.nxg * d.nyg, plR = (d.nxg - 2) * (d.nyg - 2);
   auto at = [](int z, int pl) { return (int64_t)z * pl; };     // 32 x 32 -> 64 bits
-  auto xfold = [&](int gi) { return gi == 1 ? d.Nx + 1 : (gi >= d.Nx + 2 ? gi - d.Nx : gi); };
+  auto xfold = [&](int gi) { return gi == 1 ? d.Nx + 1 : 2 + (gi - 2) % d.Nx; };
   auto zfold = [&](int k) { return PROJ ? (k == 1 ? d.Nz + 1 : (k >= d.Nz + 2 ? k - d.Nz : k)) : k; };
 
   // places in the fields, inside a plane (always legal; what is read at a
-  // position that is not needed is not used)
+  // position that is not needed is not used).  Columns past the grid fold back
+  // into it like the periodic images: with one clamped address for all of them
+  // a part-filled tile took twice as long as a full one, and copies left out by
+  // a condition slowed every tile (105 -> 141 us at 192 x 128 x 192).
   struct Pos {
     int u, v, w;
     bool neg, wall;          // u, w: wall reflection; v: zero
   };
   auto place = [&](int x, int y) {
     Pos p;
-    int gi = min(i0 - 1 + x, d.Nx + 2), gj = min(j0 - 1 + y, d.Ny + 2), gv = min(gj, d.Ny + 1);
+    int gi = i0 - 1 + x, gj = min(j0 - 1 + y, d.Ny + 2), gv = min(gj, d.Ny + 1);
     p.neg = p.wall = false;
     if (PROJ) {
       p.neg = gj == 1 || gj == d.Ny + 2;
@@ -259,13 +262,14 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
       gj = gj == 1 ? 2 : (gj == d.Ny + 2 ? d.Ny + 1 : gj);
       gv = min(gj, d.Ny);
     }
+    if (gi > d.Nx + 2) gi = xfold(gi);
     p.u = (int)idxU(d, gi, gj, 1);
     p.v = (int)idxV(d, gi, gv, 1);
     p.w = (int)idxW(d, gi, gj, 1);
     return p;
   };
   auto phi_place = [&](int x, int y) {      // rows 1 and ny+1: the gradient there is not used as it stands
-    const int gi = xfold(min(i0 - 1 + x, d.Nx + 3)), gj = min(max(j0 - 1 + y, 2), d.Ny + 1);
+    const int gi = xfold(i0 - 1 + x), gj = min(max(j0 - 1 + y, 2), d.Ny + 1);
     return (int)idxR(d, gi, gj, 2);
   };
   // second position of this thread: rows 0 and PY-1 of the tile, then the side
@@ -303,7 +307,7 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
   };
   // the last plane whose velocities are needed is k1+1; its w needs phi of k1+2
   const int kend = PROJ ? k1 + 2 : k1 + 1;
-  for (int q = 0; q < 7; ++q) {
+  for (int q = 0; q < NSLOT; ++q) {
     if (k0 - 1 + q <= kend) issue(k0 - 1 + q, q);
     cp_async_commit();
   }
@@ -319,12 +323,13 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
   }
   for (int t = tid; t < a.kc; t += RHS_THREADS) {
     const int kk = min(k0 + t, k1);
-    sZ[t] = make_double2(0.25 * m.rdz[kk], 0.25 * m.rdzg[kk]);
-    sZ[a.kc + t] = make_double2(m.czpC[kk], m.czmC[kk]);
-    sZ[2 * a.kc + t] = make_double2(m.czpF[kk], m.czmF[kk]);
+    sZ1[t] = make_double2(m.czpC[kk], m.czmC[kk]);
+    sZ1[a.kc + t] = make_double2(m.czpF[kk], m.czmF[kk]);
   }
-  if (PROJ)
-    for (int t = tid; t < a.kc + 2; t += RHS_THREADS) sGz[t] = m.rdzg[zfold(min(k0 - 1 + t, k1 + 1))];
+  for (int t = tid; t < a.kc + 2; t += RHS_THREADS) {
+    const int kk = zfold(min(k0 - 1 + t, k1 + 1));
+    sZ[t] = make_double2(0.25 * m.rdz[kk], 0.25 * m.rdzg[kk]);
+  }
   const bool edge = j0 + TY > d.Ny + 1;     // the tile holds wall rows of v or rows past them
   const int ic = min(i, d.Nx + 1);
   const double2 x0 = make_double2(0.25 * m.rdxg[ic], 0.25 * m.rdx[ic]);
@@ -361,14 +366,14 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
       return;
     }
     const double* Sn = rhs_smem + sn * L::SLOT;
-    const double gz = sGz[kz];
+    const double gz = 4.0 * sZ[kz].y;
     form(P0, S, Sn, c, cf, sGx[tx + 1], sGy[ty + 1], gz, edge, p0, u, v, w);
     double hu, hv, hw;
     if (halo) form(P1, S, Sn, ch, chf, sGx[hx], sGy[hy], gz, true, ph, hu, hv, hw);
   };
 
   // planes k0-1, k0, k0+1 formed (k0+2 has landed), slots 0, 1, 2
-  cp_async_wait<3>();
+  cp_async_wait<NSLOT - 4>();
   __syncthreads();
   if (PROJ) {
     p0 = rhs_smem[3 * PN + cf];
@@ -399,16 +404,16 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
     const int t = k - k0;
     const int s1 = next(s0), s2 = next(s1), s3 = next(s2);
     // planes up to k+3 have landed and those up to k+1 are formed; every
-    // thread is done with plane k-1, whose slot takes plane k+6
-    cp_async_wait<2>();
+    // thread is done with plane k-1, whose slot takes plane k+NSLOT-1
+    cp_async_wait<NSLOT - 5>();
     __syncthreads();
-    if (k + 6 <= kend) issue(k + 6, s0 == 0 ? NSLOT - 1 : s0 - 1);
+    if (k + NSLOT - 1 <= kend) issue(k + NSLOT - 1, s0 == 0 ? NSLOT - 1 : s0 - 1);
     cp_async_commit();
     double u2 = 0.0, v2 = 0.0, w2 = 0.0;
     if (k < k1) form_plane(t + 3, s2, s3, u2, v2, w2);
     const double *U0 = rhs_smem + s0 * L::SLOT + c, *V0 = U0 + PN, *W0 = U0 + 2 * PN;
     const double *U1 = rhs_smem + s1 * L::SLOT + c, *V1 = U1 + PN;
-    const double2 z0 = sZ[t], z1 = sZ[a.kc + t];
+    const double2 z0 = sZ[t + 1], z1 = sZ1[t];
     const double2 y0 = sY[0][ty], y1 = sY[1][ty];
     const double uxm = U0[-1], uxp = U0[1], uym = U0[-PX], uyp = U0[PX];
     const double vxm = V0[-1], vxp = V0[1], vym = V0[-PX], vyp = V0[PX];
@@ -436,7 +441,7 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
         store(a.Us, a.Hu, dPdx, a.Gu_out, conv, visc, u0, gu, zu, P0.u);
       }
       {
-        const double2 z2 = sZ[2 * a.kc + t];
+        const double2 z2 = sZ1[a.kc + t];
         const double wxm = W0[-1];
         const double exzm = mul(uxm + U1[-1], wxm + w0), eyzm = mul(vym + V1[-PX], wym + w0);
         const double cz = mul(w0 + w1, w0 + w1);
