@@ -168,15 +168,18 @@ __global__ void __launch_bounds__(256) k_rhs(RhsArgs a) {
 // The planes (tile plus halo) come by cp.async into a ring of NSLOT slots,
 // three planes ahead of the one whose velocities are formed, which in turn is
 // two ahead of the one that is computed, so one barrier a plane orders
-// everything; each thread forms the velocities of its own cell and some
-// threads those of one halo cell, in place.  Loads one plane ahead into
+// everything; each thread forms the velocities of its own cell and most
+// threads one component of a halo cell, in place (the three components of a
+// cell in one thread: 105 us in place of 103 at 192 x 128 x 192, one warp in
+// three held the others at the barrier).  Loads one plane ahead into
 // registers took 166-197 us a stage at 192 x 128 x 192 (two to three
 // microseconds a plane: the memory's latency under load).
 //
-// Measured (B200, us a stage): 192 x 128 x 192 97 in stage 1 and 105 in 2 and
-// 3, where the separate projection took 53 and the update 92; 384 x 256 x 384
-// 785 (369 and 692); 32 x 64 x 32 8 (6 and 31: that update marched 64 planes
-// whatever the grid).  Bound by instruction issue (0.55 a cycle at 16 warps,
+// Measured (B200, us a stage 2 or 3): 192 x 128 x 192 101, where the separate
+// projection took 53 and the update 92; 384 x 256 x 384 740 (369 and 692);
+// 32 x 64 x 32 8 (6 and 31: that update marched 64 planes whatever the grid).
+// Two or three planes a turn of the loop took 133 and 147 us: the code of one
+// plane is as much as the instruction cache feeds.  Bound by instruction issue (0.55 a cycle at 16 warps,
 // 400 a cell) and by the shared-memory pipe (0.7 busy: an 8-byte access of a
 // warp is two wavefronts); memory runs at 3.5 TB/s.
 //
@@ -193,8 +196,8 @@ constexpr int FX = PX + 1, FY = PY + 1, FN = FX * FY;     // phi: one more colum
 constexpr int RHS_THREADS = TX * TY;
 constexpr int NHALO = PN - TX * TY;       // halo cells of a tile, at most one a thread
 constexpr int RHS_CTAS = 2;               // resident CTAs per SM
-constexpr int NSLOT = 6;                  // planes k .. k+6
-static_assert(NHALO <= RHS_THREADS && FN - TX * TY <= RHS_THREADS, "one halo cell per thread");
+constexpr int NSLOT = 6;                  // planes k .. k+5
+static_assert(3 * NHALO <= RHS_THREADS && FN - TX * TY <= RHS_THREADS, "one halo value per thread");
 
 __device__ __forceinline__ void cp_async8(unsigned sdst, const double* gsrc) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sdst), "l"(gsrc));
@@ -272,17 +275,24 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
     const int gi = xfold(i0 - 1 + x), gj = min(max(j0 - 1 + y, 2), d.Ny + 1);
     return (int)idxR(d, gi, gj, 2);
   };
-  // second position of this thread: rows 0 and PY-1 of the tile, then the side
-  // columns; of phi: row 0, the last two rows, the side columns
-  int hx = 1, hy = 1, fx = 1, fy = 1;
-  const bool halo = tid < NHALO, fhalo = PROJ && tid < FN - TX * TY;
-  if (tid < 2 * PX) { hy = tid < PX ? 0 : PY - 1; hx = tid < PX ? tid : tid - PX; }
-  else if (halo) { const int t = tid - 2 * PX; hx = t < TY ? 0 : PX - 1; hy = 1 + (t < TY ? t : t - TY); }
+  // halo value of this thread: component hf at a tile position of rows 0 and
+  // PY-1 or the side columns (the threads past 3 * NHALO copy the last one too and form nothing);
+  // of phi: row 0, the last two rows, the side columns
+  const int hv = min(tid, 3 * NHALO - 1), hf = hv / NHALO, hp = hv - hf * NHALO;
+  int hx, hy, fx = 1, fy = 1;
+  const bool fhalo = PROJ && tid < FN - TX * TY;
+  if (hp < 2 * PX) { hy = hp < PX ? 0 : PY - 1; hx = hp < PX ? hp : hp - PX; }
+  else { const int t = hp - 2 * PX; hx = t < TY ? 0 : PX - 1; hy = 1 + (t < TY ? t : t - TY); }
   if (tid < 3 * FX) { const int r = tid / FX; fy = r == 0 ? 0 : PY - 2 + r; fx = tid - r * FX; }
   else if (fhalo) { const int t = tid - 3 * FX, q = t / TY; fx = q == 0 ? 0 : PX - 2 + q; fy = 1 + (t - q * TY); }
-  const int c = (ty + 1) * PX + (tx + 1), ch = hy * PX + hx;
+  const int c = (ty + 1) * PX + (tx + 1);
   const int cf = (ty + 1) * FX + (tx + 1), chf = hy * FX + hx;      // the same places in phi's tile
+  const int hs = hf * PN + hy * PX + hx;                            // the halo value's place in a slot
+  const int hq = 3 * PN + chf + (hf == 0 ? 1 : (hf == 1 ? FX : 0)); // the other end of its gradient
   const Pos P0 = place(tx + 1, ty + 1), P1 = place(hx, hy);
+  const double* const hsrc = hf == 0 ? a.U + P1.u : (hf == 1 ? a.V + P1.v : a.W + P1.w);
+  const int hpl = hf == 0 ? plU : (hf == 1 ? plV : plW);
+  const bool hneg = hf != 1 && P1.neg, hzero = hf == 1 && P1.wall;
   const int f0 = PROJ ? phi_place(tx + 1, ty + 1) : 0, f1 = PROJ ? phi_place(fx, fy) : 0;
   const unsigned sbase = (unsigned)__cvta_generic_to_shared(rhs_smem);
 
@@ -294,11 +304,7 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
     cp_async8(s + 8 * c, Uz + P0.u);
     cp_async8(s + 8 * (PN + c), Vz + P0.v);
     cp_async8(s + 8 * (2 * PN + c), Wz + P0.w);
-    if (halo) {
-      cp_async8(s + 8 * ch, Uz + P1.u);
-      cp_async8(s + 8 * (PN + ch), Vz + P1.v);
-      cp_async8(s + 8 * (2 * PN + ch), Wz + P1.w);
-    }
+    cp_async8(s + 8 * hs, hsrc + at(z, hpl));
     if (PROJ) {
       const double* Fz = a.phi + at(z - 1, plR);
       cp_async8(s + 8 * (3 * PN + cf), Fz + f0);
@@ -337,26 +343,12 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
   const double shift = MODE == 1 && PROJ && a.ushift ? *a.ushift : 0.0;
   const double dPdx = a.sc->dPdx, dPdy = a.sc->dPdy, dPdz = a.sc->dPdz;
 
+  const double hshift = hf == 0 ? shift : 0.0;
   // velocities of plane k0-1+kz in place: slot s, phi of the next plane in slot
-  // sn; p0, ph: phi of the own and the halo cell (carried from plane to plane);
-  // the own cell's velocities to u, v, w
-  double p0 = 0.0, ph = 0.0;
-  auto form = [&](const Pos& p, double* S, const double* Sn, int at, int atf, double gx, double gy, double gz, bool bc,
-                  double& pc, double& u, double& v, double& w) {
-    const double pz = Sn[3 * PN + atf];
-    u = __fma_rn(pc - S[3 * PN + atf + 1], gx, S[at]);
-    v = __fma_rn(pc - S[3 * PN + atf + FX], gy, S[PN + at]);
-    w = __fma_rn(pc - pz, gz, S[2 * PN + at]);
-    pc = pz;
-    if (MODE == 1) u += shift;
-    if (bc) {
-      if (p.neg) { u = -u; w = -w; }
-      if (p.wall) v = 0.0;
-    }
-    S[at] = u;
-    S[PN + at] = v;
-    S[2 * PN + at] = w;
-  };
+  // sn; p0: phi of the own cell (carried from plane to plane); the own cell's
+  // velocities to u, v, w.  The halo goes one component a thread, so that every
+  // warp has the same work before the barrier.
+  double p0 = 0.0;
   auto form_plane = [&](int kz, int s, int sn, double& u, double& v, double& w) {
     double* S = rhs_smem + s * L::SLOT;
     if (!PROJ) {
@@ -367,9 +359,23 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
     }
     const double* Sn = rhs_smem + sn * L::SLOT;
     const double gz = 4.0 * sZ[kz].y;
-    form(P0, S, Sn, c, cf, sGx[tx + 1], sGy[ty + 1], gz, edge, p0, u, v, w);
-    double hu, hv, hw;
-    if (halo) form(P1, S, Sn, ch, chf, sGx[hx], sGy[hy], gz, true, ph, hu, hv, hw);
+    const double pz = Sn[3 * PN + cf];
+    u = __fma_rn(p0 - S[3 * PN + cf + 1], sGx[tx + 1], S[c]);
+    v = __fma_rn(p0 - S[3 * PN + cf + FX], sGy[ty + 1], S[PN + c]);
+    w = __fma_rn(p0 - pz, gz, S[2 * PN + c]);
+    p0 = pz;
+    if (MODE == 1) u += shift;
+    if (edge) {
+      if (P0.neg) { u = -u; w = -w; }
+      if (P0.wall) v = 0.0;
+    }
+    S[c] = u;
+    S[PN + c] = v;
+    S[2 * PN + c] = w;
+    const double g = hf == 0 ? sGx[hx] : (hf == 1 ? sGy[hy] : gz);
+    double h = __fma_rn(S[3 * PN + chf] - (hf == 2 ? Sn : S)[hq], g, S[hs]);
+    if (MODE == 1) h += hshift;
+    if (tid < 3 * NHALO) S[hs] = hzero ? 0.0 : (hneg ? -h : h);
   };
 
   // planes k0-1, k0, k0+1 formed (k0+2 has landed), slots 0, 1, 2
@@ -377,7 +383,6 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
   __syncthreads();
   if (PROJ) {
     p0 = rhs_smem[3 * PN + cf];
-    ph = rhs_smem[3 * PN + chf];
   }
   double ua, va, wa, u0, v0, w0, u1, v1, w1;
   form_plane(0, 0, 1, ua, va, wa);
@@ -423,7 +428,8 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_CTAS) k_rhs_march(RhsArgs a) 
     const int64_t zu = at(k - 1, plU), zv = at(k - 1, plV), zw = at(k - 1, plW);
     auto store = [&](double* S, const double* Hm, double dP, double* Go, double conv, double visc, double f, double g,
                      int64_t z, int o) {
-      const double F = Hm ? __fma_rn(dP, __ldg(Hm + z + o), conv + visc) : (conv + visc) + dP;
+      // the mask of an immersed body: only without PROJ
+      const double F = !PROJ && Hm ? __fma_rn(dP, __ldg(Hm + z + o), conv + visc) : (conv + visc) + dP;
       if (MODE == 1) {
         (S + z)[o] = __fma_rn(a.cs, F, f);
         (Go + z)[o] = __fma_rn(a.cg, F, f);
