@@ -24,8 +24,8 @@
 // slab of 128 x 192 values takes 2 SMs' shared memory and one of 256 x 384
 // takes 7, so a cluster that holds it runs 8 to 12 warps per SM, in whole
 // waves of clusters, with the sweeps of 16 to 32 rows one after another.
-// 384 x 256 x 384: 1237 us in clusters, 467 here (1.5 GB moved: 230 us at the
-// copy rate); what is left is latency at 24 warps per SM and about 130
+// 384 x 256 x 384: 1237 us in clusters, 417 here (1.4 GB moved: 210 us at the
+// copy rate); what is left is latency at 24 warps per SM and about 100
 // instructions a value.  Four rounds of 64 registers or 16 rows a block were
 // slower there (553 and 603 us with 256 threads, against 539).
 #include <algorithm>
@@ -42,9 +42,16 @@ namespace {
 
 constexpr int kRows = 8;            // rows of j per block, held in registers per column
 constexpr int kMaxR = 8;            // largest FFT radix
+constexpr unsigned kRecRows = (unsigned)((1ull << 32) / kRows);   // reciprocal of kRows for div_by
 // one column per thread up to 384: the row's columns in two rounds of 192
 // threads took 539 us at 384 x 256 x 384 against 467
 constexpr int kSlabThreads = 384;
+
+// row stride in shared memory: FP64 1 mod 8, FP32 odd
+template <typename T>
+constexpr int slab_stride(int Nz) {
+  return sizeof(T) == 8 ? (Nz + 6) / 8 * 8 + 1 : Nz | 1;
+}
 
 template <typename T>
 struct SlabArgs {
@@ -245,26 +252,32 @@ __device__ __forceinline__ void slab_correct(const SlabArgs<T>& a, const SlabSme
   }
 }
 
-template <typename T>
+template <typename T, int NZ>
 __global__ void __launch_bounds__(kSlabThreads, 2) k_slab_fwd(SlabArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char slab_smem_raw[];
   __shared__ bool s_last;
   const int m = blockIdx.y, b = a.b0 + blockIdx.x;
-  const int Ny = a.d.Ny, Nz = a.d.Nz, RS = a.rs;
+  constexpr int R0 = plan_radix(NZ > 0 ? NZ : 2, kMaxR);
+  const int Ny = a.d.Ny, Nz = NZ > 0 ? NZ : a.d.Nz, RS = NZ > 0 ? slab_stride<T>(NZ) : a.rs;
   const int j0 = b * a.jr, jn = min(a.jr, Ny - j0);
   const int blo = max(a.rlo - j0, 0), bhi = min(a.rhi + 1 - j0, jn);   // rows [blo, bhi) of the band
   const bool full = bhi - blo == kRows;
   const SlabSmem<T> s = slab_carve<T>(slab_smem_raw, a);
   C* const g = a.spec + ((int64_t)m * Ny + j0) * a.pz;
   slab_tables(a, s, m, j0, jn);
-  ct_edge_any<T, false>(
-      bhi - blo, a.tw1, a.P, [&](int l, int e) { return g[(blo + l) * a.pz + e]; },
-      [&](int l, int e, C v) { s.data[(blo + l) * RS + e] = v; });
+  auto first_in = [&](int l, int e) { return g[(blo + l) * a.pz + e]; };
+  auto first_out = [&](int l, int e, C v) { s.data[(blo + l) * RS + e] = v; };
+  if constexpr (NZ > 0) ct_edge<T, false, R0>(bhi - blo, NZ, a.tw1, a.P.rec[0], first_in, first_out);
+  else ct_edge_any<T, false>(bhi - blo, a.tw1, a.P, first_in, first_out);
   asm volatile("cp.async.wait_group 0;\n" ::);
   __syncthreads();
-  if (full) fft_rows_dif<T, kMaxR, kRows>(s.data, kRows, RS, s.tw, a.P, 1);
-  else fft_rows_dif<T, kMaxR>(s.data + blo * RS, bhi - blo, RS, s.tw, a.P, 1);
+  if constexpr (NZ > 0) {
+    if (full) fft_fixed_dif<T, NZ, kMaxR, NZ / R0>(s.data, kRows, kRecRows, RS, s.tw);
+  } else if (full) {
+    fft_rows_dif<T, kMaxR, kRows>(s.data, kRows, RS, s.tw, a.P, 1);
+  }
+  if (!full) fft_rows_dif<T, kMaxR>(s.data + blo * RS, bhi - blo, RS, s.tw, a.P, 1);
   C* const e = a.ends + ((int64_t)m * a.nblk + b) * 2 * Nz;
   for (int col = threadIdx.x; col < Nz; col += blockDim.x) {
     if (full) slab_sweeps<true>(a, s, col, blo, bhi, jn, g, e);
@@ -284,12 +297,15 @@ __global__ void __launch_bounds__(kSlabThreads, 2) k_slab_fwd(SlabArgs<T> a) {
   }
 }
 
-template <typename T>
+template <typename T, int NZ>
 __global__ void __launch_bounds__(kSlabThreads, 2) k_slab_inv(SlabArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char slab_smem_raw[];
-  const int m = blockIdx.y, b = a.b0 + blockIdx.x;
-  const int Ny = a.d.Ny, Nz = a.d.Nz, RS = a.rs;
+  // the slabs that k_slab_fwd left last, and L2 still holds, come first (473 ->
+  // 448 us at 384 x 256 x 384)
+  const int m = (int)gridDim.y - 1 - (int)blockIdx.y, b = a.b0 + blockIdx.x;
+  constexpr int R0 = plan_radix(NZ > 0 ? NZ : 2, kMaxR);
+  const int Ny = a.d.Ny, Nz = NZ > 0 ? NZ : a.d.Nz, RS = NZ > 0 ? slab_stride<T>(NZ) : a.rs;
   const int j0 = b * a.jr, jn = min(a.jr, Ny - j0);
   const int blo = max(a.rlo - j0, 0), bhi = min(a.rhi + 1 - j0, jn);
   const bool full = bhi - blo == kRows;
@@ -318,11 +334,16 @@ __global__ void __launch_bounds__(kSlabThreads, 2) k_slab_inv(SlabArgs<T> a) {
     else slab_correct<false>(a, s, col, blo, bhi, j0, jn, zero, v, Y, X);
   }
   __syncthreads();
-  if (full) fft_rows_dit_inv<T, kMaxR, kRows>(s.data, kRows, RS, s.tw, a.P, 1);
-  else fft_rows_dit_inv<T, kMaxR>(s.data + blo * RS, bhi - blo, RS, s.tw, a.P, 1);
-  ct_edge_any<T, true>(
-      bhi - blo, a.tw1, a.P, [&](int l, int q) { return s.data[(blo + l) * RS + q]; },
-      [&](int l, int q, C v) { g[(blo + l) * a.pz + q] = v; });
+  if constexpr (NZ > 0) {
+    if (full) fft_fixed_dit_inv<T, NZ, kMaxR, NZ / R0>(s.data, kRows, kRecRows, RS, s.tw);
+  } else if (full) {
+    fft_rows_dit_inv<T, kMaxR, kRows>(s.data, kRows, RS, s.tw, a.P, 1);
+  }
+  if (!full) fft_rows_dit_inv<T, kMaxR>(s.data + blo * RS, bhi - blo, RS, s.tw, a.P, 1);
+  auto last_in = [&](int l, int q) { return s.data[(blo + l) * RS + q]; };
+  auto last_out = [&](int l, int q, C v) { g[(blo + l) * a.pz + q] = v; };
+  if constexpr (NZ > 0) ct_edge<T, true, R0>(bhi - blo, NZ, a.tw1, a.P.rec[0], last_in, last_out);
+  else ct_edge_any<T, true>(bhi - blo, a.tw1, a.P, last_in, last_out);
 }
 
 // factors across a block, per mode: h(last), p(first), g(first)
@@ -353,14 +374,27 @@ __global__ void k_slab_link(Dims d, int jr, int nblk, const double* __restrict__
   }
 }
 
-template <typename T>
-int slab_rs(int Nz) {
-  int rs = Nz;
-  while (rs % (sizeof(T) == 8 ? 8 : 2) != 1) ++rs;
-  return rs;
-}
-
 constexpr int kSlabSmemMax = 220 * 1024;
+
+// The kernels for rows of Nz columns.  FP64 rows of 192 to 512 columns have the
+// length compiled in (384 x 256 x 384: 448 -> 417 us); shorter rows reach these
+// kernels only with very many of them, and FP32 takes the run-time stages.
+template <typename T>
+struct SlabKernels {
+  void (*fwd)(SlabArgs<T>);
+  void (*inv)(SlabArgs<T>);
+};
+template <typename T, int... NZ>
+SlabKernels<T> slab_pick(int Nz) {
+  SlabKernels<T> k{k_slab_fwd<T, 0>, k_slab_inv<T, 0>};
+  ((Nz == NZ ? (void)(k = {k_slab_fwd<T, NZ>, k_slab_inv<T, NZ>}) : (void)0), ...);
+  return k;
+}
+template <typename T>
+SlabKernels<T> slab_kernels(int Nz) {
+  if constexpr (sizeof(T) == 8) return slab_pick<T, 192, 216, 256, 288, 324, 384, 432, 486, 512>(Nz);
+  else return slab_pick<T>(Nz);
+}
 
 }  // namespace
 
@@ -374,7 +408,7 @@ static int slab_setup_t(Handle* h, SlabTables<T>& t) {
   int rc;
   if (t.link == nullptr) {
     t.jr = kRows;
-    while (t.jr > 1 && slab_smem<T>(d.Nz, d.nkzs, t.jr, slab_rs<T>(d.Nz)) > (size_t)kSlabSmemMax) t.jr /= 2;
+    while (t.jr > 1 && slab_smem<T>(d.Nz, d.nkzs, t.jr, slab_stride<T>(d.Nz)) > (size_t)kSlabSmemMax) t.jr /= 2;
     t.nblk = (d.Ny + t.jr - 1) / t.jr;
     FftPasses P;
     make_fft_passes(d.Nz, P, kMaxR);
@@ -391,8 +425,9 @@ static int slab_setup_t(Handle* h, SlabTables<T>& t) {
     if ((rc = dev_alloc(h, &t.ticket, d.nkx))) return rc;
     C3D_CUDA_TRY(h, cudaMemcpyAsync(t.tw1, tw1.data(), sizeof(C) * d.Nz, cudaMemcpyHostToDevice, h->stream));
     C3D_CUDA_TRY(h, cudaMemcpyAsync(t.kzs, kzs.data(), sizeof(int) * d.Nz, cudaMemcpyHostToDevice, h->stream));
-    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_slab_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemMax));
-    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_slab_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemMax));
+    const SlabKernels<T> k = slab_kernels<T>(d.Nz);
+    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemMax));
+    C3D_CUDA_TRY(h, cudaFuncSetAttribute(k.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemMax));
     C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));   // the host copies end here
   }
   k_slab_link<T><<<dim3((d.nkzs + 63) / 64, d.nkx), 64, 0, h->stream>>>(d, t.jr, t.nblk, S.rdp, S.dl, S.du, t.link);
@@ -424,7 +459,7 @@ int launch_slab(Handle* h, typename SlabTables<T>::C* spec, int zero00, int rlo,
   a.tw1 = t->tw1; a.link = t->link; a.kzs = t->kzs; a.ends = t->ends; a.ticket = t->ticket;
   make_fft_passes(d.Nz, a.P, kMaxR);
   a.jr = t->jr; a.nblk = t->nblk;
-  a.rs = slab_rs<T>(d.Nz);
+  a.rs = slab_stride<T>(d.Nz);
   a.zero00 = zero00; a.rlo = rlo; a.rhi = rhi;
   a.b0 = rlo / a.jr;
   const dim3 grid(rhi / a.jr - a.b0 + 1, d.nkx);
@@ -433,9 +468,10 @@ int launch_slab(Handle* h, typename SlabTables<T>::C* spec, int zero00, int rlo,
   const int rounds = (d.Nz + kSlabThreads - 1) / kSlabThreads;
   const int nt = std::max(64, ((d.Nz + rounds - 1) / rounds + 31) / 32 * 32);
   const size_t smem = slab_smem<T>(d.Nz, d.nkzs, a.jr, a.rs);
-  k_slab_fwd<T><<<grid, nt, smem, h->stream>>>(a);
+  const SlabKernels<T> k = slab_kernels<T>(d.Nz);
+  k.fwd<<<grid, nt, smem, h->stream>>>(a);
   C3D_LAUNCH_CHECK(h);
-  k_slab_inv<T><<<grid, nt, smem, h->stream>>>(a);
+  k.inv<<<grid, nt, smem, h->stream>>>(a);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
