@@ -315,6 +315,10 @@ __host__ __device__ constexpr int plan_radix(int m, int maxr) {
     if (c <= maxr && m % c == 0) return c;
   return m;
 }
+__host__ __device__ constexpr int plan_last_radix(int m, int maxr) {
+  while (m > plan_radix(m, maxr)) m /= plan_radix(m, maxr);
+  return m;
+}
 template <typename T, bool INV, int N, int R, int L>
 __device__ __forceinline__ void ct_stage_fixed(typename cplx<T>::t* data, int nrows, unsigned nrec, int rs,
                                                const typename cplx<T>::t* tw) {
@@ -345,21 +349,22 @@ __device__ __forceinline__ void ct_stage_fixed(typename cplx<T>::t* data, int nr
   }
   __syncthreads();
 }
-template <typename T, int N, int MAXR, int L = N>
+// L / STOP: only the stages of spans L down to above STOP.
+template <typename T, int N, int MAXR, int L = N, int STOP = 1>
 __device__ __forceinline__ void fft_fixed_dif(typename cplx<T>::t* data, int nrows, unsigned nrec, int rs,
                                               const typename cplx<T>::t* tw) {
-  if constexpr (L > 1) {
+  if constexpr (L > STOP) {
     constexpr int R = plan_radix(L, MAXR);
     ct_stage_fixed<T, false, N, R, L>(data, nrows, nrec, rs, tw);
-    fft_fixed_dif<T, N, MAXR, L / R>(data, nrows, nrec, rs, tw);
+    fft_fixed_dif<T, N, MAXR, L / R, STOP>(data, nrows, nrec, rs, tw);
   }
 }
-template <typename T, int N, int MAXR, int L = N>
+template <typename T, int N, int MAXR, int L = N, int STOP = 1>
 __device__ __forceinline__ void fft_fixed_dit_inv(typename cplx<T>::t* data, int nrows, unsigned nrec, int rs,
                                                   const typename cplx<T>::t* tw) {
-  if constexpr (L > 1) {
+  if constexpr (L > STOP) {
     constexpr int R = plan_radix(L, MAXR);
-    fft_fixed_dit_inv<T, N, MAXR, L / R>(data, nrows, nrec, rs, tw);
+    fft_fixed_dit_inv<T, N, MAXR, L / R, STOP>(data, nrows, nrec, rs, tw);
     ct_stage_fixed<T, true, N, R, L>(data, nrows, nrec, rs, tw);
   }
 }

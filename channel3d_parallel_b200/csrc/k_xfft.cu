@@ -28,6 +28,13 @@ constexpr int kLines = 8;        // complex lines per CTA
 constexpr int kFwdThreads = 384;
 constexpr int kInvThreads = 192;
 constexpr int kMaxR = 8;         // largest radix (register budget)
+constexpr unsigned kRecLines = (unsigned)((1ull << 32) / kLines);   // reciprocal of kLines for div_by
+
+// shared-memory row stride: FP64 1 mod 8, FP32 odd (conflict-free across rows)
+template <typename T>
+constexpr int x_stride(int Nx) {
+  return sizeof(T) == 8 ? (Nx + 6) / 8 * 8 + 1 : Nx | 1;
+}
 
 // what the first stage reads
 enum { FROM_RHS = 0, FROM_DIV = 1, FROM_DIV_FLUX = 2, FROM_RESIDUAL = 3 };
@@ -107,7 +114,7 @@ struct LineLoads {
   double x1, x0, y1, y0, z1, z0;
 };
 template <int SRC, typename T>
-__device__ __forceinline__ LineLoads<SRC> line_load(const XfwdArgs<T>& a, const LineInfo& L, int i) {
+__device__ __forceinline__ LineLoads<SRC> line_load(const XfwdArgs<T>& a, const LineInfo& L, int N, int i) {
   LineLoads<SRC> v;
   v.x1 = v.x0 = v.y1 = v.y0 = v.z1 = v.z0 = 0.0;
   if (L.u < 0) return v;
@@ -115,7 +122,7 @@ __device__ __forceinline__ LineLoads<SRC> line_load(const XfwdArgs<T>& a, const 
     v.x1 = a.rhs[L.u + i];
     return v;
   }
-  const int N = a.d.Nx, xo = (i == 0 ? N : i) - 1;    // u(i-1) of i = 2 is u(N+1)
+  const int xo = (i == 0 ? N : i) - 1;    // u(i-1) of i = 2 is u(N+1)
   v.x1 = a.U[L.u + i];
   v.x0 = a.U[L.u + xo];
   if (L.v >= 0) v.y1 = a.V[L.v + i];
@@ -150,24 +157,24 @@ __device__ __forceinline__ double line_value(const LineInfo& L, const LineLoads<
 // from the loads (8 points a thread, 96 loads in batches of 24) the kernel
 // waited for memory, 49 us against 46 at 192 x 128 x 192.
 // FP32: the FP64 values also to val [2*kLines][Nx], for the line sums.
-template <int SRC, typename T>
-__device__ __forceinline__ void xfwd_values(const XfwdArgs<T>& a, const LineInfo* L, typename cplx<T>::t* buf,
+template <int SRC, int NX, typename T>
+__device__ __forceinline__ void xfwd_values(const XfwdArgs<T>& a, const LineInfo* L, typename cplx<T>::t* buf, int RS,
                                             double* val, double& flux) {
   constexpr int kBatch = SRC == FROM_RESIDUAL ? 2 : 4;
-  const int N = a.d.Nx;
+  const int N = NX > 0 ? NX : a.d.Nx;
   T* out = reinterpret_cast<T*>(buf);
   for (int t = threadIdx.x; t < N * (2 * kLines / kBatch); t += blockDim.x) {
-    const int g = div_by(t, a.recN), i = t - g * N;
+    const int g = NX > 0 ? t / N : div_by(t, a.recN), i = t - g * N;
     const LineInfo* l = L + g * kBatch;
     LineLoads<SRC> v[kBatch];
 #pragma unroll
-    for (int u = 0; u < kBatch; ++u) v[u] = line_load<SRC>(a, l[u], i);
+    for (int u = 0; u < kBatch; ++u) v[u] = line_load<SRC>(a, l[u], N, i);
     const double rdx = SRC == FROM_RHS ? 0.0 : a.m.rdx[2 + i];
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
       const double x = line_value<SRC>(l[u], v[u], rdx, flux);
       const int rl = g * kBatch + u;
-      out[2 * ((rl >> 1) * a.rs + i) + (rl & 1)] = (T)x;
+      out[2 * ((rl >> 1) * RS + i) + (rl & 1)] = (T)x;
       if (sizeof(T) == 4) val[rl * N + i] = x;
     }
   }
@@ -176,17 +183,18 @@ __device__ __forceinline__ void xfwd_values(const XfwdArgs<T>& a, const LineInfo
 // last stage and split: the butterflies of wavenumbers k0 + s K and of their
 // mirror images N - k0 - s K = (K - k0) + (R-1-s) K, K = N/R
 template <int R, typename T>
-__device__ __forceinline__ void xfwd_last(const XfwdArgs<T>& a, const LineInfo* L, const typename cplx<T>::t* buf) {
+__device__ __forceinline__ void xfwd_last(const XfwdArgs<T>& a, const LineInfo* L, const typename cplx<T>::t* buf,
+                                          int N, int RS) {
   using C = typename cplx<T>::t;
-  const int N = a.d.Nx, K = N / R, slab = a.d.Ny * a.pz;
+  const int K = N / R, slab = a.d.Ny * a.pz;
   for (int t = threadIdx.x; t < kLines * (K / 2 + 1); t += blockDim.x) {
     const int l = t % kLines, k0 = t / kLines, kp = k0 == 0 ? 0 : K - k0;
     const LineInfo &La = L[2 * l], &Lb = L[2 * l + 1];
     if (La.u < 0) continue;
     const bool self = kp == k0;
     C v[R], w[R];
-    const C* pv = buf + l * a.rs + a.pos[k0];
-    const C* pw = buf + l * a.rs + a.pos[kp];
+    const C* pv = buf + l * RS + a.pos[k0];
+    const C* pw = buf + l * RS + a.pos[kp];
 #pragma unroll
     for (int s = 0; s < R; ++s) { v[s] = pv[s]; w[s] = pw[s]; }
     Dft<T, false, R>::run(v);
@@ -227,39 +235,46 @@ __device__ __forceinline__ void two_sum(double& hi, double& lo, double b, double
 // U - grad(phi), formed as the projection update forms it, so that field is
 // neither written nor read back (32 bytes a cell read in place of 56 for the
 // update and 24 for its divergence).
-template <int SRC, typename T>
+template <int SRC, typename T, int NX>
 __global__ void __launch_bounds__(kFwdThreads, 2) k_xfft_fwd(XfwdArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char xf_smem[];
   __shared__ LineInfo L[2 * kLines];
   C* buf = reinterpret_cast<C*>(xf_smem);
-  C* tw = buf + (size_t)kLines * a.rs;
-  double* val = reinterpret_cast<double*>(tw + a.d.Nx);
+  const int Nx = NX > 0 ? NX : a.d.Nx, RS = NX > 0 ? x_stride<T>(NX) : a.rs;
+  C* tw = buf + (size_t)kLines * RS;
+  double* val = reinterpret_cast<double*>(tw + Nx);
   const int tid = threadIdx.x, nt = blockDim.x;
   const int r0 = a.rbase + (int)blockIdx.x * 2 * kLines, rend = a.rbase + a.nlines;
   if (tid < 2 * kLines) line_info<SRC>(a.d, a.m, a.pz, r0 + tid, rend, L[tid]);
-  for (int t = tid; t < a.d.Nx; t += nt) tw[t] = a.tw[t];
+  for (int t = tid; t < Nx; t += nt) tw[t] = a.tw[t];
   __syncthreads();
   double flux = 0.0;
-  xfwd_values<SRC>(a, L, buf, val, flux);
+  xfwd_values<SRC, NX>(a, L, buf, RS, val, flux);
   __syncthreads();
   if (sizeof(T) == 4 && a.linesum) {   // FP64 line sums: one warp per line, a fixed shuffle tree
-    const int warp = tid >> 5, lane = tid & 31, N = a.d.Nx;
+    const int warp = tid >> 5, lane = tid & 31;
     for (int rl = warp; rl < 2 * kLines; rl += nt >> 5) {
       double sum = 0.0;
-      for (int q = lane; q < N; q += 32) sum += val[rl * N + q];
+      for (int q = lane; q < Nx; q += 32) sum += val[rl * Nx + q];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       if (lane == 0 && L[rl].u >= 0) a.linesum[r0 + rl] = sum;
     }
   }
-  fft_rows_dif<T, kMaxR, kLines>(buf, kLines, a.rs, tw, a.P, 0, a.P.npass - 1);
-  switch (a.P.radix[a.P.npass - 1]) {
-    case 8: xfwd_last<8>(a, L, buf); break;
-    case 6: xfwd_last<6>(a, L, buf); break;
-    case 4: xfwd_last<4>(a, L, buf); break;
-    case 3: xfwd_last<3>(a, L, buf); break;
-    default: xfwd_last<2>(a, L, buf); break;
+  if constexpr (NX > 0) {
+    constexpr int RL = plan_last_radix(NX, kMaxR);
+    fft_fixed_dif<T, NX, kMaxR, NX, RL>(buf, kLines, kRecLines, RS, tw);
+    xfwd_last<RL>(a, L, buf, NX, RS);
+  } else {
+    fft_rows_dif<T, kMaxR, kLines>(buf, kLines, RS, tw, a.P, 0, a.P.npass - 1);
+    switch (a.P.radix[a.P.npass - 1]) {
+      case 8: xfwd_last<8>(a, L, buf, Nx, RS); break;
+      case 6: xfwd_last<6>(a, L, buf, Nx, RS); break;
+      case 4: xfwd_last<4>(a, L, buf, Nx, RS); break;
+      case 3: xfwd_last<3>(a, L, buf, Nx, RS); break;
+      default: xfwd_last<2>(a, L, buf, Nx, RS); break;
+    }
   }
   if (SRC == FROM_DIV_FLUX) {
     // block partial by a fixed tree (any thread count up to kFwdThreads); the
@@ -333,9 +348,10 @@ struct OutLine {
 };
 
 template <int R, typename T>
-__device__ __forceinline__ void xinv_first(const XinvArgs<T>& a, const OutLine* L, typename cplx<T>::t* buf) {
+__device__ __forceinline__ void xinv_first(const XinvArgs<T>& a, const OutLine* L, typename cplx<T>::t* buf, int N,
+                                           int RS) {
   using C = typename cplx<T>::t;
-  const int N = a.d.Nx, K = N / R, slab = a.d.Ny * a.pz;
+  const int K = N / R, slab = a.d.Ny * a.pz;
   for (int t = threadIdx.x; t < kLines * (K / 2 + 1); t += blockDim.x) {
     const int l = t % kLines, k0 = t / kLines, kp = k0 == 0 ? 0 : K - k0;
     const OutLine &La = L[2 * l], &Lb = L[2 * l + 1];
@@ -359,12 +375,12 @@ __device__ __forceinline__ void xinv_first(const XinvArgs<T>& a, const OutLine* 
       v[s] = C{As.x - Bs.y, As.y + Bs.x};
       w[R - 1 - s] = C{As.x + Bs.y, Bs.x - As.y};
     }
-    C* pv = buf + l * a.rs + a.pos[k0];
+    C* pv = buf + l * RS + a.pos[k0];
     Dft<T, true, R>::run(v);
 #pragma unroll
     for (int s = 0; s < R; ++s) pv[s] = v[s];
     if (kp != k0) {
-      C* pw = buf + l * a.rs + a.pos[kp];
+      C* pw = buf + l * RS + a.pos[kp];
       Dft<T, true, R>::run(w);
 #pragma unroll
       for (int s = 0; s < R; ++s) pw[s] = w[s];
@@ -375,9 +391,8 @@ __device__ __forceinline__ void xinv_first(const XinvArgs<T>& a, const OutLine* 
 // phi at x index i of a line, with the copies of apply_periodic_xz_centers
 // (src/poisson.f90:106-125): x plane nxg-1 and z plane nzp+2 duplicate plane 2
 template <typename T>
-__device__ __forceinline__ void put_phi(const XinvArgs<T>& a, const OutLine& L, int i, double v) {
+__device__ __forceinline__ void put_phi(const XinvArgs<T>& a, const OutLine& L, int N, int i, double v) {
   if (L.o < 0) return;
-  const int N = a.d.Nx;
   if (a.phi00) v += L.p00;
   if (a.accumulate) v += a.rhs[L.o + i];
   auto put = [&](double* f) {
@@ -392,13 +407,14 @@ __device__ __forceinline__ void put_phi(const XinvArgs<T>& a, const OutLine& L, 
   if (a.phi1) put(a.phi1);
 }
 
-template <typename T>
+template <typename T, int NX>
 __global__ void __launch_bounds__(kInvThreads, 4) k_xfft_inv(XinvArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char xi_smem[];
   __shared__ OutLine L[2 * kLines];
   C* buf = reinterpret_cast<C*>(xi_smem);
-  C* tw = buf + (size_t)kLines * a.rs;
+  const int Nx = NX > 0 ? NX : a.d.Nx, RS = NX > 0 ? x_stride<T>(NX) : a.rs;
+  C* tw = buf + (size_t)kLines * RS;
   const Dims& d = a.d;
   const int tid = threadIdx.x;
   if (tid < 2 * kLines) {
@@ -413,32 +429,32 @@ __global__ void __launch_bounds__(kInvThreads, 4) k_xfft_inv(XinvArgs<T> a) {
     }
     L[tid] = o;
   }
-  for (int t = tid; t < d.Nx; t += blockDim.x) tw[t] = a.tw[t];
+  for (int t = tid; t < Nx; t += blockDim.x) tw[t] = a.tw[t];
   __syncthreads();
-  switch (a.P.radix[a.P.npass - 1]) {
-    case 8: xinv_first<8>(a, L, buf); break;
-    case 6: xinv_first<6>(a, L, buf); break;
-    case 4: xinv_first<4>(a, L, buf); break;
-    case 3: xinv_first<3>(a, L, buf); break;
-    default: xinv_first<2>(a, L, buf); break;
-  }
-  __syncthreads();
-  fft_rows_dit_inv<T, kMaxR, kLines>(buf, kLines, a.rs, tw, a.P, 1, a.P.npass - 1);
   const double rsd = a.inv_scale;
-  ct_edge_any<T, true>(
-      kLines, a.tw1, a.P, [&](int l, int e) { return buf[l * a.rs + e]; },
-      [&](int l, int e, C v) {
-        put_phi(a, L[2 * l], e, (double)v.x * rsd);
-        put_phi(a, L[2 * l + 1], e, (double)v.y * rsd);
-      });
-}
-
-// shared-memory row stride: FP64 1 mod 8, FP32 odd (conflict-free across rows)
-template <typename T>
-int x_rs(int Nx) {
-  int rs = Nx;
-  while (rs % (sizeof(T) == 8 ? 8 : 2) != 1) ++rs;
-  return rs;
+  auto in = [&](int l, int e) { return buf[l * RS + e]; };
+  auto out = [&](int l, int e, C v) {
+    put_phi(a, L[2 * l], Nx, e, (double)v.x * rsd);
+    put_phi(a, L[2 * l + 1], Nx, e, (double)v.y * rsd);
+  };
+  if constexpr (NX > 0) {
+    constexpr int R0 = plan_radix(NX, kMaxR), RL = plan_last_radix(NX, kMaxR);
+    xinv_first<RL>(a, L, buf, NX, RS);
+    __syncthreads();
+    fft_fixed_dit_inv<T, NX, kMaxR, NX / R0, RL>(buf, kLines, kRecLines, RS, tw);
+    ct_edge<T, true, R0>(kLines, NX, a.tw1, a.P.rec[0], in, out);
+  } else {
+    switch (a.P.radix[a.P.npass - 1]) {
+      case 8: xinv_first<8>(a, L, buf, Nx, RS); break;
+      case 6: xinv_first<6>(a, L, buf, Nx, RS); break;
+      case 4: xinv_first<4>(a, L, buf, Nx, RS); break;
+      case 3: xinv_first<3>(a, L, buf, Nx, RS); break;
+      default: xinv_first<2>(a, L, buf, Nx, RS); break;
+    }
+    __syncthreads();
+    fft_rows_dit_inv<T, kMaxR, kLines>(buf, kLines, RS, tw, a.P, 1, a.P.npass - 1);
+    ct_edge_any<T, true>(kLines, a.tw1, a.P, in, out);
+  }
 }
 
 // at least two stages (a first and a last)
@@ -465,8 +481,33 @@ int x_threads(const FftPasses& P, int most) {
 
 template <typename T>
 size_t x_smem(const FftPasses& P, bool fwd) {
-  return sizeof(typename cplx<T>::t) * ((size_t)kLines * x_rs<T>(P.n) + P.n) +
+  return sizeof(typename cplx<T>::t) * ((size_t)kLines * x_stride<T>(P.n) + P.n) +
          (fwd && sizeof(T) == 4 ? sizeof(double) * 2 * kLines * P.n : 0);
+}
+
+// The kernels for lines of Nx points: FP64 lines of 32 to 512 points have the
+// length compiled in (inverse at 384 x 256 x 384 188 -> 170 us, forward 288 ->
+// 281; time step 4969 -> 4874 us there, 661 -> 653 at 192 x 128 x 192, 368 ->
+// 358 at 162 x 113 x 108, 83 -> 82 at 32 x 64 x 32).  FP32, and right-hand sides from memory (the Poisson
+// solve called by itself), take the run-time stages.
+template <typename T>
+struct XKernels {
+  void (*div)(XfwdArgs<T>);
+  void (*flux)(XfwdArgs<T>);
+  void (*inv)(XinvArgs<T>);
+};
+template <typename T, int... NX>
+XKernels<T> x_pick(int Nx) {
+  XKernels<T> k{k_xfft_fwd<FROM_DIV, T, 0>, k_xfft_fwd<FROM_DIV_FLUX, T, 0>, k_xfft_inv<T, 0>};
+  ((Nx == NX ? (void)(k = {k_xfft_fwd<FROM_DIV, T, NX>, k_xfft_fwd<FROM_DIV_FLUX, T, NX>, k_xfft_inv<T, NX>})
+             : (void)0), ...);
+  return k;
+}
+template <typename T>
+XKernels<T> x_kernels(int Nx) {
+  if constexpr (sizeof(T) == 8)
+    return x_pick<T, 32, 48, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 486, 512>(Nx);
+  else return x_pick<T>(Nx);
 }
 
 template <typename T>
@@ -496,7 +537,7 @@ int launch_xfft_fwd(Handle* h, bool from_div, const double* U, const double* V, 
   XfwdArgs<T> a{};
   a.d = d; a.m = h->m; a.U = U; a.V = V; a.W = W; a.rhs = rhs;
   a.spec = t.spec; a.tw = t.tw; a.linesum = linesum; a.pos = h->sp.posx;
-  a.P = x_plan(d.Nx); a.pz = t.pz; a.rs = x_rs<T>(d.Nx);
+  a.P = x_plan(d.Nx); a.pz = t.pz; a.rs = x_stride<T>(d.Nx);
   a.recN = (unsigned)(((1ull << 32) + d.Nx - 1) / d.Nx);
   a.rbase = blo * d.Nz; a.nlines = (bhi - blo + 1) * d.Nz;
   const unsigned nb = (unsigned)((a.nlines + 2 * kLines - 1) / (2 * kLines));
@@ -509,13 +550,13 @@ int launch_xfft_fwd(Handle* h, bool from_div, const double* U, const double* V, 
     }
     a.flux_part = h->flux_part; a.scw = h->sc;
     a.q0 = h->Qflow_x_0; a.norm = h->norm_u; a.dt = flux_dt;
-    k_xfft_fwd<FROM_DIV_FLUX, T><<<nb, nt, smem, h->stream>>>(a);
+    x_kernels<T>(d.Nx).flux<<<nb, nt, smem, h->stream>>>(a);
   } else if (from_div && rhs) {
-    if constexpr (sizeof(T) == 4) k_xfft_fwd<FROM_RESIDUAL, T><<<nb, nt, smem, h->stream>>>(a);
+    if constexpr (sizeof(T) == 4) k_xfft_fwd<FROM_RESIDUAL, T, 0><<<nb, nt, smem, h->stream>>>(a);
   } else if (from_div) {
-    k_xfft_fwd<FROM_DIV, T><<<nb, nt, smem, h->stream>>>(a);
+    x_kernels<T>(d.Nx).div<<<nb, nt, smem, h->stream>>>(a);
   } else {
-    k_xfft_fwd<FROM_RHS, T><<<nb, nt, smem, h->stream>>>(a);
+    k_xfft_fwd<FROM_RHS, T, 0><<<nb, nt, smem, h->stream>>>(a);
   }
   C3D_LAUNCH_CHECK(h);
   return 0;
@@ -533,11 +574,11 @@ int launch_xfft_inv(Handle* h, double* out, double* phi1, const double* phi00, i
   XinvArgs<T> a{};
   a.d = d; a.spec = t.spec; a.tw = t.tw; a.tw1 = t.tw1; a.rhs = out; a.phi1 = phi1; a.phi00 = phi00;
   a.accumulate = accumulate; a.pos = h->sp.posx;
-  a.P = x_plan(d.Nx); a.pz = t.pz; a.rs = x_rs<T>(d.Nx);
+  a.P = x_plan(d.Nx); a.pz = t.pz; a.rs = x_stride<T>(d.Nx);
   a.rbase = blo * d.Nz; a.nlines = (bhi - blo + 1) * d.Nz;
   a.inv_scale = 1.0 / ((double)d.Nx * (double)d.Nz);
   const unsigned nb = (unsigned)((a.nlines + 2 * kLines - 1) / (2 * kLines));
-  k_xfft_inv<T><<<nb, x_threads(a.P, kInvThreads), x_smem<T>(a.P, false), h->stream>>>(a);
+  x_kernels<T>(d.Nx).inv<<<nb, x_threads(a.P, kInvThreads), x_smem<T>(a.P, false), h->stream>>>(a);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
@@ -571,11 +612,12 @@ int xfft_setup(Handle* h) {
   FftPasses longest = x_plan(512);
   const int smem = (int)x_smem<T>(longest, true);
   auto limit = [&](auto* k) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); };
-  C3D_CUDA_TRY(h, limit(k_xfft_fwd<FROM_RHS, T>));
-  C3D_CUDA_TRY(h, limit(k_xfft_fwd<FROM_DIV, T>));
-  C3D_CUDA_TRY(h, limit(k_xfft_fwd<FROM_DIV_FLUX, T>));
-  if constexpr (sizeof(T) == 4) C3D_CUDA_TRY(h, limit(k_xfft_fwd<FROM_RESIDUAL, T>));
-  C3D_CUDA_TRY(h, limit(k_xfft_inv<T>));
+  C3D_CUDA_TRY(h, limit(k_xfft_fwd<FROM_RHS, T, 0>));
+  const XKernels<T> k = x_kernels<T>(d.Nx);
+  C3D_CUDA_TRY(h, limit(k.div));
+  C3D_CUDA_TRY(h, limit(k.flux));
+  if constexpr (sizeof(T) == 4) C3D_CUDA_TRY(h, limit(k_xfft_fwd<FROM_RESIDUAL, T, 0>));
+  C3D_CUDA_TRY(h, limit(k.inv));
   return 0;
 }
 template int xfft_setup<double>(Handle*);

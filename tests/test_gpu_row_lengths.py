@@ -1,7 +1,9 @@
-"""The y-z solves with the row length compiled in, against the oracle's Poisson
-solve, 1e-11 relative max-norm: every such length, in clusters (few rows of j
-and many: columns per thread differ) and by blocks, with a part-filled last
-block."""
+"""Kernels with the row length compiled in, at every such length, 1e-11 relative
+max-norm: the y-z solves against the oracle's Poisson solve, in clusters (few
+rows of j and many: columns per thread differ) and by blocks, with a
+part-filled last block; the x transforms against the oracle's time step (its
+divergence with and without the bulk flux), with a part-filled last group of
+lines."""
 import numpy as np
 import pytest
 
@@ -32,3 +34,24 @@ def test_poisson_solve(nz, rows):
         got = ch.download("RHS_P")
     ref = co.solve_poisson_equation(g, rhs)[2:, 2:, 2:]
     assert np.abs(got - ref)[:, :, :-1].max() < 1e-11 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nx", (32, 48, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 486, 512))
+def test_time_step(nx):
+    import channel3d_parallel_b200 as c3d
+    p = co.channel_params(nx + 2, 8, 8, 0.06 * nx, 0.3, 1.0 / 5600.0)
+    g = co.Grid(p)
+    st = co.seeded_initial_state(g, p["dpdx"])
+    with c3d.Channel(nx_global=nx + 2, ny_global=8, nz_global=8, Lxp=p["lxp"], Lzp=p["lzp"], nu=p["nu"], CFL=-1e-3,
+                     x_mass_cte=1, grid_type=1, alpha_stretch=2.0, dPdx=p["dpdx"]) as ch:
+        ch.set_grid(g.x[1:], g.y[1:], g.z[1:])
+        for n in ("U", "V", "W"):
+            ch.upload(n, getattr(st, n)[1:, 1:, 1:])
+        ch.set_scalars(dPdx=st.dPdx, t=0.0, Qflow_x_0=st.Qflow_x_0)
+        ch.compute_dt()
+        ch.compute_time_step_RK3(2)
+        for _ in range(2):
+            co.compute_time_step_RK3(g, st, 1e-3)
+        for n in ("U", "V", "W"):
+            ref = getattr(st, n)[1:, 1:, 1:]
+            assert np.abs(ch.download(n) - ref).max() < 1e-11 * np.abs(ref).max(), n
