@@ -10,6 +10,11 @@ namespace c3d {
 
 struct BandState;   // banded z-Fourier preconditioner (k_ib_band.cu)
 
+// grid point with spread entries: place in the field, first entry, count
+struct SpPoint {
+  int p, o, n;
+};
+
 struct IbState {
   std::string kind;
   bool moving = false;
@@ -41,6 +46,8 @@ struct IbState {
   int* sp_off[3] = {nullptr, nullptr, nullptr};
   uint32_t* sp_ent[3] = {nullptr, nullptr, nullptr};
   double* sp_w[3] = {nullptr, nullptr, nullptr};
+  SpPoint* sp_pts[3] = {nullptr, nullptr, nullptr};   // the points with entries
+  int* sp_npts = nullptr;            // how many, per component
   int* sp_sums = nullptr;            // prefix-sum chunk totals
   double* amp = nullptr;             // [3][nb] spread amplitudes
   // fields

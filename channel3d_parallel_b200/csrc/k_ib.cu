@@ -497,6 +497,18 @@ __global__ void k_ib_weights(IbGeomArgs a) {
       a.off[tslot(a.nb, t, 1, q, l)] = yg - yb;
       a.off[tslot(a.nb, t, 2, q, l)] = zg - zb;
     }
+    // The support is four cells, so one of a marker's end points lies at or
+    // past its edge, where the function is zero: the 1e-17 that rounding leaves
+    // of it at a marker on a grid line is taken out, and with it the fifth
+    // entry of the sums below.
+    for (int ax = 0; ax < 3; ++ax) {
+      const int64_t e0 = tslot(a.nb, t, ax, 0, l), e4 = tslot(a.nb, t, ax, 4, l);
+      const double w0 = a.w1[e0], w4 = a.w1[e4], dr = ax == 0 ? a.dx : (ax == 1 ? a.dymin : a.dz);
+      if (w0 != 0.0 && w4 != 0.0) {
+        const bool first = fabs(w0) < fabs(w4);
+        if (fabs(first ? w0 : w4) * dr < 1e-13) a.w1[first ? e0 : e4] = 0.0;
+      }
+    }
   }
 }
 
@@ -541,6 +553,7 @@ struct GatherArgs {
   Dims d;
   GComp comp[4];      // blockIdx.y picks the component
   int ncomp;
+  int lat, tw, tx;    // markers per lattice row, markers of a tile along it, tiles along it
   double* out;
 };
 
@@ -552,60 +565,83 @@ __device__ __forceinline__ int64_t lin(int n1, int n2, int i, int j, int k, int 
 // Gather of grid values to the markers, E (src/immersed_boundary_operators.f90
 // regT) and E1n (regT_1n, weights times the stencil point's offset along the
 // normal), with the field box of a tile of markers staged in shared memory: a
-// CTA takes kTileMarkers consecutive markers of one component (one thread
-// each), finds the box of grid points their stencils touch (periodic x and z
-// indices unwrapped around the tile's first marker), copies that box from the
-// field once (consecutive threads along x, eight loads in flight) and gathers
+// CTA takes kTileMarkers markers of one component (one thread each), a patch of
+// the marker lattice, finds the box of grid points their stencils touch
+// (periodic x and z indices unwrapped around the tile's first marker), copies
+// that box from the field by cp.async, all of it in flight at once, and gathers
 // from shared memory.  Per stencil row (qj, qk) the thread forms the row sums
 // s0 = sum_qi wx v and, for E1n, s1 = sum_qi wx ox v, and adds
 // scale wy wz (s1 + (oy + oz) s0) -- the regT / regT_1n sums
 // (src/immersed_boundary_operators.f90) regrouped by rows.  A stencil point of
 // zero weight reads a point inside the box and adds an exact zero.  A tile
 // whose box does not fit gathers from the field directly.
+//
+// Bound by latency.  Tiles of 64 markers in a row, with a thread a column of
+// the box and eight loads in flight, took 34 us for four components of 36,864
+// markers on a wavy wall and 96 us for 51,200 on two cylinders, where a row of
+// markers goes round both and tiles that held some of each had no box; patches
+// of 16 x 4 (boxes a third the size) by cp.async, and the four points of an axis
+// that can have a weight in place of five, take 18 and 41 (all with cold caches).
 constexpr int kTileMarkers = 64;
-constexpr int kTileBox = 3072;     // doubles of shared memory for the box (24 KB)
+constexpr int kTileBox = 2048;     // doubles of shared memory for the box (16 KB)
+constexpr int kTileRows = 512;     // and rows of it
 // Components of both variants may share one launch (the Schur operator's
 // E1n of phi beside the three E components); each CTA runs one variant.
 template <bool E1N>
 __device__ __forceinline__ void gather_tile(const GatherArgs& a, const GComp& cp, int c, double* box,
-                                            int* s_ref, int* s_lo, int* s_hi) {
+                                            int* s_row, int* s_ref, int* s_lo, int* s_hi) {
   const int nb = a.T.nb;
   const int tid = threadIdx.x;
-  const int l = blockIdx.x * kTileMarkers + tid;
-  const bool valid = l < nb;
+  // the patch: tw markers along the lattice rows, kTileMarkers / tw rows
+  const int tz = blockIdx.x / a.tx, x0 = (blockIdx.x - tz * a.tx) * a.tw, z0 = tz * (kTileMarkers / a.tw);
+  const int dz_ = tid / a.tw, xl = x0 + tid - dz_ * a.tw;
+  const int l = xl + a.lat * (z0 + dz_);
+  const bool valid = xl < a.lat && l < nb;
   const int t = cp.type;
   const OpTables& T = a.T;
   const GField& g = cp.f;
   const int px = a.d.Nx, pz = a.d.Nz;        // index periods of x and z (indices 2 .. N+1)
-  if (tid == 0) {
-    const int l0 = blockIdx.x * kTileMarkers;
-    s_ref[0] = T.idx[tslot(nb, t, 0, 2, l0)];
-    s_ref[1] = T.idx[tslot(nb, t, 2, 2, l0)];
+  // the four points of each axis that can have a weight: 0..3, or 1..4 when
+  // point 0 has none; a grid where five do (spacing below the widths of the
+  // delta function) is summed from the tables
+  int ix[4], iy[4], iz[4], sx = 0, sy = 0, sz = 0;
+  double wx[4], wy[4], wz[4];
+  bool five = false;
+  auto axis = [&](int ax, int (&i4)[4], double (&w4)[4], int& sh) {
+    int i5[5] = {0, 0, 0, 0, 0};
+    double w5[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int a3 = 0; a3 < 3; ++a3) { s_lo[a3] = INT_MAX; s_hi[a3] = INT_MIN; }
-  }
+    for (int q = 0; q < 5; ++q)
+      if (valid) {
+        i5[q] = T.idx[tslot(nb, t, ax, q, l)];
+        w5[q] = T.w1[tslot(nb, t, ax, q, l)];
+      }
+    sh = w5[0] == 0.0 ? 1 : 0;
+    five = five || (w5[0] != 0.0 && w5[4] != 0.0);
+    if (tid == 0) s_ref[ax] = i5[2];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      i4[q] = sh ? i5[q + 1] : i5[q];
+      w4[q] = sh ? w5[q + 1] : w5[q];
+    }
+  };
+  axis(0, ix, wx, sx);
+  axis(1, iy, wy, sy);
+  axis(2, iz, wz, sz);
+  if (tid < 3) { s_lo[tid] = INT_MAX; s_hi[tid] = INT_MIN; }
   __syncthreads();
-  const int rx = s_ref[0], rz = s_ref[1];
+  // periodic indices unwrapped around the tile's first marker, and the box
+  const int rx = s_ref[0], rz = s_ref[2];
   auto unwrap = [](int i, int r, int p) {
     if (i - r > p / 2) return i - p;
     if (r - i > p / 2) return i + p;
     return i;
   };
-  int ix[5], iy[5], iz[5];
-  double wx[5], wy[5], wz[5];
   int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    ix[q] = iy[q] = iz[q] = 0;
-    wx[q] = wy[q] = wz[q] = 0.0;
-    if (valid) {
-      ix[q] = unwrap(T.idx[tslot(nb, t, 0, q, l)], rx, px);
-      iy[q] = T.idx[tslot(nb, t, 1, q, l)];
-      iz[q] = unwrap(T.idx[tslot(nb, t, 2, q, l)], rz, pz);
-      wx[q] = T.w1[tslot(nb, t, 0, q, l)];
-      wy[q] = T.w1[tslot(nb, t, 1, q, l)];
-      wz[q] = T.w1[tslot(nb, t, 2, q, l)];
-    }
+  for (int q = 0; q < 4; ++q) {
+    ix[q] = unwrap(ix[q], rx, px);
+    iz[q] = unwrap(iz[q], rz, pz);
     if (wx[q] != 0.0) { lo[0] = min(lo[0], ix[q]); hi[0] = max(hi[0], ix[q]); }
     if (wy[q] != 0.0) { lo[1] = min(lo[1], iy[q]); hi[1] = max(hi[1], iy[q]); }
     if (wz[q] != 0.0) { lo[2] = min(lo[2], iz[q]); hi[2] = max(hi[2], iz[q]); }
@@ -619,80 +655,54 @@ __device__ __forceinline__ void gather_tile(const GatherArgs& a, const GComp& cp
     }
     if ((tid & 31) == 0) { atomicMin(&s_lo[a3], lo[a3]); atomicMax(&s_hi[a3], hi[a3]); }
   }
-  __syncthreads();
+  const bool tables = __syncthreads_or(five);
   const int bx0 = s_lo[0], by0 = s_lo[1], bz0 = s_lo[2];
   const bool any = s_hi[0] >= bx0 && s_hi[1] >= by0 && s_hi[2] >= bz0;
   const int bx = any ? s_hi[0] - bx0 + 1 : 0, by = any ? s_hi[1] - by0 + 1 : 0,
             bz = any ? s_hi[2] - bz0 + 1 : 0;
-  const bool staged = any && bx <= 2 * kTileMarkers && (int64_t)bx * by * bz <= kTileBox;
-  // periodic index back into 2 .. p+1 (one period away after the unwrap)
-  auto wrap = [](int i, int p) {
-    i = i < 2 ? i + p : (i > p + 1 ? i - p : i);
-    if (i < 2 || i > p + 1) i = 2 + ((i - 2) % p + p) % p;
-    return i;
-  };
-  auto field = [&](int i, int j, int k) { return g.F[lin(g.n1, g.n2, wrap(i, px), j, wrap(k, pz), g.rhsp)]; };
+  const bool staged = any && !tables && by * bz <= kTileRows && (int64_t)bx * by * bz <= kTileBox;
+  // periodic index back into 2 .. p+1 (at most half a period outside it)
+  auto wrap = [](int i, int p) { return i < 2 ? i + p : (i > p + 1 ? i - p : i); };
   if (staged) {
-    // the box row by row (j fastest, then k), four rows per round with two
-    // x points per thread and row: eight loads in flight
-    const int nrow = by * bz;
-    const int xa = wrap(bx0 + tid, px), xb = wrap(bx0 + tid + kTileMarkers, px);
-    const bool ha = tid < bx, hb = tid + kTileMarkers < bx;
-    int jj = 0, kk = 0;
-    for (int r0 = 0; r0 < nrow; r0 += 4) {
-      double ta[4], tb[4];
-      int cj = jj, ck = kk;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        ta[u] = tb[u] = 0.0;
-        if (r0 + u < nrow) {
-          const int j = by0 + cj, k = wrap(bz0 + ck, pz);
-          if (ha) ta[u] = g.F[lin(g.n1, g.n2, xa, j, k, g.rhsp)];
-          if (hb) tb[u] = g.F[lin(g.n1, g.n2, xb, j, k, g.rhsp)];
-        }
-        if (++cj == by) { cj = 0; ++ck; }
-      }
-      jj = cj; kk = ck;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (r0 + u < nrow) {
-          if (ha) box[tid + bx * (r0 + u)] = ta[u];
-          if (hb) box[tid + kTileMarkers + bx * (r0 + u)] = tb[u];
-        }
-      }
+    // places of the box's rows (at x = 0), then its points
+    for (int r = tid; r < by * bz; r += kTileMarkers) {
+      const int k = r / by;
+      s_row[r] = (int)lin(g.n1, g.n2, 0, by0 + r - k * by, wrap(bz0 + k, pz), g.rhsp);
     }
+    __syncthreads();
+    const unsigned rcx = 0xffffffffu / (unsigned)bx + 1u;       // ceil(2^32 / bx)
+    const unsigned sb = (unsigned)__cvta_generic_to_shared(box);
+    for (int e = tid; e < bx * by * bz; e += kTileMarkers) {
+      const int r = bx > 1 ? (int)__umulhi((unsigned)e, rcx) : e;
+      const double* src = g.F + (s_row[r] + wrap(bx0 + e - r * bx, px));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sb + 8u * (unsigned)e), "l"(src));
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::);
   }
   __syncthreads();
   if (!valid) return;
-  double ox[5], oy[5], oz[5];
-#pragma unroll
-  for (int q = 0; q < 5; ++q) ox[q] = oy[q] = oz[q] = 0.0;
-  if (E1N) {
-    const double nx_ = T.nrm[l], ny_ = T.nrm[nb + l], nz_ = T.nrm[2 * nb + l];
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      ox[q] = nx_ * T.off[tslot(nb, t, 0, q, l)];
-      oy[q] = ny_ * T.off[tslot(nb, t, 1, q, l)];
-      oz[q] = nz_ * T.off[tslot(nb, t, 2, q, l)];
-    }
-  }
+  const double nx_ = E1N ? T.nrm[l] : 0.0, ny_ = E1N ? T.nrm[nb + l] : 0.0, nz_ = E1N ? T.nrm[2 * nb + l] : 0.0;
   double acc = 0.0;
   if (staged) {
-    int offx[5], offy[5], offz[5];
+    double ox[4], oy[4], oz[4];
+    int offx[4], offy[4], offz[4];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {        // zero-weight points read the box's first point
+    for (int q = 0; q < 4; ++q) {        // zero-weight points read the box's first point
+      ox[q] = E1N ? nx_ * T.off[tslot(nb, t, 0, q + sx, l)] : 0.0;
+      oy[q] = E1N ? ny_ * T.off[tslot(nb, t, 1, q + sy, l)] : 0.0;
+      oz[q] = E1N ? nz_ * T.off[tslot(nb, t, 2, q + sz, l)] : 0.0;
       offx[q] = wx[q] != 0.0 ? ix[q] - bx0 : 0;
       offy[q] = wy[q] != 0.0 ? bx * (iy[q] - by0) : 0;
       offz[q] = wz[q] != 0.0 ? bx * by * (iz[q] - bz0) : 0;
     }
 #pragma unroll
-    for (int qk = 0; qk < 5; ++qk) {
+    for (int qk = 0; qk < 4; ++qk) {
 #pragma unroll
-      for (int qj = 0; qj < 5; ++qj) {
+      for (int qj = 0; qj < 4; ++qj) {
         const double* row = box + offy[qj] + offz[qk];
         double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-        for (int qi = 0; qi < 5; ++qi) {
+        for (int qi = 0; qi < 4; ++qi) {
           const double wv = wx[qi] * row[offx[qi]];
           s0 += wv;
           if (E1N) s1 = fma(wv, ox[qi], s1);
@@ -704,22 +714,19 @@ __device__ __forceinline__ void gather_tile(const GatherArgs& a, const GComp& cp
   } else {
 #pragma unroll 1
     for (int r = 0; r < 25; ++r) {
-      const int qj = r % 5, qk = r / 5;
-      double wyq = 0.0, wzq = 0.0, oyz = 0.0;
-      int jy = 0, kz = 0;
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        if (q == qj) { wyq = wy[q]; jy = iy[q]; oyz += oy[q]; }
-        if (q == qk) { wzq = wz[q]; kz = iz[q]; oyz += oz[q]; }
-      }
+      const int qk = r / 5, qj = r - 5 * qk;
+      const double wyq = T.w1[tslot(nb, t, 1, qj, l)], wzq = T.w1[tslot(nb, t, 2, qk, l)];
       if (wyq == 0.0 || wzq == 0.0) continue;
+      const int64_t row = lin(g.n1, g.n2, 0, T.idx[tslot(nb, t, 1, qj, l)], T.idx[tslot(nb, t, 2, qk, l)], g.rhsp);
+      const double oyz = E1N ? ny_ * T.off[tslot(nb, t, 1, qj, l)] + nz_ * T.off[tslot(nb, t, 2, qk, l)] : 0.0;
       double s0 = 0.0, s1 = 0.0;
 #pragma unroll
       for (int qi = 0; qi < 5; ++qi) {
-        if (wx[qi] == 0.0) continue;
-        const double wv = wx[qi] * field(ix[qi], jy, kz);
+        const double wq = T.w1[tslot(nb, t, 0, qi, l)];
+        if (wq == 0.0) continue;
+        const double wv = wq * g.F[row + T.idx[tslot(nb, t, 0, qi, l)]];
         s0 += wv;
-        if (E1N) s1 = fma(wv, ox[qi], s1);
+        if (E1N) s1 = fma(wv, nx_ * T.off[tslot(nb, t, 0, qi, l)], s1);
       }
       acc = fma(T.scale * wyq * wzq, E1N ? fma(oyz, s0, s1) : s0, acc);
     }
@@ -733,15 +740,20 @@ __device__ __forceinline__ void gather_tile(const GatherArgs& a, const GComp& cp
 
 __global__ void __launch_bounds__(kTileMarkers) k_ib_gather_tile(GatherArgs a) {
   __shared__ double box[kTileBox];
-  __shared__ int s_ref[2], s_lo[3], s_hi[3];
+  __shared__ int s_row[kTileRows], s_ref[3], s_lo[3], s_hi[3];
   const int c = blockIdx.y;
   const GComp& cp = a.comp[c];
-  if (cp.mode == G_E1N) gather_tile<true>(a, cp, c, box, s_ref, s_lo, s_hi);
-  else gather_tile<false>(a, cp, c, box, s_ref, s_lo, s_hi);
+  if (cp.mode == G_E1N) gather_tile<true>(a, cp, c, box, s_row, s_ref, s_lo, s_hi);
+  else gather_tile<false>(a, cp, c, box, s_row, s_ref, s_lo, s_hi);
 }
 
-static void launch_gather_tile(const GatherArgs& a, cudaStream_t st) {
-  const dim3 grid((a.T.nb + kTileMarkers - 1) / kTileMarkers, a.ncomp);
+static void launch_gather_tile(GatherArgs& a, int lat, cudaStream_t st) {
+  a.lat = lat > 0 ? lat : a.T.nb;
+  const int rows = (a.T.nb + a.lat - 1) / a.lat;
+  a.tw = rows >= 4 ? 16 : kTileMarkers;
+  a.tx = (a.lat + a.tw - 1) / a.tw;
+  const int th = kTileMarkers / a.tw;
+  const dim3 grid(a.tx * ((rows + th - 1) / th), a.ncomp);
   k_ib_gather_tile<<<grid, kTileMarkers, 0, st>>>(a);
 }
 
@@ -800,14 +812,22 @@ __global__ void k_sp_fill(OpTables T, int c, int n1, int n2, const int* __restri
 }
 
 // sort each point's entries (insertion sort: a point has at most a few
-// dozen) and attach the tensor weights
+// dozen), attach the tensor weights and list the points that have any
 __global__ void k_sp_sort(OpTables T, int c, int64_t npts, const int* __restrict__ cnt, const int* __restrict__ off,
-                          uint32_t* __restrict__ ent, double* __restrict__ w) {
+                          uint32_t* __restrict__ ent, double* __restrict__ w, SpPoint* __restrict__ pts,
+                          int* __restrict__ npt) {
   const int nb = T.nb;
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= npts) return;
-  const int n = cnt[p];
+  const int n = p < npts ? cnt[p] : 0;
+  // the point joins the list of those with entries (in any order: every point
+  // is summed by itself), one slot request a warp
+  const unsigned have = __ballot_sync(0xffffffffu, n > 0);
   if (n == 0) return;
+  const int lane = threadIdx.x & 31, lead = __ffs(have) - 1;
+  int slot = 0;
+  if (lane == lead) slot = atomicAdd(npt, __popc(have));
+  slot = __shfl_sync(have, slot, lead) + __popc(have & ((1u << lane) - 1u));
+  pts[slot] = SpPoint{(int)p, off[p], n};
   uint32_t* e = ent + off[p];
   constexpr int kSortLocal = 64;
   if (n <= kSortLocal) {
@@ -837,104 +857,98 @@ __global__ void k_sp_sort(OpTables T, int c, int64_t npts, const int* __restrict
   }
 }
 
-// per (component, marker) amplitude scale*factor*sb*f_c of the spread
+// per (component, marker) amplitude scale*factor*sb*f_c of the spread, and
+// zeros into the rows that it writes
+struct SpRows {
+  double* F;
+  int n1, n2, n3;     // extents
+  int jlo, jhi;       // Fortran rows
+};
 __global__ void k_sp_amp(OpTables T, int comp0, int ncomp, int mode, const double* __restrict__ f, double dtnu,
-                         double dt, double* __restrict__ amp) {
+                         double dt, double* __restrict__ amp, SpRows z0, SpRows z1, SpRows z2) {
   const int nb = T.nb;
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= nb * ncomp) return;
-  const int cc = gid / nb, l = gid - cc * nb;
-  const int c = comp0 + cc;
-  double fl;
-  if (mode == S_RAW) fl = f[l];
-  else if (mode == S_NORMAL) fl = T.nrm[c * nb + l];
-  else fl = dtnu * f[c * nb + l] - dt * f[3 * nb + l] * T.nrm[c * nb + l];
-  amp[c * nb + l] = T.scale * T.factor * T.sb[l] * fl;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int t = gid; t < nb * ncomp; t += step) {
+    const int cc = t / nb, l = t - cc * nb;
+    const int c = comp0 + cc;
+    double fl;
+    if (mode == S_RAW) fl = f[l];
+    else if (mode == S_NORMAL) fl = T.nrm[c * nb + l];
+    else fl = dtnu * f[c * nb + l] - dt * f[3 * nb + l] * T.nrm[c * nb + l];
+    amp[c * nb + l] = T.scale * T.factor * T.sb[l] * fl;
+  }
+  const int lane = threadIdx.x & 31, warps = step >> 5;
+  auto clear = [&](const SpRows& z) {          // a warp a row
+    const int nr = z.jhi - z.jlo + 1;
+    for (int r = gid >> 5; r < nr * z.n3; r += warps) {
+      const int k = r / nr, j = z.jlo - 1 + r - k * nr;
+      double* o = z.F + (int64_t)z.n1 * (j + (int64_t)z.n2 * k);
+      for (int t = lane; t < z.n1; t += 32) o[t] = 0.0;
+    }
+  };
+  clear(z0);
+  if (ncomp > 1) clear(z1);
+  if (ncomp > 2) clear(z2);
 }
 
 struct SpGather {
-  const int* cnt;
-  const int* off;
   const uint32_t* ent;
   const double* w;
+  const SpPoint* pts; // the points with entries
+  const int* npts;    // how many
   double* F;
-  int n1, n2, n3;
-  int jlo, jhi;       // Fortran rows written (every point of them)
 };
 
-// F(i, j, k) = sum over the point's entries of w * amp(marker), for the
-// rows jlo..jhi of up to three fields; points without entries get 0.
-// A warp takes 32 consecutive points, whose entries are one contiguous run
-// of the map: the run streams through shared memory in chunks (weights and
-// marker amplitudes loaded by consecutive lanes), and each lane then adds
-// its own point's terms in entry order.
-constexpr int kSpChunk = 128;
-__global__ void __launch_bounds__(256) k_sp_gather(SpGather g0, SpGather g1, SpGather g2, int ncomp,
+// F(p) = sum over the point's entries of w * amp(marker) at the points with
+// entries of up to three fields (the others were cleared).  kSpLanes lanes take
+// a point, so that its entries come in whole sectors, kSpBatch rounds in flight
+// at once; a lane adds its entries in order and the lanes' sums meet in a fixed
+// tree.
+//
+// Bound by the latency of entry -> amplitude.  Few of the points of the rows
+// that a body reaches have entries, and those have many (13 of 36,864 markers
+// on a wavy wall, 48 of 51,200 on two cylinders): with a lane a point over all
+// points, a warp waited for its fullest point, 39 and 110 us for three
+// components; points with entries alone, four lanes each, take 16 and 29 (cold
+// caches; eight lanes and the entries looked up by point: 31 and 46).
+constexpr int kSpLanes = 4, kSpBatch = 4;
+__global__ void __launch_bounds__(256) k_sp_gather(SpGather g0, SpGather g1, SpGather g2,
                                                    const double* __restrict__ amp, int nb) {
-  __shared__ double sw[8][kSpChunk], sa[8][kSpChunk];
-  if ((int)blockIdx.y >= ncomp) return;
   // field description of this component, picked member by member (a
   // reference to one of the parameters would copy them to local memory)
   const int by = blockIdx.y;
 #define SP_PICK(m) (by == 0 ? g0.m : (by == 1 ? g1.m : g2.m))
   SpGather g;
-  g.cnt = SP_PICK(cnt); g.off = SP_PICK(off); g.ent = SP_PICK(ent); g.w = SP_PICK(w); g.F = SP_PICK(F);
-  g.n1 = SP_PICK(n1); g.n2 = SP_PICK(n2); g.n3 = SP_PICK(n3); g.jlo = SP_PICK(jlo); g.jhi = SP_PICK(jhi);
+  g.ent = SP_PICK(ent); g.w = SP_PICK(w);
+  g.pts = SP_PICK(pts); g.npts = SP_PICK(npts); g.F = SP_PICK(F);
 #undef SP_PICK
-  const int nrow = g.jhi - g.jlo + 1;
-  const int64_t tot = (int64_t)g.n1 * nrow * g.n3;
-  const double* a = amp + (int64_t)blockIdx.y * nb;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* ws = sw[warp];
-  double* as = sa[warp];
-  for (int64_t t0 = (blockIdx.x * (int64_t)blockDim.x + warp * 32); t0 < tot;
-       t0 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t t = t0 + lane;
-    const bool valid = t < tot;
-    int64_t p = 0;
-    int n = 0, o = 0;
-    if (valid) {
-      const int i = (int)(t % g.n1);
-      const int64_t r = t / g.n1;
-      const int j = g.jlo + (int)(r % nrow);
-      const int k = (int)(r / nrow);
-      p = (int64_t)i + (int64_t)g.n1 * ((j - 1) + (int64_t)g.n2 * k);
-      n = g.cnt[p];
-      o = g.off[p];
-    }
-    // the warp's run of entries [lo, hi)
-    int lo = n ? o : INT_MAX, hi = n ? o + n : INT_MIN;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, s));
-      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, s));
-    }
+  const double* a = amp + (int64_t)by * nb;
+  const int np = *g.npts, sub = threadIdx.x % kSpLanes;
+  constexpr int kPer = 256 / kSpLanes;
+  int t = blockIdx.x * kPer + threadIdx.x / kSpLanes;
+  SpPoint nxt{0, 0, 0};
+  if (t < np) nxt = g.pts[t];
+  for (int t0 = blockIdx.x * kPer; t0 < np; t0 += gridDim.x * kPer, t += gridDim.x * kPer) {
+    const SpPoint q = nxt;
+    const int n = t < np ? q.n : 0, o = q.o;
+    if (t + (int)gridDim.x * kPer < np) nxt = g.pts[t + gridDim.x * kPer];
     double acc = 0.0;
-    for (int cb = lo; cb < hi; cb += kSpChunk) {
-      const int m = min(kSpChunk, hi - cb);
-      // all loads of the chunk in flight before the marker amplitudes they
-      // index, then the stores
-      double wv[kSpChunk / 32], av[kSpChunk / 32];
-      uint32_t ev[kSpChunk / 32];
+    for (int e0 = sub; e0 < n; e0 += kSpLanes * kSpBatch) {
+      double wv[kSpBatch];
+      uint32_t ev[kSpBatch];
 #pragma unroll
-      for (int u = 0; u < kSpChunk / 32; ++u) {
-        const int e = lane + 32 * u;
-        wv[u] = e < m ? g.w[cb + e] : 0.0;
-        ev[u] = e < m ? g.ent[cb + e] : 0u;
+      for (int u = 0; u < kSpBatch; ++u) {
+        const int e = e0 + kSpLanes * u;
+        wv[u] = e < n ? g.w[o + e] : 0.0;
+        ev[u] = e < n ? g.ent[o + e] : 0u;
       }
 #pragma unroll
-      for (int u = 0; u < kSpChunk / 32; ++u) av[u] = lane + 32 * u < m ? a[ev[u] >> 7] : 0.0;
-#pragma unroll
-      for (int u = 0; u < kSpChunk / 32; ++u) {
-        ws[lane + 32 * u] = wv[u];
-        as[lane + 32 * u] = av[u];
-      }
-      __syncwarp();
-      const int e1 = min(o + n, cb + m);
-      for (int e = max(o, cb); e < e1; ++e) acc += ws[e - cb] * as[e - cb];
-      __syncwarp();
+      for (int u = 0; u < kSpBatch; ++u)
+        if (e0 + kSpLanes * u < n) acc += wv[u] * a[ev[u] >> 7];
     }
-    if (valid) g.F[p] = acc;
+#pragma unroll
+    for (int s = kSpLanes / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (t < np && sub == 0) g.F[q.p] = acc;
   }
 }
 
@@ -1101,56 +1115,71 @@ __global__ void k_remove_mean(double* __restrict__ v, const int* __restrict__ bo
   v[l] = x;
 }
 
-// partial dot products: up to 2 pairs
+// BiCGSTAB scalars on the device: sc[0] rho_o, [1] alpha, [2] om, [3] rho_n,
+// [4] bta, [5] err
+enum BcgOp { BCG_RHO = 0, BCG_ALPHA = 1, BCG_OM = 2, BCG_ERR = 3 };
+
+// End of a reduction of 256-thread blocks: the block's two sums by a fixed
+// tree, and in the last block to finish (ticket) those of all blocks by
+// another, with the scalars that follow from them.  A kernel of one block for
+// the second tree took 3.5 us, four times an iteration.
+__device__ __forceinline__ void bcg_reduce(double s0, double s1, double* __restrict__ part,
+                                           unsigned* __restrict__ ticket, double* __restrict__ sc, int op) {
+  __shared__ double sa[256], sb_[256];
+  __shared__ bool last;
+  auto tree = [&](double v0, double v1) {
+    sa[threadIdx.x] = v0;
+    sb_[threadIdx.x] = v1;
+    __syncthreads();
+    for (int s = 128; s > 0; s >>= 1) {
+      if (threadIdx.x < s) { sa[threadIdx.x] += sa[threadIdx.x + s]; sb_[threadIdx.x] += sb_[threadIdx.x + s]; }
+      __syncthreads();
+    }
+  };
+  tree(s0, s1);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = sa[0];
+    part[2 * blockIdx.x + 1] = sb_[0];
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  s0 = s1 = 0.0;
+  for (int t = threadIdx.x; t < (int)gridDim.x; t += 256) {
+    s0 += __ldcg(part + 2 * t);
+    s1 += __ldcg(part + 2 * t + 1);
+  }
+  tree(s0, s1);
+  if (threadIdx.x == 0) {
+    const double d0 = sa[0], d1 = sb_[0];
+    if (op == BCG_RHO) {             // rho_n = <rhat, r>; bta; rho_o = rho_n
+      sc[3] = d0;
+      sc[4] = (d0 / sc[0]) * (sc[1] / sc[2]);
+      sc[0] = d0;
+    } else if (op == BCG_ALPHA) {    // alpha = rho_n / <rhat, nu>
+      sc[1] = sc[3] / d0;
+    } else if (op == BCG_OM) {       // om = <t, s>/<t, t>
+      sc[2] = d0 / d1;
+    } else {                         // err = <r, r>
+      sc[5] = d0;
+    }
+    *ticket = 0u;
+  }
+}
+
+// dot products <a, b> and, with c, <c, e>
 __global__ void __launch_bounds__(256) k_dot2(const double* __restrict__ a, const double* __restrict__ b,
                                              const double* __restrict__ c, const double* __restrict__ e,
-                                             int64_t n, double* __restrict__ part) {
+                                             int64_t n, double* __restrict__ part, unsigned* __restrict__ ticket,
+                                             double* __restrict__ sc, int op) {
   double s0 = 0.0, s1 = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     s0 += a[i] * b[i];
     if (c) s1 += c[i] * e[i];
   }
-  __shared__ double sa[256], sb_[256];
-  sa[threadIdx.x] = s0;
-  sb_[threadIdx.x] = s1;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) { sa[threadIdx.x] += sa[threadIdx.x + s]; sb_[threadIdx.x] += sb_[threadIdx.x + s]; }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { part[2 * blockIdx.x] = sa[0]; part[2 * blockIdx.x + 1] = sb_[0]; }
-}
-
-// BiCGSTAB scalars on the device: sc[0] rho_o, [1] alpha, [2] om, [3] rho_n,
-// [4] bta, [5] err, [6] dot1, [7] dot2
-__global__ void k_dot_final(const double* __restrict__ part, int np, double* sc, int slot0, int op) {
-  __shared__ double sa[256], sb_[256];
-  double s0 = 0.0, s1 = 0.0;
-  for (int t = threadIdx.x; t < np; t += blockDim.x) { s0 += part[2 * t]; s1 += part[2 * t + 1]; }
-  sa[threadIdx.x] = s0;
-  sb_[threadIdx.x] = s1;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) { sa[threadIdx.x] += sa[threadIdx.x + s]; sb_[threadIdx.x] += sb_[threadIdx.x + s]; }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const double d0 = sa[0], d1 = sb_[0];
-    if (op == 0) {            // rho_n = <rhat, r>; bta; rho_o = rho_n
-      sc[3] = d0;
-      sc[4] = (d0 / sc[0]) * (sc[1] / sc[2]);
-      sc[0] = d0;
-    } else if (op == 1) {     // alpha = rho_n / <rhat, nu>
-      sc[1] = sc[3] / d0;
-    } else if (op == 2) {     // om = <t, s>/<t, t>
-      sc[2] = d0 / d1;
-    } else if (op == 3) {     // err = <r, r>
-      sc[5] = d0;
-    } else {
-      sc[slot0] = d0;
-      sc[slot0 + 1] = d1;
-    }
-  }
+  bcg_reduce(s0, s1, part, ticket, sc, op);
 }
 
 // p = r + bta*(p - om*nu);  ph = M p
@@ -1179,11 +1208,11 @@ __global__ void k_bcg_s(int64_t n, const double* __restrict__ r, const double* _
   }
 }
 
-// x = h + om*sh; r = s - om*t; partial <r, r>
+// x = h + om*sh; r = s - om*t; err = <r, r>
 __global__ void __launch_bounds__(256) k_bcg_x(int64_t n, double* __restrict__ x, double* __restrict__ r,
                                               const double* __restrict__ s, const double* __restrict__ sh,
-                                              const double* __restrict__ t, const double* __restrict__ sc,
-                                              double* __restrict__ part) {
+                                              const double* __restrict__ t, double* __restrict__ sc,
+                                              double* __restrict__ part, unsigned* __restrict__ ticket) {
   const double om = sc[2];
   double acc = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1192,14 +1221,7 @@ __global__ void __launch_bounds__(256) k_bcg_x(int64_t n, double* __restrict__ x
     r[i] = v;
     acc += v * v;
   }
-  __shared__ double sa[256];
-  sa[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sa[threadIdx.x] += sa[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { part[2 * blockIdx.x] = sa[0]; part[2 * blockIdx.x + 1] = 0.0; }
+  bcg_reduce(acc, 0.0, part, ticket, sc, BCG_ERR);
 }
 
 __global__ void k_axpby(int64_t n, double a, const double* __restrict__ x, double b,
@@ -1378,7 +1400,6 @@ static OpTables tables(Handle* h) {
   return T;
 }
 
-static unsigned thread_blocks(int64_t n) { return (unsigned)((n + 127) / 128); }
 
 static int upload_geometry(Handle* h) {
   IbState* s = h->ib;
@@ -1577,24 +1598,24 @@ __global__ void __launch_bounds__(256) k_grad_minus_reg(Dims d, Metric m, const 
                                                        const double* __restrict__ Wr, double* __restrict__ Gu,
                                                        double* __restrict__ Gv, double* __restrict__ Gw, int jlo,
                                                        int jhi) {
-  const int nxi = d.Nx, nzi = d.Nz, nr = jhi - jlo + 1;
-  const int64_t tot = (int64_t)nxi * nr * nzi;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = 2 + (int)(t % nxi);
-    const int64_t r = t / nxi;
-    const int j = jlo + (int)(r % nr);
-    const int k = 2 + (int)(r / nr);
+  // blockDim.x threads a row of x (two 64-bit divisions a point took as many
+  // instructions as the rest of it)
+  const int nr = jhi - jlo + 1;
+  for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < nr * d.Nz; r += gridDim.x * blockDim.y) {
+    const int kk = r / nr, k = 2 + kk, j = jlo + r - kk * nr;
     const bool centre = j >= 2 && j <= d.ny;       // u and w rows
-    const double p0 = centre ? P[idxR(d, i, j, k)] : 0.0;
-    if (centre) {
-      const int64_t iu = idxU(d, i, j, k), iw = idxW(d, i, j, k);
-      Gu[iu] = (P[idxR(d, i + 1, j, k)] - p0) * m.rdxg[i] - Ur[iu];
-      Gw[iw] = (P[idxR(d, i, j, k + 1)] - p0) * m.rdzg[k] - Wr[iw];
-    }
-    if (j >= 1 && j <= d.ny) {                     // v faces
-      const double gv = (j >= 2 && j <= d.ny - 1) ? (P[idxR(d, i, j + 1, k)] - p0) * m.rdyg[j] : 0.0;
-      const int64_t iv = idxV(d, i, j, k);
-      Gv[iv] = gv - Vr[iv];
+    for (int i = 2 + threadIdx.x; i <= d.Nx + 1; i += blockDim.x) {
+      const double p0 = centre ? P[idxR(d, i, j, k)] : 0.0;
+      if (centre) {
+        const int64_t iu = idxU(d, i, j, k), iw = idxW(d, i, j, k);
+        Gu[iu] = (P[idxR(d, i + 1, j, k)] - p0) * m.rdxg[i] - Ur[iu];
+        Gw[iw] = (P[idxR(d, i, j, k + 1)] - p0) * m.rdzg[k] - Wr[iw];
+      }
+      if (j >= 1 && j <= d.ny) {                   // v faces
+        const double gv = (j >= 2 && j <= d.ny - 1) ? (P[idxR(d, i, j + 1, k)] - p0) * m.rdyg[j] : 0.0;
+        const int64_t iv = idxV(d, i, j, k);
+        Gv[iv] = gv - Vr[iv];
+      }
     }
   }
 }
@@ -1612,7 +1633,7 @@ static int gather3(Handle* h, int mode, const double* U, const double* V, const 
   const GField fs[3] = {gf_u(h->d, U), gf_v(h->d, V), gf_w(h->d, W)};
   for (int c = 0; c < 3; ++c) a.comp[c] = GComp{fs[c], c, mode, sign, sub, subv, addv};
   a.ncomp = 3; a.out = out;
-  launch_gather_tile(a, h->stream);
+  launch_gather_tile(a, h->ib->lat_nx, h->stream);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
@@ -1622,7 +1643,7 @@ static int gather_c(Handle* h, const double* P, double mul, double* out, double 
   a.T = tables(h); a.d = h->d;
   a.comp[0] = GComp{GField{P, h->d.nxg - 2, h->d.nyg - 2, 1, mul}, 3, G_E1N, sign, nullptr, nullptr, nullptr};
   a.ncomp = 1; a.out = out;
-  launch_gather_tile(a, h->stream);
+  launch_gather_tile(a, h->ib->lat_nx, h->stream);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
@@ -1642,11 +1663,13 @@ static int build_spread_maps(Handle* h) {
       if ((rc = dev_alloc(h, &s->sp_off[c], npts[c]))) return rc;
       if ((rc = dev_alloc(h, &s->sp_ent[c], ne))) return rc;
       if ((rc = dev_alloc(h, &s->sp_w[c], ne))) return rc;
+      if ((rc = dev_alloc(h, &s->sp_pts[c], std::min(ne, npts[c])))) return rc;
     }
   }
   const int64_t maxpts = std::max(npts[0], std::max(npts[1], npts[2]));
   const int nchunks = (int)((maxpts + kScanChunk - 1) / kScanChunk);
   if (!s->sp_sums && (rc = dev_alloc(h, &s->sp_sums, nchunks))) return rc;
+  if (!s->sp_npts && (rc = dev_alloc(h, &s->sp_npts, 3))) return rc;
   if (!s->amp && (rc = dev_alloc(h, &s->amp, 3 * (int64_t)s->nb))) return rc;
   const unsigned gq = (unsigned)((25 * (int64_t)s->nb + 255) / 256);
   for (int c = 0; c < 3; ++c) {
@@ -1665,8 +1688,9 @@ static int build_spread_maps(Handle* h) {
     C3D_CUDA_TRY(h, cudaMemsetAsync(s->sp_cnt[c], 0, 4 * (size_t)n, h->stream));
     k_sp_fill<<<gq, 256, 0, h->stream>>>(T, c, n1s[c], n2s[c], s->sp_off[c], s->sp_cnt[c], s->sp_ent[c]);
     C3D_LAUNCH_CHECK(h);
+    C3D_CUDA_TRY(h, cudaMemsetAsync(s->sp_npts + c, 0, 4, h->stream));
     k_sp_sort<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(T, c, n, s->sp_cnt[c], s->sp_off[c], s->sp_ent[c],
-                                                                  s->sp_w[c]);
+                                                                  s->sp_w[c], s->sp_pts[c], s->sp_npts + c);
     C3D_LAUNCH_CHECK(h);
   }
   return 0;
@@ -1679,25 +1703,19 @@ static int spread(Handle* h, int mode, int comp0, int ncomp, const double* f, do
   IbState* s = h->ib;
   const Dims& d = h->d;
   const OpTables T = tables(h);
-  k_sp_amp<<<thread_blocks((int64_t)ncomp * s->nb), 128, 0, h->stream>>>(T, comp0, ncomp, mode, f, dt * h->p.nu, dt,
-                                                                         s->amp);
-  C3D_LAUNCH_CHECK(h);
   double* Fs[3] = {F0, F1, F2};
   const int n1s[3] = {d.nx, d.nxg, d.nxg}, n2s[3] = {d.nyg, d.ny, d.nyg}, n3s[3] = {d.nzg, d.nzg, d.nz};
   SpGather g[3]{};
-  int64_t most = 0;
+  SpRows z[3]{};
   for (int cc = 0; cc < ncomp; ++cc) {
     const int c = comp0 + cc;
-    g[cc].cnt = s->sp_cnt[c]; g[cc].off = s->sp_off[c]; g[cc].ent = s->sp_ent[c]; g[cc].w = s->sp_w[c];
-    g[cc].F = Fs[cc]; g[cc].n1 = n1s[c]; g[cc].n2 = n2s[c]; g[cc].n3 = n3s[c];
-    g[cc].jlo = std::max(jlo, 1);
-    g[cc].jhi = std::min(jhi, n2s[c]);
-    if (g[cc].jhi < g[cc].jlo) { g[cc].jlo = 1; g[cc].jhi = 0; }
-    most = std::max(most, (int64_t)g[cc].n1 * (g[cc].jhi - g[cc].jlo + 1) * g[cc].n3);
+    g[cc] = SpGather{s->sp_ent[c], s->sp_w[c], s->sp_pts[c], s->sp_npts + c, Fs[cc]};
+    z[cc] = SpRows{Fs[cc], n1s[c], n2s[c], n3s[c], std::max(jlo, 1), std::min(jhi, n2s[c])};
+    if (z[cc].jhi < z[cc].jlo) z[cc].jhi = z[cc].jlo - 1;
   }
-  if (most == 0) return 0;
-  dim3 grid((unsigned)std::min<int64_t>((most + 255) / 256, 148 * 8), (unsigned)ncomp);
-  k_sp_gather<<<grid, 256, 0, h->stream>>>(g[0], g[1], g[2], ncomp, s->amp + (int64_t)comp0 * s->nb, s->nb);
+  k_sp_amp<<<148 * 8, 256, 0, h->stream>>>(T, comp0, ncomp, mode, f, dt * h->p.nu, dt, s->amp, z[0], z[1], z[2]);
+  C3D_LAUNCH_CHECK(h);
+  k_sp_gather<<<dim3(148 * 8 / ncomp, ncomp), 256, 0, h->stream>>>(g[0], g[1], g[2], s->amp + (int64_t)comp0 * s->nb, s->nb);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
@@ -1772,8 +1790,9 @@ int ib_schur(Handle* h, const double* f, double* Sf, double dt) {
   // Sf(p) = -E1n_c(phi/dt), gathered in the same launch;
   // then the mean removal and -E1nHc_ext*p_jump                       :123-126
   const Dims& d = h->d;
-  const int64_t npts = (int64_t)d.Nx * (s->iy_hi - s->iy_lo + 1) * d.Nz;
-  k_grad_minus_reg<<<(unsigned)std::min<int64_t>((npts + 255) / 256, 148 * 8), 256, 0, h->stream>>>(
+  const int64_t rows = (int64_t)(s->iy_hi - s->iy_lo + 1) * d.Nz;
+  const unsigned bx = std::min(256, (d.Nx + 31) / 32 * 32), by = 256 / bx;
+  k_grad_minus_reg<<<(unsigned)std::min<int64_t>((rows + by - 1) / by, 148 * 64), dim3(bx, by), 0, h->stream>>>(
       d, h->m, h->rhs_p, s->Ureg, s->Vreg, s->Wreg, s->Ut, s->Vt, s->Wt, s->iy_lo, s->iy_hi);
   C3D_LAUNCH_CHECK(h);
   GatherArgs a{};
@@ -1782,18 +1801,14 @@ int ib_schur(Handle* h, const double* f, double* Sf, double dt) {
   for (int c = 0; c < 3; ++c) a.comp[c] = GComp{fs[c], c, G_E, 1.0, s->E1nH, f, nullptr};
   a.comp[3] = GComp{GField{h->rhs_p, d.nxg - 2, d.nyg - 2, 1, 1.0 / dt}, 3, G_E1N, -1.0, nullptr, nullptr, nullptr};
   a.ncomp = 4; a.out = Sf;
-  launch_gather_tile(a, h->stream);
+  launch_gather_tile(a, h->ib->lat_nx, h->stream);
   C3D_LAUNCH_CHECK(h);
   return remove_mean(h, Sf + 3 * nb, f + 3 * nb);
 }
 
-static int dot(Handle* h, const double* a, const double* b, const double* c, const double* e, int op,
-               int slot0 = 6) {
+static int dot(Handle* h, const double* a, const double* b, const double* c, const double* e, BcgOp op) {
   IbState* s = h->ib;
-  const int64_t n = 4 * (int64_t)s->nb;
-  k_dot2<<<kIbRedBlocks, 256, 0, h->stream>>>(a, b, c, e, n, s->red);
-  C3D_LAUNCH_CHECK(h);
-  k_dot_final<<<1, 256, 0, h->stream>>>(s->red, kIbRedBlocks, s->sc, slot0, op);
+  k_dot2<<<kIbRedBlocks, 256, 0, h->stream>>>(a, b, c, e, 4 * (int64_t)s->nb, s->red, s->ticket, s->sc, op);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
@@ -1849,7 +1864,7 @@ static int bcg_iteration(Handle* h, double* x, double dt, const double* blk, boo
   const unsigned gb = 148 * 4;
   const unsigned gm = (unsigned)((nb + 255) / 256);
   int rc;
-  if ((rc = dot(h, s->rhat, s->r, nullptr, nullptr, 0))) return rc;           // rho_n, bta
+  if ((rc = dot(h, s->rhat, s->r, nullptr, nullptr, BCG_RHO))) return rc;     // rho_n, bta
   k_bcg_p<<<gb, 256, 0, h->stream>>>(n, s->r, s->p, s->nu, s->ph, nullptr, s->sc);
   C3D_LAUNCH_CHECK(h);
   if (band) {
@@ -1859,7 +1874,7 @@ static int bcg_iteration(Handle* h, double* x, double dt, const double* blk, boo
     C3D_LAUNCH_CHECK(h);
   }
   if ((rc = ib_schur(h, s->ph, s->nu, dt))) return rc;
-  if ((rc = dot(h, s->rhat, s->nu, nullptr, nullptr, 1))) return rc;          // alpha
+  if ((rc = dot(h, s->rhat, s->nu, nullptr, nullptr, BCG_ALPHA))) return rc;  // alpha
   k_bcg_s<<<gb, 256, 0, h->stream>>>(n, s->r, s->nu, s->s, s->sh, x, s->ph, nullptr, s->sc);
   C3D_LAUNCH_CHECK(h);
   if (band) {
@@ -1869,10 +1884,8 @@ static int bcg_iteration(Handle* h, double* x, double dt, const double* blk, boo
     C3D_LAUNCH_CHECK(h);
   }
   if ((rc = ib_schur(h, s->sh, s->t, dt))) return rc;
-  if ((rc = dot(h, s->t, s->s, s->t, s->t, 2))) return rc;                    // om
-  k_bcg_x<<<kIbRedBlocks, 256, 0, h->stream>>>(n, x, s->r, s->s, s->sh, s->t, s->sc, s->red);
-  C3D_LAUNCH_CHECK(h);
-  k_dot_final<<<1, 256, 0, h->stream>>>(s->red, kIbRedBlocks, s->sc, 0, 3);   // err
+  if ((rc = dot(h, s->t, s->s, s->t, s->t, BCG_OM))) return rc;               // om
+  k_bcg_x<<<kIbRedBlocks, 256, 0, h->stream>>>(n, x, s->r, s->s, s->sh, s->t, s->sc, s->red, s->ticket);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
