@@ -710,8 +710,8 @@ int poisson_setup(Handle* h) {
     h->flux_part_len = nbx;
   }
   if ((rc = build_tri_table(h))) return rc;
-  if (S.spec32 && (rc = slab_setup(h, true))) return rc;
-  return slab_setup(h, false);
+  if (S.spec32 && slab_by_blocks(d, S.cluster32) && (rc = slab_setup(h, true))) return rc;
+  return slab_by_blocks(d, S.cluster) ? slab_setup(h, false) : 0;
 }
 
 int mixed_setup(Handle* h) {
@@ -729,7 +729,7 @@ int mixed_setup(Handle* h) {
   if ((rc = dev_alloc(h, &S.phi00, d.Ny))) return rc;
   if ((rc = xfft_setup<float>(h))) return rc;
   if ((rc = build_tri_table(h))) return rc;       // with the FP32 pivots
-  if ((rc = slab_setup(h, true))) return rc;
+  if (slab_by_blocks(d, S.cluster32) && (rc = slab_setup(h, true))) return rc;
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return 0;
 }
