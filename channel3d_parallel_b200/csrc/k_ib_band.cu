@@ -504,8 +504,9 @@ __global__ void __launch_bounds__(256) k_band_inv(int nb, int lat, int nzl, int 
 // at most 4 apart, so with blocks of 4 consecutive positions (16 rows: 4
 // markers x 4 components) each system is block tridiagonal; a block LU
 // without interchanges between blocks (Gauss-Jordan with partial pivoting
-// inside each 16 x 16 diagonal block) makes the solve 2 x (4 len / 16)
-// dependent block steps instead of 2 x 4 len scalar ones.
+// inside each 16 x 16 diagonal block), from both ends to the middle block row,
+// makes the solve 4 len / 16 dependent block steps instead of 2 x 4 len scalar
+// ones.
 // ---------------------------------------------------------------------------
 constexpr int kBs = 16;
 
@@ -549,17 +550,21 @@ __global__ void k_blk_pad(int nq, int nseg, int NBq, const int* __restrict__ seg
     if (kBs * i + rr >= m) Bb[o + rr * kBs + rr] = make_double2(1.0, 0.0);
 }
 
-// Block LU of one system by one warp: Delta_0 = B_0, Delta_i = B_i -
-// A_i G_{i-1}, P_i = Delta_i^-1, G_i = P_i C_i, and Q_i = P_i A_i, which
-// replaces A_i (the forward sweep is then y_i = P_i b_i - Q_i y_{i-1}: one
-// dependent product per block row).  The block products run over the 256
-// entries of a block in shared memory; the inverse is Gauss-Jordan with
+// Block LU of one system from both ends, a warp each (part 0: block rows 0 ..
+// M-1 downwards, part 1: N-1 .. M+1 upwards, M = N/2), then the middle row
+// (part 2, a launch of its own).  Downwards Delta_i = B_i - A_i G_{i-1}, P_i =
+// Delta_i^-1, G_i = P_i C_i, and Q_i = P_i A_i, which replaces A_i (the forward
+// sweep is then y_i = P_i b_i - Q_i y_{i-1}: one dependent product per block
+// row); upwards the same with A and C exchanged; Delta_M = B_M - A_M G_{M-1} -
+// C_M G_{M+1}, with P_M A_M in place of A_M and P_M C_M in G_M.  The block
+// products run over the 256 entries of a block in shared memory; the inverse is
+// Gauss-Jordan with
 // partial pivoting on [Delta_i | I] held by columns in registers (lane c < 16
 // holds column c of Delta_i, lane 16 + c column c of the identity), a pivot
 // row being marked used rather than swapped, so that row perm[k] ends as row
 // k of the inverse.  A pivot below 1e-12 of the block's largest entry sets
 // flag[1]: the caller then uses the pivoted banded LU instead.
-__global__ void __launch_bounds__(32) k_blk_factor(int nseg, int NBq, const int* __restrict__ nblk,
+__global__ void __launch_bounds__(32) k_blk_factor(int part0, int nseg, int NBq, const int* __restrict__ nblk,
                                                    const int* __restrict__ blkoff, double2* __restrict__ Ab,
                                                    const double2* __restrict__ Bb, const double2* __restrict__ Cb,
                                                    double2* __restrict__ Pb, double2* __restrict__ Gb,
@@ -582,42 +587,58 @@ __global__ void __launch_bounds__(32) k_blk_factor(int nseg, int NBq, const int*
     fence_mbar_init();
   }
   __syncwarp();
-  auto fetch = [&](int i) {          // lane 0: block row i into buffer i & 1
-    const int64_t o = b0 + (int64_t)i * kBs * kBs;
-    uint64_t* b = &bar[i & 1];
+  const int M = N / 2, part = part0 + (int)blockIdx.y;
+  const int n = part == 0 ? M : (part == 1 ? N - 1 - M : 1);      // block rows of this part
+  if (n == 0) return;
+  auto row = [&](int s) { return part == 0 ? s : (part == 1 ? N - 1 - s : M); };
+  const int first = part == 1 ? 2 : 0;     // A or, upwards, C: the block that meets the row before
+  auto fetch = [&](int s) {          // lane 0: the part's row s into buffer s & 1
+    const int64_t o = b0 + (int64_t)row(s) * kBs * kBs;
+    uint64_t* b = &bar[s & 1];
     fence_async_shared();
     mbar_arrive_expect_tx(b, 3 * kBlkBytes);
-    bulk_load(sIn[i & 1][0], Ab + o, kBlkBytes, b);
-    bulk_load(sIn[i & 1][1], Bb + o, kBlkBytes, b);
-    bulk_load(sIn[i & 1][2], Cb + o, kBlkBytes, b);
+    bulk_load(sIn[s & 1][0], Ab + o, kBlkBytes, b);
+    bulk_load(sIn[s & 1][1], Bb + o, kBlkBytes, b);
+    bulk_load(sIn[s & 1][2], Cb + o, kBlkBytes, b);
   };
-  if (lane == 0) fetch(0);
-  bool ok = true;
-  for (int i = 0; i < N; ++i) {
-    const int64_t o = b0 + (int64_t)i * kBs * kBs;
-    if (!mbar_wait(&bar[i & 1], (unsigned)(i >> 1) & 1u, kWaitCycles)) ok = false;
-    __syncwarp();
-    if (lane == 0 && i + 1 < N) fetch(i + 1);
-    const double2* sA = sIn[i & 1][0];
-    const double2* sB = sIn[i & 1][1];
-    const double2* sC = sIn[i & 1][2];
-    // Delta_i = B_i - A_i G_{i-1} (eight entries per lane, interleaved)
+  // Delta -= X G (eight entries per lane, interleaved)
+  auto subtract = [&](const double2* X) {
 #pragma unroll 4
     for (int e = lane; e < kBs * kBs; e += 32) {
       const int rr = e / kBs, cc = e % kBs;
-      double2 d = sB[e];
-      if (i > 0) {
-        double2 a0 = zero, a1 = zero;
+      double2 a0 = zero, a1 = zero;
 #pragma unroll
-        for (int k = 0; k < kBs; k += 2) {
-          a0 = cadd(a0, cmul(sA[rr * kBs + k], sG[k * kBs + cc]));
-          a1 = cadd(a1, cmul(sA[rr * kBs + k + 1], sG[(k + 1) * kBs + cc]));
-        }
-        d = csub(d, cadd(a0, a1));
+      for (int k = 0; k < kBs; k += 2) {
+        a0 = cadd(a0, cmul(X[rr * kBs + k], sG[k * kBs + cc]));
+        a1 = cadd(a1, cmul(X[rr * kBs + k + 1], sG[(k + 1) * kBs + cc]));
       }
-      sD[e] = d;
+      sD[e] = csub(sD[e], cadd(a0, a1));
     }
     __syncwarp();
+  };
+  if (lane == 0) fetch(0);
+  bool ok = true;
+  for (int s = 0; s < n; ++s) {
+    const int64_t o = b0 + (int64_t)row(s) * kBs * kBs;
+    if (!mbar_wait(&bar[s & 1], (unsigned)(s >> 1) & 1u, kWaitCycles)) ok = false;
+    __syncwarp();
+    if (lane == 0 && s + 1 < n) fetch(s + 1);
+    const double2* sA = sIn[s & 1][first];
+    const double2* sB = sIn[s & 1][1];
+    const double2* sC = sIn[s & 1][2 - first];
+    for (int e = lane; e < kBs * kBs; e += 32) sD[e] = sB[e];
+    __syncwarp();
+    if (part < 2) {
+      if (s > 0) subtract(sA);
+    } else {
+      for (int side = 0; side < 2; ++side) {       // the rows M - 1 and M + 1
+        if (side == 0 ? M == 0 : M + 1 == N) continue;
+        const double2* G = Gb + o + (side == 0 ? -1 : 1) * kBs * kBs;
+        for (int e = lane; e < kBs * kBs; e += 32) sG[e] = G[e];
+        __syncwarp();
+        subtract(side == 0 ? sA : sC);
+      }
+    }
     double2 col[kBs];
 #pragma unroll
     for (int rr = 0; rr < kBs; ++rr)
@@ -628,7 +649,7 @@ __global__ void __launch_bounds__(32) k_blk_factor(int nseg, int NBq, const int*
 #pragma unroll
       for (int rr = 0; rr < kBs; ++rr) dmax = fmax(dmax, cabs1(col[rr]));
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, s));
+    for (int w = 16; w > 0; w >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, w));
     unsigned used = 0;
     unsigned long long perm = 0;       // 4 bits per pivot step: the row it took
 #pragma unroll 1
@@ -685,13 +706,14 @@ __global__ void __launch_bounds__(32) k_blk_factor(int nseg, int NBq, const int*
       }
     }
     __syncwarp();
-    // G_i = P_i C_i (kept for the next block row) and Q_i = P_i A_i
+    // G_i = P_i C_i (kept for the next block row) and Q_i = P_i A_i, where the
+    // block row on that side exists
 #pragma unroll 4
     for (int e = lane; e < 2 * kBs * kBs; e += 32) {
       const bool isg = e < kBs * kBs;
       const int f = isg ? e : e - kBs * kBs;
       const int rr = f / kBs, cc = f % kBs;
-      if (isg ? (i + 1 >= N) : (i == 0)) continue;
+      if (part < 2 ? (!isg && s == 0) : (isg ? M + 1 == N : M == 0)) continue;
       const double2* R = isg ? sC : sA;
       double2 a0 = zero, a1 = zero;
 #pragma unroll
@@ -711,17 +733,26 @@ __global__ void __launch_bounds__(32) k_blk_factor(int nseg, int NBq, const int*
   if (!ok && lane == 0) atomicOr(flag + 3, 1);
 }
 
-// Block forward and back substitution of one system by one CTA of four
-// warps: thread (r, p) = (tid / 8, tid % 8) forms the terms of columns p and
-// p + 8 of row r of each 16 x 16 product (a quarter warp reads 128
-// consecutive bytes of a block row: no bank conflicts), eight threads add
-// them by shuffles, and one barrier per block row publishes the new 16-vector
-// (double-buffered).  The blocks stream through a shared-memory ring of bulk
-// copies (kBlkRing - 1 block rows ahead, issued by thread 0), and the
-// system's right-hand side and solution sit in shared memory for the whole
-// solve.
-constexpr int kBlkRing = 16;    // one 16x16 block per stage: 15 blocks (60 KB) in flight
-constexpr int kBlkThreads = 128;
+// Block forward and back substitution of one system by one CTA, from both ends
+// at once: four warps take the block rows 0 .. M (M = N/2) downwards, four the
+// rows N-1 .. M+1 upwards, they meet in row M and go back outwards.  In a group
+// of four warps thread (r, p) = (tid / 8, tid % 8) forms the terms of columns p
+// and p + 8 of row r of each 16 x 16 product (a quarter warp reads 128
+// consecutive bytes of a block row: no bank conflicts), eight threads add them
+// by shuffles, and one barrier per block row publishes the new 16-vectors
+// (double-buffered).  A group's blocks stream through a shared-memory ring of
+// bulk copies that a warp of its own issues, which waits for the slots the group
+// has read and takes no part in its barriers; the system's right-hand side and
+// solution sit in shared memory for the whole solve.
+//
+// 97 systems of 48 block rows: from one end alone, a thread of the four warps
+// issuing the copies behind a proxy fence, 42 us; from both ends 40, the issue
+// holding every step's barrier (fewer dependent FP64 operations in a step and
+// blocks read ahead into registers changed nothing either); with the copies out
+// of the barriers 28.
+constexpr int kBlkRing = 16;    // one 16x16 block per stage, half of them per group (32 KB)
+constexpr int kBlkGroup = 128;
+constexpr int kBlkThreads = 2 * kBlkGroup + 64;   // and a warp a group that issues its copies
 static size_t blk_solve_smem(int nmax) {
   return sizeof(double2) * ((size_t)kBlkRing * kBs * kBs + 2 * (size_t)kBs * nmax);
 }
@@ -759,15 +790,20 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
   const int m = 4 * seglen[sg];
   double2* xs = bs_smem + (size_t)kBlkRing * kBs * kBs;   // [kBs * N] right-hand side b
   double2* ys = xs + (size_t)kBs * N;                     // [kBs * N] t, then y, then x
-  __shared__ double2 vv[2][kBs];
-  __shared__ __align__(8) uint64_t bar[kBlkRing];
+  __shared__ double2 vv[2][2][kBs], mid[2][kBs];
+  __shared__ __align__(8) uint64_t bar[kBlkRing], empty[kBlkRing];   // block arrived, slot read
   const int64_t b0 = ((int64_t)q * NBq + blkoff[sg]) * (kBs * kBs);
   double2* x = rhs + (int64_t)q * 4 * lat + 4 * segstart[sg];
   const int tid = threadIdx.x;
-  const int r = tid >> 3, pp = tid & 7;
+  const bool copies = tid >= 2 * kBlkGroup;
+  const int gr = copies ? (tid - 2 * kBlkGroup) / 32 : tid / kBlkGroup, gt = tid % kBlkGroup;   // 0 downwards, 1 upwards
+  const int r = gt >> 3, pp = gt & 7;
   const double2 zero = make_double2(0.0, 0.0);
   if (tid == 0) {
-    for (int k = 0; k < kBlkRing; ++k) mbar_init(&bar[k], 1);
+    for (int k = 0; k < kBlkRing; ++k) {
+      mbar_init(&bar[k], 1);
+      mbar_init(&empty[k], 1);
+    }
     fence_mbar_init();
   }
   for (int e0 = tid; e0 < kBs * N; e0 += 4 * kBlkThreads) {   // four loads in flight
@@ -782,46 +818,62 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
       if (e0 + kBlkThreads * u < kBs * N) xs[e0 + kBlkThreads * u] = tv[u];
   }
   __syncthreads();
-  // `used` counts the blocks consumed (uniform across the CTA); slot and
-  // phase follow from it.
-  unsigned used = 0;
   bool ok = true;
   constexpr unsigned kBlkBytes = kBs * kBs * sizeof(double2);
-  auto blk = [&](const double2* base, int i) { return base + b0 + (int64_t)i * kBs * kBs; };
-  // The three passes consume one sequence of blocks, g = 0 .. 3N-3: P_0 ..
-  // P_{N-1}, then Q_1 .. Q_{N-1}, then G_{N-2} .. G_0; block g goes to slot
-  // g % kBlkRing.  The first kBlkRing are issued at g = 0, and at every
-  // g = 4, 8, ... the four blocks g+12 .. g+15, into the slots of g-4 .. g-1,
-  // which the barriers of their block rows have released (one proxy fence
-  // per group), so each pass's first blocks arrive during the previous one.
-  const int total = 3 * N - 2;
+  constexpr int kRing = kBlkRing / 2;
+  double2 (*const gring)[kBs * kBs] = ring + gr * kRing;
+  uint64_t *const gbar = bar + gr * kRing, *const gempty = empty + gr * kRing;
+  // the group's block rows s = 0, 1, ... from its end; row K is the middle one,
+  // whose P the first group takes
+  const int M = N / 2, K = gr == 0 ? M : N - 1 - M, np = gr == 0 ? M + 1 : K;
+  auto row = [&](int s) { return gr == 0 ? s : N - 1 - s; };
+  // Each group consumes one sequence of blocks: its P, Q of its rows 1 .. K
+  // (of the middle row the half that meets this group), then G of K-1 .. 0;
+  // block g goes to slot g % kRing once the group has read block g - kRing, so
+  // each pass's first blocks arrive during the previous one.
+  const int total = np + 2 * K;
   auto src = [&](int g) -> const double2* {
-    if (g < N) return blk(Pb, g);
-    if (g < 2 * N - 1) return blk(Ab, g - N + 1);
-    return blk(Gb, N - 2 - (g - (2 * N - 1)));
-  };
-  auto refill = [&](int g) {
-    const int lo = g == 0 ? 0 : g + kBlkRing - 4, hi = min(total, g + kBlkRing);
-    if (tid == 0 && lo < hi) {
-      fence_async_shared();            // the CTA's reads of the slots come first
-      for (int k = lo; k < hi; ++k) {
-        const unsigned slot = (unsigned)k % kBlkRing;
-        mbar_arrive_expect_tx(&bar[slot], kBlkBytes);
-        bulk_load(ring[slot], src(k), kBlkBytes, &bar[slot]);
-      }
+    const double2* base;
+    int i;
+    if (g < np) {
+      base = Pb;
+      i = row(g);
+    } else if (g < np + K) {
+      const int s = g - np + 1;
+      base = gr == 1 && s == K ? Gb : Ab;
+      i = row(s);
+    } else {
+      base = Gb;
+      i = row(np + 2 * K - 1 - g);
     }
+    return base + b0 + (int64_t)i * kBs * kBs;
   };
-  auto acquire = [&]() -> const double2* {
-    const unsigned slot = used % kBlkRing;
-    if (!mbar_wait(&bar[slot], (used / kBlkRing) & 1u, kWaitCycles)) ok = false;
-    ++used;
-    return ring[slot];
+  if (copies) {
+    if ((tid & 31) == 0)
+      for (int g = 0; g < total; ++g) {
+        const int slot = g % kRing;
+        if (g >= kRing && !mbar_wait(&gempty[slot], (unsigned)(g / kRing - 1) & 1u, kWaitCycles)) break;
+        mbar_arrive_expect_tx(&gbar[slot], kBlkBytes);
+        bulk_load(gring[slot], src(g), kBlkBytes, &gbar[slot]);
+      }
+    return;
+  }
+  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + gr), "n"(kBlkGroup) : "memory"); };
+  auto both_sync = [&] { asm volatile("bar.sync 3, %0;" ::"n"(2 * kBlkGroup) : "memory"); };
+  auto acquire = [&](int g) -> const double2* {
+    if (ok && !mbar_wait(&gbar[g % kRing], (unsigned)(g / kRing) & 1u, kWaitCycles)) ok = false;
+    return gring[g % kRing];
   };
-  // row r of M times v: columns pp and pp + 8 here, the other six pairs in
+  // after the barrier behind the group's reads of block g
+  auto release = [&](int g) {
+    if (gt == 0) mbar_arrive(&gempty[g % kRing]);
+  };
+  // row r of block g times v: columns pp and pp + 8 here, the other six pairs in
   // the seven neighbouring threads (shuffle sum over the group of eight)
-  auto rowdot = [&](const double2* M, const double2* v) {
-    const double2 p0 = M[r * kBs + pp], y0 = v[pp];
-    const double2 p1 = M[r * kBs + pp + 8], y1 = v[pp + 8];
+  auto rowdot = [&](int g, const double2* v) {
+    const double2* B = acquire(g);
+    const double2 p0 = B[r * kBs + pp], y0 = v[pp];
+    const double2 p1 = B[r * kBs + pp + 8], y1 = v[pp + 8];
     double2 a;
     a.x = p0.x * y0.x - p0.y * y0.y;
     a.y = p0.x * y0.y + p0.y * y0.x;
@@ -835,16 +887,15 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
     return a;
   };
   // t_i = P_i b_i for every block row (independent products): four block
-  // rows per step, one per warp; lane (r2, hh) forms half (eight terms, in a
-  // row-rotated order) of row r2.  P_i is block g = i of the sequence.
+  // rows per step and group, one per warp; lane (r2, hh) forms half (eight terms,
+  // in a row-rotated order) of row r2.  P of the group's row s is block g = s.
   {
-    const int warp = tid >> 5, lane = tid & 31, r2 = lane & 15, hh = lane >> 4;
-    for (int s4 = 0; s4 < N; s4 += 4) {
-      refill(s4);
-      const int i = s4 + warp;
-      if (i < N) {
-        if (!mbar_wait(&bar[i % kBlkRing], (unsigned)(i / kBlkRing) & 1u, kWaitCycles)) ok = false;
-        const double2* Pi = ring[i % kBlkRing];
+    const int warp = gt >> 5, lane = tid & 31, r2 = lane & 15, hh = lane >> 4;
+    for (int s4 = 0; s4 < np; s4 += 4) {
+      const int sr = s4 + warp;
+      if (sr < np) {
+        const double2* Pi = acquire(sr);
+        const int i = row(sr);
         const double2* v = xs + kBs * i;
         double2 a0 = zero, a1 = zero;
 #pragma unroll
@@ -863,41 +914,56 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
         a0.y += __shfl_xor_sync(0xffffffffu, a0.y, 16);
         if (hh == 0) ys[kBs * i + r2] = a0;
       }
-      __syncthreads();
+      group_sync();
+      for (int g = s4; g < min(s4 + 4, np); ++g) release(g);
     }
-    used = (unsigned)N;
   }
-  // forward: y_i = t_i - Q_i y_{i-1} (Q_i = P_i A_i, stored in place of A_i);
-  // vv[i & 1] carries y_i to the next block row
-  for (int i = 0; i < N; ++i) {
-    if (i > 0 && ((N + i - 1) & 3) == 0) refill(N + i - 1);
-    const int row = kBs * i + r;
-    double2 y = ys[row];
-    if (i > 0) {
-      const double2* Qi = acquire();
-      y = csub(y, rowdot(Qi, vv[(i - 1) & 1]));
-    }
+  // inwards: y_s = t_s - Q_s y_{s-1}, and for the middle row the product alone;
+  // vv[group][s & 1] carries y_s to the next step
+  if (pp == 0) {
+    if (K > 0) vv[gr][0][r] = ys[kBs * row(0) + r];
+    mid[gr][r] = zero;
+  }
+  group_sync();
+  for (int s = 1; s <= K; ++s) {
+    const double2 a = rowdot(np + s - 1, vv[gr][(s - 1) & 1]);
     if (pp == 0) {
-      vv[i & 1][r] = y;
-      ys[row] = y;
+      if (s == K) {
+        mid[gr][r] = a;
+      } else {
+        const int e = kBs * row(s) + r;
+        const double2 y = csub(ys[e], a);
+        vv[gr][s & 1][r] = y;
+        ys[e] = y;
+      }
     }
-    __syncthreads();
+    group_sync();
+    release(np + s - 1);
   }
-  // backward: x_i = y_i - G_i x_{i+1}; vv[(i + 1) & 1] holds x_{i+1}
-  for (int i = N - 2; i >= 0; --i) {
-    if (((3 * N - 3 - i) & 3) == 0) refill(3 * N - 3 - i);
-    const double2* Gi = acquire();
-    const double2 a = rowdot(Gi, vv[(i + 1) & 1]);
-    const int row = kBs * i + r;
+  // the middle row, then outwards: x_s = y_s - G_s x_{s+1}
+  both_sync();
+  double2 xm = zero;
+  if (pp == 0) {
+    xm = csub(csub(ys[kBs * M + r], mid[0][r]), mid[1][r]);
+    vv[gr][K & 1][r] = xm;
+  }
+  both_sync();                         // both groups have read t of the middle row
+  if (gr == 0 && pp == 0) ys[kBs * M + r] = xm;
+  for (int s = K - 1; s >= 0; --s) {
+    const int g = np + 2 * K - 1 - s;
+    const double2 a = rowdot(g, vv[gr][(s + 1) & 1]);
     if (pp == 0) {
-      const double2 xr = csub(ys[row], a);
-      vv[i & 1][r] = xr;
-      ys[row] = xr;
+      const int e = kBs * row(s) + r;
+      const double2 xr = csub(ys[e], a);
+      vv[gr][s & 1][r] = xr;
+      ys[e] = xr;
     }
-    __syncthreads();
+    group_sync();
+    release(g);
   }
-  for (int e = tid; e < m; e += kBlkThreads) x[e] = ys[e];
-  if (!ok && tid == 0) atomicOr(flag + 3, 1);
+  both_sync();
+  for (int e = tid; e < m; e += 2 * kBlkGroup) x[e] = ys[e];
+  if (!ok && gt == 0) atomicOr(flag + 3, 1);
 }
 
 // Forward and back substitution of one system (LAPACK zgbtrs, no transpose)
@@ -1233,7 +1299,10 @@ static int band_factor_that(Handle* h) {
   k_blk_pad<<<nq * B->nseg, 32, 0, h->stream>>>(nq, B->nseg, B->NBq, B->seglen_d, B->nblk_d, B->blkoff_d, B->Bb_d);
   C3D_LAUNCH_CHECK(h);
   C3D_CUDA_TRY(h, cudaMemsetAsync(B->flag_d, 0, 8, h->stream));
-  k_blk_factor<<<nq * B->nseg, 32, 0, h->stream>>>(B->nseg, B->NBq, B->nblk_d, B->blkoff_d, B->Ab_d, B->Bb_d,
+  k_blk_factor<<<dim3(nq * B->nseg, 2), 32, 0, h->stream>>>(0, B->nseg, B->NBq, B->nblk_d, B->blkoff_d, B->Ab_d, B->Bb_d,
+                                                   B->Cb_d, B->Pb_d, B->Gb_d, B->flag_d);
+  C3D_LAUNCH_CHECK(h);
+  k_blk_factor<<<nq * B->nseg, 32, 0, h->stream>>>(2, B->nseg, B->NBq, B->nblk_d, B->blkoff_d, B->Ab_d, B->Bb_d,
                                                    B->Cb_d, B->Pb_d, B->Gb_d, B->flag_d);
   C3D_LAUNCH_CHECK(h);
   int flag[2] = {0, 0};
