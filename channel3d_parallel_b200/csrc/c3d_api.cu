@@ -266,7 +266,6 @@ static void free_handle(Handle* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   ib_free(h);
   mlp_free(h);
-  mixed_free(h);
   drop_step_graphs(h);
   for (void* p : h->allocations) cudaFree(p);
   if (h->h2d) cudaStreamSynchronize(h->h2d);

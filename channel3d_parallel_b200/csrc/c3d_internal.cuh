@@ -237,10 +237,6 @@ struct Handle {
   StepGraph graphs[G_COUNT];
   double graph_dt = 0;
   bool write_pinterim = false;   // projection also stores P_interim = phi/dt
-  // programmatic dependent launch of the time step's kernels: off, the
-  // captured step graph ran slower with it (1118 against 1124 steps/s at
-  // 192x129x192) although each kernel alone starts 2-3 us earlier
-  bool use_pdl = false;
 };
 
 void drop_step_graphs(Handle* h);   // after any change of what they bake in
@@ -274,32 +270,6 @@ struct Status {
     }                                                                           \
   } while (0)
 
-// ---- programmatic dependent launch ----------------------------------------
-// The time step's kernels are launched so that a kernel's CTAs may start
-// while its predecessor in the stream finishes: each kernel reads only
-// set-up tables (twiddles, metric, digit reversal) before pdl_wait(), which
-// returns once the preceding grid has completed and its writes are visible;
-// it then calls pdl_trigger(), so the next kernel launches once every CTA of
-// this one has passed its wait.  Both are no-ops for an ordinary launch.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                              cudaStream_t stream, Args&&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
 // ---- kernels / drivers implemented in the .cu files ----------------------
 // boundary conditions (k_bc.cu)
 enum FieldKind { KIND_U = 0, KIND_V = 1, KIND_W = 2 };
@@ -330,7 +300,6 @@ int rebuild_pressure(Handle* h);
 int compute_pressure(Handle* h);
 int profile_spectral(Handle* h, int part);   // 0 div_xfft, 1 spectral_yz, 2 xfft inv
 int mixed_setup(Handle* h);
-void mixed_free(Handle* h);
 // x transforms (k_xfft.cu)
 int64_t xfft_blocks(const Dims& d);
 template <typename T>

@@ -1934,8 +1934,6 @@ static int bcg_graph_ready(Handle* h, double* x, double dt, const double* blk, b
     return 0;
   }
   cudaGraph_t body = np.conditional.phGraph_out[0];
-  const bool pdl = h->use_pdl;
-  h->use_pdl = false;                 // plain kernel nodes in the body
   const int64_t l0 = h->launches;
   C3D_CUDA_TRY(h, cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
   int rc = bcg_iteration(h, x, dt, blk, band);
@@ -1946,7 +1944,6 @@ static int bcg_graph_ready(Handle* h, double* x, double dt, const double* blk, b
   }
   cudaGraph_t captured = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(h->stream, &captured);
-  h->use_pdl = pdl;
   s->bcg_body_launches = h->launches - l0;
   h->launches = l0;
   if (rc) return rc;

@@ -169,8 +169,6 @@ __global__ void __launch_bounds__(256) k_spectral_band(BandYzArgs a) {
   const int tid = threadIdx.x, nt = blockDim.x;
   double2* g = a.spec + ((int64_t)m * Ny + a.rlo) * a.pz;
   for (int t = tid; t < Nz; t += nt) tw[t] = a.tw[t];
-  pdl_wait();
-  pdl_trigger();
   // eight loads in flight per thread before any store
   for (int t0 = tid; t0 < nr * Nz; t0 += 8 * nt) {
     double2 tv[8];
@@ -289,7 +287,7 @@ static int launch_band_yz(Handle* h, int blo, int bhi, bool* done) {
   BandYzArgs a{};
   a.d = d; a.spec = S.spec; a.tw = S.twz; a.rdp = S.rdp; a.tail = S.tail; a.dl = S.dl; a.du = S.du;
   a.P = get_passes(d.Nz, kBandMaxR); a.rs = rs; a.pz = S.pz64; a.rlo = blo; a.rhi = bhi;
-  C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_spectral_band, dim3((unsigned)d.nkx), dim3(256), smem, h->stream, a));
+  k_spectral_band<<<(unsigned)d.nkx, 256, smem, h->stream>>>(a);
   C3D_LAUNCH_CHECK(h);
   *done = true;
   return 0;
@@ -520,8 +518,6 @@ __global__ void __launch_bounds__(256, 4) k_grad_sub2(Dims d, Metric m, const do
   const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 2 + blockIdx.y * blockDim.y + threadIdx.y;
   const int k = 2 + 2 * (int)blockIdx.z;
-  pdl_wait();
-  pdl_trigger();
   if (i > d.Nx + 1 || j > d.Ny + 1) return;
   const bool two = k + 1 <= d.Nz + 1;
   const bool hv = j <= d.Ny;
@@ -601,8 +597,7 @@ int launch_gradient_subtract(Handle* h, const double* Ui, const double* Vi, cons
   double* Pint = (h->ib != nullptr || h->write_pinterim) ? h->P_interim : nullptr;
   if (!dup_plane && !Pint) {
     const dim3 b2(32, 8, 1), g2((d.Nx + 31) / 32, (d.Ny + 7) / 8, (d.Nz + 1) / 2);
-    C3D_CUDA_TRY(h, launch_pdl(h->use_pdl, k_grad_sub2, g2, b2, 0, h->stream, d, h->m, Ui, Vi, Wi, phi, Uo, Vo, Wo,
-                               with_ghosts ? 1 : 0, ushift));
+    k_grad_sub2<<<g2, b2, 0, h->stream>>>(d, h->m, Ui, Vi, Wi, phi, Uo, Vo, Wo, with_ghosts ? 1 : 0, ushift);
     C3D_LAUNCH_CHECK(h);
     return 0;
   }
@@ -733,7 +728,5 @@ int mixed_setup(Handle* h) {
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return 0;
 }
-
-void mixed_free(Handle* h) { (void)h; }
 
 }  // namespace c3d

@@ -108,7 +108,8 @@ typedef struct c3d_stats {
   int32_t precond_mode;        /* preconditioner of the last Schur solve      */
   double  last_bicgstab_ms;    /* device time of the last Schur solve (ms)    */
   double  bicgstab_ms;         /* accumulated device time of Schur solves     */
-  int32_t slab_cluster[2];     /* CTAs per kx-slab cluster of the y-z solve: FP64, FP32 */
+  int32_t slab_cluster[2];     /* CTAs per kx-slab cluster of the y-z solve: FP64, FP32 (above 8,
+                                  or with more than 256 columns, blocks of rows solve instead) */
   int32_t slab_narrow[2];      /* 1: narrow slab CTAs (<= 192 threads, 3 per SM); FP64, FP32 */
   double  qflow_y_0, qflow_z_0;/* targets of the y and z constant-flux corrections */
   int64_t precond_builds;      /* probed (or predicted) band preconditioners built */
@@ -271,7 +272,8 @@ int c3d_kernel_launches(int handle, int64_t* count);
  * times between CUDA events on the handle's stream (the fields are used as
  * scratch); ms[c] = average device time of class c in the order
  * rhs_stage, ghosts, div_xfft, spectral_yz, xfft_inv, grad_sub, massflow
- * (FP64 kernels).  Writes min(nmax, 7) entries.                              */
+ * (FP64 kernels; rhs_stage: the update of stage 2 or 3 with the projection of
+ * the stage before it).  Writes min(nmax, 7) entries.                              */
 int c3d_profile_kernels(int handle, int nrep, double* ms, int nmax);
 
 /* ---- learned preconditioner / warm start of the IB Schur solve ------------
