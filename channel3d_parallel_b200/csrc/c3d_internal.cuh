@@ -313,7 +313,7 @@ int launch_xfft_inv(Handle* h, double* out, double* phi1, const double* phi00, i
 int slab_setup(Handle* h, bool f32);
 template <typename T>
 int launch_slab(Handle* h, typename SlabTables<T>::C* spec, int zero00, int rlo, int rhi);
-// the same in one kernel (k_slab_cluster.cu)
+// the same in one kernel (slab_cluster.cuh)
 template <typename T>
 int cluster_setup(Handle* h);
 template <typename T>

@@ -376,9 +376,10 @@ __global__ void k_slab_link(Dims d, int jr, int nblk, const double* __restrict__
 
 constexpr int kSlabSmemMax = 220 * 1024;
 
-// The kernels for rows of Nz columns.  FP64 rows of 192 to 512 columns have the
-// length compiled in (384 x 256 x 384: 448 -> 417 us); shorter rows reach these
-// kernels only with very many of them, and FP32 takes the run-time stages.
+// The kernels for rows of Nz columns.  Rows of 192 to 512 columns have the
+// length compiled in (384 x 256 x 384: 448 -> 417 us, FP32 mixed steps
+// 7480 -> 7370);
+// shorter rows reach these kernels only with very many of them.
 template <typename T>
 struct SlabKernels {
   void (*fwd)(SlabArgs<T>);
@@ -392,8 +393,7 @@ SlabKernels<T> slab_pick(int Nz) {
 }
 template <typename T>
 SlabKernels<T> slab_kernels(int Nz) {
-  if constexpr (sizeof(T) == 8) return slab_pick<T, 192, 216, 256, 288, 324, 384, 432, 486, 512>(Nz);
-  else return slab_pick<T>(Nz);
+  return slab_pick<T, 192, 216, 256, 288, 324, 384, 432, 486, 512>(Nz);
 }
 
 }  // namespace

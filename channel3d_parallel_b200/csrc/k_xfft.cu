@@ -485,29 +485,35 @@ size_t x_smem(const FftPasses& P, bool fwd) {
          (fwd && sizeof(T) == 4 ? sizeof(double) * 2 * kLines * P.n : 0);
 }
 
-// The kernels for lines of Nx points: FP64 lines of 32 to 512 points have the
-// length compiled in (inverse at 384 x 256 x 384 188 -> 170 us, forward 288 ->
+// The kernels for lines of Nx points: lines of 32 to 512 points have the length
+// compiled in (FP64: inverse at 384 x 256 x 384 188 -> 170 us, forward 288 ->
 // 281; time step 4969 -> 4874 us there, 661 -> 653 at 192 x 128 x 192, 368 ->
-// 358 at 162 x 113 x 108, 83 -> 82 at 32 x 64 x 32).  FP32, and right-hand sides from memory (the Poisson
-// solve called by itself), take the run-time stages.
+// 358 at 162 x 113 x 108, 83 -> 82 at 32 x 64 x 32; FP32 mixed steps 1117 -> 1064
+// us at 192 x 128 x 192, 7771 -> 7535 at 384 x 256 x 384).  Right-hand
+// sides from memory (the Poisson solve called by itself) take the run-time
+// stages.
 template <typename T>
 struct XKernels {
   void (*div)(XfwdArgs<T>);
   void (*flux)(XfwdArgs<T>);
+  void (*residual)(XfwdArgs<T>);     // FP32
   void (*inv)(XinvArgs<T>);
 };
+template <typename T, int NX>
+XKernels<T> x_set() {
+  XKernels<T> k{k_xfft_fwd<FROM_DIV, T, NX>, k_xfft_fwd<FROM_DIV_FLUX, T, NX>, nullptr, k_xfft_inv<T, NX>};
+  if constexpr (sizeof(T) == 4) k.residual = k_xfft_fwd<FROM_RESIDUAL, T, NX>;
+  return k;
+}
 template <typename T, int... NX>
 XKernels<T> x_pick(int Nx) {
-  XKernels<T> k{k_xfft_fwd<FROM_DIV, T, 0>, k_xfft_fwd<FROM_DIV_FLUX, T, 0>, k_xfft_inv<T, 0>};
-  ((Nx == NX ? (void)(k = {k_xfft_fwd<FROM_DIV, T, NX>, k_xfft_fwd<FROM_DIV_FLUX, T, NX>, k_xfft_inv<T, NX>})
-             : (void)0), ...);
+  XKernels<T> k = x_set<T, 0>();
+  ((Nx == NX ? (void)(k = x_set<T, NX>()) : (void)0), ...);
   return k;
 }
 template <typename T>
 XKernels<T> x_kernels(int Nx) {
-  if constexpr (sizeof(T) == 8)
-    return x_pick<T, 32, 48, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 486, 512>(Nx);
-  else return x_pick<T>(Nx);
+  return x_pick<T, 32, 48, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 486, 512>(Nx);
 }
 
 template <typename T>
@@ -552,7 +558,7 @@ int launch_xfft_fwd(Handle* h, bool from_div, const double* U, const double* V, 
     a.q0 = h->Qflow_x_0; a.norm = h->norm_u; a.dt = flux_dt;
     x_kernels<T>(d.Nx).flux<<<nb, nt, smem, h->stream>>>(a);
   } else if (from_div && rhs) {
-    if constexpr (sizeof(T) == 4) k_xfft_fwd<FROM_RESIDUAL, T, 0><<<nb, nt, smem, h->stream>>>(a);
+    if constexpr (sizeof(T) == 4) x_kernels<T>(d.Nx).residual<<<nb, nt, smem, h->stream>>>(a);
   } else if (from_div) {
     x_kernels<T>(d.Nx).div<<<nb, nt, smem, h->stream>>>(a);
   } else {
@@ -616,7 +622,7 @@ int xfft_setup(Handle* h) {
   const XKernels<T> k = x_kernels<T>(d.Nx);
   C3D_CUDA_TRY(h, limit(k.div));
   C3D_CUDA_TRY(h, limit(k.flux));
-  if constexpr (sizeof(T) == 4) C3D_CUDA_TRY(h, limit(k_xfft_fwd<FROM_RESIDUAL, T, 0>));
+  if constexpr (sizeof(T) == 4) C3D_CUDA_TRY(h, limit(k.residual));
   C3D_CUDA_TRY(h, limit(k.inv));
   return 0;
 }
