@@ -127,8 +127,9 @@ struct SpectralState {
   double* tri = nullptr;                     // diagonal, kxx and kzz behind the tables
   double *dl = nullptr, *du = nullptr;       // Dyy(j+1, j) and Dyy(j, j+1), j = 0..Ny-1 (0 past the end)
   // x(j)/y(j) of the homogeneous tail (right-hand side zero from row j on),
-  // same layout as rdp; built on first use by the band-restricted solve
+  // same layout as rdp; built by the band-restricted solve on its first use on a grid
   double* tail = nullptr;
+  bool tail_current = false;                 // of the current grid's tables
   float *dl32 = nullptr, *du32 = nullptr;
   // spectra, layout [m][j][k] = [(m*Ny + (j-2))*pz + (k-2)]: one kx slab is
   // Ny rows of pz complex values (pz*sizeof(complex) a multiple of 16 bytes)

@@ -1453,8 +1453,19 @@ static int upload_grids(Handle* h) {
   return 0;
 }
 
+// after a change of the grid: what the immersed body keeps between solves and
+// holds the old spacings (the captured iteration loop, whose kernels take the
+// cell volume by value, and the preconditioners) or was learned on them
 void ib_grids_changed(Handle* h) {
-  if (h->ib) h->ib->grids_current = false;
+  IbState* s = h->ib;
+  if (!s) return;
+  s->grids_current = false;
+  s->bcg_key.clear();          // no key matches: the next solve captures its loop anew
+  s->have_jac = s->have_lrn = false;
+  band_invalidate(h);
+  for (int& n : s->nhist) n = 0;
+  s->band_iters_ref = 0.0;
+  s->lrn_slow = 0;
 }
 
 int ib_create(Handle* h) {
@@ -1907,8 +1918,8 @@ __global__ void k_bcg_loop(cudaGraphConditionalHandle cond, const double* __rest
 // whose body (one iteration and k_bcg_loop) runs until k_bcg_loop stops it,
 // so a solve costs one graph launch and one host synchronisation instead of
 // one per iteration.  What the body bakes in (mode, factors, operand
-// pointers, dt, tolerance, the band of stencil rows) is the graph's key;
-// the graph is re-captured when it changes.  Sets bcg_graph_off, and
+// pointers, dt, tolerance, the band of stencil rows) is the graph's key; the
+// graph is re-captured when it or the grid (ib_grids_changed) changes.  Sets bcg_graph_off, and
 // leaves the loop to the host, when conditional nodes are unavailable.
 static int bcg_graph_ready(Handle* h, double* x, double dt, const double* blk, bool band, int mode, double eps) {
   IbState* s = h->ib;

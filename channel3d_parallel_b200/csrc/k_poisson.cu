@@ -132,6 +132,7 @@ static int build_tri_table(Handle* h) {
   k_tri_table<<<dim3((nkzs + 63) / 64, nkx), 64, 0, s>>>(d, S.tri, S.dl, S.du, S.tri + Ny, S.tri + Ny + nkx, S.rdp,
                                                          S.rdp32, S.mult00);
   C3D_LAUNCH_CHECK(h);
+  S.tail_current = false;
   C3D_CUDA_TRY(h, cudaStreamSynchronize(s));   // the host copies end here
   return 0;
 }
@@ -143,7 +144,7 @@ static int build_tri_table(Handle* h) {
 // band alone: the forward sweep starts at rlo from zero, and the back
 // substitution starts from x(rhi+1) = S(rhi+1) y(rhi+1), y(rhi+1) =
 // -MULT(rhi) y(rhi), where S(j) = x(j)/y(j) of the homogeneous tail is
-// tabulated once (build_tail_table).  One CTA per kx slab, the band rows in
+// tabulated once per grid (build_tail_table).  One CTA per kx slab, the band rows in
 // shared memory; the band's own z transform, there and back.
 // ---------------------------------------------------------------------------
 struct BandYzArgs {
@@ -256,9 +257,10 @@ static int build_tail_table(Handle* h) {
       }
     }
   int rc;
-  if ((rc = dev_alloc(h, &S.tail, nt))) return rc;
+  if (!S.tail && (rc = dev_alloc(h, &S.tail, nt))) return rc;
   C3D_CUDA_TRY(h, cudaMemcpyAsync(S.tail, tail.data(), 8 * nt, cudaMemcpyHostToDevice, h->stream));
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  S.tail_current = true;
   return 0;
 }
 
@@ -279,7 +281,7 @@ static int launch_band_yz(Handle* h, int blo, int bhi, bool* done) {
   const size_t smem = band_yz_smem(d, rs, nr);
   if (nr <= 0 || smem > kBandYzSmemMax) return 0;
   int rc;
-  if (!S.tail) {   // first use (outside any graph capture: the table build synchronises)
+  if (!S.tail_current) {   // first use on this grid (outside any graph capture: the table build synchronises)
     if ((rc = build_tail_table(h))) return rc;
     C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_spectral_band, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kBandYzSmemMax));
