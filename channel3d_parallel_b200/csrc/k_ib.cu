@@ -36,8 +36,11 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
   const int nxb = p.nxb, nzb = p.nzb;
   const double Lxp = h->Lxp, Lzp = h->Lzp;
   // every body type writes the same entries at every time, so the arrays
-  // are cleared only when their size changes
+  // are cleared only when their size changes.  The device arrays hold the
+  // marker count of the first geometry: another one (double_cylinders_z takes it
+  // from the grid's spacings) is refused before anything is changed.
   auto resize = [&](int nb) {
+    if (s->xb_d != nullptr && s->nb != nb) { err = "marker count changed"; return false; }
     if (s->nb != nb || (int)s->xb.size() != nb) {
       s->nb = nb;
       s->xb.assign(nb, 0); s->yb.assign(nb, 0); s->zb.assign(nb, 0);
@@ -46,6 +49,7 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
       s->yref.assign(nb, 1); s->body.assign(nb, 0);
     }
     s->lat_nx = nb;
+    return true;
   };
   // Lattices whose markers differ from row to row only in z (every value
   // but zb depends on the x index and the time): the first row is computed
@@ -68,7 +72,7 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
   if (s->kind == "center_wall") {                                     // :80-115
     if (p.grid_type != 0) { err = "Error: body type is incompatible with grid type"; return C3D_ERR_PARAM; }
     const int nb = nxb * nzb;
-    resize(nb);
+    if (!resize(nb)) return C3D_ERR_PARAM;
     s->lat_nx = nxb;
     const double dxb = Lxp / nxb, dzb = Lzp / nzb;
     for (int j = 1; j <= nzb; ++j)
@@ -94,7 +98,7 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
     }
     const int nw = two ? 2 : 1;
     const int nb = nw * nxb * nzb;
-    resize(nb);
+    if (!resize(nb)) return C3D_ERR_PARAM;
     s->lat_nx = nw * nxb;
     const double dxb = Lxp / nxb, dzb = Lzp / nzb;
     const double A = p.body_param_1, om = p.body_param_2, b3 = p.body_param_3;
@@ -163,7 +167,7 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
     s->nbodies = nw;
   } else if (s->kind == "traveling_wave_x") {                          // :271-390
     const int nb = 2 * nxb * nzb;
-    resize(nb);
+    if (!resize(nb)) return C3D_ERR_PARAM;
     s->lat_nx = 2 * nxb;
     const double dxb = Lxp / nxb, dzb = Lzp / nzb;
     const double b1 = p.body_param_1, b2 = p.body_param_2, b3 = p.body_param_3, tr = p.body_ramp_up_time;
@@ -226,7 +230,7 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
     const int nxb1 = (int)(2 * 3.14159 * r1 / dxb), nxb2 = (int)(2 * 3.14159 * r2 / dxb);
     const int nxbt = nxb1 + nxb2;
     const int nb = nxbt * nzb;
-    resize(nb);
+    if (!resize(nb)) return C3D_ERR_PARAM;
     s->lat_nx = nxbt;
     const double xc = 0.5 * Lxp, yc = 0.5 * p.Ly_channel;
     const double dsb1 = 2 * 3.14159 * r1 / nxb1, dsb2 = 2 * 3.14159 * r2 / nxb2;
@@ -273,7 +277,7 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
     const double r = p.body_param_1, us = p.body_param_2;
     const double dzb = Lzp / nzb, dsb = 2.0 * kPiIb * r / nxb;
     const int nb = 2 * nxb * nzb;
-    resize(nb);
+    if (!resize(nb)) return C3D_ERR_PARAM;
     s->lat_nx = 2 * nxb;
     const double xc[2] = {p.body_param_3, 2.0 * p.body_param_3};
     const double yc[2] = {0.5 * p.Ly_channel, 0.5 * p.Ly_channel + p.body_param_4};
@@ -312,7 +316,7 @@ static int geometry_host(Handle* h, IbState* s, double t, std::string& err) {
     const double hh = p.body_param_1, amp = p.body_param_2, om = p.body_param_3;
     const double pitchx = Lxp / nxb, pitchz = Lzp / nzb, wz = 0.5 * pitchz;
     const int nb = nxb * nzb * my * mz;
-    resize(nb);
+    if (!resize(nb)) return C3D_ERR_PARAM;
     s->lat_nx = nxb * my;
     uint64_t st = (uint64_t)(int64_t)std::llround(p.body_param_4);
     std::vector<double> phase(nxb * nzb);
@@ -1545,10 +1549,8 @@ int ib_setup_geometry(Handle* h, double t) {
   IbState* s = h->ib;
   if (!s) return C3D_ERR_UNSUPPORTED;
   std::string err;
-  const int nb0 = s->nb;
   int rc = geometry_host(h, s, t, err);
   if (rc) { h->last_error = err; return rc; }
-  if (s->nb != nb0) { h->last_error = "marker count changed"; return C3D_ERR_PARAM; }
   return upload_geometry(h);
 }
 

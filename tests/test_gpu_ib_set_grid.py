@@ -50,3 +50,25 @@ def test_new_grid_equals_a_fresh_handle(mode):
                 out.append(res + [ch.download(n) for n in ("U", "V", "W", "FB")])
         for name, a, b in zip(("schur", "precond", "U", "V", "W", "FB"), *out):
             assert np.array_equal(a, b), (name, np.abs(a - b).max() / np.abs(b).max())
+
+
+def test_grid_that_changes_the_marker_count_is_refused_whole():
+    """double_cylinders_z takes its marker count from the spacings; the device
+    arrays keep the first one, so another count is refused without a change: the
+    body works on, and with the first grid set again as before."""
+    import channel3d_parallel_b200 as c3d
+    kw = dict(nx_global=34, ny_global=33, nz_global=14, Lzp=1.0, nu=3e-4, CFL=-0.01, grid_type=0, alpha_stretch=0.0,
+              body_type="double_cylinders_z", nxb=0, nzb=6, body_param_1=0.15, body_param_2=0.3, body_param_3=0.015)
+    with c3d.Channel(**dict(kw, Lxp=2.0)) as ch, c3d.Channel(**dict(kw, Lxp=1.0)) as wide:
+        first, second, nb = ch.grid(), wide.grid(), ch.dims["nb"]
+        assert wide.dims["nb"] > nb
+        ch.compute_dt()
+        ch.compute_heaviside()
+        f = np.random.default_rng(2).standard_normal(4 * nb)
+        before = ch.schur(f)
+        with pytest.raises(c3d.C3DError, match="marker count"):
+            ch.set_grid(second["x"], second["y"], second["z"])
+        assert len(ch.download("XB")) == nb and np.isfinite(ch.schur(f)).all()
+        ch.set_grid(first["x"], first["y"], first["z"])
+        ch.compute_heaviside()
+        assert np.array_equal(ch.schur(f), before)
