@@ -1136,6 +1136,10 @@ static size_t solve_smem_bytes(int lat) {
 static size_t fwd_smem_bytes(int nzl) { return sizeof(double) * (32 * (size_t)nzl + 2 * (size_t)nzl); }
 static size_t inv_smem_bytes(int nzl, int nq) { return sizeof(double) * (64 * (size_t)nq + 2 * (size_t)nzl); }
 
+// the largest of these that are accepted (k_band_inv takes at most kInvExtra
+// more than k_band_fwd: nq <= nzl/2 + 1)
+constexpr size_t kBandSmemMax = 220 * 1024, kBlkSmemMax = 200 * 1024, kInvExtra = 512;
+
 static int band_setup(Handle* h) {
   IbState* s = h->ib;
   if (s->band) return 0;
@@ -1148,7 +1152,7 @@ static int band_setup(Handle* h) {
   B->nzl = s->nb / lat;
   B->nq = B->nzl / 2 + 1;
   B->nseg = (int)B->seg_start.size();
-  if (B->nzl * lat != s->nb || solve_smem_bytes(lat) > 220 * 1024 || fwd_smem_bytes(B->nzl) > 220 * 1024) {
+  if (B->nzl * lat != s->nb || solve_smem_bytes(lat) > kBandSmemMax || fwd_smem_bytes(B->nzl) > kBandSmemMax) {
     B->ok = false;
     return 0;
   }
@@ -1212,7 +1216,7 @@ static int band_setup(Handle* h) {
     B->NBq += B->nblk[sgi];
     B->nblk_max = std::max(B->nblk_max, B->nblk[sgi]);
   }
-  if (blk_solve_smem(B->nblk_max) > 200 * 1024) {
+  if (blk_solve_smem(B->nblk_max) > kBlkSmemMax) {
     h->last_error = "band preconditioner: a lattice segment is too long for the block solve";
     return C3D_ERR_UNSUPPORTED;
   }
@@ -1261,16 +1265,15 @@ static int band_setup(Handle* h) {
   C3D_CUDA_TRY(h, cudaMemcpyAsync(B->nblk_d, B->nblk.data(), 4 * B->nseg, cudaMemcpyHostToDevice, st));
   C3D_CUDA_TRY(h, cudaMemcpyAsync(B->blkoff_d, B->blkoff.data(), 4 * B->nseg, cudaMemcpyHostToDevice, st));
   C3D_CUDA_TRY(h, cudaStreamSynchronize(st));
-  const size_t solve_smem = solve_smem_bytes(lat);
-  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem));
-  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_band_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)fwd_smem_bytes(nzl)));
-  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_band_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)inv_smem_bytes(nzl, nq)));
-  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_band_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(sizeof(double2) * kFactorWin * kLdab)));
-  C3D_CUDA_TRY(h, cudaFuncSetAttribute(k_blk_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)blk_solve_smem(B->nblk_max)));
+  // process-wide, and handles of other lattices share them: the most any needs
+  auto limit = [&](auto* k, size_t b) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+  };
+  C3D_CUDA_TRY(h, limit(k_band_solve, kBandSmemMax));
+  C3D_CUDA_TRY(h, limit(k_band_fwd, kBandSmemMax));
+  C3D_CUDA_TRY(h, limit(k_band_inv, kBandSmemMax + kInvExtra));
+  C3D_CUDA_TRY(h, limit(k_band_factor, sizeof(double2) * kFactorWin * kLdab));
+  C3D_CUDA_TRY(h, limit(k_blk_solve, kBlkSmemMax));
   return 0;
 }
 
