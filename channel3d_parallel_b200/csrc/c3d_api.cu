@@ -469,16 +469,25 @@ static int sync_scalars_to_device(Handle* h) {
   return 0;
 }
 
+static int device_error(Handle* h, unsigned long long err) {
+  if (!err) return 0;
+  h->last_error = "a kernel gave up waiting for an asynchronous copy (device state is suspect)";
+  return C3D_ERR_CUDA;
+}
+
 static int sync_scalars_from_device(Handle* h) {
   DevScalars s{};
   C3D_CUDA_TRY(h, cudaMemcpyAsync(&s, h->sc, sizeof(s), cudaMemcpyDeviceToHost, h->stream));
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   h->dPdx = s.dPdx; h->dPdy = s.dPdy; h->dPdz = s.dPdz;
-  if (s.err) {
-    h->last_error = "a kernel gave up waiting for an asynchronous copy (device state is suspect)";
-    return C3D_ERR_CUDA;
-  }
-  return 0;
+  return device_error(h, s.err);
+}
+
+int check_device_error(Handle* h) {
+  unsigned long long e = 0;
+  C3D_CUDA_TRY(h, cudaMemcpyAsync(&e, &h->sc->err, sizeof(e), cudaMemcpyDeviceToHost, h->stream));
+  C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  return device_error(h, e);
 }
 
 void drop_step_graphs(Handle* h) {
@@ -1244,7 +1253,9 @@ int c3d_bicgstab(int id, const double* rhs) {
   const int64_t n = 4 * (int64_t)ib_nb(h);
   double* dr = ib_scratch(h, 2);
   C3D_CUDA_TRY(h, cudaMemcpyAsync(dr, rhs, n * 8, cudaMemcpyHostToDevice, h->stream));
-  RET(h, ib_bicgstab(h, dr, h->dt));
+  rc = ib_bicgstab(h, dr, h->dt);
+  const int err = rc < 0 ? 0 : check_device_error(h);
+  RET(h, err ? err : rc);
 }
 int c3d_precond_apply(int id, const double* in, double* out) {
   GET_HANDLE(id);
@@ -1254,13 +1265,15 @@ int c3d_precond_apply(int id, const double* in, double* out) {
   double* dout = ib_scratch(h, 0);
   C3D_CUDA_TRY(h, cudaMemcpyAsync(din, in, n * 8, cudaMemcpyHostToDevice, h->stream));
   rc = ib_precond_apply(h, din, dout, h->dt);
-  if (rc) RET(h, rc);
-  RET(h, marker_out(h, dout, out, n));
+  if (rc || (rc = marker_out(h, dout, out, n))) RET(h, rc);
+  RET(h, check_device_error(h));
 }
 int c3d_compute_IB_projection(int id) {
   GET_HANDLE(id);
   int rc = need_ib(h); if (rc) RET(h, rc);
-  RET(h, ib_projection(h, h->dt, 0));
+  rc = ib_projection(h, h->dt, 0);
+  const int err = rc < 0 ? 0 : check_device_error(h);
+  RET(h, err ? err : rc);
 }
 
 }  // extern "C"

@@ -240,6 +240,7 @@ struct Handle {
   bool write_pinterim = false;   // projection also stores P_interim = phi/dt
 };
 
+int check_device_error(Handle* h);  // waits for the stream; C3D_ERR_CUDA once a kernel gave up a wait
 void drop_step_graphs(Handle* h);   // after any change of what they bake in
 const double* ib_hu(Handle* h);
 const double* ib_hv(Handle* h);

@@ -2129,7 +2129,11 @@ int ib_bicgstab(Handle* h, const double* b, double dt) {
   h->stats.bicgstab_iters += it;
   h->stats.last_bicgstab_iters = it;
   h->stats.last_residual = std::sqrt(err);
-  if (!(err == err)) { h->last_error = "BiCGSTAB produced a non-finite residual"; return C3D_ERR_NAN; }
+  if (!(err == err)) {
+    if ((rc = check_device_error(h))) return rc;      // products of blocks that never arrived
+    h->last_error = "BiCGSTAB produced a non-finite residual";
+    return C3D_ERR_NAN;
+  }
   if (it == h->p.cg_max_iter && err >= eps) return C3D_WARN_NOT_CONVERGED;
   return 0;
 }

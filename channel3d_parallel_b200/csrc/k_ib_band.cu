@@ -40,6 +40,7 @@
 #include "c3d_internal.cuh"
 #include "ib_state.cuh"
 #include "bulk.cuh"
+#include "copy_ring.cuh"
 #include "fft.cuh"
 
 namespace c3d {
@@ -105,7 +106,7 @@ struct BandState {
   FftPasses fftP{};
   double2* ftw_d = nullptr;        // [nzl] exp(-2 pi i m / nzl)
   int* fpos_d = nullptr;           // [nzl] digit-reversed position of coefficient m
-  int* flag_d = nullptr;           // [0] zero pivot seen
+  int* flag_d = nullptr;           // [0] zero pivot seen, [1] small pivot in a diagonal block
   bool built = false;
   std::vector<double> yb_at, xb_at;
   double dt_at = 0;
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(32) k_blk_factor(int part0, int nseg, int NBq,
                                                    const int* __restrict__ blkoff, double2* __restrict__ Ab,
                                                    const double2* __restrict__ Bb, const double2* __restrict__ Cb,
                                                    double2* __restrict__ Pb, double2* __restrict__ Gb,
-                                                   int* __restrict__ flag) {
+                                                   int* __restrict__ flag, unsigned long long* __restrict__ err) {
   // A_i, B_i, C_i of block row i arrive by bulk copies into buffer i & 1
   // while block row i - 1 is factored
   __shared__ __align__(128) double2 sIn[2][3][kBs * kBs];
@@ -617,11 +618,14 @@ __global__ void __launch_bounds__(32) k_blk_factor(int part0, int nseg, int NBq,
     __syncwarp();
   };
   if (lane == 0) fetch(0);
-  bool ok = true;
   for (int s = 0; s < n; ++s) {
     const int64_t o = b0 + (int64_t)row(s) * kBs * kBs;
-    if (!mbar_wait(&bar[s & 1], (unsigned)(s >> 1) & 1u, kWaitCycles)) ok = false;
-    __syncwarp();
+    const unsigned phase = (unsigned)(s >> 1) & 1u;
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar[s & 1], phase, kWaitCycles))) {
+      if (lane == 0) atomicOr(err, 1ull);
+      mbar_wait(&bar[s & 1], phase, kWaitCycles);    // row s alone is in flight
+      return;
+    }
     if (lane == 0 && s + 1 < n) fetch(s + 1);
     const double2* sA = sIn[s & 1][first];
     const double2* sB = sIn[s & 1][1];
@@ -730,7 +734,6 @@ __global__ void __launch_bounds__(32) k_blk_factor(int part0, int nseg, int NBq,
     for (int e = lane; e < kBs * kBs; e += 32) sG[e] = sD[e];
     __syncwarp();
   }
-  if (!ok && lane == 0) atomicOr(flag + 3, 1);
 }
 
 // Block forward and back substitution of one system by one CTA, from both ends
@@ -742,7 +745,8 @@ __global__ void __launch_bounds__(32) k_blk_factor(int part0, int nseg, int NBq,
 // by shuffles, and one barrier per block row publishes the new 16-vectors
 // (double-buffered).  A group's blocks stream through a shared-memory ring of
 // bulk copies that a warp of its own issues, which waits for the slots the group
-// has read and takes no part in its barriers; the system's right-hand side and
+// has read and takes no part in its barriers (copy_ring.cuh; a wait that gives
+// up is recorded in the handle's error word); the system's right-hand side and
 // solution sit in shared memory for the whole solve.
 //
 // 97 systems of 48 block rows: from one end alone, a thread of the four warps
@@ -764,7 +768,8 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
                                                            const double2* __restrict__ Ab,
                                                            const double2* __restrict__ Pb,
                                                            const double2* __restrict__ Gb,
-                                                           double2* __restrict__ rhs, int* __restrict__ flag);
+                                                           double2* __restrict__ rhs,
+                                                           unsigned long long* __restrict__ err);
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -782,7 +787,8 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
                                                            const double2* __restrict__ Ab,
                                                            const double2* __restrict__ Pb,
                                                            const double2* __restrict__ Gb,
-                                                           double2* __restrict__ rhs, int* __restrict__ flag) {
+                                                           double2* __restrict__ rhs,
+                                                           unsigned long long* __restrict__ err) {
   extern __shared__ __align__(128) double2 bs_smem[];
   double2 (*ring)[kBs * kBs] = reinterpret_cast<double2 (*)[kBs * kBs]>(bs_smem);
   const int q = blockIdx.x / nseg, sg = blockIdx.x % nseg;
@@ -849,13 +855,8 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
     return base + b0 + (int64_t)i * kBs * kBs;
   };
   if (copies) {
-    if ((tid & 31) == 0)
-      for (int g = 0; g < total; ++g) {
-        const int slot = g % kRing;
-        if (g >= kRing && !mbar_wait(&gempty[slot], (unsigned)(g / kRing - 1) & 1u, kWaitCycles)) break;
-        mbar_arrive_expect_tx(&gbar[slot], kBlkBytes);
-        bulk_load(gring[slot], src(g), kBlkBytes, &gbar[slot]);
-      }
+    if ((tid & 31) == 0 && !copy_ring<kRing>(total, gring, gbar, gempty, kBlkBytes, kWaitCycles, src))
+      atomicOr(err, 1ull);
     return;
   }
   auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + gr), "n"(kBlkGroup) : "memory"); };
@@ -963,7 +964,7 @@ __global__ void __launch_bounds__(kBlkThreads) k_blk_solve(int lat, int nseg, in
   }
   both_sync();
   for (int e = tid; e < m; e += 2 * kBlkGroup) x[e] = ys[e];
-  if (!ok && gt == 0) atomicOr(flag + 3, 1);
+  if (!ok) atomicOr(err, 1ull);
 }
 
 // Forward and back substitution of one system (LAPACK zgbtrs, no transpose)
@@ -1229,7 +1230,7 @@ static int band_setup(Handle* h) {
   if ((rc = dev_alloc(h, &B->Pb_d, nbe))) return rc;
   if ((rc = dev_alloc(h, &B->Gb_d, nbe))) return rc;
   if ((rc = dev_alloc(h, &B->tw_d, 2 * (int64_t)nzl))) return rc;
-  if ((rc = dev_alloc(h, &B->flag_d, 4))) return rc;
+  if ((rc = dev_alloc(h, &B->flag_d, 2))) return rc;
   B->fft = make_fft_passes(nzl, B->fftP, 16) && fft_smem_bytes(nzl) <= 48 * 1024;
   std::vector<double2> ftw;
   std::vector<int> fpos;
@@ -1303,14 +1304,15 @@ static int band_factor_that(Handle* h) {
   C3D_LAUNCH_CHECK(h);
   C3D_CUDA_TRY(h, cudaMemsetAsync(B->flag_d, 0, 8, h->stream));
   k_blk_factor<<<dim3(nq * B->nseg, 2), 32, 0, h->stream>>>(0, B->nseg, B->NBq, B->nblk_d, B->blkoff_d, B->Ab_d, B->Bb_d,
-                                                   B->Cb_d, B->Pb_d, B->Gb_d, B->flag_d);
+                                                   B->Cb_d, B->Pb_d, B->Gb_d, B->flag_d, &h->sc->err);
   C3D_LAUNCH_CHECK(h);
   k_blk_factor<<<nq * B->nseg, 32, 0, h->stream>>>(2, B->nseg, B->NBq, B->nblk_d, B->blkoff_d, B->Ab_d, B->Bb_d,
-                                                   B->Cb_d, B->Pb_d, B->Gb_d, B->flag_d);
+                                                   B->Cb_d, B->Pb_d, B->Gb_d, B->flag_d, &h->sc->err);
   C3D_LAUNCH_CHECK(h);
   int flag[2] = {0, 0};
   C3D_CUDA_TRY(h, cudaMemcpyAsync(flag, B->flag_d, 8, cudaMemcpyDeviceToHost, h->stream));
-  C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  const int rc = check_device_error(h);
+  if (rc) return rc;
   B->block = flag[1] == 0;
   if (B->block) return 0;
   // pivoted banded LU
@@ -1407,7 +1409,7 @@ int band_apply(Handle* h, const double* in, double* out) {
   if (B->block) {
     k_blk_solve<<<nq * B->nseg, kBlkThreads, blk_solve_smem(B->nblk_max), h->stream>>>(
         lat, B->nseg, B->NBq, B->segstart_d, B->seglen_d, B->nblk_d, B->blkoff_d, B->Ab_d, B->Pb_d, B->Gb_d,
-        B->rhs_d, B->flag_d);
+        B->rhs_d, &h->sc->err);
   } else {
     const size_t smem = solve_smem_bytes(lat);
     k_band_solve<<<nq * B->nseg, 32, smem, h->stream>>>(lat, B->nseg, B->segstart_d, B->seglen_d, B->AB_d,
