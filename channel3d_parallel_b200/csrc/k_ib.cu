@@ -2041,9 +2041,9 @@ int ib_bicgstab(Handle* h, const double* b, double dt) {
   C3D_CUDA_TRY(h, cudaMemcpyAsync(s->scr1, x, 8 * n, cudaMemcpyDeviceToDevice, h->stream));
   if ((rc = bcg_restart(h, b, x, dt, gb))) return rc;
   if (mode == C3D_PRECOND_LEARNED) {
-    // warm start x0 += M r0
-    if ((rc = band_apply(h, s->r, s->scr2))) return rc;
-    k_axpby<<<gb, 256, 0, h->stream>>>(n, 1.0, x, 1.0, s->scr2, x);
+    // warm start x0 += M r0 (ph: the caller's right-hand side may be scratch)
+    if ((rc = band_apply(h, s->r, s->ph))) return rc;
+    k_axpby<<<gb, 256, 0, h->stream>>>(n, 1.0, x, 1.0, s->ph, x);
     C3D_LAUNCH_CHECK(h);
     if ((rc = bcg_restart(h, b, x, dt, gb))) return rc;
   }
