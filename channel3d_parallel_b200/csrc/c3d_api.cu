@@ -661,7 +661,7 @@ static int run_steps(Handle* h, int nsteps, bool euler = false) {
   h->last_step_ms = nsteps > 0 ? ms / nsteps : 0.0;
   C3D_CUDA_TRY(h, cudaGetLastError());
   if ((rc = sync_scalars_from_device(h))) return rc;
-  if (warn) h->last_error = "a Schur solve stopped at cg_max_iter before reaching cg_tol";
+  if (warn) h->last_error = "a Schur solve stopped (cg_max_iter, or no further iteration) before reaching cg_tol";
   return warn;
 }
 

@@ -1903,16 +1903,23 @@ static int bcg_iteration(Handle* h, double* x, double dt, const double* blk, boo
   return 0;
 }
 
+// After an iteration rho_o and om divide in the next one's bta: once either is
+// exactly zero (on a system that does not converge <rhat, r> sinks to rounding,
+// and it is a sum that can come out as zero) there is no further iteration, and
+// the iterate, still finite, is where the solve ends.
+__host__ __device__ inline bool bcg_ended(double rho, double om) { return rho == 0.0 || om == 0.0; }
+
 // End of a captured iteration: count it, record its squared residual and
 // keep the WHILE node looping while the residual is finite and at or above
-// the tolerance and the launch's iteration limit is not reached.
+// the tolerance, a next iteration exists and the launch's iteration limit is
+// not reached.
 __global__ void k_bcg_loop(cudaGraphConditionalHandle cond, const double* __restrict__ sc, int* __restrict__ loop,
                            double* __restrict__ hist, double eps) {
   const double err = sc[5];
   const int it = loop[0] + 1;
   loop[0] = it;
   hist[it - 1] = err;
-  const bool go = isfinite(err) && err >= eps && it < loop[1];
+  const bool go = isfinite(err) && err >= eps && !bcg_ended(sc[0], sc[2]) && it < loop[1];
   cudaGraphSetConditional(cond, go ? 1u : 0u);
 }
 
@@ -2062,6 +2069,7 @@ int ib_bicgstab(Handle* h, const double* b, double dt) {
     // run the whole solve in one launch
     const int lim = mode == C3D_PRECOND_LEARNED ? std::min(maxit, it + kBcgChunk) : maxit;
     int done = it;
+    bool ended = false;                  // no further iteration exists
     if (!s->bcg_graph_off && (rc = bcg_graph_ready(h, x, dt, blk, band, mode, eps)) == 0 && !s->bcg_graph_off) {
       const int lc[2] = {it, lim};
       C3D_CUDA_TRY(h, cudaMemcpyAsync(s->loop_d, lc, sizeof(lc), cudaMemcpyHostToDevice, h->stream));
@@ -2070,12 +2078,17 @@ int ib_bicgstab(Handle* h, const double* b, double dt) {
       C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
       if (done <= it || done > lim) { h->last_error = "BiCGSTAB graph: bad iteration count"; return C3D_ERR_CUDA; }
       h->launches += s->bcg_body_launches * (done - it);
+      ended = done < lim;                // before its limit, by the residual or for good
     } else {
       if (rc) return rc;
       // host-driven iteration (conditional graphs unavailable)
       if ((rc = bcg_iteration(h, x, dt, blk, band))) return rc;
       done = it + 1;
       C3D_CUDA_TRY(h, cudaMemcpyAsync(s->hist_d + it, s->sc + 5, 8, cudaMemcpyDeviceToDevice, h->stream));
+      double q[3];
+      C3D_CUDA_TRY(h, cudaMemcpyAsync(q, s->sc, sizeof(q), cudaMemcpyDeviceToHost, h->stream));
+      C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+      ended = bcg_ended(q[0], q[2]);
     }
     const size_t h0 = hist.size();
     hist.resize(h0 + (done - it));
@@ -2084,8 +2097,9 @@ int ib_bicgstab(Handle* h, const double* b, double dt) {
     C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     it = done;
     err = hist.back();
+    ended = ended && std::isfinite(err) && err >= eps;
     if (mode == C3D_PRECOND_LEARNED) {
-      const bool broke = !(err == err) || std::isinf(err);
+      const bool broke = !(err == err) || std::isinf(err) || ended;
       // stall: the best residual of the last kStallWindow iterations is not
       // 1 % below the best one before them
       bool stalled = false;
@@ -2111,8 +2125,10 @@ int ib_bicgstab(Handle* h, const double* b, double dt) {
         if ((rc = bcg_restart(h, b, x, dt, gb))) return rc;
         hist.clear();
         err = 1.0;
+        continue;
       }
     }
+    if (ended) break;
   }
   if (err == err && (rc = push_history(h, x))) return rc;
   if (pure_band && err < eps)
@@ -2134,7 +2150,7 @@ int ib_bicgstab(Handle* h, const double* b, double dt) {
     h->last_error = "BiCGSTAB produced a non-finite residual";
     return C3D_ERR_NAN;
   }
-  if (it == h->p.cg_max_iter && err >= eps) return C3D_WARN_NOT_CONVERGED;
+  if (err >= eps) return C3D_WARN_NOT_CONVERGED;      // at cg_max_iter, or no further iteration
   return 0;
 }
 

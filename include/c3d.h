@@ -41,7 +41,7 @@ extern "C" {
 #define C3D_ERR_IO             -5   /* file could not be read                 */
 #define C3D_ERR_UNSUPPORTED    -6   /* option not available for this set-up  */
 #define C3D_ERR_NO_DEVICE      -7   /* no CUDA device visible                 */
-#define C3D_WARN_NOT_CONVERGED  1   /* BiCGSTAB stopped at cg_max_iter        */
+#define C3D_WARN_NOT_CONVERGED  1   /* BiCGSTAB stopped at cg_max_iter, or where rho or omega came out as zero */
 
 /* ---- field identifiers (Fortran extents, lower bound 1 unless stated) ---- */
 #define C3D_FIELD_U             1   /* U(nx, nyg, nzg)        src/global.f90:106 */
