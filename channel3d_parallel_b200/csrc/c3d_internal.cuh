@@ -104,9 +104,10 @@ struct SlabTables {
 };
 
 // cluster of CTAs that holds a kx slab: cs CTAs of jc rows of j, shared memory
-// row stride rs complex values, nt threads, smem bytes; narrow CTAs or not
+// row stride rs complex values, nt threads, smem bytes; narrow CTAs or not; jmax
+// rows that a CTA can hold, clusters resident at once
 struct SlabCluster {
-  int cs = 1, jc = 1, rs = 0, nt = 256, smem = 0, narrow = 0;
+  int cs = 1, jc = 1, rs = 0, nt = 256, smem = 0, narrow = 0, jmax = 0, active = 0;
 };
 
 // Spectral Poisson state: twiddles, Thomas factor tables and spectra for the

@@ -341,13 +341,28 @@ __global__ void __launch_bounds__(1024) k_mode00(Dims d, const double* __restric
 // host drivers
 // ---------------------------------------------------------------------------
 // Which form of the z transforms and y solves: the cluster that keeps a slab on
-// chip moves the spectrum once in place of twice, but needs 16 CTAs of an SM
-// each for the large slabs, and past 256 columns a thread has several.
-// Measured, cluster against blocks (us, B200): 192x128x192 45 / 67,
-// 256x128x256 93 / 114, 64x256x64 19 / 33; 16 CTAs: 192x256x192 156 / 134,
-// 256x192x256 276 / 165, 384x256x384 1237 / 467; 8 CTAs with Nz = 384:
-// 128x64x384 89 / 65, 384x64x384 222 / 145.
-static bool slab_by_blocks(const Dims& d, const SlabCluster& c) { return c.cs > 8 || d.Nz > 256; }
+// chip moves the spectrum once in place of twice and has no chain through
+// memory, but past 256 columns a thread of it has several, and slabs of many
+// rows or columns need 16 CTAs.  Few such slabs, resident at once, are still
+// better off there (at most two of their CTAs an SM, three with up to 64 columns;
+// where the CTAs are more than three quarters full, two waves of up to four an
+// SM): in thin channels the chain over the blocks is what the other form waits
+// for.
+// Measured, cluster against blocks (us, B200, FP64), clusters of up to 8 CTAs:
+// 192x128x192 45 / 67, 256x128x256 93 / 114, 64x256x64 19 / 33; more than 256
+// columns: 48x8x384 30 / 18, 12x64x288 34 / 21, 128x64x384 89 / 65, 384x256x384
+// 1237 / 417; 16 CTAs: 12x300x12 15 / 25, 36x160x64 17 / 21, 24x160x128 21 / 25,
+// 36x160x128 27 / 25, 64x160x128 42 / 32, 24x500x64 21 / 39, 48x500x64 38 / 45, 64x500x64 51 / 50,
+// 24x300x36 17 / 25, 36x300x36 30 / 27, 96x300x64 61 / 41, 192x256x192 156 / 134.
+// FP32 (mixed steps, six solves): 24x300x64 390 / 429, 36x500x64 723 / 823,
+// 96x300x36 670 / 537, 48x8x288 378 / 211.
+static bool slab_by_blocks(const Dims& d, const SlabCluster& c) {
+  if (d.Nz > 256) return true;
+  if (c.cs <= 8) return false;
+  const bool filled = 4 * c.jc > 3 * c.jmax;
+  const int most = filled ? std::min(2 * c.active, 4 * 148 / c.cs) : std::min(c.active, (d.Nz > 64 ? 2 : 3) * 148 / c.cs);
+  return d.nkx > most;
+}
 
 // parts: bit0 x FFT, bit1 y-z solve, bit2 inverse x FFT.  rhs_in: the
 // right-hand side, or with from_div the potential whose residual

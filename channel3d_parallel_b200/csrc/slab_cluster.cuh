@@ -415,22 +415,22 @@ static int active_clusters(int cs, int nt, int smem) {
 // Picks the shape whose kx slabs (one cluster each) run in fewer waves of
 // co-resident clusters, as the device reports them; the narrow shape on a tie.
 template <typename T>
-static bool choose_cluster(const Dims& d, int pz, int& cs, int& jc, int& rs, int& nt, int& smem, int& narrow) {
-  rs = pz;
+static bool choose_cluster(const Dims& d, int pz, SlabCluster& c) {
+  int rs = pz;
   if (sizeof(T) == 8) { while (rs % 8 != 1) ++rs; }
   else { while (rs % 4 != 2) ++rs; }
   int ncs, njc, nnt, nsm, wcs, wjc, wnt, wsm;
   const bool okn = choose_shape<T, true>(d, rs, ncs, njc, nnt, nsm);
   const bool okw = choose_shape<T, false>(d, rs, wcs, wjc, wnt, wsm);
   auto waves = [&](int active) { return active > 0 ? (d.nkx + active - 1) / active : 1 << 30; };
-  const int wn = okn ? waves(active_clusters<T, true>(ncs, nnt, nsm)) : 1 << 30;
-  const int ww = okw ? waves(active_clusters<T, false>(wcs, wnt, wsm)) : 1 << 30;
-  if (okn && (!okw || wn <= ww)) {
-    narrow = 1; cs = ncs; jc = njc; nt = nnt; smem = nsm;
+  const int an = okn ? active_clusters<T, true>(ncs, nnt, nsm) : 0;
+  const int aw = okw ? active_clusters<T, false>(wcs, wnt, wsm) : 0;
+  if (okn && (!okw || waves(an) <= waves(aw))) {
+    c = SlabCluster{ncs, njc, rs, nnt, nsm, 1, yz_jmax<T, true>(), an};
     return true;
   }
   if (!okw) return false;
-  narrow = 0; cs = wcs; jc = wjc; nt = wnt; smem = wsm;
+  c = SlabCluster{wcs, wjc, rs, wnt, wsm, 0, yz_jmax<T, false>(), aw};
   return true;
 }
 
@@ -498,7 +498,7 @@ int cluster_setup(Handle* h) {
   SpectralState& S = h->sp;
   constexpr bool f32 = sizeof(T) == 4;
   SlabCluster& c = f32 ? S.cluster32 : S.cluster;
-  if (!choose_cluster<T>(d, f32 ? S.pz32 : S.pz64, c.cs, c.jc, c.rs, c.nt, c.smem, c.narrow)) {
+  if (!choose_cluster<T>(d, f32 ? S.pz32 : S.pz64, c)) {
     h->last_error = f32 ? "ny_global too large for the FP32 cluster decomposition"
                         : "ny_global too large for one 16-CTA cluster per kx slab";
     return C3D_ERR_UNSUPPORTED;

@@ -108,8 +108,8 @@ typedef struct c3d_stats {
   int32_t precond_mode;        /* preconditioner of the last Schur solve      */
   double  last_bicgstab_ms;    /* device time of the last Schur solve (ms)    */
   double  bicgstab_ms;         /* accumulated device time of Schur solves     */
-  int32_t slab_cluster[2];     /* CTAs per kx-slab cluster of the y-z solve: FP64, FP32 (above 8,
-                                  or with more than 256 columns, blocks of rows solve instead) */
+  int32_t slab_cluster[2];     /* CTAs per kx-slab cluster of the y-z solve: FP64, FP32 (with more than
+                                  256 columns, or above 8 with many slabs, blocks of rows solve instead) */
   int32_t slab_narrow[2];      /* 1: narrow slab CTAs (<= 192 threads, 3 per SM); FP64, FP32 */
   double  qflow_y_0, qflow_z_0;/* targets of the y and z constant-flux corrections */
   int64_t precond_builds;      /* probed (or predicted) band preconditioners built */
