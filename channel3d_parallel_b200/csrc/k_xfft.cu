@@ -24,9 +24,12 @@ constexpr int kLines = 8;        // complex lines per CTA
 // through L1, which many CTAs' rows leave little of (four CTAs of 192 threads
 // at 384 x 256 x 384: 400 us, two of 384: 289; 43 either way at 192 x 128 x
 // 192); the inverse is bound by its stages (288 columns: 86 us with 192
-// threads, 97 with 384)
+// threads, 97 with 384) as long as several CTAs share an SM: with one or none
+// its rounds follow one another, and up to 384 threads take fewer of them
+// (512x16x16 12.4 -> 10.4 us, 486x20x24 14.5 -> 10.4, 384x64x24 10.4 -> 8.3)
 constexpr int kFwdThreads = 384;
 constexpr int kInvThreads = 192;
+constexpr int kInvFewThreads = 384;
 constexpr int kMaxR = 8;         // largest radix (register budget)
 constexpr unsigned kRecLines = (unsigned)((1ull << 32) / kLines);   // reciprocal of kLines for div_by
 
@@ -408,7 +411,7 @@ __device__ __forceinline__ void put_phi(const XinvArgs<T>& a, const OutLine& L, 
 }
 
 template <typename T, int NX>
-__global__ void __launch_bounds__(kInvThreads, 4) k_xfft_inv(XinvArgs<T> a) {
+__global__ void __launch_bounds__(kInvFewThreads, 2) k_xfft_inv(XinvArgs<T> a) {
   using C = typename cplx<T>::t;
   extern __shared__ __align__(16) unsigned char xi_smem[];
   __shared__ OutLine L[2 * kLines];
@@ -584,7 +587,7 @@ int launch_xfft_inv(Handle* h, double* out, double* phi1, const double* phi00, i
   a.rbase = blo * d.Nz; a.nlines = (bhi - blo + 1) * d.Nz;
   a.inv_scale = 1.0 / ((double)d.Nx * (double)d.Nz);
   const unsigned nb = (unsigned)((a.nlines + 2 * kLines - 1) / (2 * kLines));
-  x_kernels<T>(d.Nx).inv<<<nb, x_threads(a.P, kInvThreads), x_smem<T>(a.P, false), h->stream>>>(a);
+  x_kernels<T>(d.Nx).inv<<<nb, x_threads(a.P, nb <= 148 ? kInvFewThreads : kInvThreads), x_smem<T>(a.P, false), h->stream>>>(a);
   C3D_LAUNCH_CHECK(h);
   return 0;
 }
