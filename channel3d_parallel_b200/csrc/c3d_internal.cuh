@@ -172,7 +172,6 @@ void set_global_error(const std::string& msg);
 
 struct IbState;   // immersed-boundary state (k_ib.cu)
 struct MlpState;  // learned preconditioner network (k_mlp.cu)
-struct MixedState;  // mixed-precision work buffers (k_poisson.cu)
 
 struct Handle {
   Params p;
@@ -226,7 +225,6 @@ struct Handle {
   std::vector<cudaEvent_t> ev_slab;
   double last_step_ms = 0;
   IbState* ib = nullptr;
-  MixedState* mixed = nullptr;
   MlpState* mlp = nullptr;
   // the time step's captured CUDA graphs (valid for graph_dt): a whole step,
   // a step that leaves its last projection to the next one, and two steps
@@ -294,7 +292,7 @@ int launch_poisson_of_div(Handle* h, const double* U, const double* V, const dou
 int launch_poisson_of_div_band(Handle* h, const double* U, const double* V, const double* W, double* out,
                                int jlo, int jhi);
 int launch_stage_solve(Handle* h, double* const star[3], int rk_step, double dt, bool flux, double** phi);
-int launch_projection_step(Handle* h, int rk_step, double dt, const double* ushift = nullptr);
+int launch_projection_step(Handle* h, int rk_step, double dt);
 int launch_gradient_subtract(Handle* h, const double* Ui, const double* Vi, const double* Wi,
                              const double* phi, double dt, double* Uo, double* Vo, double* Wo,
                              bool dup_plane = true, bool with_ghosts = false,

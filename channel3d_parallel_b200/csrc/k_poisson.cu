@@ -654,14 +654,13 @@ int launch_stage_solve(Handle* h, double* const star[3], int rk_step, double dt,
 }
 
 // compute_non_IB_projection with U* in (Us,Vs,Ws) and the result in (U,V,W),
-// all ghost entries included (and the x mass-flow correction when ushift is
-// given)
-int launch_projection_step(Handle* h, int rk_step, double dt, const double* ushift) {
+// all ghost entries included
+int launch_projection_step(Handle* h, int rk_step, double dt) {
   double* const star[3] = {h->Us, h->Vs, h->Ws};
   double* phi = nullptr;
-  const int rc = launch_stage_solve(h, star, rk_step, dt, ushift != nullptr, &phi);
+  const int rc = launch_stage_solve(h, star, rk_step, dt, false, &phi);
   if (rc) return rc;
-  return launch_gradient_subtract(h, h->Us, h->Vs, h->Ws, phi, dt, h->U, h->V, h->W, false, true, ushift);
+  return launch_gradient_subtract(h, h->Us, h->Vs, h->Ws, phi, dt, h->U, h->V, h->W, false, true);
 }
 
 // P = phi1/(dt*rk_coef(1,1)) with the copies of src/poisson.f90:92-98
