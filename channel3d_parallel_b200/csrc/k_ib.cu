@@ -10,8 +10,9 @@
 //    values, grid offsets and folded grid indices of each axis; a stencil
 //    weight is dx*dymin*dz*dx_w*dy_w*dz_w in the reference's multiplication
 //    order;
-//  - E / E1n gather one warp per (marker, component); R spreads with FP64
-//    atomics (so R is order-dependent at round-off level);
+//  - E / E1n gather a patch of markers per CTA from a box of the field in
+//    shared memory; R is a gather over an inverse map of the stencils, its sums
+//    in a fixed order, so both repeat bit for bit;
 //  - the reference's marker partition, support planes and MPI gathers are
 //    replaced by direct indexing of the resident fields: a stencil point on
 //    the periodic duplicate centre plane nzg-1 is folded onto plane 2.
@@ -501,10 +502,13 @@ __global__ void k_ib_weights(IbGeomArgs a) {
       a.off[tslot(a.nb, t, 1, q, l)] = yg - yb;
       a.off[tslot(a.nb, t, 2, q, l)] = zg - zb;
     }
-    // The support is four cells, so one of a marker's end points lies at or
-    // past its edge, where the function is zero: the 1e-17 that rounding leaves
-    // of it at a marker on a grid line is taken out, and with it the fifth
-    // entry of the sums below.
+    // The support is four widths, and five neighbouring points span at least four
+    // (dx, dz, dymin are the least spacings of the centres, and two cells
+    // together are twice one of them): one of a marker's end points lies at or
+    // past the edge.  Both weights are nonzero only by rounding of the positions,
+    // delta/dr < 1e-12, where the function is 0.66 delta^3/dr^3 and its formula
+    // leaves up to 5e-16: that is taken out, and with it the fifth entry of the
+    // sums below.
     for (int ax = 0; ax < 3; ++ax) {
       const int64_t e0 = tslot(a.nb, t, ax, 0, l), e4 = tslot(a.nb, t, ax, 4, l);
       const double w0 = a.w1[e0], w4 = a.w1[e4], dr = ax == 0 ? a.dx : (ax == 1 ? a.dymin : a.dz);
@@ -606,8 +610,8 @@ __device__ __forceinline__ void gather_tile(const GatherArgs& a, const GComp& cp
   const GField& g = cp.f;
   const int px = a.d.Nx, pz = a.d.Nz;        // index periods of x and z (indices 2 .. N+1)
   // the four points of each axis that can have a weight: 0..3, or 1..4 when
-  // point 0 has none; a grid where five do (spacing below the widths of the
-  // delta function) is summed from the tables
+  // point 0 has none; a tile where five do (an x grid that is not uniform) is summed
+  // from the tables
   int ix[4], iy[4], iz[4], sx = 0, sy = 0, sz = 0;
   double wx[4], wy[4], wz[4];
   bool five = false;
@@ -766,9 +770,11 @@ enum SpreadMode { S_RAW = 0, S_JUMP = 1, S_NORMAL = 2 };
 // ---- spreading R f as a gather over an inverse map of the stencils ------
 // The reference adds each marker's 125 stencil contributions to the field
 // (local_reg, src/immersed_boundary_operators.f90:544-603).  Here every grid
-// point sums the contributions that reach it, in increasing (marker, stencil
-// point) order -- the order in which the markers are visited -- so R f is
-// bitwise reproducible (no atomics, no order that depends on scheduling).
+// point sums the contributions that reach it: its entries are sorted by (marker,
+// stencil point), lane s of the four that share the point adds entries s, s+4,
+// ... in that order, and the four sums meet in a fixed tree.  So R f is bitwise
+// reproducible (no atomics, no order that depends on scheduling), though not the
+// sum in the order in which the reference visits the markers.
 // Per component the map is CSR over the field's points: cnt[p] entries from
 // off[p] in ent (marker << 7 | stencil point q = qi + 5 qj + 25 qk) with the
 // tensor weight w = wx (wy wz) beside each entry.  It is rebuilt whenever the

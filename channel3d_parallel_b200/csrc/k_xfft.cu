@@ -488,8 +488,8 @@ size_t x_smem(const FftPasses& P, bool fwd) {
          (fwd && sizeof(T) == 4 ? sizeof(double) * 2 * kLines * P.n : 0);
 }
 
-// The kernels for lines of Nx points: lines of 32 to 512 points have the length
-// compiled in (FP64: inverse at 384 x 256 x 384 188 -> 170 us, forward 288 ->
+// The kernels for lines of Nx points: lines of 32 to 512 points, but 36 and 54,
+// have the length compiled in (FP64: inverse at 384 x 256 x 384 188 -> 170 us, forward 288 ->
 // 281; time step 4969 -> 4874 us there, 661 -> 653 at 192 x 128 x 192, 368 ->
 // 358 at 162 x 113 x 108, 83 -> 82 at 32 x 64 x 32; FP32 mixed steps 1117 -> 1064
 // us at 192 x 128 x 192, 7771 -> 7535 at 384 x 256 x 384).  Right-hand
