@@ -136,6 +136,7 @@ struct SpectralState {
   // Ny rows of pz complex values (pz*sizeof(complex) a multiple of 16 bytes)
   double2* spec = nullptr;
   float2* spec32 = nullptr;
+  bool mixed_ready = false;                  // everything of the FP32 path is there
   int pz64 = 0, pz32 = 0;
   // FP64 kx = kz = 0 mode of the FP32 path
   double* linesum = nullptr;                 // per (j, k) line sum of the right-hand side

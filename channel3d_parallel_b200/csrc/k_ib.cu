@@ -1677,7 +1677,7 @@ static int build_spread_maps(Handle* h) {
   const int64_t npts[3] = {sizeU(d), sizeV(d), sizeW(d)};
   int rc;
   for (int c = 0; c < 3; ++c) {
-    if (!s->sp_cnt[c]) {
+    if (!s->sp_pts[c]) {            // the last of them
       if ((rc = dev_alloc(h, &s->sp_cnt[c], npts[c]))) return rc;
       if ((rc = dev_alloc(h, &s->sp_off[c], npts[c]))) return rc;
       if ((rc = dev_alloc(h, &s->sp_ent[c], ne))) return rc;

@@ -75,7 +75,7 @@ __device__ __forceinline__ double2 crcp(double2 a) {
 }  // namespace
 
 struct BandState {
-  bool ok = false;                 // lattice supports the band form
+  bool ok = false;                 // lattice supports the band form, buffers are there
   int lat = 0, nzl = 0, nq = 0, nseg = 0;
   std::vector<int> seg_start, seg_len;
   int spacing[4] = {8, 8, 8, 32};
@@ -1141,22 +1141,29 @@ static size_t inv_smem_bytes(int nzl, int nq) { return sizeof(double) * (64 * (s
 // more than k_band_fwd: nq <= nzl/2 + 1)
 constexpr size_t kBandSmemMax = 220 * 1024, kBlkSmemMax = 200 * 1024, kInvExtra = 512;
 
-static int band_setup(Handle* h) {
+// B->ok only at the end: a lattice that is not supported, or buffers that could
+// not be had, leave none of the pointers below to a later call
+static int band_fill(Handle* h, BandState* B) {
   IbState* s = h->ib;
-  if (s->band) return 0;
-  BandState* B = new BandState();
-  s->band = B;
-  B->ok = lattice_segments(s, h->p, B->seg_start, B->seg_len);
-  if (!B->ok) return 0;
+  if (!lattice_segments(s, h->p, B->seg_start, B->seg_len)) return 0;
   const int lat = s->lat_nx;
   B->lat = lat;
   B->nzl = s->nb / lat;
   B->nq = B->nzl / 2 + 1;
   B->nseg = (int)B->seg_start.size();
-  if (B->nzl * lat != s->nb || solve_smem_bytes(lat) > kBandSmemMax || fwd_smem_bytes(B->nzl) > kBandSmemMax) {
-    B->ok = false;
+  if (B->nzl * lat != s->nb || solve_smem_bytes(lat) > kBandSmemMax || fwd_smem_bytes(B->nzl) > kBandSmemMax)
     return 0;
+  B->nblk.resize(B->nseg);
+  B->blkoff.resize(B->nseg);
+  B->NBq = 0;
+  B->nblk_max = 0;
+  for (int sgi = 0; sgi < B->nseg; ++sgi) {
+    B->nblk[sgi] = (4 * B->seg_len[sgi] + kBs - 1) / kBs;
+    B->blkoff[sgi] = B->NBq;
+    B->NBq += B->nblk[sgi];
+    B->nblk_max = std::max(B->nblk_max, B->nblk[sgi]);
   }
+  if (blk_solve_smem(B->nblk_max) > kBlkSmemMax) return 0;     // a segment too long for the block solve
   // folded positions, neighbours, colours
   std::vector<int> pos(lat), seg(lat), nbr((size_t)lat * kNd), col((size_t)4 * lat);
   for (int sgi = 0; sgi < B->nseg; ++sgi) {
@@ -1172,10 +1179,7 @@ static int band_setup(Handle* h) {
   // the folded order keeps every band entry within kKl of the diagonal
   for (int i = 0; i < lat; ++i)
     for (int d = 0; d < kNd; ++d)
-      if (std::abs(pos[nbr[(size_t)i * kNd + d]] - pos[i]) > 2 * kKb) {
-        B->ok = false;
-        return 0;
-      }
+      if (std::abs(pos[nbr[(size_t)i * kNd + d]] - pos[i]) > 2 * kKb) return 0;
   B->colours.assign(4, {});
   for (int c = 0; c < 4; ++c) {
     const int P = B->spacing[c];
@@ -1207,20 +1211,6 @@ static int band_setup(Handle* h) {
   if ((rc = dev_alloc(h, &B->AB_d, (int64_t)nq * kLdab * 4 * lat))) return rc;
   if ((rc = dev_alloc(h, &B->ipiv_d, (int64_t)nq * 4 * lat))) return rc;
   if ((rc = dev_alloc(h, &B->rhs_d, (int64_t)nq * 4 * lat))) return rc;
-  B->nblk.resize(B->nseg);
-  B->blkoff.resize(B->nseg);
-  B->NBq = 0;
-  B->nblk_max = 0;
-  for (int sgi = 0; sgi < B->nseg; ++sgi) {
-    B->nblk[sgi] = (4 * B->seg_len[sgi] + kBs - 1) / kBs;
-    B->blkoff[sgi] = B->NBq;
-    B->NBq += B->nblk[sgi];
-    B->nblk_max = std::max(B->nblk_max, B->nblk[sgi]);
-  }
-  if (blk_solve_smem(B->nblk_max) > kBlkSmemMax) {
-    h->last_error = "band preconditioner: a lattice segment is too long for the block solve";
-    return C3D_ERR_UNSUPPORTED;
-  }
   const int64_t nbe = (int64_t)nq * B->NBq * kBs * kBs;
   if ((rc = dev_alloc(h, &B->nblk_d, B->nseg))) return rc;
   if ((rc = dev_alloc(h, &B->blkoff_d, B->nseg))) return rc;
@@ -1275,7 +1265,17 @@ static int band_setup(Handle* h) {
   C3D_CUDA_TRY(h, limit(k_band_inv, kBandSmemMax + kInvExtra));
   C3D_CUDA_TRY(h, limit(k_band_factor, sizeof(double2) * kFactorWin * kLdab));
   C3D_CUDA_TRY(h, limit(k_blk_solve, kBlkSmemMax));
+  B->ok = true;
   return 0;
+}
+
+static int band_setup(Handle* h) {
+  IbState* s = h->ib;
+  if (s->band) return 0;
+  s->band = new BandState();
+  const int rc = band_fill(h, s->band);
+  if (rc) band_free(s);
+  return rc;
 }
 
 bool band_supported(Handle* h) {

@@ -698,10 +698,7 @@ __global__ void k_to_bf16(int64_t n, const float4* __restrict__ x, uint2* __rest
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static int mlp_ensure(Handle* h) {
-  if (h->mlp) return 0;
-  MlpState* M = new MlpState();
-  h->mlp = M;
+static int mlp_fill(Handle* h, MlpState* M) {
   int rc;
   if ((rc = dev_alloc(h, &M->w, kNParam))) return rc;
   if ((rc = dev_alloc(h, &M->g, kNParam))) return rc;
@@ -729,6 +726,15 @@ static int mlp_ensure(Handle* h) {
     attr = true;
   }
   return cudaStreamSynchronize(h->stream) == cudaSuccess ? 0 : C3D_ERR_CUDA;
+}
+
+static int mlp_ensure(Handle* h) {
+  if (h->mlp) return 0;
+  MlpState* M = new MlpState();
+  const int rc = mlp_fill(h, M);
+  if (rc) delete M;              // device buffers are tracked by the handle
+  else h->mlp = M;
+  return rc;
 }
 
 static int upload_sig(Handle* h) {
@@ -792,11 +798,12 @@ static int ensure_rows(Handle* h, int rows) {
   MlpState* S = h->mlp;
   if (S->cap_rows >= rows) return 0;
   int rc;
-  S->cap_rows = rows;
+  S->cap_rows = 0;               // none until all four are there
   if ((rc = dev_alloc(h, &S->H1, (int64_t)rows * kH))) return rc;
   if ((rc = dev_alloc(h, &S->H2, (int64_t)rows * kH))) return rc;
   if ((rc = dev_alloc(h, &S->dO, (int64_t)rows * kO))) return rc;
   if ((rc = dev_alloc(h, &S->out, (int64_t)rows * kO))) return rc;
+  S->cap_rows = rows;
   return 0;
 }
 

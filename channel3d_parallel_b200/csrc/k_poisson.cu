@@ -721,14 +721,14 @@ int poisson_setup(Handle* h) {
     h->flux_part_len = nbx;
   }
   if ((rc = build_tri_table(h))) return rc;
-  if (S.spec32 && slab_by_blocks(d, S.cluster32) && (rc = slab_setup(h, true))) return rc;
+  if (S.mixed_ready && slab_by_blocks(d, S.cluster32) && (rc = slab_setup(h, true))) return rc;
   return slab_by_blocks(d, S.cluster) ? slab_setup(h, false) : 0;
 }
 
 int mixed_setup(Handle* h) {
   const Dims& d = h->d;
   SpectralState& S = h->sp;
-  if (S.spec32 != nullptr) return 0;
+  if (S.mixed_ready) return 0;
   S.pz32 = d.Nz + (d.Nz & 1);
   int rc;
   if ((rc = cluster_setup<float>(h))) return rc;
@@ -742,6 +742,7 @@ int mixed_setup(Handle* h) {
   if ((rc = build_tri_table(h))) return rc;       // with the FP32 pivots
   if (slab_by_blocks(d, S.cluster32) && (rc = slab_setup(h, true))) return rc;
   C3D_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  S.mixed_ready = true;
   return 0;
 }
 

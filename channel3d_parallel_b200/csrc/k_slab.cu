@@ -407,7 +407,7 @@ static int slab_setup_t(Handle* h, SlabTables<T>& t) {
   const Dims& d = h->d;
   SpectralState& S = h->sp;
   int rc;
-  if (t.link == nullptr) {
+  if (t.ticket == nullptr) {      // the last of its buffers
     t.jr = kRows;
     while (t.jr > 1 && slab_smem<T>(d.Nz, d.nkzs, t.jr, slab_stride<T>(d.Nz)) > (size_t)kSlabSmemMax) t.jr /= 2;
     t.nblk = (d.Ny + t.jr - 1) / t.jr;
