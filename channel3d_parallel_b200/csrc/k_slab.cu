@@ -25,10 +25,11 @@
 // takes 7, so a cluster that holds it runs 8 to 12 warps per SM, in whole
 // waves of clusters, with the sweeps of 16 to 32 rows one after another.
 // 384 x 256 x 384: 1237 us in clusters, 417 here (1.4 GB moved: 210 us at the
-// copy rate); few slabs in a thin channel are the other way round, the chain
-// over the blocks being what they wait for (slab_by_blocks, k_poisson.cu).  What is left is latency at 24 warps per SM and about 100
-// instructions a value.  Four rounds of 64 registers or 16 rows a block were
-// slower there (553 and 603 us with 256 threads, against 539).
+// copy rate); what is left is latency at 24 warps per SM and about 100
+// instructions a value.  Few slabs in a thin channel are the other way round:
+// the chain over the blocks is what they wait for (slab_by_blocks,
+// k_poisson.cu).  Four rounds of 64 registers or 16 rows a block were
+// slower at 384 x 256 x 384 (553 and 603 us with 256 threads, against 539).
 #include <algorithm>
 #include <cmath>
 #include <vector>
